@@ -307,6 +307,7 @@ struct DeviceOptimizer
 	double2 *x, *xn, *dirs, *res, *ug;
 	double* scratch;   // projected-gradient output of HVP evaluations
 	std::vector<double2> hx;
+	CircuitSpec orbits;   // the columns of every evaluation
 	int hvp_prec;
 	long evals_hvp = 0, evals_grad = 0, evals_f = 0;
 
@@ -328,6 +329,7 @@ struct DeviceOptimizer
 		res = ug + 16 * nu;
 		scratch = reinterpret_cast<double*>(res + nres);
 		hx.assign(x0, x0 + 16 * nu);
+		if ((ret = use_orbits(rt, pb, th, orbits))) return ret;
 		return RQC_CUDA(cudaMemcpyAsync(x, x0, 16 * nu * sizeof(double2), cudaMemcpyHostToDevice, rt.stream));
 	}
 
@@ -343,7 +345,7 @@ struct DeviceOptimizer
 
 	CircuitSpec spec(bool with_dirs) const
 	{
-		CircuitSpec cs;
+		CircuitSpec cs = orbits;
 		cs.L = pb.L;
 		cs.ngates = pb.G;
 		cs.gates = pb.gates.data();

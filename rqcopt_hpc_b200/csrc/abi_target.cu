@@ -8,6 +8,7 @@
 
 #include "engine.h"
 #include "manifold.cuh"
+
 #include "rqc_runtime.h"
 #include "rqcopt_gpu.h"
 #include "target_problem.h"
@@ -149,6 +150,7 @@ bool TargetHolder::set(linear_func ufunc, void* udata, int L)
 		if (!t || !p.set_brickwall(L, t->nlayers, t->vlist, nullptr, t->perms)) return false;
 		gates = p.gates;
 		wires = p.wires;
+		spec.per = p.per;
 	} else if (ufunc == rqcopt_circuit_ufunc) {
 		const struct rqcopt_circuit_target* t = static_cast<const struct rqcopt_circuit_target*>(udata);
 		Problem p;
@@ -164,6 +166,28 @@ bool TargetHolder::set(linear_func ufunc, void* udata, int L)
 	spec.gates = gates.data();
 	spec.wires = wires.data();
 	return true;
+}
+
+int use_orbits(Runtime& rt, const Problem& pb, const TargetHolder& th, CircuitSpec& cs)
+{
+	const int per = pb.L / 2;
+	// beyond 20 qubits no evaluation over all columns ends in reasonable time: the list is not worth its memory
+	if (pb.L < 4 || pb.L > 20 || pb.per != per || th.spec.ufunc || th.spec.per != per || rt.col_begin != 0 ||
+	    rt.col_end != 0)
+		return OK;
+	std::vector<const int*> layers;
+	for (int k = 0; k < pb.G; k += per) layers.push_back(&pb.wires[2 * (size_t)k]);
+	for (int k = 0; k < th.spec.ngates; k += per) layers.push_back(&th.wires[2 * (size_t)k]);
+	const std::vector<int> sym = wire_symmetries(pb.L, layers);
+	if ((int)sym.size() == pb.L) return OK;
+	std::vector<BasisCol> cols = orbit_columns(pb.L, sym);
+	if (rt.real_pairs) cols = pair_columns(cols);
+	const size_t bytes = cols.size() * sizeof(BasisCol);
+	int ret = ensure_device(rt.columns, bytes);
+	if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(rt.columns.ptr, cols.data(), bytes, cudaMemcpyHostToDevice, rt.stream));
+	cs.columns = static_cast<const BasisCol*>(rt.columns.ptr);
+	cs.ncolumns = (int64_t)cols.size();
+	return ret;
 }
 
 // Fold per-gate sums into per-unit sums and project (src/target.c:410-430, 526-535, 652-672).
@@ -222,12 +246,13 @@ int run_target(const Problem& pb, const TargetHolder& th, int mode, numeric* fva
 	cs.dirs = mode == EVAL_HVP ? pb.dirs.data() : nullptr;
 	cs.wires = pb.wires.data();
 	const int prec = rt->precision == PREC_C128 ? PREC_C128 : PREC_C64;
+	int ret = prec == PREC_C128 ? use_orbits(*rt, pb, th, cs) : OK;
+	if (ret) return ret;
 	const size_t nres = result_count(pb.G);
 	const size_t nu = (size_t)pb.nunits;
 	// device layout in rt.opt: res | ugates | udirs | dunits | hunits | grad | hvp
 	const size_t bytes = (nres + 4 * 16 * nu) * sizeof(double2) + 2 * 16 * nu * sizeof(double);
-	int ret = ensure_device(rt->result, bytes);
-	if (ret) return ret;
+	if ((ret = ensure_device(rt->result, bytes))) return ret;
 	double2* d_res = reinterpret_cast<double2*>(rt->result.ptr);
 	double2* d_ug = d_res + nres;
 	double2* d_uz = d_ug + 16 * nu;

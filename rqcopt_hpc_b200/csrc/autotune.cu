@@ -9,7 +9,7 @@
 // recompute them from the pass input, and for complex64 whether the passes run on the
 // FP32 FMA pipe or on the TF32 tensor-core MMA.
 //
-// On the first evaluation of a problem shape (qubits, gates, target gates, precision,
+// On the first evaluation of a problem shape (columns, qubits, gates, target gates, precision,
 // mode, target kind, paired columns) large enough for the choice to matter, every
 // candidate runs over the same contiguous sample of basis columns (the column range of
 // rqcopt_gpu_set_column_range) and is timed with CUDA events on the library stream;
@@ -92,7 +92,7 @@ double time_config(Runtime& rt, const Config& k, const CircuitSpec& c, const Tar
 int evaluate_autotuned(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int mode, int precision, double2* d_out)
 {
 	const int64_t N = (int64_t)1 << c.L;
-	const int64_t ncols = rt.real_pairs ? N / 2 : N;
+	const int64_t ncols = column_count(rt, c);
 	const double work = (double)ncols * (double)N * (double)(c.ngates + t.ngates);
 	// host-callback targets are not tuned: the sample runs would call the caller's ufunc
 	if (!rt.autotune || rt.tuning || c.L < 4 || work < TUNE_MIN_WORK || t.ufunc ||
@@ -100,7 +100,7 @@ int evaluate_autotuned(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, i
 		rt.last_choice = {rt.gates_per_pass, rt.column_chunk, rt.recon_c128, rt.c64_ffma, 0.0, 0};
 		return evaluate_configured(rt, c, t, mode, precision, d_out);
 	}
-	const std::array<long, 11> key = {c.L, c.ngates, t.ngates, precision, mode, t.ufunc ? 1 : 0, rt.real_pairs,
+	const std::array<long, 12> key = {(long)ncols, c.L, c.ngates, t.ngates, precision, mode, t.ufunc ? 1 : 0, rt.real_pairs,
 	                                  rt.pin_gpp ? rt.gates_per_pass : 0, rt.pin_chunk ? rt.column_chunk : -1,
 	                                  rt.pin_recon ? rt.recon_c128 : -1, rt.pin_ffma ? rt.c64_ffma : -1};
 	const Saved saved(rt);

@@ -37,16 +37,6 @@ constexpr int NPART = 64;   // doubles of partial sums per block and gate: 16 co
 
 // ---------------------------------------------------------------------------------- helpers
 
-// Paired basis columns (real-orthogonal problems): with c_pair_half = N/2 the column
-// with basis index b (< N/2) is e_b + i e_{b + N/2}; 0 selects plain basis columns.
-__constant__ int64_t c_pair_half = 0;
-
-template <typename T>
-__device__ __forceinline__ cplx<T> basis_amp(int64_t loc, int64_t b)
-{
-	return mk<T>(loc == b ? T(1) : T(0), (c_pair_half != 0 && loc == b + c_pair_half) ? T(1) : T(0));
-}
-
 __device__ __forceinline__ void block_add_f(double fx, double fy, double2* __restrict__ fpart)
 {
 	__shared__ double red[2][TPB / 32];
@@ -66,12 +56,12 @@ __device__ __forceinline__ void block_add_f(double fx, double fy, double2* __res
 // ---------------------------------------------------------------------------------- kernels
 
 // out = G in over all groups of a chunk.
-//   IN  0: read `in`; 1: column c of the chunk is the basis vector e_{b0 + c}
+//   IN  0: read `in`; 1: column c of the chunk is basis column c of src
 //   OUT 0: store; 1: store -conj(.); 2: no store, accumulate f += <phi, out> into fpart
 template <typename T, int IN, int OUT>
 __global__ void __launch_bounds__(TPB) k_apply(const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out,
                                                const cplx<T>* __restrict__ phi, Gate4<T> g, WirePair w, int L,
-                                               int64_t ngroups, int64_t b0, double2* __restrict__ fpart)
+                                               int64_t ngroups, ColumnSource src, double2* __restrict__ fpart)
 {
 	using V = cplx<T>;
 	const int lg = L - 2;
@@ -85,7 +75,7 @@ __global__ void __launch_bounds__(TPB) k_apply(const cplx<T>* __restrict__ in, c
 		const int64_t base = (c << L) + loc;
 		V x[4], y[4];
 #pragma unroll
-		for (int m = 0; m < 4; m++) x[m] = IN == 0 ? in[base + off[m]] : basis_amp<T>(loc + off[m], b0 + c);
+		for (int m = 0; m < 4; m++) x[m] = IN == 0 ? in[base + off[m]] : basis_amp<T>(src, loc + off[m], c);
 		gate_apply(g, x, y);
 #pragma unroll
 		for (int m = 0; m < 4; m++) {
@@ -109,7 +99,7 @@ template <typename T, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(TPB) k_forward(const cplx<T>* __restrict__ psi, const cplx<T>* __restrict__ dpsi,
                                                  cplx<T>* __restrict__ psi_o, cplx<T>* __restrict__ dpsi_o,
                                                  const cplx<T>* __restrict__ phi, Gate4<T> g, Gate4<T> z, WirePair w,
-                                                 int L, int64_t ngroups, int64_t b0, double2* __restrict__ fpart)
+                                                 int L, int64_t ngroups, ColumnSource src, double2* __restrict__ fpart)
 {
 	using V = cplx<T>;
 	const int lg = L - 2;
@@ -123,7 +113,7 @@ __global__ void __launch_bounds__(TPB) k_forward(const cplx<T>* __restrict__ psi
 		const int64_t base = (c << L) + loc;
 		V x[4], y[4];
 #pragma unroll
-		for (int m = 0; m < 4; m++) x[m] = FIRST ? basis_amp<T>(loc + off[m], b0 + c) : psi[base + off[m]];
+		for (int m = 0; m < 4; m++) x[m] = FIRST ? basis_amp<T>(src, loc + off[m], c) : psi[base + off[m]];
 		gate_apply(g, x, y);
 		if (LAST) {
 #pragma unroll
@@ -164,7 +154,7 @@ __global__ void __launch_bounds__(TPB) k_reverse(const cplx<T>* __restrict__ phi
                                                  const cplx<T>* __restrict__ psi, const cplx<T>* __restrict__ dpsi,
                                                  cplx<T>* __restrict__ phi_o, cplx<T>* __restrict__ dphi_o,
                                                  Gate4<T> g, Gate4<T> z, WirePair w, int L, int64_t ngroups,
-                                                 int64_t b0, double* __restrict__ part)
+                                                 ColumnSource src, double* __restrict__ part)
 {
 	using V = cplx<T>;
 	constexpr int NA = TAN ? 16 : 8;          // complex accumulators per thread
@@ -196,7 +186,7 @@ __global__ void __launch_bounds__(TPB) k_reverse(const cplx<T>* __restrict__ phi
 #pragma unroll
 		for (int m = 0; m < 4; m++) {
 			p[m] = phi[base + off[m]];
-			x[m] = LAST ? basis_amp<T>(loc + off[m], b0 + c) : psi[base + off[m]];
+			x[m] = LAST ? basis_amp<T>(src, loc + off[m], c) : psi[base + off[m]];
 			if (TAN) {
 				dp[m] = FIRST ? czero<V>() : dphi[base + off[m]];
 				dx[m] = LAST ? czero<V>() : dpsi[base + off[m]];
@@ -366,12 +356,12 @@ static Gate4<T> to_gate(const double2* g)
 
 template <typename T>
 static int launch_apply(Runtime& rt, int in_mode, int out_mode, const cplx<T>* in, cplx<T>* out, const cplx<T>* phi,
-                        const Gate4<T>& g, const WirePair& w, int L, int64_t ngroups, int64_t b0, double2* fpart, int fgrid)
+                        const Gate4<T>& g, const WirePair& w, int L, int64_t ngroups, const ColumnSource& src, double2* fpart, int fgrid)
 {
 	const int grid = out_mode == 2 ? fgrid : grid_for(rt, ngroups, 8);
 #define RQC_APPLY_CASE(I, O)                                                                             \
 	if (in_mode == I && out_mode == O) {                                                                 \
-		RQC_LAUNCH(rt, KC_APPLY, (k_apply<T, I, O>), grid, in, out, phi, g, w, L, ngroups, b0, fpart); \
+		RQC_LAUNCH(rt, KC_APPLY, (k_apply<T, I, O>), grid, in, out, phi, g, w, L, ngroups, src, fpart); \
 		return OK;                                                                                       \
 	}
 	RQC_APPLY_CASE(0, 0) RQC_APPLY_CASE(0, 1) RQC_APPLY_CASE(0, 2)
@@ -383,13 +373,13 @@ static int launch_apply(Runtime& rt, int in_mode, int out_mode, const cplx<T>* i
 template <typename T>
 static int launch_forward(Runtime& rt, bool first, bool last, const cplx<T>* psi, const cplx<T>* dpsi, cplx<T>* psi_o,
                           cplx<T>* dpsi_o, const cplx<T>* phi, const Gate4<T>& g, const Gate4<T>& z, const WirePair& w,
-                          int L, int64_t ngroups, int64_t b0, double2* fpart, int fgrid)
+                          int L, int64_t ngroups, const ColumnSource& src, double2* fpart, int fgrid)
 {
 	const int grid = last ? fgrid : grid_for(rt, ngroups, 8);
 #define RQC_FWD_CASE(F, LA)                                                                                         \
 	if (first == F && last == LA) {                                                                                 \
 		RQC_LAUNCH(rt, KC_FORWARD, (k_forward<T, F, LA>), grid, psi, dpsi, psi_o, dpsi_o, phi, g, z, w, L, ngroups, \
-		           b0, fpart);                                                                                      \
+		           src, fpart);                                                                                      \
 		return OK;                                                                                                  \
 	}
 	RQC_FWD_CASE(false, false) RQC_FWD_CASE(true, false) RQC_FWD_CASE(false, true) RQC_FWD_CASE(true, true)
@@ -400,13 +390,13 @@ static int launch_forward(Runtime& rt, bool first, bool last, const cplx<T>* psi
 template <typename T>
 static int launch_reverse(Runtime& rt, bool tan, bool first, bool last, const cplx<T>* phi, const cplx<T>* dphi,
                           const cplx<T>* psi, const cplx<T>* dpsi, cplx<T>* phi_o, cplx<T>* dphi_o, const Gate4<T>& g,
-                          const Gate4<T>& z, const WirePair& w, int L, int64_t ngroups, int64_t b0, double* part,
+                          const Gate4<T>& z, const WirePair& w, int L, int64_t ngroups, const ColumnSource& src, double* part,
                           int grid)
 {
 #define RQC_REV_CASE(TA, F, LA)                                                                                        \
 	if (tan == TA && first == F && last == LA) {                                                                       \
 		RQC_LAUNCH(rt, KC_REVERSE, (k_reverse<T, TA, F, LA>), grid, phi, dphi, psi, dpsi, phi_o, dphi_o, g, z, w, L,   \
-		           ngroups, b0, part);                                                                                 \
+		           ngroups, src, part);                                                                                 \
 		return OK;                                                                                                     \
 	}
 	RQC_REV_CASE(false, false, false) RQC_REV_CASE(false, true, false)
@@ -446,7 +436,7 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 	using V = cplx<T>;
 	const int L = c.L, G = c.ngates;
 	const int64_t N = (int64_t)1 << L;
-	const int64_t ncols = rt.real_pairs ? N / 2 : N;   // (paired) basis columns
+	const int64_t ncols = column_count(rt, c);
 	const bool tan = mode == EVAL_HVP;
 	const bool host_target = t.ufunc != nullptr;
 
@@ -504,6 +494,13 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 	for (int64_t b0 = cbeg; b0 < cend; b0 += C) {
 		const int64_t Cc = std::min(C, cend - b0);
 		const int64_t ngroups = Cc * (N / 4);
+		ColumnSource src;
+		src.tab = c.columns;
+		src.b0 = b0;
+		src.end = cend;
+		src.pair_half = rt.real_pairs ? N / 2 : 0;
+		ColumnSource tsrc = src;
+		tsrc.weighted = 1;
 
 		// target columns phi = -conj(U e_b)
 		if (host_target) {
@@ -535,7 +532,7 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 				const V* in = first ? nullptr : P[(k - 1) & 1];
 				V* out = last ? PHI : P[k & 1];
 				if ((ret = launch_apply<T>(rt, first ? 1 : 0, last ? 1 : 0, in, out, nullptr, tg[k], tw[k], L, ngroups,
-				                           b0, nullptr, nblk)))
+				                           tsrc, nullptr, nblk)))
 					return ret;
 			}
 		}
@@ -545,7 +542,7 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 				const bool first = k == 0, last = k == G - 1;
 				const V* in = first ? nullptr : P[(k - 1) & 1];
 				if ((ret = launch_apply<T>(rt, first ? 1 : 0, last ? 2 : 0, in, last ? nullptr : P[k & 1], PHI, gg[k], gw[k],
-				                           L, ngroups, b0, fpart, nblk)))
+				                           L, ngroups, src, fpart, nblk)))
 					return ret;
 			}
 			continue;
@@ -557,11 +554,11 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 			if (tan) {
 				if ((ret = launch_forward<T>(rt, first, last, first ? nullptr : cache_at(k), first ? nullptr : dcache_at(k),
 				                             last ? nullptr : cache_at(k + 1), last ? nullptr : dcache_at(k + 1), PHI, gg[k],
-				                             zz[k], gw[k], L, ngroups, b0, fpart, nblk)))
+				                             zz[k], gw[k], L, ngroups, src, fpart, nblk)))
 					return ret;
 			} else {
 				if ((ret = launch_apply<T>(rt, first ? 1 : 0, last ? 2 : 0, first ? nullptr : cache_at(k),
-				                           last ? nullptr : cache_at(k + 1), PHI, gg[k], gw[k], L, ngroups, b0, fpart, nblk)))
+				                           last ? nullptr : cache_at(k + 1), PHI, gg[k], gw[k], L, ngroups, src, fpart, nblk)))
 					return ret;
 			}
 		}
@@ -576,7 +573,7 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 			if ((ret = launch_reverse<T>(rt, tan, first, last, ph, dph, last ? nullptr : cache_at(k),
 			                             (last || !tan) ? nullptr : dcache_at(k), last ? nullptr : P[nxt],
 			                             (last || !tan) ? nullptr : D[nxt], gg[k], tan ? zz[k] : zero_gate, gw[k], L,
-			                             ngroups, b0, part + (size_t)k * nblk * NPART, nblk)))
+			                             ngroups, src, part + (size_t)k * nblk * NPART, nblk)))
 				return ret;
 		}
 	}
@@ -586,20 +583,12 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 	return RQC_CUDA(cudaGetLastError());
 }
 
-int set_pair_half_fused(Runtime& rt, int64_t half);
-
 namespace {
 
 __global__ void k_real_part(double2* __restrict__ d, int64_t n)
 {
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
 		d[i].y = 0;
-}
-
-int set_pair_half(Runtime& rt, int64_t half)
-{
-	int ret = RQC_CUDA(cudaMemcpyToSymbolAsync(c_pair_half, &half, sizeof(half), 0, cudaMemcpyHostToDevice, rt.stream));
-	return ret ? ret : set_pair_half_fused(rt, half);
 }
 
 }  // namespace
@@ -613,19 +602,24 @@ int evaluate_configured(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, 
 	return evaluate_columns(rt, c, t, mode, precision, d_out);
 }
 
-// With rt.real_pairs (real gates, real target): the 2^(L-1) paired columns
-// e_b + i e_{b + N/2}.  Every sum the engine forms pairs an adjoint-type state (from
+// With rt.real_pairs (real gates, real target): paired columns e_b + i e_b' (b' = b + N/2,
+// or the pairs of a column list).  Every sum the engine forms pairs an adjoint-type state (from
 // -conj(U psi)) with a forward-type state, both propagated by real matrices, so its
 // real part is the sum of the two real columns' terms; the imaginary parts (cross
 // terms) are cleared.
-int evaluate(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int mode, int precision, double2* d_out)
+int evaluate(Runtime& rt, const CircuitSpec& spec, const TargetSpec& t, int mode, int precision, double2* d_out)
 {
+	CircuitSpec c = spec;
+	if (precision != PREC_C128) {
+		// complex64 sums run over every column: their rounding errors (1e-6 of the result)
+		// average over the columns, and the results stay those of the sum over all of them
+		// bit by bit (over one column per orbit they move by 1e-6)
+		c.columns = nullptr;
+		c.ncolumns = 0;
+	}
 	if (!rt.real_pairs) return evaluate_autotuned(rt, c, t, mode, precision, d_out);
 	if (c.L < 2) return E_ARG;
-	int ret = set_pair_half(rt, (int64_t)1 << (c.L - 1));
-	if (!ret) ret = evaluate_autotuned(rt, c, t, mode, precision, d_out);
-	const int reset = set_pair_half(rt, 0);
-	if (!ret) ret = reset;
+	int ret = evaluate_autotuned(rt, c, t, mode, precision, d_out);
 	if (ret) return ret;
 	k_real_part<<<1, 256, 0, rt.stream>>>(d_out, (int64_t)result_count(c.ngates));
 	rt.launches++;
@@ -661,7 +655,7 @@ static int evaluate_columns(Runtime& rt, const CircuitSpec& c, const TargetSpec&
 int gate_apply_device(Runtime& rt, int L, const double2* gate, int i, int j, const double2* d_in, double2* d_out, long ncols)
 {
 	const int64_t ngroups = (int64_t)ncols << (L - 2);
-	return launch_apply<double>(rt, 0, 0, d_in, d_out, nullptr, to_gate<double>(gate), make_pair_(L, i, j), L, ngroups, 0,
+	return launch_apply<double>(rt, 0, 0, d_in, d_out, nullptr, to_gate<double>(gate), make_pair_(L, i, j), L, ngroups, ColumnSource{},
 	                            nullptr, 0);
 }
 
@@ -698,7 +692,7 @@ int apply_circuit_device_c64(Runtime& rt, int L, int ngates, const double2* gate
 	for (int k = 0; k < ngates; k++) {
 		float2* dst = ((ngates - 1 - k) % 2 == 0) ? d_out : tmp;
 		if ((ret = launch_apply<float>(rt, 0, 0, src, dst, nullptr, to_gate<float>(gates + 16 * k),
-		                               make_pair_(L, wires[2 * k], wires[2 * k + 1]), L, ngroups, 0, nullptr, 0)))
+		                               make_pair_(L, wires[2 * k], wires[2 * k + 1]), L, ngroups, ColumnSource{}, nullptr, 0)))
 			return ret;
 		src = dst;
 	}
@@ -718,7 +712,7 @@ int gate_backward_device(Runtime& rt, int L, const double2* gate, int i, int j, 
 	if ((ret = RQC_CUDA(cudaMemsetAsync(part, 0, part_doubles * sizeof(double), rt.stream)))) return ret;
 	const Gate4<double> zero_gate{};
 	if ((ret = launch_reverse<double>(rt, false, true, false, d_dout, nullptr, d_psi, nullptr, d_dpsi, nullptr,
-	                                  to_gate<double>(gate), zero_gate, make_pair_(L, i, j), L, ngroups, 0, part, nblk)))
+	                                  to_gate<double>(gate), zero_gate, make_pair_(L, i, j), L, ngroups, ColumnSource{}, part, nblk)))
 		return ret;
 	if ((ret = ensure_device(rt.result, result_count(1) * sizeof(double2)))) return ret;
 	double2* res = reinterpret_cast<double2*>(rt.result.ptr);
@@ -728,7 +722,7 @@ int gate_backward_device(Runtime& rt, int L, const double2* gate, int i, int j, 
 	return RQC_CUDA(cudaMemcpyAsync(d_dgate, res + 1, 16 * sizeof(double2), cudaMemcpyDeviceToDevice, rt.stream));
 }
 
-int target_columns_device(Runtime& rt, const TargetSpec& t, int L, int64_t b0, int64_t ncols, double2* phi,
+int target_columns_device(Runtime& rt, const TargetSpec& t, int L, const ColumnSource& src, int64_t ncols, double2* phi,
                           double2* p0, double2* p1)
 {
 	const int64_t N = (int64_t)1 << L;
@@ -741,7 +735,7 @@ int target_columns_device(Runtime& rt, const TargetSpec& t, int L, int64_t b0, i
 		const linear_func uf = reinterpret_cast<linear_func>(t.ufunc);
 		for (int64_t c = 0; c < ncols; c++) {
 			memset(hbasis, 0, N * sizeof(double2));
-			hbasis[b0 + c].x = 1;
+			hbasis[src.b0 + c].x = 1;
 			statevector e = { reinterpret_cast<numeric*>(hbasis), L };
 			statevector u = { reinterpret_cast<numeric*>(hcols + c * N), L };
 			const int r = uf(&e, t.udata, &u);
@@ -763,7 +757,7 @@ int target_columns_device(Runtime& rt, const TargetSpec& t, int L, int64_t b0, i
 		const bool first = k == 0, last = k == t.ngates - 1;
 		if ((ret = launch_apply<double>(rt, first ? 1 : 0, last ? 1 : 0, first ? nullptr : P[(k - 1) & 1],
 		                                last ? phi : P[k & 1], nullptr, to_gate<double>(t.gates + 16 * k),
-		                                make_pair_(L, t.wires[2 * k], t.wires[2 * k + 1]), L, ngroups, b0, nullptr, 0)))
+		                                make_pair_(L, t.wires[2 * k], t.wires[2 * k + 1]), L, ngroups, src, nullptr, 0)))
 			return ret;
 	}
 	return OK;
@@ -804,7 +798,7 @@ int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2*
 		const bool first = k == 0, last = k == t.ngates - 1;
 		if ((ret = launch_apply<double>(rt, 0, last ? 1 : 0, first ? states : P[(k - 1) & 1], last ? phi : P[k & 1],
 		                                nullptr, to_gate<double>(t.gates + 16 * k),
-		                                make_pair_(L, t.wires[2 * k], t.wires[2 * k + 1]), L, ngroups, 0, nullptr, 0)))
+		                                make_pair_(L, t.wires[2 * k], t.wires[2 * k + 1]), L, ngroups, ColumnSource{}, nullptr, 0)))
 			return ret;
 	}
 	return OK;
@@ -862,10 +856,10 @@ int column_passes_device(Runtime& rt, int L, int ngates, const double2* gates, c
 		if (tan) {
 			V* dout = k + 1 < G ? dcache + (int64_t)(k + 1) * N : sink;
 			if ((ret = launch_forward<double>(rt, false, false, psi_at(k), dcache + (int64_t)k * N, out, dout, nullptr,
-			                                  gg[k], zz[k], gw[k], L, ngroups, 0, nullptr, 0)))
+			                                  gg[k], zz[k], gw[k], L, ngroups, ColumnSource{}, nullptr, 0)))
 				return ret;
 		} else {
-			if ((ret = launch_apply<double>(rt, 0, 0, psi_at(k), out, nullptr, gg[k], gw[k], L, ngroups, 0, nullptr, 0)))
+			if ((ret = launch_apply<double>(rt, 0, 0, psi_at(k), out, nullptr, gg[k], gw[k], L, ngroups, ColumnSource{}, nullptr, 0)))
 				return ret;
 		}
 	}
@@ -877,7 +871,7 @@ int column_passes_device(Runtime& rt, int L, int ngates, const double2* gates, c
 		V* po = k > 0 ? P[nxt] : sink;
 		V* dpo = tan ? (k > 0 ? D[nxt] : sink + N) : nullptr;
 		if ((ret = launch_reverse<double>(rt, tan, first, false, ph, (first || !tan) ? nullptr : D[cur], psi_at(k),
-		                                  tan ? dcache + (int64_t)k * N : nullptr, po, dpo, gg[k], zz[k], gw[k], L, ngroups, 0,
+		                                  tan ? dcache + (int64_t)k * N : nullptr, po, dpo, gg[k], zz[k], gw[k], L, ngroups, ColumnSource{},
 		                                  part + (size_t)k * nblk * NPART, nblk)))
 			return ret;
 	}

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include "rqc_common.cuh"
 #include "rqc_runtime.h"
 
 namespace rqc {
@@ -19,7 +20,17 @@ struct CircuitSpec
 	const double2* gates = nullptr;   // [ngates][16]
 	const double2* dirs = nullptr;    // [ngates][16], EVAL_HVP only
 	const int* wires = nullptr;       // [2 * ngates]
+	// columns to sum over instead of all basis states (device; rt.columns, see orbits.h)
+	const BasisCol* columns = nullptr;
+	int64_t ncolumns = 0;
 };
+
+// columns of an evaluation: the listed ones, or all (paired) basis states
+inline int64_t column_count(const Runtime& rt, const CircuitSpec& c)
+{
+	if (c.columns) return c.ncolumns;
+	return ((int64_t)1 << c.L) >> (rt.real_pairs ? 1 : 0);
+}
 
 // The target U: either a circuit evaluated on the device (gates, wires) or a
 // host callback `linear_func` applied to one basis column at a time.
@@ -30,6 +41,7 @@ struct TargetSpec
 	const int* wires = nullptr;
 	void* ufunc = nullptr;
 	void* udata = nullptr;
+	int per = 1;   // consecutive gates that are copies of one (brickwall layer)
 };
 
 // Device result layout (double2): [0] f, [1 + 16 g + e] dG_g[e], [1 + 16 G + 16 g + e] (H Z)_g[e]
@@ -76,10 +88,10 @@ int gate_backward_device(Runtime& rt, int L, const double2* gate, int i, int j, 
 int column_passes_device(Runtime& rt, int L, int ngates, const double2* gates, const double2* dirs, const int* wires,
                          const double2* d_psi, const double2* d_phi, double2* d_psi_out, double2* d_dgates,
                          double2* d_hess);
-// Target columns of one chunk: phi[c] = -conj(U e_{b0 + c}) for c < ncols (states of
-// 2^L amplitudes one after another), through the device circuit of t or its host
-// callback; p0 and p1 are two chunk-sized scratch arrays.
-int target_columns_device(Runtime& rt, const TargetSpec& t, int L, int64_t b0, int64_t ncols, double2* phi,
+// Target columns of one chunk: phi[c] = -conj(U e_c), e_c column c of src, for c < ncols
+// (states of 2^L amplitudes one after another), through the device circuit of t or its host
+// callback (plain basis states only); p0 and p1 are two chunk-sized scratch arrays.
+int target_columns_device(Runtime& rt, const TargetSpec& t, int L, const ColumnSource& src, int64_t ncols, double2* phi,
                           double2* p0, double2* p1);
 // The same for given input states: phi[c] = -conj(U states[c]).
 int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2* states, int64_t ncols, double2* phi,

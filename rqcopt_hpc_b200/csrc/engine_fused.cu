@@ -44,7 +44,6 @@ constexpr int TPB2 = 256;
 constexpr int MAXK = 4;
 constexpr int MAXNB = 8;
 constexpr int NPART2 = 64;
-constexpr int EPT = (1 << MAXNB) * 4 / TPB2;   // complex128 tile elements per thread (4 columns per row)
 
 template <typename T> struct ColsPer;
 template <> struct ColsPer<double> { static constexpr int v = 4; };   // 4 x 16 B = 64 B runs
@@ -61,22 +60,9 @@ struct PassGeom
 	int64_t C;             // allocated columns of the chunk (row pitch)
 	int64_t ncg;           // column groups of CW columns covering the valid columns
 	int64_t ntiles;        // row tiles (2^(L-NB)) x column groups
-	int64_t b0;            // basis index of the chunk's first column
+	ColumnSource src;      // the chunk's columns
 	uint32_t rest_mask;    // state row bits that are not tile bits
 };
-
-// Paired basis columns (real-orthogonal problems): with c_pair_half = N/2 the column
-// with basis index b (< N/2) is e_b + i e_{b + N/2}; 0 selects plain basis columns.
-__constant__ int64_t c_pair_half = 0;
-// End of the column range of the current evaluation: the columns of a chunk's last
-// column group at or beyond it are zero (they add nothing to any sum).
-__constant__ int64_t c_col_end = INT64_MAX;
-
-__device__ __forceinline__ float basis_re(int64_t row, int64_t b) { return (row == b && b < c_col_end) ? 1.f : 0.f; }
-__device__ __forceinline__ float basis_im(int64_t row, int64_t b)
-{
-	return (c_pair_half != 0 && b < c_col_end && row == b + c_pair_half) ? 1.f : 0.f;
-}
 
 template <typename T> struct PassGates { Gate4<T> g[MAXK]; Gate4<T> z[MAXK]; };
 // W_k = G_k^+ Z_k G_k^+ of each gate of a pass (adjoint reconstruction of the tangent state)
@@ -92,6 +78,13 @@ __device__ __forceinline__ int64_t deposit(int64_t v, uint32_t mask)
 		mask &= mask - 1;
 	}
 	return r;
+}
+
+// amplitude `row` of columns col and col + 1 (complex64)
+__device__ __forceinline__ float4 basis_pair(const ColumnSource& s, int64_t row, int64_t col)
+{
+	const float2 a = basis_amp<float>(s, row, col), b = basis_amp<float>(s, row, col + 1);
+	return make_float4(a.x, a.y, b.x, b.y);
 }
 
 template <typename T>
@@ -137,324 +130,6 @@ __device__ __forceinline__ cplx<T> sel4(const cplx<T> v[4], int q)
 __device__ __forceinline__ int sel4_int(const int v[4], int q)
 {
 	return q == 0 ? v[0] : q == 1 ? v[1] : q == 2 ? v[2] : v[3];
-}
-
-// ------------------------------------------------------------------------------ forward kernel
-
-// One pass forward over tiles.  IN: 0 read psi/dpsi, 1 basis columns (dpsi = 0).
-// OUT: 0 store psi/dpsi, 1 store -conj(psi) (no tangent), 2 f += <phi, psi> (no store).
-template <typename T, bool TAN, int IN, int OUT>
-__global__ void __launch_bounds__(TPB2) k2_fwd(const cplx<T>* __restrict__ psi, const cplx<T>* __restrict__ dpsi,
-                                               cplx<T>* __restrict__ psi_o, cplx<T>* __restrict__ dpsi_o,
-                                               const cplx<T>* __restrict__ phi, PassGeom pg, PassGates<T> gates,
-                                               double2* __restrict__ fpart)
-{
-	using V = cplx<T>;
-	constexpr int CW = ColsPer<T>::v;
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	const int R = 1 << pg.NB, A = R * CW;
-	V* sg = reinterpret_cast<V*>(smem_raw);                       // 32 * MAXK gate entries
-	int* rowoff = reinterpret_cast<int*>(sg + 32 * MAXK);          // R
-	V* S = reinterpret_cast<V*>(rowoff + (1 << MAXNB));            // psi tile [R][CW]
-	V* dS = S + A;                                                 // dpsi tile
-	gates_to_smem<T>(gates, pg.K, TAN, sg);
-	row_offsets(pg, rowoff);
-	const int64_t rtiles = (int64_t)1 << (pg.L - pg.NB);
-	double fx = 0, fy = 0;
-	__syncthreads();
-
-	for (int64_t tile = blockIdx.x; tile < pg.ntiles; tile += gridDim.x) {
-		const int64_t rt = tile / pg.ncg, cg = tile - rt * pg.ncg;
-		(void)rtiles;
-		const int64_t rowbase = deposit(rt, pg.rest_mask);
-		const int64_t colbase = cg * CW;
-		// load
-		for (int e = threadIdx.x; e < A; e += blockDim.x) {
-			const int r = e / CW, cc = e - r * CW;
-			const int64_t row = rowbase + rowoff[r];
-			const int64_t col = colbase + cc;
-			if (IN == 0) {
-				const int64_t a = row * pg.C + col;
-				S[e] = psi[a];
-				if (TAN) dS[e] = dpsi[a];
-			} else {
-				S[e] = mk<T>(T(basis_re(row, pg.b0 + col)), T(basis_im(row, pg.b0 + col)));
-				if (TAN) dS[e] = czero<V>();
-			}
-		}
-		__syncthreads();
-		// gate steps
-		for (int k = 0; k < pg.K; k++) {
-			const V* gk = sg + 32 * k;
-			const int bi = pg.gi[k], bj = pg.gj[k];
-			for (int base = 0; base < A; base += blockDim.x) {
-				const int task = base + threadIdx.x;
-				const bool active = task < A;
-				const int g = task >> 2, q = task & 3;
-				const int cc = g % CW, b6 = g / CW;
-				int rows[4];
-				group_rows(b6, bi, bj, rows);
-				V x[4], dx[4], y = czero<V>(), dy = czero<V>();
-				if (active) {
-#pragma unroll
-					for (int m = 0; m < 4; m++) {
-						x[m] = S[rows[m] * CW + cc];
-						if (TAN) dx[m] = dS[rows[m] * CW + cc];
-					}
-#pragma unroll
-					for (int m = 0; m < 4; m++) {
-						y = cfma(gk[4 * q + m], x[m], y);
-						if (TAN) {
-							dy = cfma(gk[4 * q + m], dx[m], dy);
-							dy = cfma(gk[16 + 4 * q + m], x[m], dy);
-						}
-					}
-				}
-				__syncwarp();
-				if (active) {
-					const int r = sel4_int(rows, q);
-					S[r * CW + cc] = y;
-					if (TAN) dS[r * CW + cc] = dy;
-				}
-			}
-			__syncthreads();
-		}
-		// store / reduce
-		for (int e = threadIdx.x; e < A; e += blockDim.x) {
-			const int r = e / CW, cc = e - r * CW;
-			const int64_t a = (rowbase + rowoff[r]) * pg.C + colbase + cc;
-			if (OUT == 2) {
-				const V p = phi[a];
-				const V s = S[e];
-				fx += (double)p.x * s.x - (double)p.y * s.y;
-				fy += (double)p.x * s.y + (double)p.y * s.x;
-			} else if (OUT == 1) {
-				psi_o[a] = cneg_conj(S[e]);
-			} else {
-				psi_o[a] = S[e];
-				if (TAN) dpsi_o[a] = dS[e];
-			}
-		}
-		__syncthreads();
-	}
-	if (OUT == 2) {
-		__shared__ double red[2][TPB2 / 32];
-		fx = warp_sum(fx);
-		fy = warp_sum(fy);
-		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-		if (lane == 0) { red[0][warp] = fx; red[1][warp] = fy; }
-		__syncthreads();
-		if (threadIdx.x == 0) {
-			double sx = 0, sy = 0;
-			for (int w = 0; w < TPB2 / 32; w++) { sx += red[0][w]; sy += red[1][w]; }
-			fpart[blockIdx.x].x += sx;
-			fpart[blockIdx.x].y += sy;
-		}
-	}
-}
-
-// ------------------------------------------------------------------------------ reverse kernel
-
-// One pass in reverse over tiles.  FIRST: the pass ends the circuit (dphi = 0).
-// LAST: the pass starts the circuit (psi is the basis column, dpsi = 0, no outputs).
-// part: per-gate partial sums of the pass, gate k at part + k * nblk * 64, block b at + b * 64.
-template <typename T, bool TAN, bool FIRST, bool LAST>
-__global__ void __launch_bounds__(TPB2, 1) k2_rev(const cplx<T>* __restrict__ psi, const cplx<T>* __restrict__ dpsi,
-                                                  const cplx<T>* __restrict__ phi, const cplx<T>* __restrict__ dphi,
-                                                  cplx<T>* __restrict__ phi_o, cplx<T>* __restrict__ dphi_o,
-                                                  PassGeom pg, PassGates<T> gates, double* __restrict__ part, int nblk)
-{
-	using V = cplx<T>;
-	constexpr int CW = ColsPer<T>::v;
-	constexpr bool FLUSH = sizeof(T) == 4;
-	constexpr int RUN = 4;
-	constexpr int NV = TAN ? 16 : 8;   // accumulator reals per gate: row q of dG (and of HZ)
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	const int R = 1 << pg.NB, A = R * CW, K = pg.K;
-	V* sg = reinterpret_cast<V*>(smem_raw);
-	int* rowoff = reinterpret_cast<int*>(sg + 32 * MAXK);
-	V* tiles = reinterpret_cast<V*>(rowoff + (1 << MAXNB));
-	V* Psi = tiles;                               // K tiles: state entering gate k
-	V* dPsi = TAN ? tiles + K * A : nullptr;      // K tiles
-	V* Phi = tiles + (TAN ? 2 * K : K) * A;       // adjoint
-	V* dPhi = TAN ? Phi + A : nullptr;
-	gates_to_smem<T>(gates, K, TAN, sg);
-	row_offsets(pg, rowoff);
-	const int q = threadIdx.x & 3;
-
-	T acc[MAXK][NV];
-	double accd[MAXK][FLUSH ? NV : 1];
-#pragma unroll
-	for (int k = 0; k < MAXK; k++)
-#pragma unroll
-		for (int v = 0; v < NV; v++) {
-			acc[k][v] = 0;
-			if (FLUSH) accd[k][v] = 0;
-		}
-	int run = 0;
-	__syncthreads();
-
-	for (int64_t tile = blockIdx.x; tile < pg.ntiles; tile += gridDim.x) {
-		const int64_t rt = tile / pg.ncg, cg = tile - rt * pg.ncg;
-		const int64_t rowbase = deposit(rt, pg.rest_mask);
-		const int64_t colbase = cg * CW;
-		for (int e = threadIdx.x; e < A; e += blockDim.x) {
-			const int r = e / CW, cc = e - r * CW;
-			const int64_t row = rowbase + rowoff[r], col = colbase + cc;
-			const int64_t a = row * pg.C + col;
-			if (LAST) {
-				Psi[e] = mk<T>(T(basis_re(row, pg.b0 + col)), T(basis_im(row, pg.b0 + col)));
-				if (TAN) dPsi[e] = czero<V>();
-			} else {
-				Psi[e] = psi[a];
-				if (TAN) dPsi[e] = dpsi[a];
-			}
-			Phi[e] = phi[a];
-			if (TAN) dPhi[e] = FIRST ? czero<V>() : dphi[a];
-		}
-		__syncthreads();
-		// recompute the states entering gates 1..K-1
-#pragma unroll
-		for (int k = 0; k < MAXK - 1; k++) {
-			if (k + 1 >= K) break;
-			const V* gk = sg + 32 * k;
-			const V* src = Psi + k * A;
-			V* dst = Psi + (k + 1) * A;
-			const V* dsrc = TAN ? dPsi + k * A : nullptr;
-			V* ddst = TAN ? dPsi + (k + 1) * A : nullptr;
-			for (int base = 0; base < A; base += blockDim.x) {
-				const int task = base + threadIdx.x;
-				if (task >= A) break;
-				const int g = task >> 2;
-				const int cc = g % CW, b6 = g / CW;
-				int rows[4];
-				group_rows(b6, pg.gi[k], pg.gj[k], rows);
-				V y = czero<V>(), dy = czero<V>();
-#pragma unroll
-				for (int m = 0; m < 4; m++) {
-					const V x = src[rows[m] * CW + cc];
-					y = cfma(gk[4 * q + m], x, y);
-					if (TAN) {
-						dy = cfma(gk[16 + 4 * q + m], x, dy);
-						dy = cfma(gk[4 * q + m], dsrc[rows[m] * CW + cc], dy);
-					}
-				}
-				const int r = sel4_int(rows, q);
-				dst[r * CW + cc] = y;
-				if (TAN) ddst[r * CW + cc] = dy;
-			}
-			__syncthreads();
-		}
-		// reverse through the pass
-#pragma unroll
-		for (int k = MAXK - 1; k >= 0; k--) {
-			if (k >= K) continue;
-			const V* gk = sg + 32 * k;
-			const V* X = Psi + k * A;
-			const V* dX = TAN ? dPsi + k * A : nullptr;
-			const bool first_gate = FIRST && k == K - 1;   // adjoint tangent still zero
-			const bool last_gate = LAST && k == 0;         // entering state is the basis column, dpsi = 0
-			for (int base = 0; base < A; base += blockDim.x) {
-				const int task = base + threadIdx.x;
-				const bool active = task < A;
-				const int g = task >> 2;
-				const int cc = g % CW, b6 = g / CW;
-				int rows[4];
-				group_rows(b6, pg.gi[k], pg.gj[k], rows);
-				V p[4], dp[4], x[4], dx[4];
-				V np = czero<V>(), ndp = czero<V>();
-				if (active) {
-#pragma unroll
-					for (int m = 0; m < 4; m++) {
-						const int a = rows[m] * CW + cc;
-						p[m] = Phi[a];
-						x[m] = X[a];
-						if (TAN) {
-							dp[m] = dPhi[a];
-							dx[m] = dX[a];
-						}
-					}
-					const V pq = sel4<T>(p, q);
-					const V dpq = TAN ? sel4<T>(dp, q) : czero<V>();
-#pragma unroll
-					for (int c = 0; c < 4; c++) {
-						acc[k][2 * c]     = fma(pq.x, x[c].x, fma(-pq.y, x[c].y, acc[k][2 * c]));
-						acc[k][2 * c + 1] = fma(pq.x, x[c].y, fma(pq.y, x[c].x, acc[k][2 * c + 1]));
-						if (TAN) {
-							T hx = acc[k][8 + 2 * c], hy = acc[k][8 + 2 * c + 1];
-							if (!last_gate) {
-								hx = fma(pq.x, dx[c].x, fma(-pq.y, dx[c].y, hx));
-								hy = fma(pq.x, dx[c].y, fma(pq.y, dx[c].x, hy));
-							}
-							if (!first_gate) {
-								hx = fma(dpq.x, x[c].x, fma(-dpq.y, x[c].y, hx));
-								hy = fma(dpq.x, x[c].y, fma(dpq.y, x[c].x, hy));
-							}
-							acc[k][8 + 2 * c] = hx;
-							acc[k][8 + 2 * c + 1] = hy;
-						}
-					}
-					if (!(LAST && k == 0)) {
-#pragma unroll
-						for (int r = 0; r < 4; r++) {
-							np = cfma(gk[4 * r + q], p[r], np);
-							if (TAN) {
-								ndp = cfma(gk[16 + 4 * r + q], p[r], ndp);
-								if (!first_gate) ndp = cfma(gk[4 * r + q], dp[r], ndp);
-							}
-						}
-					}
-				}
-				__syncwarp();
-				if (active && !(LAST && k == 0)) {
-					const int r = sel4_int(rows, q);
-					Phi[r * CW + cc] = np;
-					if (TAN) dPhi[r * CW + cc] = ndp;
-				}
-			}
-			if (FLUSH && ++run == RUN) {
-				run = 0;
-#pragma unroll
-				for (int kk = 0; kk < MAXK; kk++)
-#pragma unroll
-					for (int v = 0; v < NV; v++) { accd[kk][v] += acc[kk][v]; acc[kk][v] = 0; }
-			}
-			__syncthreads();
-		}
-		if (!LAST) {
-			for (int e = threadIdx.x; e < A; e += blockDim.x) {
-				const int r = e / CW, cc = e - r * CW;
-				const int64_t a = (rowbase + rowoff[r]) * pg.C + colbase + cc;
-				phi_o[a] = Phi[e];
-				if (TAN) dphi_o[a] = dPhi[e];
-			}
-		}
-		__syncthreads();
-	}
-
-	// reduce: lanes with equal q (xor 16, 8, 4), then over warps
-	double* red = reinterpret_cast<double*>(tiles);   // [warps][4][MAXK * NV]
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-	for (int k = 0; k < MAXK; k++)
-#pragma unroll
-		for (int v = 0; v < NV; v++) {
-			double x = FLUSH ? accd[k][v] + (double)acc[k][v] : (double)acc[k][v];
-			x += __shfl_xor_sync(0xffffffffu, x, 16);
-			x += __shfl_xor_sync(0xffffffffu, x, 8);
-			x += __shfl_xor_sync(0xffffffffu, x, 4);
-			if (lane < 4) red[(warp * 4 + lane) * (MAXK * NV) + k * NV + v] = x;
-		}
-	__syncthreads();
-	const int nwarps = blockDim.x >> 5;
-	for (int idx = threadIdx.x; idx < 4 * K * NV; idx += blockDim.x) {
-		const int qq = idx / (K * NV), rem = idx % (K * NV), k = rem / NV, v = rem % NV;
-		double s = 0;
-		for (int w = 0; w < nwarps; w++) s += red[(w * 4 + qq) * (MAXK * NV) + k * NV + v];
-		// v < 8: dG row qq (complex c = v/2); v >= 8: HZ row qq
-		const int dst = v < 8 ? 8 * qq + v : 32 + 8 * qq + (v - 8);
-		part[(size_t)k * nblk * NPART2 + (size_t)blockIdx.x * NPART2 + dst] += s;
-	}
 }
 
 // ------------------------------------------------------------------------------ complex128 kernels on the FP64 MMA
@@ -678,8 +353,10 @@ inline size_t k3_fwd_smem(int NB, bool tan)
 	return 32 * MAXK * sizeof(double2) + (1 << MAXNB) * sizeof(int) + (tan ? 4 : 2) * ((size_t)1 << NB) * 4 * sizeof(double2);
 }
 
-// Forward pass (complex128).  Same contract as k2_fwd; OUT 3 writes the pass output
-// and adds f, as the last pass does when the reverse pass rebuilds states from it.
+// One pass forward over tiles (complex128).  IN: 0 read psi/dpsi, 1 basis columns (dpsi = 0).
+// OUT: 0 store psi/dpsi, 1 store -conj(psi) (no tangent), 2 f += <phi, psi> (no store),
+// 3 store the pass output and add f, as the last pass does when the reverse pass rebuilds
+// states from it.
 // Tiles are double-buffered in shared memory: the next tile position's state arrives
 // by cp.async while the gates run on the current one.
 template <bool TAN, int IN, int OUT>
@@ -737,7 +414,7 @@ __global__ void __launch_bounds__(NTF, TAN ? 3 : 6) k3_fwd(const double2* __rest
 				const int r = e >> 2, cc = e & 3;
 				const int pe = sidx(r, cc);
 				const int64_t row = rowbase + rowoff[r], col = colbase + cc;
-				S[pe] = make_double2(basis_re(row, pg.b0 + col), basis_im(row, pg.b0 + col));
+				S[pe] = basis_amp<double>(pg.src, row, col);
 				if (TAN) dS[pe] = make_double2(0, 0);
 			}
 		}
@@ -826,7 +503,9 @@ __global__ void __launch_bounds__(NTF, TAN ? 3 : 6) k3_fwd(const double2* __rest
 	}
 }
 
-// Reverse pass (complex128).  Same contract as k2_rev; partials are raw 8x8 sums
+// One pass in reverse (complex128), from the checkpoint psi, dpsi at the pass input and
+// phi, dphi at its output.  FIRST: the circuit's last pass (dphi = 0); LAST: its first one
+// (psi the basis columns, dpsi = 0, no outputs).  Partials are raw 8x8 sums
 // (part + k * nblk * 128 + blockIdx.x * 128: [0, 64) dG, [64, 128) HZ, index m*8 + n).
 template <bool TAN, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(NTR, 1) k3_rev(const double2* __restrict__ psi, const double2* __restrict__ dpsi,
@@ -884,7 +563,7 @@ __global__ void __launch_bounds__(NTR, 1) k3_rev(const double2* __restrict__ psi
 			const int pe = sidx(r, cc);
 			if (LAST) {
 				const int64_t row = rowbase + rowoff[r], col = colbase + cc;
-				Psi[pe] = make_double2(basis_re(row, pg.b0 + col), basis_im(row, pg.b0 + col));
+				Psi[pe] = basis_amp<double>(pg.src, row, col);
 				if (TAN) dPsi[pe] = make_double2(0, 0);
 			} else {
 				Psi[pe] = ra[i];
@@ -1209,7 +888,7 @@ inline size_t k4_fwd_smem(int NB, bool tan, bool with_phi)
 	       MAXK * 32 * sizeof(int) + 2 * ns * A * sizeof(float2);
 }
 
-// Forward pass (complex64).  Same contract as k2_fwd.  The next tile streams into a
+// Forward pass (complex64).  Same contract as k3_fwd.  The next tile streams into a
 // second set of shared-memory buffers with cp.async while the current one is processed.
 template <bool TAN, int IN, int OUT>
 __global__ void __launch_bounds__(NT4F, 3) k4_fwd(const float2* __restrict__ psi, const float2* __restrict__ dpsi,
@@ -1272,8 +951,7 @@ __global__ void __launch_bounds__(NT4F, 3) k4_fwd(const float2* __restrict__ psi
 			} else {
 				const int64_t row = rowbase + ro[i], col = colbase + c2i;
 				*reinterpret_cast<float4*>(stage(buf, 0) + pe) =
-				    make_float4(basis_re(row, pg.b0 + col), basis_im(row, pg.b0 + col), basis_re(row, pg.b0 + col + 1),
-				                basis_im(row, pg.b0 + col + 1));
+				    basis_pair(pg.src, row, col);
 				if (TAN) *reinterpret_cast<float4*>(stage(buf, 1) + pe) = make_float4(0.f, 0.f, 0.f, 0.f);
 			}
 			if (FSUM) cp_async16(stage(buf, NS - 1) + pe, phi + a);
@@ -1355,7 +1033,7 @@ inline size_t k4_rev_smem(int NB, int K, bool tan)
 }
 
 
-// Reverse pass (complex64).  Same contract as k2_rev; partials are raw sums
+// Reverse pass (complex64).  Same contract as k3_rev; partials are raw sums
 // (part + k * nblk * NRAW4 + blockIdx.x * NRAW4 + lane * 4 + v).
 // scratch: per-block FP64 lane sums, blockIdx.x * (NT4R/32 * 32 * MAXK * 4) doubles.
 // The next tile's inputs stream into a second set of shared-memory buffers with
@@ -1443,8 +1121,7 @@ __global__ void __launch_bounds__(NT4R, 1) k4_rev(const float2* __restrict__ psi
 			if (LAST) {
 				const int64_t row = rowbase + ro[i], col = colbase + c2i;
 				*reinterpret_cast<float4*>(stage(buf, 0) + pe) =
-				    make_float4(basis_re(row, pg.b0 + col), basis_im(row, pg.b0 + col), basis_re(row, pg.b0 + col + 1),
-				                basis_im(row, pg.b0 + col + 1));
+				    basis_pair(pg.src, row, col);
 				if (TAN) *reinterpret_cast<float4*>(stage(buf, 2) + pe) = make_float4(0.f, 0.f, 0.f, 0.f);
 			} else {
 				cp_async16(stage(buf, 0) + pe, psi + a);
@@ -2082,8 +1759,7 @@ __global__ void __launch_bounds__(NT7, 3) k7_fwd(const float2* __restrict__ psi,
 			} else {
 				const int64_t row = rowbase + ro[i], col = colbase + c2i;
 				*reinterpret_cast<float4*>(S + pe) =
-				    make_float4(basis_re(row, pg.b0 + col), basis_im(row, pg.b0 + col), basis_re(row, pg.b0 + col + 1),
-				                basis_im(row, pg.b0 + col + 1));
+				    basis_pair(pg.src, row, col);
 				if (TAN) *reinterpret_cast<float4*>(dS + pe) = make_float4(0.f, 0.f, 0.f, 0.f);
 			}
 		}
@@ -2463,7 +2139,7 @@ std::vector<Pass> schedule(int L, int G, const int* wires, int maxk)
 		}
 		for (int b = 0; __builtin_popcount(bits) < NB && b < L; b++) bits |= 1u << b;
 		Pass p;
-		memset(&p.geom, 0, sizeof(p.geom));
+		p.geom = PassGeom{};
 		p.first = i;
 		p.K = K;
 		p.geom.K = K;
@@ -2871,7 +2547,7 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 	constexpr int CW = ColsPer<T>::v;
 	const int L = c.L, G = c.ngates;
 	const int64_t N = (int64_t)1 << L;
-	const int64_t ncols = rt.real_pairs ? N / 2 : N;   // (paired) basis columns
+	const int64_t ncols = column_count(rt, c);
 	const bool tan = mode == EVAL_HVP;
 	const bool host_target = t.ufunc != nullptr;
 	std::vector<Pass> passes = schedule(L, G, c.wires, maxk);
@@ -2946,11 +2622,6 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 		dstage = reinterpret_cast<double2*>(rt.stage[2].ptr);
 	}
 
-	if (cend != rt.col_end_dev) {   // a copy from host memory waits for the stream: only when it changes
-		if ((ret = RQC_CUDA(cudaMemcpyToSymbolAsync(c_col_end, &cend, sizeof(cend), 0, cudaMemcpyHostToDevice, rt.stream))))
-			return ret;
-		rt.col_end_dev = cend;
-	}
 	for (int64_t b0 = cbeg; b0 < cend; b0 += C) {
 		const int64_t Cc = std::min(C, cend - b0);
 		const int64_t ncg = (Cc + CW - 1) / CW;
@@ -2959,7 +2630,10 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 			g.C = C;
 			g.ncg = ncg;
 			g.ntiles = ((int64_t)1 << (L - g.NB)) * ncg;
-			g.b0 = b0;
+			g.src.tab = c.columns;
+			g.src.b0 = b0;
+			g.src.end = cend;
+			g.src.pair_half = rt.real_pairs ? N / 2 : 0;
 			return g;
 		};
 
@@ -2986,7 +2660,8 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 			if ((ret = RQC_CUDA(cudaStreamSynchronize(rt.stream)))) return ret;
 		} else {
 			for (int p = 0; p < Pt; p++) {
-				const PassGeom g = geom(tpasses[p]);
+				PassGeom g = geom(tpasses[p]);
+				g.src.weighted = 1;
 				const bool first = p == 0, last = p == Pt - 1;
 				const V* in = first ? nullptr : Pb[(p - 1) & 1];
 				V* out = last ? PHI : Pb[p & 1];
@@ -3104,11 +2779,6 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 }
 
 }  // namespace
-
-int set_pair_half_fused(Runtime& rt, int64_t half)
-{
-	return RQC_CUDA(cudaMemcpyToSymbolAsync(c_pair_half, &half, sizeof(half), 0, cudaMemcpyHostToDevice, rt.stream));
-}
 
 int evaluate_fused(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int mode, int precision, int maxk, double2* d_out)
 {

@@ -880,7 +880,7 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 		if (samp) {
 			if ((ret = haar_states_device(rt, *samp, L, b0, Cc, states))) return ret;
 			if ((ret = target_states_device(rt, t, L, states, Cc, phi_at(G - 1), tq[0], tq[1]))) return ret;
-		} else if ((ret = target_columns_device(rt, t, L, b0, Cc, phi_at(G - 1), tq[0], tq[1]))) {
+		} else if ((ret = target_columns_device(rt, t, L, plain_columns(b0), Cc, phi_at(G - 1), tq[0], tq[1]))) {
 			return ret;
 		}
 		if ((ret = sw.reverse_chain(phi_at, ngroups, nullptr))) return ret;
@@ -973,7 +973,7 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	double2* fres = hess ? part2 + (size_t)m * m : jac;
 	if ((ret = RQC_CUDA(cudaMemsetAsync(fres, 0, nres * sizeof(double2), rt.stream)))) return ret;
 	if (hess && (ret = RQC_CUDA(cudaMemsetAsync(part2, 0, (size_t)m * m * sizeof(double2), rt.stream)))) return ret;
-	if ((ret = target_columns_device(rt, t, half, 0, s, hneg, sc0, sc1))) return ret;
+	if ((ret = target_columns_device(rt, t, half, plain_columns(0), s, hneg, sc0, sc1))) return ret;
 
 	Sweep sw(rt, c);
 	sw.keep_final = hess;

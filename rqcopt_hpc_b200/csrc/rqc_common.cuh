@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "orbits.h"
+
 namespace rqc {
 
 // ---------------------------------------------------------------- complex types
@@ -43,6 +45,45 @@ __device__ __forceinline__ double2 to_d(float2 a) { return make_double2(a.x, a.y
 
 // One 4x4 gate in arithmetic precision T, row-major (row = 2*b_i + b_j).
 template <typename T> struct Gate4 { cplx<T> m[16]; };
+
+// ---------------------------------------------------------------- basis columns
+
+// Where the columns of a chunk come from.  Column c of the chunk is number b0 + c: entry of
+// tab if there is one, otherwise basis state b0 + c (paired with b0 + c + pair_half if that
+// is not 0).  Columns at or beyond end are zero (they add nothing to any sum).  The weights
+// multiply the input of the target passes (weighted), so that phi carries them into every
+// sum, all of which are linear in phi.
+struct ColumnSource
+{
+	const BasisCol* tab = nullptr;
+	int64_t b0 = 0, end = INT64_MAX, pair_half = 0;
+	int weighted = 0;
+};
+
+inline ColumnSource plain_columns(int64_t b0)
+{
+	ColumnSource s;
+	s.b0 = b0;
+	return s;
+}
+
+// amplitude `row` of column c of the chunk
+template <typename T>
+__device__ __forceinline__ cplx<T> basis_amp(const ColumnSource& s, int64_t row, int64_t c)
+{
+	const int64_t k = s.b0 + c;
+	cplx<T> v = mk<T>(T(0), T(0));
+	if (k >= s.end) return v;
+	if (s.tab) {
+		const BasisCol e = s.tab[k];
+		if (row == e.re) v.x = s.weighted ? (T)e.wre : T(1);
+		if (row == e.im) v.y = s.weighted ? (T)e.wim : T(1);
+	} else {
+		if (row == k) v.x = T(1);
+		if (s.pair_half != 0 && row == k + s.pair_half) v.y = T(1);
+	}
+	return v;
+}
 
 // ---------------------------------------------------------------- amplitude groups
 

@@ -38,6 +38,7 @@ struct Runtime
 	Buffer scratch;       // FP64 per-lane sums of the complex64 reverse passes
 	Buffer stage[4];      // staging of host statevectors
 	Buffer arrays;        // statevector arrays and gate-input caches of the full-Hessian calls
+	Buffer columns;       // column list of the current call (orbits.h)
 	Buffer hpin;          // pinned host scratch
 	Buffer status;        // device status word of kernels with bounded waits (non-zero: a wait gave up)
 
@@ -49,7 +50,6 @@ struct Runtime
 	// basis columns the target sums run over: [col_begin, col_end), col_end 0 = to the last
 	// column (rqcopt_gpu_set_column_range)
 	int64_t col_begin = 0, col_end = 0;
-	int64_t col_end_dev = -1;    // the column end the fused kernels hold (__constant__), -1 unset
 	int real_pairs = 0;          // evaluate(): paired basis columns of a real problem (rqcopt_gpu_set_real_pairs)
 	int gates_per_pass = 4;   // 1: one kernel per gate; 2..4: fused passes
 	int recon_c128 = 1;       // complex128 reverse passes rebuild states with adjoint gates (unitary gates)
@@ -61,7 +61,7 @@ struct Runtime
 	int autotune = 1;
 	bool tuning = false;
 	bool pin_gpp = false, pin_chunk = false, pin_recon = false, pin_ffma = false;   // set explicitly by the caller
-	std::map<std::array<long, 11>, TuneChoice> tune_cache;
+	std::map<std::array<long, 12>, TuneChoice> tune_cache;
 	TuneChoice last_choice = {0, 0, 0, 0, 0.0, 0};
 
 	// instrumentation

@@ -36,6 +36,12 @@ struct TargetHolder
 	bool set(linear_func ufunc, void* udata, int L);
 };
 
+// Sum over the orbits of the wire relabellings that circuit and target share, instead of
+// over all basis states (orbits.h): a brickwall against a device-native brickwall whose
+// results are per-layer sums, over all columns.  Fills cs.columns and cs.ncolumns, the list
+// in rt.columns (held until the next call).
+int use_orbits(Runtime& rt, const Problem& pb, const TargetHolder& th, CircuitSpec& cs);
+
 int post_launch(Runtime& rt, const double2* d_res, const Problem& pb, const double2* d_ugates, const double2* d_udirs,
                 int with_hvp, double2* d_dunits, double2* d_hunits, double* d_grad, double* d_hvp);
 
