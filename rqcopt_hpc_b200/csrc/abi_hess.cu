@@ -281,6 +281,7 @@ int hessian_target(const char* fn, linear_func ufunc, void* udata, const struct 
 	c.nlayers = nlayers;
 	c.ugates = ug.data();
 	c.wires = wires.data();
+	if (!samp && (ret = use_orbits(*rt, nqubits, nlayers, wires.data(), th, &c.columns, &c.ncolumns))) return ret;
 	if ((ret = hessian_target_device(*rt, c, th.spec, rec, samp))) return ret;
 	if (H) {
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(d_ug, ug.data(), 16 * (size_t)nlayers * sizeof(double2), cudaMemcpyHostToDevice,
@@ -451,6 +452,7 @@ int blockenc(const char* fn, linear_func hfunc, void* hdata, const struct mat4x4
 	c.nlayers = nlayers;
 	c.ugates = ug.data();
 	c.wires = wires.data();
+	if ((ret = use_orbits_blockenc(*rt, nqubits, nlayers, wires.data(), th, &c.columns, &c.ncolumns))) return ret;
 	if ((ret = blockenc_device(*rt, c, th.spec, mode, rec, d_h2))) return ret;
 	if (grad_vec) {
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(d_ug, ug.data(), 16 * (size_t)nlayers * sizeof(double2), cudaMemcpyHostToDevice,

@@ -329,7 +329,8 @@ struct DeviceOptimizer
 		res = ug + 16 * nu;
 		scratch = reinterpret_cast<double*>(res + nres);
 		hx.assign(x0, x0 + 16 * nu);
-		if ((ret = use_orbits(rt, pb, th, orbits))) return ret;
+		if (pb.brickwall && (ret = use_orbits(rt, pb.L, pb.nunits, pb.wires.data(), th, &orbits.columns, &orbits.ncolumns)))
+			return ret;
 		return RQC_CUDA(cudaMemcpyAsync(x, x0, 16 * nu * sizeof(double2), cudaMemcpyHostToDevice, rt.stream));
 	}
 
@@ -488,6 +489,8 @@ struct DeviceOptimizer
 		c.L = pb.L;
 		c.nlayers = nl;
 		c.wires = pb.wires.data();
+		c.columns = orbits.columns;
+		c.ncolumns = orbits.ncolumns;
 		const int threads = 64, blocks = (nl + threads - 1) / threads;
 		for (int k = 0; k < niter && !ret; k++) {
 			// f, gradient vector and Hessian matrix at x (src/trust_region.c:263)

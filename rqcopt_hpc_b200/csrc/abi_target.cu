@@ -82,6 +82,7 @@ bool Problem::set_brickwall(int L_, int nlayers, const struct mat4x4* vlist, con
 	L = L_;
 	if (L < 2 || L % 2 || nlayers < 1 || !perms || !vlist) return false;
 	per = L / 2;
+	brickwall = true;
 	nunits = nlayers;
 	G = nunits * per;
 	gates.assign(16 * (size_t)G, make_double2(0, 0));
@@ -108,6 +109,7 @@ bool Problem::set_circuit(int L_, int ngates, const struct mat4x4* g, const stru
 	L = L_;
 	if (L < 2 || ngates < 1 || !g || !w) return false;
 	per = 1;
+	brickwall = false;
 	nunits = G = ngates;
 	gates.assign(reinterpret_cast<const double2*>(g), reinterpret_cast<const double2*>(g) + 16 * (size_t)G);
 	dirs.clear();
@@ -168,26 +170,60 @@ bool TargetHolder::set(linear_func ufunc, void* udata, int L)
 	return true;
 }
 
-int use_orbits(Runtime& rt, const Problem& pb, const TargetHolder& th, CircuitSpec& cs)
+namespace {
+
+int upload_columns(Runtime& rt, const std::vector<BasisCol>& cols, const BasisCol** columns, int64_t* ncolumns)
 {
-	const int per = pb.L / 2;
-	// beyond 20 qubits no evaluation over all columns ends in reasonable time: the list is not worth its memory
-	if (pb.L < 4 || pb.L > 20 || pb.per != per || th.spec.ufunc || th.spec.per != per || rt.col_begin != 0 ||
-	    rt.col_end != 0)
-		return OK;
-	std::vector<const int*> layers;
-	for (int k = 0; k < pb.G; k += per) layers.push_back(&pb.wires[2 * (size_t)k]);
-	for (int k = 0; k < th.spec.ngates; k += per) layers.push_back(&th.wires[2 * (size_t)k]);
-	const std::vector<int> sym = wire_symmetries(pb.L, layers);
-	if ((int)sym.size() == pb.L) return OK;
-	std::vector<BasisCol> cols = orbit_columns(pb.L, sym);
-	if (rt.real_pairs) cols = pair_columns(cols);
 	const size_t bytes = cols.size() * sizeof(BasisCol);
 	int ret = ensure_device(rt.columns, bytes);
 	if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(rt.columns.ptr, cols.data(), bytes, cudaMemcpyHostToDevice, rt.stream));
-	cs.columns = static_cast<const BasisCol*>(rt.columns.ptr);
-	cs.ncolumns = (int64_t)cols.size();
+	*columns = static_cast<const BasisCol*>(rt.columns.ptr);
+	*ncolumns = (int64_t)cols.size();
 	return ret;
+}
+
+// beyond 20 qubits no evaluation over all columns ends in reasonable time: the list is not
+// worth its memory
+constexpr int MAX_ORBIT_QUBITS = 20;
+
+}  // namespace
+
+int use_orbits(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th, const BasisCol** columns,
+               int64_t* ncolumns)
+{
+	const int per = L / 2;
+	if (L < 4 || L > MAX_ORBIT_QUBITS || th.spec.ufunc || th.spec.per != per || rt.col_begin != 0 || rt.col_end != 0)
+		return OK;
+	std::vector<const int*> layers;
+	for (int l = 0; l < nlayers; l++) layers.push_back(wires + (size_t)l * L);
+	for (int k = 0; k < th.spec.ngates; k += per) layers.push_back(&th.wires[2 * (size_t)k]);
+	const std::vector<int> sym = wire_symmetries(L, layers);
+	if ((int)sym.size() == L) return OK;
+	const std::vector<BasisCol> cols = orbit_columns(L, sym);
+	return upload_columns(rt, rt.real_pairs ? pair_columns(cols) : cols, columns, ncolumns);
+}
+
+int use_orbits_blockenc(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th,
+                        const BasisCol** columns, int64_t* ncolumns)
+{
+	const int half = L / 2, hper = half / 2;
+	if (L < 4 || half > MAX_ORBIT_QUBITS || th.spec.ufunc || hper < 1 || half % 2 || th.spec.per != hper) return OK;
+	std::vector<const int*> layers, hlayers;
+	for (int l = 0; l < nlayers; l++) layers.push_back(wires + (size_t)l * L);
+	for (int k = 0; k < th.spec.ngates; k += hper) hlayers.push_back(&th.wires[2 * (size_t)k]);
+	const std::vector<int> sym = wire_symmetries(L, layers);
+	std::vector<int> hsym;   // wire 2 k of the full register is wire k of the half register
+	for (size_t g = 0; g < sym.size(); g += L) {
+		std::vector<int> h(half);
+		bool ok = true;
+		for (int k = 0; k < half && ok; k++) {
+			ok = sym[g + 2 * k] % 2 == 0;
+			h[k] = sym[g + 2 * k] / 2;
+		}
+		if (ok && preserves_layers(half, hlayers, h.data())) hsym.insert(hsym.end(), h.begin(), h.end());
+	}
+	if ((int)hsym.size() == half) return OK;
+	return upload_columns(rt, orbit_columns(half, hsym), columns, ncolumns);
 }
 
 // Fold per-gate sums into per-unit sums and project (src/target.c:410-430, 526-535, 652-672).
@@ -246,7 +282,7 @@ int run_target(const Problem& pb, const TargetHolder& th, int mode, numeric* fva
 	cs.dirs = mode == EVAL_HVP ? pb.dirs.data() : nullptr;
 	cs.wires = pb.wires.data();
 	const int prec = rt->precision == PREC_C128 ? PREC_C128 : PREC_C64;
-	int ret = prec == PREC_C128 ? use_orbits(*rt, pb, th, cs) : OK;
+	int ret = prec == PREC_C128 && pb.brickwall ? use_orbits(*rt, pb.L, pb.nunits, pb.wires.data(), th, &cs.columns, &cs.ncolumns) : OK;
 	if (ret) return ret;
 	const size_t nres = result_count(pb.G);
 	const size_t nu = (size_t)pb.nunits;

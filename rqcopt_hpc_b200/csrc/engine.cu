@@ -417,17 +417,6 @@ static int partial_grid(const Runtime& rt)
 	return rt.num_sms * per_sm;
 }
 
-static size_t workspace_limit(Runtime& rt)
-{
-	if (rt.workspace_limit) return rt.workspace_limit;
-	size_t free_b = 0, total_b = 0;
-	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-		cudaGetLastError();
-		return (size_t)1 << 30;
-	}
-	return (size_t)((free_b + rt.work.bytes) * 0.75);
-}
-
 // ---------------------------------------------------------------------------------- evaluation
 
 template <typename T>
@@ -457,10 +446,10 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 	const size_t col_bytes = (size_t)nstates * N * sizeof(V);
 	const int64_t cbeg = std::min<int64_t>(rt.col_begin, ncols);
 	const int64_t cend = rt.col_end > 0 ? std::min<int64_t>(rt.col_end, ncols) : ncols;
-	int64_t C = (int64_t)(workspace_limit(rt) / col_bytes);
+	int64_t C = std::max<int64_t>(1, cend - cbeg);
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
 	if (host_target) C = std::min<int64_t>(C, std::max<int64_t>(1, ((int64_t)256 << 20) / (N * 16)));
-	C = std::min(C, std::max<int64_t>(1, cend - cbeg));
+	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
 	if (C < 1) {
 		fprintf(stderr, "rqcopt_gpu: one basis column needs %zu bytes of workspace, more than the limit\n", col_bytes);
 		return E_ALLOC;

@@ -2529,17 +2529,6 @@ int rev_grid(Runtime& rt, bool tan)
 	return rt.num_sms * per_sm;
 }
 
-size_t workspace_limit2(Runtime& rt)
-{
-	if (rt.workspace_limit) return rt.workspace_limit;
-	size_t free_b = 0, total_b = 0;
-	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-		cudaGetLastError();
-		return (size_t)1 << 30;
-	}
-	return (size_t)((free_b + rt.work.bytes) * 0.75);
-}
-
 template <typename T>
 int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int mode, int maxk, double2* d_out)
 {
@@ -2573,12 +2562,11 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 	const size_t col_bytes = (size_t)nstates * N * sizeof(V);
 	const int64_t cbeg = std::min<int64_t>(rt.col_begin, ncols);
 	const int64_t cend = rt.col_end > 0 ? std::min<int64_t>(rt.col_end, ncols) : ncols;
-	const int64_t C_mem = (int64_t)(workspace_limit2(rt) / col_bytes);
-	int64_t C = C_mem;
+	int64_t C = ((std::max<int64_t>(1, cend - cbeg) + CW - 1) / CW) * CW;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, ((rt.column_chunk + CW - 1) / CW) * CW);
 	if (host_target) C = std::min<int64_t>(C, std::max<int64_t>(CW, ((int64_t)256 << 20) / (N * 16)));
-	C = std::min<int64_t>(C, ((std::max<int64_t>(1, cend - cbeg) + CW - 1) / CW) * CW);
-	C = (C / CW) * CW;
+	const int64_t C_mem = (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes);
+	C = (std::min(C, C_mem) / CW) * CW;
 	if (C < CW || C > C_mem) {
 		fprintf(stderr, "rqcopt_gpu: %d columns need %zu bytes of workspace, more than the limit\n", CW, CW * col_bytes);
 		return E_ALLOC;

@@ -98,13 +98,13 @@ __device__ __forceinline__ void contract(double (&acc)[32], const double2 p[4], 
 
 // One gate of the forward sweep (see the file comment).  Block (s, bx): state s
 // (0: psi, 1 + t: tangent t of layer t / 16, entry t % 16), column range bx.
-//   basis_b0 >= 0: psi_in is the basis column basis_b0 + c of chunk column c
+//   basis: psi_in is basis column c of src for chunk column c
 //   fresh:  the tangents of `layer` are zero before this gate
 //   carry:  carry the tangents through the gate (0 at the last gate)
 //   psi_out: G psi_in, or null where the next input state is given (one-state pass)
 //   fpart:  non-null at the last gate of a target sum: f += phi . (G psi)
 __global__ void __launch_bounds__(HT, 2)
-k_hsweep(const double2* __restrict__ psi_in, int64_t basis_b0, double2* __restrict__ psi_out,
+k_hsweep(const double2* __restrict__ psi_in, int basis, ColumnSource src, double2* __restrict__ psi_out,
          const double2* __restrict__ phi, double2* __restrict__ tan, Gate4<double> g, WirePair w, int L,
          int64_t ngroups, int64_t sstride, int layer, int fresh, int carry, double* __restrict__ part, int S,
          double2* __restrict__ fpart)
@@ -133,7 +133,7 @@ k_hsweep(const double2* __restrict__ psi_in, int64_t basis_b0, double2* __restri
 		if (s == 0) {
 #pragma unroll
 			for (int m = 0; m < 4; m++)
-				x[m] = basis_b0 >= 0 ? make_double2(loc + off[m] == basis_b0 + c ? 1.0 : 0.0, 0.0) : psi_in[base + off[m]];
+				x[m] = basis ? basis_amp<double>(src, loc + off[m], c) : psi_in[base + off[m]];
 		} else if (zero_in) {
 #pragma unroll
 			for (int m = 0; m < 4; m++) x[m] = make_double2(0, 0);
@@ -164,8 +164,7 @@ k_hsweep(const double2* __restrict__ psi_in, int64_t basis_b0, double2* __restri
 				gate_apply(g, x, y);
 			}
 			if (own) {
-				const double2 v = basis_b0 >= 0 ? make_double2(loc + off[ec] == basis_b0 + c ? 1.0 : 0.0, 0.0)
-				                                : psi_in[base + off[ec]];
+				const double2 v = basis ? basis_amp<double>(src, loc + off[ec], c) : psi_in[base + off[ec]];
 				y[er].x += v.x;
 				y[er].y += v.y;
 			}
@@ -208,12 +207,12 @@ struct LayerGates
 // and writes them back once; one thread per amplitude group and gate.  Block
 // (s, bx): state s as in k_hsweep, column blocks bx, bx + nbx, ...  psi_q comes
 // from the forward cache psi + q * sstride, except psi_0 of a basis-column sum
-// (basis_b0 >= 0), which is the basis column basis_b0 + c.  The tangents of
+// (from_basis), which is basis column c of src.  The tangents of
 // `layer` start at zero (they are created at its first gate).  last: the layer
 // holds the circuit's last gate (no G at that gate, no store of the tiles, f
 // summed by the psi blocks).
 __global__ void __launch_bounds__(HT, 2)
-k_hlayer(const double2* __restrict__ psi, int64_t basis_b0, const double2* __restrict__ phi, double2* __restrict__ tan,
+k_hlayer(const double2* __restrict__ psi, int from_basis, ColumnSource src, const double2* __restrict__ phi, double2* __restrict__ tan,
          Gate4<double> g, LayerGates lgts, int L, int64_t ncols, int64_t sstride, int layer, int last,
          double* __restrict__ part, int S, double2* __restrict__ fpart)
 {
@@ -253,7 +252,7 @@ k_hlayer(const double2* __restrict__ psi, int64_t basis_b0, const double2* __res
 			const double2* __restrict__ ph = phi + (int64_t)q * sstride + gofs;
 			const double2* __restrict__ ps = psi + (int64_t)q * sstride + gofs;
 			const bool zero_in = own && k == 0;
-			const bool basis = q == 0 && basis_b0 >= 0;
+			const bool basis = q == 0 && from_basis;
 			const int64_t offc = ((ec & 2) ? w.si : 0) + ((ec & 1) ? w.sj : 0);
 			for (int gi = threadIdx.x; gi < ngr; gi += HT) {
 				const int cc = gi >> lg;
@@ -265,7 +264,7 @@ k_hlayer(const double2* __restrict__ psi, int64_t basis_b0, const double2* __res
 				if (s == 0) {
 #pragma unroll
 					for (int m = 0; m < 4; m++)
-						x[m] = basis ? make_double2(loc + off[m] == basis_b0 + col0 + cc ? 1.0 : 0.0, 0.0) : ps[li + off[m]];
+						x[m] = basis ? basis_amp<double>(src, loc + off[m], col0 + cc) : ps[li + off[m]];
 				} else if (zero_in) {
 #pragma unroll
 					for (int m = 0; m < 4; m++) x[m] = make_double2(0, 0);
@@ -301,8 +300,7 @@ k_hlayer(const double2* __restrict__ psi, int64_t basis_b0, const double2* __res
 						gate_apply(g, x, y);
 					}
 					if (own) {
-						const double2 v = basis ? make_double2(loc + offc == basis_b0 + col0 + cc ? 1.0 : 0.0, 0.0)
-						                        : ps[li + offc];
+						const double2 v = basis ? basis_amp<double>(src, loc + offc, col0 + cc) : ps[li + offc];
 						y[er].x += v.x;
 						y[er].y += v.y;
 					}
@@ -346,20 +344,25 @@ __host__ __device__ __forceinline__ int64_t blockenc_index(int64_t b, int half)
 	return c;
 }
 
+// half-register basis state and weight of column k (tab null: state k, weight 1)
+__device__ __forceinline__ int64_t benc_state(const BasisCol* tab, int64_t k) { return tab ? tab[k].re : k; }
+__device__ __forceinline__ double benc_weight(const BasisCol* tab, int64_t k) { return tab ? tab[k].wre : 1.0; }
+
 // psi_0 of columns b0 .. b0 + ncols - 1: the basis states P e_b
-__global__ void k_benc_init(double2* __restrict__ states, int L, int64_t b0, int64_t ncols)
+__global__ void k_benc_init(double2* __restrict__ states, int L, const BasisCol* __restrict__ tab, int64_t b0, int64_t ncols)
 {
 	const int64_t N = (int64_t)1 << L;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ncols * N; i += (int64_t)gridDim.x * blockDim.x) {
 		const int64_t c = i >> L, a = i & (N - 1);
-		states[i] = make_double2(a == blockenc_index(b0 + c, L / 2) ? 1.0 : 0.0, 0.0);
+		states[i] = make_double2(a == blockenc_index(benc_state(tab, b0 + c), L / 2) ? 1.0 : 0.0, 0.0);
 	}
 }
 
-// residual d = P^dag W P e_b - H e_b on the P rows: f += |d|^2 / 2 (per block), chi = P conj(d)
-// (zero elsewhere: chi is cleared before).  hneg[b][a] = -conj((H e_b)[a]).
-__global__ void k_benc_residual(const double2* __restrict__ wout, const double2* __restrict__ hneg, int L, int64_t b0,
-                                int64_t ncols, double2* __restrict__ chi, double2* __restrict__ fpart)
+// residual d = P^dag W P e_b - H e_b on the P rows: f += w |d|^2 / 2 (per block), chi = w P conj(d)
+// (zero elsewhere: chi is cleared before), w the column's weight.  hneg[b][a] = -conj((H e_b)[a]).
+__global__ void k_benc_residual(const double2* __restrict__ wout, const double2* __restrict__ hneg, int L,
+                                const BasisCol* __restrict__ tab, int64_t b0, int64_t ncols, double2* __restrict__ chi,
+                                double2* __restrict__ fpart)
 {
 	__shared__ double red[HT / 32];
 	const int half = L / 2;
@@ -368,11 +371,12 @@ __global__ void k_benc_residual(const double2* __restrict__ wout, const double2*
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ncols * s; i += (int64_t)gridDim.x * blockDim.x) {
 		const int64_t c = i >> half, a = i & (s - 1);
 		const int64_t idx = (c << L) + blockenc_index(a, half);
-		const double2 hn = hneg[(b0 + c) * s + a];
+		const double2 hn = hneg[benc_state(tab, b0 + c) * s + a];
+		const double wt = benc_weight(tab, b0 + c);
 		const double2 w = wout[idx];
 		const double dx = w.x + hn.x, dy = w.y - hn.y;   // w - H e_b with H e_b = -conj(hn)
-		acc += 0.5 * (dx * dx + dy * dy);
-		if (chi) chi[idx] = make_double2(dx, -dy);
+		acc += 0.5 * wt * (dx * dx + dy * dy);
+		if (chi) chi[idx] = make_double2(wt * dx, -wt * dy);
 	}
 	acc = warp_sum(acc);
 	if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -396,9 +400,10 @@ __global__ void k_benc_gather(const double2* __restrict__ tan, int L, int64_t nc
 	}
 }
 
-// Gauss-Newton term: part2[(l i), (k j)] += sum_r conj(jac[l i][r]) jac[k j][r] for layer l >= k
-// (src/target.c:1570-1580); one block per entry
-__global__ void k_benc_gram(const double2* __restrict__ jac, int64_t K, int nl, double2* __restrict__ part2)
+// Gauss-Newton term: part2[(l i), (k j)] += sum_r w conj(jac[l i][r]) jac[k j][r] for layer l >= k
+// (src/target.c:1570-1580), row r belonging to column b0 + (r >> half) of weight w; one block per entry
+__global__ void k_benc_gram(const double2* __restrict__ jac, int64_t K, int nl, const BasisCol* __restrict__ tab, int64_t b0,
+                            int half, double2* __restrict__ part2)
 {
 	__shared__ double red[2][HT / 32];
 	const int m = 16 * nl;
@@ -410,8 +415,9 @@ __global__ void k_benc_gram(const double2* __restrict__ jac, int64_t K, int nl, 
 	double sx = 0, sy = 0;
 	for (int64_t r = threadIdx.x; r < K; r += HT) {
 		const double2 a = x[r], b = y[r];
-		sx += a.x * b.x + a.y * b.y;     // conj(a) b
-		sy += a.x * b.y - a.y * b.x;
+		const double wt = benc_weight(tab, b0 + (r >> half));
+		sx += wt * (a.x * b.x + a.y * b.y);     // conj(a) b
+		sy += wt * (a.x * b.y - a.y * b.x);
 	}
 	sx = warp_sum(sx);
 	sy = warp_sum(sy);
@@ -490,9 +496,10 @@ __global__ void k_hassemble(const double* __restrict__ part, int nbx, int nl, in
 }
 
 // out = G in over `ngroups` groups of consecutive 2^L-amplitude states
-//   basis_b0 >= 0: `in` is the basis column basis_b0 + c of column c
+//   basis: `in` is basis column c of src
 __global__ void __launch_bounds__(HT) k_happly(const double2* __restrict__ in, double2* __restrict__ out, Gate4<double> g,
-                                               WirePair w, int L, int64_t ngroups, int64_t basis_b0 = -1)
+                                               WirePair w, int L, int64_t ngroups, int basis = 0,
+                                               ColumnSource src = ColumnSource{})
 {
 	const int lg = L - 2;
 	const int64_t gmask = ((int64_t)1 << lg) - 1;
@@ -504,7 +511,7 @@ __global__ void __launch_bounds__(HT) k_happly(const double2* __restrict__ in, d
 		double2 x[4], y[4];
 #pragma unroll
 		for (int m = 0; m < 4; m++)
-			x[m] = basis_b0 >= 0 ? make_double2(loc + off[m] == basis_b0 + c ? 1.0 : 0.0, 0.0) : in[base + off[m]];
+			x[m] = basis ? basis_amp<double>(src, loc + off[m], c) : in[base + off[m]];
 		gate_apply(g, x, y);
 #pragma unroll
 		for (int m = 0; m < 4; m++) out[base + off[m]] = y[m];
@@ -690,17 +697,6 @@ int checked(Runtime& rt)
 	return RQC_CUDA(cudaGetLastError());
 }
 
-size_t hess_workspace_limit(Runtime& rt)
-{
-	if (rt.workspace_limit) return rt.workspace_limit;
-	size_t free_b = 0, total_b = 0;
-	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-		cudaGetLastError();
-		return (size_t)1 << 30;
-	}
-	return (size_t)((free_b + rt.work.bytes) * 0.75);
-}
-
 // blocks per state: enough for four groups per thread, at most HMAXBX
 int blocks_per_state(int64_t ngroups)
 {
@@ -719,6 +715,7 @@ struct Sweep
 
 	bool keep_final = false;   // carry the tangents through the last gate and store them (block encoding)
 	bool psi_only = false;     // gradient only: the psi blocks of the sweep
+	ColumnSource src;          // basis columns of the chunk
 
 	Sweep(Runtime& r, const HessCircuit& hc) : rt(r), c(hc), L(hc.L), nl(hc.nlayers), per(hc.L / 2),
 	                                           G(hc.nlayers * (hc.L / 2)), S(1 + 16 * hc.nlayers), nbx(1) {}
@@ -764,7 +761,8 @@ struct Sweep
 	}
 
 	// one gate of the forward sweep
-	int gate(int q, const double2* psi_in, int64_t basis_b0, double2* psi_out, const double2* phi, double2* tan,
+	// basis: psi_in is the basis columns of the chunk (psi_0 of a column sum)
+	int gate(int q, const double2* psi_in, int basis, double2* psi_out, const double2* phi, double2* tan,
 	         int64_t ngroups, int64_t sstride, bool with_f)
 	{
 		const int a = q / per;
@@ -772,23 +770,23 @@ struct Sweep
 		const dim3 grid(psi_only ? 1 : 1 + 16 * (a + 1), nbx);
 		cudaEvent_t ev;
 		launch_begin(rt, KC_HESS, &ev);
-		k_hsweep<<<grid, HT, 0, rt.stream>>>(psi_in, basis_b0, last ? nullptr : psi_out, phi, tan, gg[a], gw[q], L,
+		k_hsweep<<<grid, HT, 0, rt.stream>>>(psi_in, basis, src, last ? nullptr : psi_out, phi, tan, gg[a], gw[q], L,
 		                                     ngroups, sstride, a, q % per == 0 ? 1 : 0, (last && !keep_final) ? 0 : 1, part,
 		                                     S, (with_f && last) ? fpart : nullptr);
 		launch_end(rt, KC_HESS, ev);
 		return RQC_CUDA(cudaGetLastError());
 	}
 
-	// psi_q = G_{q-1} psi_{q-1} for q = 1 .. G-1 into psi_at(q); psi_0 the basis columns from basis_b0
+	// psi_q = G_{q-1} psi_{q-1} for q = 1 .. G-1 into psi_at(q); psi_0 the chunk's basis columns (basis) or psi_at(0)
 	template <typename PsiAt>
-	int forward_chain(PsiAt psi_at, int64_t ngroups, int64_t basis_b0)
+	int forward_chain(PsiAt psi_at, int64_t ngroups, int basis)
 	{
 		const int grid = grid_of(rt, ngroups, 8);
 		for (int q = 1; q < G; q++) {
 			cudaEvent_t ev;
 			launch_begin(rt, KC_APPLY, &ev);
 			k_happly<<<grid, HT, 0, rt.stream>>>(psi_at(q - 1), psi_at(q), gg[(q - 1) / per], gw[q - 1], L, ngroups,
-			                                     q == 1 ? basis_b0 : -1);
+			                                     q == 1 ? basis : 0, src);
 			launch_end(rt, KC_APPLY, ev);
 			if (int e = RQC_CUDA(cudaGetLastError())) return e;
 		}
@@ -796,7 +794,7 @@ struct Sweep
 	}
 
 	// one layer with shared-memory tiles (L <= 12)
-	int layer(int a, const double2* psi, int64_t basis_b0, const double2* phi, double2* tan, int64_t ncols,
+	int layer(int a, const double2* psi, int basis, const double2* phi, double2* tan, int64_t ncols,
 	          int64_t sstride, bool with_f)
 	{
 		static bool smem_set = false;
@@ -814,7 +812,7 @@ struct Sweep
 		const dim3 grid(psi_only ? 1 : 1 + 16 * (a + 1), nbx);
 		cudaEvent_t ev;
 		launch_begin(rt, KC_HESS, &ev);
-		k_hlayer<<<grid, HT, HTILE * sizeof(double2), rt.stream>>>(psi, basis_b0, phi, tan, gg[a], lgts, L, ncols, sstride, a,
+		k_hlayer<<<grid, HT, HTILE * sizeof(double2), rt.stream>>>(psi, basis, src, phi, tan, gg[a], lgts, L, ncols, sstride, a,
 		                                                             last ? 1 : 0, part, S,
 		                                                             (with_f && last) ? fpart : nullptr);
 		launch_end(rt, KC_HESS, ev);
@@ -841,7 +839,7 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	if (samp && samp->nsamples < 1) return E_ARG;
 	const int per = L / 2, G = nl * per;
 	const int64_t N = (int64_t)1 << L;
-	const int64_t ncols = samp ? samp->nsamples : N;   // basis columns, or sample states
+	const int64_t ncols = samp ? samp->nsamples : (c.columns ? c.ncolumns : N);   // basis columns, or sample states
 	// layer kernel (shared-memory tiles) up to L = 12, one kernel per gate beyond
 	const bool layered = L <= 12 && per <= HMAXPER;
 	// states per column: phi_q of every gate, psi_q of every gate (layered) or two psi
@@ -849,10 +847,10 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	// states besides
 	const int64_t nstates = G + (layered ? G : 2) + 16 * (int64_t)nl + (samp ? (layered ? 2 : 3) : 0);
 	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
-	int64_t C = (int64_t)(hess_workspace_limit(rt) / col_bytes);
+	int64_t C = ncols;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
 	if (t.ufunc) C = std::min<int64_t>(C, std::max<int64_t>(1, ((int64_t)256 << 20) / (N * 16)));
-	C = std::min(C, ncols);
+	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
 	if (C < 1) {
 		fprintf(stderr, "rqcopt_gpu: one basis column of the Hessian sweep needs %zu bytes of workspace, more than the limit\n",
 		        col_bytes);
@@ -876,11 +874,16 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	for (int64_t b0 = 0; b0 < ncols; b0 += C) {
 		const int64_t Cc = std::min(C, ncols - b0);
 		const int64_t ngroups = Cc * (N / 4);
-		const int64_t basis = samp ? -1 : b0;
+		const int basis = samp ? 0 : 1;
+		sw.src.tab = c.columns;
+		sw.src.b0 = b0;
+		sw.src.end = ncols;
+		ColumnSource tsrc = sw.src;
+		tsrc.weighted = 1;
 		if (samp) {
 			if ((ret = haar_states_device(rt, *samp, L, b0, Cc, states))) return ret;
 			if ((ret = target_states_device(rt, t, L, states, Cc, phi_at(G - 1), tq[0], tq[1]))) return ret;
-		} else if ((ret = target_columns_device(rt, t, L, plain_columns(b0), Cc, phi_at(G - 1), tq[0], tq[1]))) {
+		} else if ((ret = target_columns_device(rt, t, L, tsrc, Cc, phi_at(G - 1), tq[0], tq[1]))) {
 			return ret;
 		}
 		if ((ret = sw.reverse_chain(phi_at, ngroups, nullptr))) return ret;
@@ -892,7 +895,7 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 		}
 		for (int q = 0; q < G; q++) {
 			const double2* in = q == 0 ? states : P[(q - 1) & 1];
-			if ((ret = sw.gate(q, in, q == 0 ? basis : -1, P[q & 1], phi_at(q), tan, ngroups, cs, true))) return ret;
+			if ((ret = sw.gate(q, in, q == 0 ? basis : 0, P[q & 1], phi_at(q), tan, ngroups, cs, true))) return ret;
 		}
 	}
 	if ((ret = sw.assemble(d_rec))) return ret;
@@ -926,10 +929,10 @@ int hessian_single_device(Runtime& rt, const HessCircuit& c, const double2* d_ca
 	if ((ret = sw.reverse_chain(phi_at, N / 4, d_dpsi))) return ret;
 	if (layered) {
 		for (int a = 0; a < nl; a++)
-			if ((ret = sw.layer(a, d_cache, -1, phi, tan, 1, N, false))) return ret;
+			if ((ret = sw.layer(a, d_cache, 0, phi, tan, 1, N, false))) return ret;
 	} else {
 		for (int q = 0; q < G; q++)
-			if ((ret = sw.gate(q, d_cache + (int64_t)q * N, -1, nullptr, phi_at(q), tan, N / 4, N, false))) return ret;
+			if ((ret = sw.gate(q, d_cache + (int64_t)q * N, 0, nullptr, phi_at(q), tan, N / 4, N, false))) return ret;
 	}
 	return sw.assemble(d_rec);
 }
@@ -946,9 +949,10 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	// buffers and the input states; W P e_b; the tangents (Hessian only)
 	const int64_t nstates = G + (layered ? G : 3) + 1 + (hess ? 16 * (int64_t)nl : 0);
 	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
-	int64_t C = (int64_t)(hess_workspace_limit(rt) / col_bytes);
+	const int64_t ncols = c.columns ? c.ncolumns : s;
+	int64_t C = ncols;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
-	C = std::min(C, s);
+	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
 	if (C < 1) return E_ALLOC;
 	int ret = ensure_device(rt.work, (size_t)nstates * C * N * sizeof(double2));
 	if (ret) return ret;
@@ -973,7 +977,7 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	double2* fres = hess ? part2 + (size_t)m * m : jac;
 	if ((ret = RQC_CUDA(cudaMemsetAsync(fres, 0, nres * sizeof(double2), rt.stream)))) return ret;
 	if (hess && (ret = RQC_CUDA(cudaMemsetAsync(part2, 0, (size_t)m * m * sizeof(double2), rt.stream)))) return ret;
-	if ((ret = target_columns_device(rt, t, half, plain_columns(0), s, hneg, sc0, sc1))) return ret;
+	if ((ret = target_columns_device(rt, t, half, ColumnSource{}, s, hneg, sc0, sc1))) return ret;
 
 	Sweep sw(rt, c);
 	sw.keep_final = hess;
@@ -985,15 +989,15 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 		sw.gw.resize(G);
 		for (int q = 0; q < G; q++) sw.gw[q] = make_pair_(L, c.wires[2 * q], c.wires[2 * q + 1]);
 	}
-	for (int64_t b0 = 0; b0 < s; b0 += C) {
-		const int64_t Cc = std::min(C, s - b0);
+	for (int64_t b0 = 0; b0 < ncols; b0 += C) {
+		const int64_t Cc = std::min(C, ncols - b0);
 		const int64_t ngroups = Cc * (N / 4);
 		const int agrid = grid_of(rt, ngroups, 8);
-		k_benc_init<<<grid_of(rt, Cc * N, 8), HT, 0, rt.stream>>>(states, L, b0, Cc);
+		k_benc_init<<<grid_of(rt, Cc * N, 8), HT, 0, rt.stream>>>(states, L, c.columns, b0, Cc);
 		if ((ret = checked(rt))) return ret;
 		// forward pass to W P e_b
 		if (layered && mode >= 1) {
-			if ((ret = sw.forward_chain(psi_at, ngroups, -1))) return ret;
+			if ((ret = sw.forward_chain(psi_at, ngroups, 0))) return ret;
 			k_happly<<<agrid, HT, 0, rt.stream>>>(psi_at(G - 1), wout, sw.gg[(G - 1) / per], sw.gw[G - 1], L, ngroups);
 			if ((ret = checked(rt))) return ret;
 		} else {
@@ -1007,23 +1011,23 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 		}
 		double2* chi = mode >= 1 ? phi_at(G - 1) : nullptr;
 		if (chi && (ret = RQC_CUDA(cudaMemsetAsync(chi, 0, (size_t)Cc * N * sizeof(double2), rt.stream)))) return ret;
-		k_benc_residual<<<nres, HT, 0, rt.stream>>>(wout, hneg, L, b0, Cc, chi, fres);
+		k_benc_residual<<<nres, HT, 0, rt.stream>>>(wout, hneg, L, c.columns, b0, Cc, chi, fres);
 		if ((ret = checked(rt))) return ret;
 		if (mode == 0) continue;
 		if ((ret = sw.reverse_chain(phi_at, ngroups, nullptr))) return ret;
 		if (layered) {
 			for (int a = 0; a < nl; a++)
-				if ((ret = sw.layer(a, psi, -1, phi, tan, Cc, cs, false))) return ret;
+				if ((ret = sw.layer(a, psi, 0, phi, tan, Cc, cs, false))) return ret;
 		} else {
 			for (int q = 0; q < G; q++) {
 				const double2* in = q == 0 ? states : P[(q - 1) & 1];
-				if ((ret = sw.gate(q, in, -1, P[q & 1], phi_at(q), tan, ngroups, cs, false))) return ret;
+				if ((ret = sw.gate(q, in, 0, P[q & 1], phi_at(q), tan, ngroups, cs, false))) return ret;
 			}
 		}
 		if (hess) {
 			k_benc_gather<<<grid_of(rt, (int64_t)m * Cc * s, 8), HT, 0, rt.stream>>>(tan, L, Cc, cs, m, jac);
 			if ((ret = checked(rt))) return ret;
-			k_benc_gram<<<m * m, HT, 0, rt.stream>>>(jac, Cc * s, nl, part2);
+			k_benc_gram<<<m * m, HT, 0, rt.stream>>>(jac, Cc * s, nl, c.columns, b0, half, part2);
 			if ((ret = checked(rt))) return ret;
 		}
 	}

@@ -17,6 +17,10 @@ struct HessCircuit
 	int nlayers = 0;
 	const double2* ugates = nullptr;   // [nlayers][16]
 	const int* wires = nullptr;        // [2 * nlayers * L/2]
+	// columns to sum over instead of all basis states (device, orbits.h); of the half register
+	// for the block encoding
+	const BasisCol* columns = nullptr;
+	int64_t ncolumns = 0;
 };
 
 // Device output record of the Hessian engine (double2 entries):

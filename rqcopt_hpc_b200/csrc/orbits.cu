@@ -50,6 +50,23 @@ std::vector<int> wire_symmetries(int L, const std::vector<const int*>& layers)
 	return sym;
 }
 
+bool preserves_layers(int L, const std::vector<const int*>& layers, const int* s)
+{
+	for (const int* w : layers) {
+		std::vector<int> after(L, -1);   // second wire of the pair that begins with a wire
+		std::vector<char> seen(L, 0);
+		for (int p = 0; p < L / 2; p++) {
+			const int i = w[2 * p], j = w[2 * p + 1];
+			if (i < 0 || j < 0 || i >= L || j >= L || i == j || seen[i] || seen[j]) return false;
+			seen[i] = seen[j] = 1;
+			after[i] = j;
+		}
+		for (int p = 0; p < L / 2; p++)
+			if (after[s[w[2 * p]]] != s[w[2 * p + 1]]) return false;
+	}
+	return true;
+}
+
 std::vector<BasisCol> orbit_columns(int L, const std::vector<int>& sym)
 {
 	const int ng = (int)sym.size() / L, nbytes = (L + 7) / 8;

@@ -29,6 +29,10 @@ struct BasisCol
 // do not connect the wires (a relabelling is then not fixed by the image of one wire).
 std::vector<int> wire_symmetries(int L, const std::vector<const int*>& layers);
 
+// Whether the relabelling s (L wires) preserves every layer; false if a layer does not cover
+// each wire once.
+bool preserves_layers(int L, const std::vector<const int*>& layers, const int* s);
+
 // The least state of every orbit under the relabellings sym, in ascending order, with the size
 // of its orbit as weight (im = -1: no second state).
 std::vector<BasisCol> orbit_columns(int L, const std::vector<int>& sym);

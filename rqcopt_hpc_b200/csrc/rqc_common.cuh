@@ -60,13 +60,6 @@ struct ColumnSource
 	int weighted = 0;
 };
 
-inline ColumnSource plain_columns(int64_t b0)
-{
-	ColumnSource s;
-	s.b0 = b0;
-	return s;
-}
-
 // amplitude `row` of column c of the chunk
 template <typename T>
 __device__ __forceinline__ cplx<T> basis_amp(const ColumnSource& s, int64_t row, int64_t c)

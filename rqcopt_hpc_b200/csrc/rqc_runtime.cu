@@ -85,6 +85,18 @@ int ensure_host_pinned(Buffer& b, size_t bytes)
 	return OK;
 }
 
+size_t workspace_budget(Runtime& rt, size_t want)
+{
+	if (rt.workspace_limit) return rt.workspace_limit;
+	if (rt.work.ptr && rt.work.bytes >= want) return want;
+	size_t free_b = 0, total_b = 0;
+	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+		cudaGetLastError();
+		return (size_t)1 << 30;
+	}
+	return (size_t)((free_b + rt.work.bytes) * 0.75);
+}
+
 bool is_device_pointer(const void* p)
 {
 	cudaPointerAttributes a;

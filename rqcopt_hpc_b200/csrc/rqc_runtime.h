@@ -94,6 +94,12 @@ void fail_arg(const char* fn, const char* msg);
 int ensure_device(Buffer& b, size_t bytes);
 int ensure_host_pinned(Buffer& b, size_t bytes);
 
+// Bytes the column-chunk workspace (rt.work) may take for a call that would like `want`: the
+// limit set by the caller, else what it already holds if that is enough, else 3/4 of the
+// memory free beside it.  The driver is asked for the free memory only to grow: the query
+// takes the driver's locks (20-40 ms now and then on a host that other processes use).
+size_t workspace_budget(Runtime& rt, size_t want);
+
 // true if the pointer is device-accessible memory of this context (device or managed)
 bool is_device_pointer(const void* p);
 

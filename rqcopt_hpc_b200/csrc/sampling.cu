@@ -144,17 +144,6 @@ __global__ void k_fsum(const double2* __restrict__ fpart, int nblk, double scale
 	f[0] = make_double2(sx * scale, sy * scale);
 }
 
-size_t sampling_workspace_limit(Runtime& rt)
-{
-	if (rt.workspace_limit) return rt.workspace_limit;
-	size_t free_b = 0, total_b = 0;
-	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-		cudaGetLastError();
-		return (size_t)1 << 30;
-	}
-	return (size_t)((free_b + rt.work.bytes) * 0.75);
-}
-
 int g_real_samples = 0;
 
 }  // namespace
@@ -189,10 +178,10 @@ int sampled_f_device(Runtime& rt, int L, int ngates, const double2* gates, const
 	if (sp.nsamples < 1) return E_ARG;
 	// chunk states: samples, target columns, C psi, two target scratch states
 	const size_t col_bytes = 5 * (size_t)N * sizeof(double2);
-	int64_t C = (int64_t)(sampling_workspace_limit(rt) / col_bytes);
+	int64_t C = sp.nsamples;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
 	if (t.ufunc) C = std::min<int64_t>(C, std::max<int64_t>(1, ((int64_t)256 << 20) / (N * 16)));
-	C = std::min<int64_t>(C, sp.nsamples);
+	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
 	if (C < 1) return E_ALLOC;
 	int ret = ensure_device(rt.work, 5 * (size_t)C * N * sizeof(double2));
 	if (ret) return ret;

@@ -16,6 +16,7 @@ struct Problem
 	int G = 0;        // sequential gates
 	int nunits = 0;   // optimisation units
 	int per = 1;      // sequential gates per unit (brickwall: L/2 copies of the layer gate)
+	bool brickwall = false;
 	std::vector<double2> gates, dirs;     // [G][16]
 	std::vector<int> wires;               // [2G]
 	std::vector<double2> ugates, udirs;   // [nunits][16]
@@ -38,9 +39,15 @@ struct TargetHolder
 
 // Sum over the orbits of the wire relabellings that circuit and target share, instead of
 // over all basis states (orbits.h): a brickwall against a device-native brickwall whose
-// results are per-layer sums, over all columns.  Fills cs.columns and cs.ncolumns, the list
-// in rt.columns (held until the next call).
-int use_orbits(Runtime& rt, const Problem& pb, const TargetHolder& th, CircuitSpec& cs);
+// results are per-layer sums, over all columns.  Sets *columns and *ncolumns where there is
+// such a symmetry; the list lies in rt.columns (held until the next call).
+int use_orbits(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th, const BasisCol** columns,
+               int64_t* ncolumns);
+// The same for the block encoding of a brickwall on L/2 qubits (the target) by one on L: the
+// relabellings keep the wires of the half register (0, 2, 4, ...) among themselves; columns
+// of the half register.
+int use_orbits_blockenc(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th,
+                        const BasisCol** columns, int64_t* ncolumns);
 
 int post_launch(Runtime& rt, const double2* d_res, const Problem& pb, const double2* d_ugates, const double2* d_udirs,
                 int with_hvp, double2* d_dunits, double2* d_hunits, double* d_grad, double* d_hvp);

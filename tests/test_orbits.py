@@ -154,3 +154,41 @@ def test_real_orbit_evaluations_equal_plain_ones(gpu, L, kind):
     ref = real.brickwall_unitary_target_projected_hessian_vector_product(ref_t, v[:3], d, perms, L)
     assert abs(got[0] - ref[0]) <= 1e-12 * 2 ** (L / 2)
     assert rel_err(got[1], ref[1]) <= 1e-12 and rel_err(got[2], ref[2]) <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,kind", [(4, "ring"), (6, "renamed"), (8, "ring"), (8, "reversed"), (8, "any"), (14, "ring")])
+@pytest.mark.parametrize("chunk", [0, 7])
+def test_orbit_hessians_equal_plain_ones(gpu, L, kind, chunk):
+    depth = 2 if L == 14 else 3
+    vlist, _, tvlist, _ = brickwall_instance(L, depth, L, 2, L + 1)
+    perms = _layers(kind, L, depth, L)
+    t = gpu.Target(brickwall=(tvlist, perms[:2]))
+    if L == 14 and chunk:
+        chunk = 700
+    try:
+        gpu.set_column_chunk(chunk)
+        got = gpu.brickwall_unitary_target_gradient_hessian(t, vlist, perms, L)
+        gpu.set_column_range(0, 1 << L)
+        ref = gpu.brickwall_unitary_target_gradient_hessian(t, vlist, perms, L)
+    finally:
+        gpu.set_column_range(0, 0)
+        gpu.set_autotune(True)
+    assert abs(got[0] - ref[0]) <= 1e-12 * 2 ** (L / 2)
+    assert rel_err(got[1], ref[1]) <= 1e-12 and rel_err(got[2], ref[2]) <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,depth,hdepth", [(4, 2, 1), (8, 3, 1), (8, 3, 2), (12, 3, 3)])
+def test_orbit_block_encodings_equal_plain_ones(gpu, L, depth, hdepth):
+    vlist, perms, _, _ = brickwall_instance(L, depth, L, 1, L + 1)
+    hv, hp, _, _ = brickwall_instance(L // 2, hdepth, 3, 1, 4)
+    dev = gpu.Target(brickwall=(hv, hp))
+    host = gpu.Target(fn=lambda x: gpu.apply_brickwall_unitary(hv, hp, x))   # a callback: all columns
+    for fn in (gpu.brickwall_blockenc_target_and_gradient, gpu.brickwall_blockenc_target_gradient_hessian,
+               gpu.brickwall_blockenc_target_gradient_vector_hessian_matrix):
+        got, ref = fn(dev, vlist, perms, L), fn(host, vlist, perms, L)
+        assert abs(got[0] - ref[0]) <= 1e-12 * abs(ref[0])
+        for a, b in zip(got[1:], ref[1:]):
+            assert rel_err(a, b) <= 1e-12
+    assert abs(gpu.brickwall_blockenc_target(dev, vlist, perms, L) - ref[0]) <= 1e-12 * abs(ref[0])
