@@ -281,6 +281,7 @@ int hessian_target(const char* fn, linear_func ufunc, void* udata, const struct 
 	c.nlayers = nlayers;
 	c.ugates = ug.data();
 	c.wires = wires.data();
+	if ((ret = th.to_device(*rt))) return ret;
 	if (!samp && (ret = use_orbits(*rt, nqubits, nlayers, wires.data(), th, &c.columns, &c.ncolumns))) return ret;
 	if ((ret = hessian_target_device(*rt, c, th.spec, rec, samp))) return ret;
 	if (H) {
@@ -361,7 +362,8 @@ int sampled_value(const char* fn, linear_func ufunc, void* udata, const std::vec
 	if (!th.set(ufunc, udata, nqubits)) return fail(fn, E_ARG);
 	Runtime* rt = runtime();
 	if (!rt) return E_CUDA;
-	int ret = ensure_device(rt->result, sizeof(double2));
+	int ret = th.to_device(*rt);
+	if (!ret) ret = ensure_device(rt->result, sizeof(double2));
 	if (ret) return ret;
 	double2* d_f = static_cast<double2*>(rt->result.ptr);
 	if ((ret = sampled_f_device(*rt, nqubits, (int)(wires.size() / 2), gates.data(), wires.data(), th.spec,
@@ -452,6 +454,7 @@ int blockenc(const char* fn, linear_func hfunc, void* hdata, const struct mat4x4
 	c.nlayers = nlayers;
 	c.ugates = ug.data();
 	c.wires = wires.data();
+	if ((ret = th.to_device(*rt))) return ret;
 	if ((ret = use_orbits_blockenc(*rt, nqubits, nlayers, wires.data(), th, &c.columns, &c.ncolumns))) return ret;
 	if ((ret = blockenc_device(*rt, c, th.spec, mode, rec, d_h2))) return ret;
 	if (grad_vec) {

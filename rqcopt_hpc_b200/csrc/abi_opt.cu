@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "engine_small.h"
 #include "hess.h"
 #include "manifold.cuh"
 #include "rqc_runtime.h"
@@ -29,50 +30,120 @@ using namespace rqc;
 namespace {
 
 // r = grad, rsq, stop tolerance, z = 0, d = -r
-__global__ void k_tcg_init(int n, const double* grad, double* r, double* d, double* z, TcgState* st, double radius,
-                           double abstol, double reltol)
+__global__ void __launch_bounds__(TR_THREADS) k_tcg_init(int n, const double* grad, double* r, double* d, double* z,
+                                                         TcgState* st, double radius, double abstol, double reltol)
 {
-	if (threadIdx.x | blockIdx.x) return;
-	tcg_init_dev(n, grad, r, d, z, st, radius, abstol, reltol);
+	__shared__ BlockDots dots;
+	tcg_init_blk(n, grad, r, d, z, st, radius, abstol, reltol, dots);
 }
 
 // One tCG step after Hd = H d
-__global__ void k_tcg_step(int n, double* d, const double* hd, double* z, double* r, TcgState* st)
+__global__ void __launch_bounds__(TR_THREADS) k_tcg_step(int n, double* d, const double* hd, double* z, double* r,
+                                                         TcgState* st)
 {
-	if (threadIdx.x | blockIdx.x) return;
-	tcg_step_dev(n, d, hd, z, r, st);
+	__shared__ BlockDots dots;
+	tcg_step_blk(n, d, hd, z, r, st, dots);
 }
 
-// Ratio test and radius update; fx / fnext read from the given device doubles unless null.
-__global__ void k_rtr_rho(int n, const double* grad, const double* eta, const double* heta, const double* fx_dev,
-                          const double* fnext_dev, RtrState* st, int on_boundary)
+// Ratio test and radius update; fx / fnext read from the given device doubles unless null,
+// the boundary flag from boundary_dev unless null.
+__global__ void __launch_bounds__(TR_THREADS) k_rtr_rho(int n, const double* grad, const double* eta, const double* heta,
+                                                        const double* fx_dev, const double* fnext_dev, RtrState* st,
+                                                        int on_boundary, const int* boundary_dev)
 {
-	if (threadIdx.x | blockIdx.x) return;
-	if (fx_dev) st->fx = *fx_dev;
-	if (fnext_dev) st->fnext = *fnext_dev;
-	rtr_rho_dev(n, grad, eta, heta, st, on_boundary);
+	__shared__ BlockDots dots;
+	if (threadIdx.x == 0) {
+		if (fx_dev) st->fx = *fx_dev;
+		if (fnext_dev) st->fnext = *fnext_dev;
+	}
+	rtr_rho_blk(n, grad, eta, heta, st, boundary_dev ? *boundary_dev : on_boundary, dots);
 }
 
-// Z_u = V_u A(vec_u) for every unit (src/matrix.c:309-314)
+// Z_u = V_u A(vec_u) for every unit (src/matrix.c:309-314), a thread per entry
 __global__ void k_real_to_tangent(int nunits, const double* vec, const double2* x, double2* dirs)
 {
-	const int u = blockIdx.x * blockDim.x + threadIdx.x;
+	const int i = blockIdx.x * blockDim.x + threadIdx.x, u = i >> 4, r = (i & 15) >> 2, c = i & 3;
 	if (u >= nunits) return;
-	M4 v, z;
-	for (int e = 0; e < 16; e++) v.a[e] = x[16 * u + e];
-	m4_real_to_tangent(vec + 16 * u, v, z);
-	for (int e = 0; e < 16; e++) dirs[16 * u + e] = z.a[e];
+	const double* a = vec + 16 * u;
+	double2 s = c_(0, 0);
+	for (int m = 0; m < 4; m++) {
+		// entry (m, c) of the anti-Hermitian matrix (src/matrix.c:218-243)
+		double2 w;
+		if (m == c) w = c_(0, a[5 * m]);
+		else if (m < c) w = c_(0.5 * (a[4 * m + c] - a[4 * c + m]), 0.5 * (a[4 * m + c] + a[4 * c + m]));
+		else w = c_(-0.5 * (a[4 * c + m] - a[4 * m + c]), 0.5 * (a[4 * c + m] + a[4 * m + c]));
+		s = c_add(s, c_mul(x[16 * u + 4 * r + m], w));
+	}
+	dirs[i] = s;
 }
 
-// polar retraction of every unit (src/matrix.c:517-531)
+__device__ __forceinline__ double2 shfl2(double2 v, int src)
+{
+	return c_(__shfl_sync(0xffffffffu, v.x, src, 16), __shfl_sync(0xffffffffu, v.y, src, 16));
+}
+
+// inverse of the 4x4 matrix whose entry (r, c) lane 4 r + c of a 16-lane group holds: m4_inverse
+// (manifold.cuh), an entry per lane
+__device__ inline double2 group_inverse(double2 m, int r, int c)
+{
+	double2 v = c_(r == c ? 1.0 : 0.0, 0);
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		// pivot row: the first largest entry of column k at or below row k
+		const double mine = c_abs(m);
+		int piv = k;
+		double best = __shfl_sync(0xffffffffu, mine, 5 * k, 16);
+#pragma unroll
+		for (int i = k + 1; i < 4; i++) {
+			const double x = __shfl_sync(0xffffffffu, mine, 4 * i + k, 16);
+			if (x > best) { best = x; piv = i; }
+		}
+		const int from = r == k ? 4 * piv + c : r == piv ? 4 * k + c : 4 * r + c;
+		m = shfl2(m, from);
+		v = shfl2(v, from);
+		const double2 d = shfl2(m, 5 * k), mk = shfl2(m, 4 * k + c), vk = shfl2(v, 4 * k + c);
+		const double2 s = c_div(shfl2(m, 4 * r + k), d);
+		if (r == k) {
+			m = c == k ? c_(1, 0) : c > k ? c_div(m, d) : m;
+			v = c_div(v, d);
+		} else {
+			m = c == k ? c_(0, 0) : c > k ? c_sub(m, c_mul(s, mk)) : m;
+			v = c_sub(v, c_mul(s, vk));
+		}
+	}
+	return v;
+}
+
+// polar retraction of every unit (src/matrix.c:517-531), 16 lanes per unit: m4_retract
+// (manifold.cuh) an entry per lane.  With a thread per unit the 6-8 Newton steps on local
+// arrays took 88 us at any number of units.
 __global__ void k_retract(int nunits, const double2* x, const double* eta, double2* xs)
 {
-	const int u = blockIdx.x * blockDim.x + threadIdx.x;
-	if (u >= nunits) return;
-	M4 v, w;
-	for (int e = 0; e < 16; e++) v.a[e] = x[16 * u + e];
-	m4_retract(v, eta + 16 * u, w);
-	for (int e = 0; e < 16; e++) xs[16 * u + e] = w.a[e];
+	const int i = blockIdx.x * blockDim.x + threadIdx.x, r = (i & 15) >> 2, c = i & 3;
+	const int u = min(i >> 4, nunits - 1);   // whole warps take part in the shuffles
+	const double* a = eta + 16 * u;
+	double2 w;
+	if (r == c) w = c_(1, a[5 * r]);
+	else if (r < c) w = c_(0.5 * (a[4 * r + c] - a[4 * c + r]), 0.5 * (a[4 * r + c] + a[4 * c + r]));
+	else w = c_(-0.5 * (a[4 * c + r] - a[4 * r + c]), 0.5 * (a[4 * c + r] + a[4 * r + c]));
+	const double2 g = x[16 * u + 4 * r + c];
+	double2 y = c_(0, 0);
+#pragma unroll
+	for (int m = 0; m < 4; m++) y = c_add(y, c_mul(shfl2(g, 4 * r + m), shfl2(w, 4 * m + c)));
+	// Newton iteration y <- (y + y^{-H}) / 2 to the unitary polar factor (src/matrix.c:488-510)
+	bool done = false;
+	for (int k = 0; k < 14; k++) {
+		const double2 inv = group_inverse(y, r, c);
+		const double2 t = c_conj(shfl2(inv, 4 * c + r));
+		const double2 next = c_scale(c_add(y, t), 0.5);
+		double d = c_abs(c_sub(next, t));
+#pragma unroll
+		for (int o = 8; o > 0; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o, 16));
+		if (!done) y = next;
+		done = done || (k >= 4 && d < 1e-14);
+		if (__all_sync(0xffffffffu, done)) break;
+	}
+	if ((i >> 4) < nunits) xs[i] = y;
 }
 
 int launched(Runtime& rt)
@@ -84,8 +155,11 @@ int launched(Runtime& rt)
 template <typename S>
 int read_state(Runtime& rt, const S* d, S* h)
 {
-	int ret = RQC_CUDA(cudaMemcpyAsync(h, d, sizeof(S), cudaMemcpyDeviceToHost, rt.stream));
-	return ret ? ret : sync(rt);
+	int ret = ensure_host_pinned(rt.out_host, sizeof(S));
+	if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(rt.out_host.ptr, d, sizeof(S), cudaMemcpyDeviceToHost, rt.stream));
+	if (!ret) ret = sync(rt);
+	if (!ret) memcpy(h, rt.out_host.ptr, sizeof(S));
+	return ret;
 }
 
 // ----------------------------------------------------------------------------- generic API
@@ -115,7 +189,7 @@ int alloc_vecs(Runtime& rt, int n, DevVecs& v, Buffer& buf)
 int tcg_host_callback(Runtime& rt, const double* x, hessian_vector_product_func f_hvp, void* fdata, int n, double radius,
                       const struct truncated_cg_params* params, DevVecs& v, std::vector<double>& hbuf, bool* on_boundary)
 {
-	k_tcg_init<<<1, 1, 0, rt.stream>>>(n, v.grad, v.r, v.d, v.z, v.tcg, radius, params->abstol, params->reltol);
+	k_tcg_init<<<1, TR_THREADS, 0, rt.stream>>>(n, v.grad, v.r, v.d, v.z, v.tcg, radius, params->abstol, params->reltol);
 	int ret = launched(rt);
 	*on_boundary = false;
 	hbuf.resize(2 * (size_t)n);
@@ -124,7 +198,7 @@ int tcg_host_callback(Runtime& rt, const double* x, hessian_vector_product_func 
 		if ((ret = sync(rt))) break;
 		f_hvp(x, fdata, hbuf.data(), hbuf.data() + n);
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(v.hd, hbuf.data() + n, n * sizeof(double), cudaMemcpyHostToDevice, rt.stream)))) break;
-		k_tcg_step<<<1, 1, 0, rt.stream>>>(n, v.d, v.hd, v.z, v.r, v.tcg);
+		k_tcg_step<<<1, TR_THREADS, 0, rt.stream>>>(n, v.d, v.hd, v.z, v.r, v.tcg);
 		if ((ret = launched(rt))) break;
 		TcgState st;
 		if ((ret = read_state(rt, v.tcg, &st))) break;
@@ -189,7 +263,7 @@ extern "C" void riemannian_trust_region_optimize_hvp(const target_func f, const 
 		rs.fnext = f(xn.data(), fdata);
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(v.heta, hheta.data(), n * sizeof(double), cudaMemcpyHostToDevice, rt->stream)))) break;
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(v.rtr, &rs, sizeof(rs), cudaMemcpyHostToDevice, rt->stream)))) break;
-		k_rtr_rho<<<1, 1, 0, rt->stream>>>(n, v.grad, v.z, v.heta, nullptr, nullptr, v.rtr, boundary ? 1 : 0);
+		k_rtr_rho<<<1, TR_THREADS, 0, rt->stream>>>(n, v.grad, v.z, v.heta, nullptr, nullptr, v.rtr, boundary ? 1 : 0, nullptr);
 		if ((ret = launched(*rt))) break;
 		if ((ret = read_state(*rt, v.rtr, &rs))) break;
 		if (rs.accept) x.swap(xn);
@@ -278,7 +352,7 @@ extern "C" void riemannian_trust_region_optimize_hmat(target_func f, target_grad
 		rs.fx = fx;
 		rs.fnext = f(xn.data(), fdata);
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(v.rtr, &rs, sizeof(rs), cudaMemcpyHostToDevice, rt->stream)))) break;
-		k_rtr_rho<<<1, 1, 0, rt->stream>>>(n, v.grad, v.z, v.heta, nullptr, nullptr, v.rtr, boundary);
+		k_rtr_rho<<<1, TR_THREADS, 0, rt->stream>>>(n, v.grad, v.z, v.heta, nullptr, nullptr, v.rtr, boundary, nullptr);
 		if ((ret = launched(*rt))) break;
 		if ((ret = read_state(*rt, v.rtr, &rs))) break;
 		if (rs.accept) x.swap(xn);
@@ -304,20 +378,25 @@ struct DeviceOptimizer
 	const TargetHolder& th;
 	int n;
 	DevVecs v;
-	double2 *x, *xn, *dirs, *res, *ug;
+	double2 *x, *xn, *dirs, *res;
 	double* scratch;   // projected-gradient output of HVP evaluations
 	std::vector<double2> hx;
 	CircuitSpec orbits;   // the columns of every evaluation
+	// complex128 evaluations of a small problem: two launches each, gates and directions
+	// straight from the device vectors (engine_small.cu)
+	bool small = false;
+	SmallEval ev;
+	const double2* at = nullptr;   // the loaded gates (device)
 	int hvp_prec;
 	long evals_hvp = 0, evals_grad = 0, evals_f = 0;
 
 	DeviceOptimizer(Runtime& r, Problem& p, const TargetHolder& t) : rt(r), pb(p), th(t), n(16 * p.nunits) {}
 
-	int init(const double2* x0)
+	int init(const double2* x0, bool c128)
 	{
 		const size_t nu = pb.nunits;
 		const size_t nres = result_count(pb.G);
-		const size_t bytes = 7 * (size_t)n * sizeof(double) + 512 + (4 * 16 * nu + nres) * sizeof(double2) + (n + 8) * sizeof(double);
+		const size_t bytes = 7 * (size_t)n * sizeof(double) + 512 + (3 * 16 * nu + nres) * sizeof(double2) + (n + 8) * sizeof(double);
 		int ret = ensure_device(rt.opt, bytes);
 		if (ret) return ret;
 		if ((ret = alloc_vecs(rt, n, v, rt.opt))) return ret;
@@ -325,22 +404,27 @@ struct DeviceOptimizer
 		x = reinterpret_cast<double2*>(base);
 		xn = x + 16 * nu;
 		dirs = xn + 16 * nu;
-		ug = dirs + 16 * nu;
-		res = ug + 16 * nu;
+		res = dirs + 16 * nu;
 		scratch = reinterpret_cast<double*>(res + nres);
 		hx.assign(x0, x0 + 16 * nu);
-		if (pb.brickwall && (ret = use_orbits(rt, pb.L, pb.nunits, pb.wires.data(), th, &orbits.columns, &orbits.ncolumns)))
-			return ret;
+		const std::vector<BasisCol> cols =
+			pb.brickwall ? orbits_of(rt, pb.L, pb.nunits, pb.wires.data(), th) : std::vector<BasisCol>();
+		if (!cols.empty() && (ret = upload_columns(rt, cols, &orbits.columns, &orbits.ncolumns))) return ret;
+		orbits.L = pb.L;
+		small = c128 && SmallEval::fits(rt, pb, th, column_count(rt, orbits));
+		if (small && (ret = ev.prepare(rt, pb, th, cols))) return ret;
 		return RQC_CUDA(cudaMemcpyAsync(x, x0, 16 * nu * sizeof(double2), cudaMemcpyHostToDevice, rt.stream));
 	}
 
-	// gates of the device array `src` become the kernel arguments of the next passes
-	int load_gates(const double2* src)
+	// gates of the device array `src` become those of the next evaluations; the pass engines
+	// and the Hessian sweep take them as kernel arguments, from the host
+	int load_gates(const double2* src, bool on_host)
 	{
+		at = src;
+		if (!on_host) return OK;
 		int ret = RQC_CUDA(cudaMemcpyAsync(hx.data(), src, hx.size() * sizeof(double2), cudaMemcpyDeviceToHost, rt.stream));
 		if (!ret) ret = sync(rt);
 		if (!ret) pb.set_gates_from_units(hx.data());
-		if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(ug, src, hx.size() * sizeof(double2), cudaMemcpyDeviceToDevice, rt.stream));
 		return ret;
 	}
 
@@ -359,6 +443,11 @@ struct DeviceOptimizer
 	int eval_f(int prec)
 	{
 		evals_f++;
+		if (small) {
+			SmallOut out;
+			out.f = res;
+			return ev.eval(rt, EVAL_F, at, nullptr, out);
+		}
 		return evaluate(rt, spec(false), th.spec, EVAL_F, prec, res);
 	}
 
@@ -366,8 +455,14 @@ struct DeviceOptimizer
 	int eval_grad(int prec)
 	{
 		evals_grad++;
+		if (small) {
+			SmallOut out;
+			out.f = res;
+			out.grad = v.grad;
+			return ev.eval(rt, EVAL_GRAD, at, nullptr, out);
+		}
 		int ret = evaluate(rt, spec(false), th.spec, EVAL_GRAD, prec, res);
-		if (!ret) ret = post_launch(rt, res, pb, ug, nullptr, 0, nullptr, nullptr, v.grad, nullptr);
+		if (!ret) ret = post_launch(rt, res, pb, at, nullptr, 0, nullptr, nullptr, v.grad, nullptr);
 		return ret;
 	}
 
@@ -375,16 +470,20 @@ struct DeviceOptimizer
 	int eval_hvp(const double* vec, double* out, int prec)
 	{
 		evals_hvp++;
-		const int threads = 64, blocks = (pb.nunits + threads - 1) / threads;
-		k_real_to_tangent<<<blocks, threads, 0, rt.stream>>>(pb.nunits, vec, ug, dirs);
+		k_real_to_tangent<<<(16 * pb.nunits + 127) / 128, 128, 0, rt.stream>>>(pb.nunits, vec, at, dirs);
 		int ret = launched(rt);
+		if (!ret && small) {
+			SmallOut o;
+			o.hvp = out;
+			return ev.eval(rt, EVAL_HVP, at, dirs, o);
+		}
 		std::vector<double2> hd(16 * (size_t)pb.nunits);
 		if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(hd.data(), dirs, hd.size() * sizeof(double2), cudaMemcpyDeviceToHost, rt.stream));
 		if (!ret) ret = sync(rt);
 		if (ret) return ret;
 		pb.set_dirs_from_units(hd.data());
 		if ((ret = evaluate(rt, spec(true), th.spec, EVAL_HVP, prec, res))) return ret;
-		return post_launch(rt, res, pb, ug, dirs, 1, nullptr, nullptr, scratch, out);
+		return post_launch(rt, res, pb, at, dirs, 1, nullptr, nullptr, scratch, out);
 	}
 
 	int run(const struct rtr_params* params, int niter, double* f_iter, double2* x_final, int precision)
@@ -400,27 +499,27 @@ struct DeviceOptimizer
 		const int fprec = precision == PREC_C64 ? PREC_C64 : PREC_C128;
 		hvp_prec = precision == PREC_C128 ? PREC_C128 : PREC_C64;
 		double* fx_slot = scratch + n;
-		const int threads = 64, blocks = (pb.nunits + threads - 1) / threads;
+		const int threads = 128, blocks = (16 * pb.nunits + threads - 1) / threads;
 		rt.opt_trace.clear();
 		for (int k = 0; k < niter && !ret; k++) {
 			// f and gradient at x (src/trust_region.c:328)
-			if ((ret = load_gates(x))) break;
+			if ((ret = load_gates(x, !small))) break;
 			if ((ret = eval_grad(fprec))) break;
 			if ((ret = RQC_CUDA(cudaMemcpyAsync(fx_slot, res, sizeof(double), cudaMemcpyDeviceToDevice, rt.stream)))) break;
-			if ((ret = RQC_CUDA(cudaMemcpyAsync(&rs, v.rtr, sizeof(rs), cudaMemcpyDeviceToHost, rt.stream)))) break;
-			if ((ret = sync(rt))) break;
 			// tCG (src/trust_region.c:159-217)
-			k_tcg_init<<<1, 1, 0, rt.stream>>>(n, v.grad, v.r, v.d, v.z, v.tcg, rs.radius, params->tcg_params.abstol,
+			k_tcg_init<<<1, TR_THREADS, 0, rt.stream>>>(n, v.grad, v.r, v.d, v.z, v.tcg, rs.radius, params->tcg_params.abstol,
 			                                   params->tcg_params.reltol);
 			if ((ret = launched(rt))) break;
 			TcgState st;
-			if ((ret = read_state(rt, v.tcg, &st))) break;
-			if (precision == PREC_MIXED && hvp_prec != PREC_C128 && sqrt(st.rsq) < rt.refine_threshold) hvp_prec = PREC_C128;
+			if (precision == PREC_MIXED && hvp_prec != PREC_C128) {
+				if ((ret = read_state(rt, v.tcg, &st))) break;
+				if (sqrt(st.rsq) < rt.refine_threshold) hvp_prec = PREC_C128;
+			}
 			bool boundary = false;
 			int inner = 0;
 			for (int it = 0; it < params->tcg_params.maxiter; it++) {
 				if ((ret = eval_hvp(v.d, v.hd, hvp_prec))) break;
-				k_tcg_step<<<1, 1, 0, rt.stream>>>(n, v.d, v.hd, v.z, v.r, v.tcg);
+				k_tcg_step<<<1, TR_THREADS, 0, rt.stream>>>(n, v.d, v.hd, v.z, v.r, v.tcg);
 				if ((ret = launched(rt))) break;
 				if ((ret = read_state(rt, v.tcg, &st))) break;
 				inner = it + 1;
@@ -432,10 +531,10 @@ struct DeviceOptimizer
 			k_retract<<<blocks, threads, 0, rt.stream>>>(pb.nunits, x, v.z, xn);
 			if ((ret = launched(rt))) break;
 			if ((ret = eval_hvp(v.z, v.heta, hvp_prec))) break;
-			if ((ret = load_gates(xn))) break;
+			if ((ret = load_gates(xn, !small))) break;
 			if ((ret = eval_f(fprec))) break;
-			k_rtr_rho<<<1, 1, 0, rt.stream>>>(n, v.grad, v.z, v.heta, fx_slot, reinterpret_cast<const double*>(res), v.rtr,
-			                                   boundary ? 1 : 0);
+			k_rtr_rho<<<1, TR_THREADS, 0, rt.stream>>>(n, v.grad, v.z, v.heta, fx_slot, reinterpret_cast<const double*>(res), v.rtr,
+			                                   boundary ? 1 : 0, nullptr);
 			if ((ret = launched(rt))) break;
 			if ((ret = read_state(rt, v.rtr, &rs))) break;
 			f_iter[k] = rs.fx;
@@ -444,7 +543,7 @@ struct DeviceOptimizer
 		}
 		if (ret) return ret;
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(x_final, x, hx.size() * sizeof(double2), cudaMemcpyDeviceToHost, rt.stream)))) return ret;
-		if ((ret = load_gates(x))) return ret;
+		if ((ret = load_gates(x, !small))) return ret;
 		if ((ret = eval_f(fprec))) return ret;
 		double2 ff;
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(&ff, res, sizeof(double2), cudaMemcpyDeviceToHost, rt.stream)))) return ret;
@@ -491,10 +590,10 @@ struct DeviceOptimizer
 		c.wires = pb.wires.data();
 		c.columns = orbits.columns;
 		c.ncolumns = orbits.ncolumns;
-		const int threads = 64, blocks = (nl + threads - 1) / threads;
+		const int threads = 128, blocks = (16 * nl + threads - 1) / threads;
 		for (int k = 0; k < niter && !ret; k++) {
 			// f, gradient vector and Hessian matrix at x (src/trust_region.c:263)
-			if ((ret = load_gates(x))) break;
+			if ((ret = load_gates(x, true))) break;
 			c.ugates = hx.data();
 			if (rng) {
 				const SampleSpec sp = sample_spec(rng, nsamples);
@@ -503,22 +602,20 @@ struct DeviceOptimizer
 			} else if ((ret = hessian_target_device(rt, c, th.spec, rec))) {
 				break;
 			}
-			if ((ret = project_hessian_device(rt, nl, ug, rec, v.grad, d_hess))) break;
+			if ((ret = project_hessian_device(rt, nl, at, rec, v.grad, d_hess))) break;
 			if ((ret = RQC_CUDA(cudaMemcpyAsync(fx_slot, rec, sizeof(double), cudaMemcpyDeviceToDevice, rt.stream)))) break;
 			// tCG on the dense Hessian (src/trust_region.c:264)
 			if ((ret = tcg_hmat_device(rt, n, v.grad, d_hess, rs.radius, params->tcg_params.maxiter,
 			                           params->tcg_params.abstol, params->tcg_params.reltol, d_work, v.z, d_status)))
 				break;
-			int boundary = 0;
-			if ((ret = RQC_CUDA(cudaMemcpyAsync(&boundary, d_status, sizeof(int), cudaMemcpyDeviceToHost, rt.stream)))) break;
 			// candidate, model decrease and ratio test (src/trust_region.c:265-281)
 			k_retract<<<blocks, threads, 0, rt.stream>>>(nl, x, v.z, xn);
 			if ((ret = launched(rt))) break;
 			if ((ret = gemv_device(rt, n, d_hess, v.z, v.heta))) break;
-			if ((ret = load_gates(xn))) break;   // synchronises: boundary is valid after this
+			if ((ret = load_gates(xn, !small || rng))) break;
 			if ((ret = rng ? eval_f_sampled(rng, nsamples) : eval_f(PREC_C128))) break;
-			k_rtr_rho<<<1, 1, 0, rt.stream>>>(n, v.grad, v.z, v.heta, fx_slot, reinterpret_cast<const double*>(res), v.rtr,
-			                                   boundary);
+			k_rtr_rho<<<1, TR_THREADS, 0, rt.stream>>>(n, v.grad, v.z, v.heta, fx_slot, reinterpret_cast<const double*>(res), v.rtr,
+			                                   0, d_status);
 			if ((ret = launched(rt))) break;
 			if ((ret = read_state(rt, v.rtr, &rs))) break;
 			f_iter[k] = rs.fx;
@@ -526,7 +623,7 @@ struct DeviceOptimizer
 		}
 		if (ret) return ret;
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(x_final, x, hx.size() * sizeof(double2), cudaMemcpyDeviceToHost, rt.stream)))) return ret;
-		if ((ret = load_gates(x))) return ret;
+		if ((ret = load_gates(x, !small || rng))) return ret;
 		if ((ret = rng ? eval_f_sampled(rng, nsamples) : eval_f(PREC_C128))) return ret;
 		double2 ff;
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(&ff, res, sizeof(double2), cudaMemcpyDeviceToHost, rt.stream)))) return ret;
@@ -551,12 +648,13 @@ void run_optimizer(const char* fn, Problem& pb, linear_func ufunc, void* udata, 
 	}
 	Runtime* rt = runtime();
 	if (!rt) { set_last_error(E_CUDA); return; }
+	if (int ret = th.to_device(*rt)) { set_last_error(ret); return; }
 	// the drivers disable the per-iteration callback (src/brickwall_opt.c:141-143)
 	params->g_func = NULL;
 	params->g_data = NULL;
 	params->g_iter = NULL;
 	DeviceOptimizer opt(*rt, pb, th);
-	int ret = opt.init(reinterpret_cast<const double2*>(start));
+	int ret = opt.init(reinterpret_cast<const double2*>(start), hmat || rt->precision == PREC_C128);
 	if (!ret)
 		ret = hmat ? opt.run_hmat(params, niter, f_iter, reinterpret_cast<double2*>(out), rng, nsamples)
 		           : opt.run(params, niter, f_iter, reinterpret_cast<double2*>(out), rt->precision);

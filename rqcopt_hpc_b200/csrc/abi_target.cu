@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "engine_small.h"
 #include "manifold.cuh"
 
 #include "rqc_runtime.h"
@@ -162,6 +163,13 @@ bool TargetHolder::set(linear_func ufunc, void* udata, int L)
 	} else {
 		spec.ufunc = reinterpret_cast<void*>(ufunc);
 		spec.udata = udata;
+		if (ufunc == rqcopt_dense_ufunc) {
+			const struct rqcopt_dense_target* t = static_cast<const struct rqcopt_dense_target*>(udata);
+			if (t && t->u && t->nqubits == L) {
+				dense_host = reinterpret_cast<const double2*>(t->u);
+				dense_L = L;
+			}
+		}
 		return true;
 	}
 	spec.ngates = (int)(wires.size() / 2);
@@ -169,8 +177,6 @@ bool TargetHolder::set(linear_func ufunc, void* udata, int L)
 	spec.wires = wires.data();
 	return true;
 }
-
-namespace {
 
 int upload_columns(Runtime& rt, const std::vector<BasisCol>& cols, const BasisCol** columns, int64_t* ncolumns)
 {
@@ -186,28 +192,33 @@ int upload_columns(Runtime& rt, const std::vector<BasisCol>& cols, const BasisCo
 // worth its memory
 constexpr int MAX_ORBIT_QUBITS = 20;
 
-}  // namespace
-
-int use_orbits(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th, const BasisCol** columns,
-               int64_t* ncolumns)
+std::vector<BasisCol> orbits_of(const Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th)
 {
 	const int per = L / 2;
-	if (L < 4 || L > MAX_ORBIT_QUBITS || th.spec.ufunc || th.spec.per != per || rt.col_begin != 0 || rt.col_end != 0)
-		return OK;
+	if (L < 4 || L > MAX_ORBIT_QUBITS || th.spec.ufunc || th.spec.dense || th.spec.per != per || rt.col_begin != 0 ||
+	    rt.col_end != 0)
+		return {};
 	std::vector<const int*> layers;
 	for (int l = 0; l < nlayers; l++) layers.push_back(wires + (size_t)l * L);
 	for (int k = 0; k < th.spec.ngates; k += per) layers.push_back(&th.wires[2 * (size_t)k]);
 	const std::vector<int> sym = wire_symmetries(L, layers);
-	if ((int)sym.size() == L) return OK;
+	if ((int)sym.size() == L) return {};
 	const std::vector<BasisCol> cols = orbit_columns(L, sym);
-	return upload_columns(rt, rt.real_pairs ? pair_columns(cols) : cols, columns, ncolumns);
+	return rt.real_pairs ? pair_columns(cols) : cols;
+}
+
+int use_orbits(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th, const BasisCol** columns,
+               int64_t* ncolumns)
+{
+	const std::vector<BasisCol> cols = orbits_of(rt, L, nlayers, wires, th);
+	return cols.empty() ? OK : upload_columns(rt, cols, columns, ncolumns);
 }
 
 int use_orbits_blockenc(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th,
                         const BasisCol** columns, int64_t* ncolumns)
 {
 	const int half = L / 2, hper = half / 2;
-	if (L < 4 || half > MAX_ORBIT_QUBITS || th.spec.ufunc || hper < 1 || half % 2 || th.spec.per != hper) return OK;
+	if (L < 4 || half > MAX_ORBIT_QUBITS || th.spec.ufunc || th.spec.dense || hper < 1 || half % 2 || th.spec.per != hper) return OK;
 	std::vector<const int*> layers, hlayers;
 	for (int l = 0; l < nlayers; l++) layers.push_back(wires + (size_t)l * L);
 	for (int k = 0; k < th.spec.ngates; k += hper) hlayers.push_back(&th.wires[2 * (size_t)k]);
@@ -224,6 +235,19 @@ int use_orbits_blockenc(Runtime& rt, int L, int nlayers, const int* wires, const
 	}
 	if ((int)hsym.size() == half) return OK;
 	return upload_columns(rt, orbit_columns(half, hsym), columns, ncolumns);
+}
+
+int TargetHolder::to_device(Runtime& rt)
+{
+	if (!dense_host || dense_L > 13) return OK;
+	const size_t bytes = sizeof(double2) << (2 * dense_L);
+	int ret = ensure_device(rt.dense, bytes);
+	if (ret == E_ALLOC) return OK;   // no room: column by column through the host
+	if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(rt.dense.ptr, dense_host, bytes, cudaMemcpyDefault, rt.stream));
+	if (ret) return ret;
+	spec.dense = static_cast<const double2*>(rt.dense.ptr);
+	spec.ufunc = nullptr;
+	return OK;
 }
 
 // Fold per-gate sums into per-unit sums and project (src/target.c:410-430, 526-535, 652-672).
@@ -269,8 +293,37 @@ int post_launch(Runtime& rt, const double2* d_res, const Problem& pb, const doub
 	return RQC_CUDA(cudaGetLastError());
 }
 
+// run_target for a small problem: inputs in one staged copy, two launches, results written to
+// pinned host memory by the second
+static int run_small(Runtime& rt, const Problem& pb, const TargetHolder& th, const std::vector<BasisCol>& cols, int mode,
+                     numeric* fval, struct mat4x4* dunits, struct mat4x4* hunits, double* grad_vec, double* hvp_vec)
+{
+	const size_t nu = 16 * (size_t)pb.nunits;
+	const bool tan = mode == EVAL_HVP;
+	SmallEval ev;
+	int ret = ev.prepare(rt, pb, th, cols, pb.ugates.data(), tan ? pb.udirs.data() : nullptr);
+	if (!ret) ret = ensure_host_pinned(rt.out_host, (1 + 2 * nu) * sizeof(double2) + 2 * nu * sizeof(double));
+	if (ret) return ret;
+	SmallOut out;
+	double2* h = static_cast<double2*>(rt.out_host.ptr);
+	double* hv = reinterpret_cast<double*>(h + 1 + 2 * nu);
+	out.f = h;
+	out.dunits = dunits ? h + 1 : nullptr;
+	out.hunits = hunits && tan ? h + 1 + nu : nullptr;
+	out.grad = grad_vec ? hv : nullptr;
+	out.hvp = hvp_vec && tan ? hv + nu : nullptr;
+	if ((ret = ev.eval(rt, mode, nullptr, nullptr, out))) return ret;
+	if ((ret = sync(rt))) return ret;
+	if (fval) memcpy(fval, out.f, sizeof(double2));
+	if (out.dunits) memcpy(dunits, out.dunits, nu * sizeof(double2));
+	if (out.hunits) memcpy(hunits, out.hunits, nu * sizeof(double2));
+	if (out.grad) memcpy(grad_vec, out.grad, nu * sizeof(double));
+	if (out.hvp) memcpy(hvp_vec, out.hvp, nu * sizeof(double));
+	return OK;
+}
+
 // One evaluation of a target function through the engine, with host outputs.
-int run_target(const Problem& pb, const TargetHolder& th, int mode, numeric* fval, struct mat4x4* dunits,
+int run_target(const Problem& pb, TargetHolder& th, int mode, numeric* fval, struct mat4x4* dunits,
                struct mat4x4* hunits, double* grad_vec, double* hvp_vec)
 {
 	Runtime* rt = runtime();
@@ -282,8 +335,15 @@ int run_target(const Problem& pb, const TargetHolder& th, int mode, numeric* fva
 	cs.dirs = mode == EVAL_HVP ? pb.dirs.data() : nullptr;
 	cs.wires = pb.wires.data();
 	const int prec = rt->precision == PREC_C128 ? PREC_C128 : PREC_C64;
-	int ret = prec == PREC_C128 && pb.brickwall ? use_orbits(*rt, pb.L, pb.nunits, pb.wires.data(), th, &cs.columns, &cs.ncolumns) : OK;
+	int ret = th.to_device(*rt);
 	if (ret) return ret;
+	if (prec == PREC_C128) {
+		const std::vector<BasisCol> cols =
+			pb.brickwall ? orbits_of(*rt, pb.L, pb.nunits, pb.wires.data(), th) : std::vector<BasisCol>();
+		if (SmallEval::fits(*rt, pb, th, cols.empty() ? column_count(*rt, cs) : (int64_t)cols.size()))
+			return run_small(*rt, pb, th, cols, mode, fval, dunits, hunits, grad_vec, hvp_vec);
+		if (!cols.empty() && (ret = upload_columns(*rt, cols, &cs.columns, &cs.ncolumns))) return ret;
+	}
 	const size_t nres = result_count(pb.G);
 	const size_t nu = (size_t)pb.nunits;
 	// device layout in rt.opt: res | ugates | udirs | dunits | hunits | grad | hvp

@@ -100,7 +100,7 @@ int evaluate_autotuned(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, i
 		rt.last_choice = {rt.gates_per_pass, rt.column_chunk, rt.recon_c128, rt.c64_ffma, 0.0, 0};
 		return evaluate_configured(rt, c, t, mode, precision, d_out);
 	}
-	const std::array<long, 12> key = {(long)ncols, c.L, c.ngates, t.ngates, precision, mode, t.ufunc ? 1 : 0, rt.real_pairs,
+	const std::array<long, 12> key = {(long)ncols, c.L, c.ngates, t.ngates, precision, mode, t.dense ? 2 : t.ufunc ? 1 : 0, rt.real_pairs,
 	                                  rt.pin_gpp ? rt.gates_per_pass : 0, rt.pin_chunk ? rt.column_chunk : -1,
 	                                  rt.pin_recon ? rt.recon_c128 : -1, rt.pin_ffma ? rt.c64_ffma : -1};
 	const Saved saved(rt);

@@ -270,6 +270,59 @@ __global__ void __launch_bounds__(TPB) k_reverse(const cplx<T>* __restrict__ phi
 	}
 }
 
+// phi[c] = -conj(U e_c) of a dense U for columns c < ncols of src, states one after another:
+// 32 x 32 tiles through shared memory, reads along U's rows and writes along the states
+template <typename T>
+__global__ void __launch_bounds__(256) k_dense_columns(const double2* __restrict__ u, int L, ColumnSource src, int64_t ncols,
+                                                       cplx<T>* __restrict__ phi)
+{
+	__shared__ double2 tile[32][33];
+	const int64_t N = (int64_t)1 << L, row0 = (int64_t)blockIdx.x * 32, col0 = (int64_t)blockIdx.y * 32;
+	const int x = threadIdx.x & 31;
+	for (int y = threadIdx.x >> 5; y < 32; y += 8)
+		if (row0 + y < N && col0 + x < ncols) tile[y][x] = dense_amp(u, L, src, row0 + y, col0 + x);
+	__syncthreads();
+	for (int y = threadIdx.x >> 5; y < 32; y += 8)
+		if (row0 + x < N && col0 + y < ncols) {
+			const double2 v = tile[x][y];
+			phi[(col0 + y) * N + row0 + x] = mk<T>((T)(-v.x), (T)v.y);
+		}
+}
+
+template <typename T>
+static int dense_columns(Runtime& rt, const double2* u, int L, const ColumnSource& src, int64_t ncols, cplx<T>* phi)
+{
+	const int64_t N = (int64_t)1 << L;
+	k_dense_columns<T><<<dim3((unsigned)((N + 31) / 32), (unsigned)((ncols + 31) / 32)), 256, 0, rt.stream>>>(u, L, src, ncols,
+	                                                                                                        phi);
+	rt.launches++;
+	return RQC_CUDA(cudaGetLastError());
+}
+
+// phi[s] = -conj(U x[s]) of a dense U for ns states one after another: a warp per row of U and
+// four states
+__global__ void __launch_bounds__(256) k_dense_states(const double2* __restrict__ u, int L, const double2* __restrict__ x,
+                                                      int64_t ns, double2* __restrict__ phi)
+{
+	const int64_t N = (int64_t)1 << L, row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), s0 = (int64_t)blockIdx.y * 4;
+	const int lane = threadIdx.x & 31;
+	if (row >= N) return;
+	double2 acc[4];
+#pragma unroll
+	for (int k = 0; k < 4; k++) acc[k] = make_double2(0, 0);
+	for (int64_t c = lane; c < N; c += 32) {
+		const double2 a = u[(row << L) + c];
+#pragma unroll
+		for (int k = 0; k < 4; k++)
+			if (s0 + k < ns) acc[k] = cfma(a, x[((s0 + k) << L) + c], acc[k]);
+	}
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		const double re = warp_sum(acc[k].x), im = warp_sum(acc[k].y);
+		if (lane == 0 && s0 + k < ns) phi[((s0 + k) << L) + row] = make_double2(-re, im);
+	}
+}
+
 // out = -conj(in), converting from complex128 host columns to the pass precision
 template <typename T>
 __global__ void k_conj_neg(const double2* __restrict__ in, cplx<T>* __restrict__ out, int64_t n)
@@ -282,32 +335,22 @@ __global__ void k_conj_neg(const double2* __restrict__ in, cplx<T>* __restrict__
 
 // Sum partials over blocks (compensated).  Block s < nslots reduces gate s, block
 // nslots reduces f.  out: [0] f, [1 + 16 s + e] grad, [1 + 16 nslots + 16 s + e] HVP.
-__global__ void k_reduce(const double* __restrict__ part, const double2* __restrict__ fpart, int nslots, int nblk,
-                         int with_hvp, double2* __restrict__ out)
+__global__ void __launch_bounds__(RED_GROUPS * NPART)
+k_reduce(const double* __restrict__ part, const double2* __restrict__ fpart, int nslots, int nblk, int with_hvp,
+         double2* __restrict__ out)
 {
+	__shared__ double red[RED_GROUPS][NPART];
 	double* o = reinterpret_cast<double*>(out);
-	const int s = blockIdx.x, t = threadIdx.x;
+	const int s = blockIdx.x, t = threadIdx.x % NPART;
+	const bool first = threadIdx.x < NPART;
 	if (s < nslots) {
-		if (t >= NPART || (!with_hvp && t >= 32)) return;
-		double sum = 0, comp = 0;
-		for (int b = 0; b < nblk; b++) {
-			const double y = part[((size_t)s * nblk + b) * NPART + t] - comp;
-			const double u = sum + y;
-			comp = (u - sum) - y;
-			sum = u;
-		}
+		const double sum = block_column_sum<NPART>(part + (size_t)s * nblk * NPART + t, nblk, NPART, red);
+		if (!first || (!with_hvp && t >= 32)) return;
 		if (t < 32) o[2 * (1 + 16 * (size_t)s) + t] = sum;
 		else o[2 * (1 + 16 * (size_t)nslots + 16 * (size_t)s) + (t - 32)] = sum;
-	} else if (t < 2) {
-		double sum = 0, comp = 0;
-		for (int b = 0; b < nblk; b++) {
-			const double v = t == 0 ? fpart[b].x : fpart[b].y;
-			const double y = v - comp;
-			const double u = sum + y;
-			comp = (u - sum) - y;
-			sum = u;
-		}
-		o[t] = sum;
+	} else {
+		const double sum = block_column_sum<NPART>(reinterpret_cast<const double*>(fpart) + (t & 1), nblk, 2, red);
+		if (first && t < 2) o[t] = sum;
 	}
 }
 
@@ -514,6 +557,8 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 			if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 			// the pinned buffer is reused by the next chunk
 			if ((ret = RQC_CUDA(cudaStreamSynchronize(rt.stream)))) return ret;
+		} else if (t.dense) {
+			if ((ret = dense_columns<T>(rt, t.dense, L, tsrc, Cc, PHI))) return ret;
 		} else {
 			const int Gt = t.ngates;
 			for (int k = 0; k < Gt; k++) {
@@ -567,7 +612,7 @@ static int evaluate_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, in
 		}
 	}
 
-	k_reduce<<<G + 1, 64, 0, rt.stream>>>(part, fpart, G, nblk, tan ? 1 : 0, d_out);
+	k_reduce<<<G + 1, RED_GROUPS * NPART, 0, rt.stream>>>(part, fpart, G, nblk, tan ? 1 : 0, d_out);
 	rt.launches++;
 	return RQC_CUDA(cudaGetLastError());
 }
@@ -627,7 +672,7 @@ static int evaluate_columns(Runtime& rt, const CircuitSpec& c, const TargetSpec&
 		if (t.wires[2 * k] < 0 || t.wires[2 * k] >= c.L || t.wires[2 * k + 1] < 0 || t.wires[2 * k + 1] >= c.L ||
 		    t.wires[2 * k] == t.wires[2 * k + 1])
 			return E_ARG;
-	if (!t.ufunc && t.ngates < 1) return E_ARG;
+	if (!t.ufunc && !t.dense && t.ngates < 1) return E_ARG;
 	if (mode != EVAL_GRAD && mode != EVAL_HVP) {
 		// f only: the reduction still writes the (zero) gradient slots
 		mode = EVAL_F;
@@ -705,7 +750,7 @@ int gate_backward_device(Runtime& rt, int L, const double2* gate, int i, int j, 
 		return ret;
 	if ((ret = ensure_device(rt.result, result_count(1) * sizeof(double2)))) return ret;
 	double2* res = reinterpret_cast<double2*>(rt.result.ptr);
-	k_reduce<<<2, 64, 0, rt.stream>>>(part, fpart, 1, nblk, 0, res);
+	k_reduce<<<2, RED_GROUPS * NPART, 0, rt.stream>>>(part, fpart, 1, nblk, 0, res);
 	rt.launches++;
 	if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 	return RQC_CUDA(cudaMemcpyAsync(d_dgate, res + 1, 16 * sizeof(double2), cudaMemcpyDeviceToDevice, rt.stream));
@@ -717,6 +762,7 @@ int target_columns_device(Runtime& rt, const TargetSpec& t, int L, const ColumnS
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ngroups = ncols * (N / 4);
 	int ret;
+	if (t.dense) return dense_columns<double>(rt, t.dense, L, src, ncols, phi);
 	if (t.ufunc) {
 		if ((ret = ensure_host_pinned(rt.hpin, (size_t)(ncols + 1) * N * sizeof(double2)))) return ret;
 		double2* hcols = reinterpret_cast<double2*>(rt.hpin.ptr);
@@ -758,6 +804,12 @@ int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2*
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ngroups = ncols * (N / 4);
 	int ret;
+	if (t.dense) {
+		k_dense_states<<<dim3((unsigned)((N + 7) / 8), (unsigned)((ncols + 3) / 4)), 256, 0, rt.stream>>>(t.dense, L, states,
+		                                                                                                 ncols, phi);
+		rt.launches++;
+		return RQC_CUDA(cudaGetLastError());
+	}
 	if (t.ufunc) {
 		if ((ret = ensure_host_pinned(rt.hpin, (size_t)(2 * ncols) * N * sizeof(double2)))) return ret;
 		double2* hin = reinterpret_cast<double2*>(rt.hpin.ptr);
@@ -866,7 +918,7 @@ int column_passes_device(Runtime& rt, int L, int ngates, const double2* gates, c
 	}
 	if ((ret = ensure_device(rt.result, result_count(G) * sizeof(double2)))) return ret;
 	double2* res = reinterpret_cast<double2*>(rt.result.ptr);
-	k_reduce<<<G + 1, 64, 0, rt.stream>>>(part, fpart, G, nblk, tan ? 1 : 0, res);
+	k_reduce<<<G + 1, RED_GROUPS * NPART, 0, rt.stream>>>(part, fpart, G, nblk, tan ? 1 : 0, res);
 	rt.launches++;
 	if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 	if ((ret = RQC_CUDA(cudaMemcpyAsync(d_dgates, res + 1, 16 * (size_t)G * sizeof(double2), cudaMemcpyDeviceToDevice,

@@ -32,7 +32,7 @@ inline int64_t column_count(const Runtime& rt, const CircuitSpec& c)
 	return ((int64_t)1 << c.L) >> (rt.real_pairs ? 1 : 0);
 }
 
-// The target U: either a circuit evaluated on the device (gates, wires) or a
+// The target U: a circuit evaluated on the device (gates, wires), a dense matrix, or a
 // host callback `linear_func` applied to one basis column at a time.
 struct TargetSpec
 {
@@ -42,6 +42,8 @@ struct TargetSpec
 	void* ufunc = nullptr;
 	void* udata = nullptr;
 	int per = 1;   // consecutive gates that are copies of one (brickwall layer)
+	// dense U, row-major 2^L x 2^L (device), instead of gates or a callback
+	const double2* dense = nullptr;
 };
 
 // Device result layout (double2): [0] f, [1 + 16 g + e] dG_g[e], [1 + 16 G + 16 g + e] (H Z)_g[e]

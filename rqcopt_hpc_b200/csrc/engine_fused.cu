@@ -659,24 +659,19 @@ __global__ void __launch_bounds__(NTR, 1) k3_rev(const double2* __restrict__ psi
 
 // Sum raw 8x8 partials over blocks (compensated) and fold them into complex dG, HZ:
 // X[r][c] = (R[2r][2c] - R[2r+1][2c+1]) + i (R[2r][2c+1] + R[2r+1][2c]).
-__global__ void k3_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* __restrict__ fpart,
-                          int nblk_f, int with_hvp, double2* __restrict__ out)
+__global__ void __launch_bounds__(RED_GROUPS * NPART3)
+k3_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* __restrict__ fpart, int nblk_f,
+          int with_hvp, double2* __restrict__ out)
 {
+	__shared__ double red[RED_GROUPS][NPART3];
 	__shared__ double raw[NPART3];
-	const int s = blockIdx.x, t = threadIdx.x;
+	const int s = blockIdx.x, t = threadIdx.x % NPART3;
+	const bool first = threadIdx.x < NPART3;
 	if (s < nslots) {
-		if (t < NPART3) {
-			double sum = 0, comp = 0;
-			for (int b = 0; b < nblk; b++) {
-				const double y = part[((size_t)s * nblk + b) * NPART3 + t] - comp;
-				const double u = sum + y;
-				comp = (u - sum) - y;
-				sum = u;
-			}
-			raw[t] = sum;
-		}
+		const double sum = block_column_sum<NPART3>(part + (size_t)s * nblk * NPART3 + t, nblk, NPART3, red);
+		if (first) raw[t] = sum;
 		__syncthreads();
-		if (t < 32) {
+		if (first && t < 32) {
 			const int which = t >> 4, e = t & 15, r = e >> 2, c = e & 3;
 			if (which == 1 && !with_hvp) return;
 			const double* R = raw + 64 * which;
@@ -684,15 +679,9 @@ __global__ void k3_reduce(const double* __restrict__ part, int nslots, int nblk,
 			const double im = R[(2 * r) * 8 + 2 * c + 1] + R[(2 * r + 1) * 8 + 2 * c];
 			out[1 + 16 * (size_t)(which ? nslots + s : s) + e] = make_double2(re, im);
 		}
-	} else if (t < 2) {
-		double sum = 0, comp = 0;
-		for (int b = 0; b < nblk_f; b++) {
-			const double y = (t == 0 ? fpart[b].x : fpart[b].y) - comp;
-			const double u = sum + y;
-			comp = (u - sum) - y;
-			sum = u;
-		}
-		reinterpret_cast<double*>(out)[t] = sum;
+	} else {
+		const double sum = block_column_sum<NPART3>(reinterpret_cast<const double*>(fpart) + (t & 1), nblk_f, 2, red);
+		if (first && t < 2) reinterpret_cast<double*>(out)[t] = sum;
 	}
 }
 
@@ -2027,31 +2016,22 @@ __global__ void __launch_bounds__(NT7, 2) k7_rev(const float2* __restrict__ psi,
 // Sum the complex64 engine's raw partials over blocks and fold them into complex dG, HZ.
 // Lane (g, t) of an outer-sum MMA holds C[g][2t..2t+1] (v 0,1) and C[g+8][2t..2t+1]
 // (v 2,3): dG raw R[g][2t+i] = v_i, HZ raw R[g][2t+i] = v_{2+i}.
-__global__ void k4_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* __restrict__ fpart,
-                          int nblk_f, int with_hvp, double2* __restrict__ out)
+__global__ void __launch_bounds__(RED_GROUPS * NRAW4)
+k4_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* __restrict__ fpart, int nblk_f,
+          int with_hvp, double2* __restrict__ out)
 {
-	__shared__ double raw[NRAW4];
+	__shared__ double red[RED_GROUPS][NRAW4];
 	__shared__ double R[2][64];
-	const int s = blockIdx.x, t = threadIdx.x;
+	const int s = blockIdx.x, t = threadIdx.x % NRAW4;
+	const bool first = threadIdx.x < NRAW4;
 	if (s < nslots) {
-		for (int v = t; v < NRAW4; v += blockDim.x) {
-			double sum = 0, comp = 0;
-			for (int b = 0; b < nblk; b++) {
-				const double y = part[((size_t)s * nblk + b) * NRAW4 + v] - comp;
-				const double u = sum + y;
-				comp = (u - sum) - y;
-				sum = u;
-			}
-			raw[v] = sum;
+		const double sum = block_column_sum<NRAW4>(part + (size_t)s * nblk * NRAW4 + t, nblk, NRAW4, red);
+		if (first) {
+			const int ln = t >> 2, v = t & 3, gg = ln >> 2, tt = ln & 3;
+			R[v >> 1][gg * 8 + 2 * tt + (v & 1)] = sum;
 		}
 		__syncthreads();
-		if (t < 64) {
-			const int ln = t >> 1, i = t & 1, gg = ln >> 2, tt = ln & 3;
-			R[0][gg * 8 + 2 * tt + i] = raw[ln * 4 + i];
-			R[1][gg * 8 + 2 * tt + i] = raw[ln * 4 + 2 + i];
-		}
-		__syncthreads();
-		if (t < 32) {
+		if (first && t < 32) {
 			const int which = t >> 4, e = t & 15, r = e >> 2, c = e & 3;
 			if (which == 1 && !with_hvp) return;
 			const double* X = R[which];
@@ -2059,15 +2039,9 @@ __global__ void k4_reduce(const double* __restrict__ part, int nslots, int nblk,
 			const double im = X[(2 * r) * 8 + 2 * c + 1] + X[(2 * r + 1) * 8 + 2 * c];
 			out[1 + 16 * (size_t)(which ? nslots + s : s) + e] = make_double2(re, im);
 		}
-	} else if (t < 2) {
-		double sum = 0, comp = 0;
-		for (int b = 0; b < nblk_f; b++) {
-			const double y = (t == 0 ? fpart[b].x : fpart[b].y) - comp;
-			const double u = sum + y;
-			comp = (u - sum) - y;
-			sum = u;
-		}
-		reinterpret_cast<double*>(out)[t] = sum;
+	} else {
+		const double sum = block_column_sum<NRAW4>(reinterpret_cast<const double*>(fpart) + (t & 1), nblk_f, 2, red);
+		if (first && t < 2) reinterpret_cast<double*>(out)[t] = sum;
 	}
 }
 
@@ -2087,32 +2061,34 @@ __global__ void k2_target_from_host(const double2* __restrict__ in, cplx<T>* __r
 	}
 }
 
-// f and per-gate sums over blocks; same record layout as the per-gate engine
-__global__ void k2_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* __restrict__ fpart,
-                          int nblk_f, int with_hvp, double2* __restrict__ out)
+// -conj(U e_c) of a dense U into the interleaved chunk [N][C]
+template <typename T>
+__global__ void k2_target_dense(const double2* __restrict__ u, int L, ColumnSource src, cplx<T>* __restrict__ out, int64_t C)
 {
+	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (C << L); i += (int64_t)gridDim.x * blockDim.x) {
+		const int64_t row = i / C;
+		const double2 v = dense_amp(u, L, src, row, i - row * C);
+		out[i] = mk<T>((T)(-v.x), (T)v.y);
+	}
+}
+
+// f and per-gate sums over blocks; same record layout as the per-gate engine
+__global__ void __launch_bounds__(RED_GROUPS * NPART2)
+k2_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* __restrict__ fpart, int nblk_f,
+          int with_hvp, double2* __restrict__ out)
+{
+	__shared__ double red[RED_GROUPS][NPART2];
 	double* o = reinterpret_cast<double*>(out);
-	const int s = blockIdx.x, t = threadIdx.x;
+	const int s = blockIdx.x, t = threadIdx.x % NPART2;
+	const bool first = threadIdx.x < NPART2;
 	if (s < nslots) {
-		if (t >= NPART2 || (!with_hvp && t >= 32)) return;
-		double sum = 0, comp = 0;
-		for (int b = 0; b < nblk; b++) {
-			const double y = part[((size_t)s * nblk + b) * NPART2 + t] - comp;
-			const double u = sum + y;
-			comp = (u - sum) - y;
-			sum = u;
-		}
+		const double sum = block_column_sum<NPART2>(part + (size_t)s * nblk * NPART2 + t, nblk, NPART2, red);
+		if (!first || (!with_hvp && t >= 32)) return;
 		if (t < 32) o[2 * (1 + 16 * (size_t)s) + t] = sum;
 		else o[2 * (1 + 16 * (size_t)nslots + 16 * (size_t)s) + (t - 32)] = sum;
-	} else if (t < 2) {
-		double sum = 0, comp = 0;
-		for (int b = 0; b < nblk_f; b++) {
-			const double y = (t == 0 ? fpart[b].x : fpart[b].y) - comp;
-			const double u = sum + y;
-			comp = (u - sum) - y;
-			sum = u;
-		}
-		o[t] = sum;
+	} else {
+		const double sum = block_column_sum<NPART2>(reinterpret_cast<const double*>(fpart) + (t & 1), nblk_f, 2, red);
+		if (first && t < 2) o[t] = sum;
 	}
 }
 
@@ -2540,7 +2516,7 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 	const bool tan = mode == EVAL_HVP;
 	const bool host_target = t.ufunc != nullptr;
 	std::vector<Pass> passes = schedule(L, G, c.wires, maxk);
-	std::vector<Pass> tpasses = host_target ? std::vector<Pass>() : schedule(L, t.ngates, t.wires, maxk);
+	std::vector<Pass> tpasses = host_target ? std::vector<Pass>() : schedule(L, t.ngates, t.wires, maxk);   // none of a dense one
 	const int P = (int)passes.size(), Pt = (int)tpasses.size();
 	std::vector<PassGates<T>> pgates(P), tgates(Pt);
 	for (int p = 0; p < P; p++) pgates[p] = pass_gates<T>(passes[p], c.gates, tan ? c.dirs : nullptr);
@@ -2583,10 +2559,13 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 
 	// complex64 reverse passes on the FP32 pipe (k7_rev) or on the TF32 MMA (k5_rev)
 	const bool ffma = !std::is_same<T, double>::value && recon && rt.c64_ffma;
-	const int nblk = recon ? (std::is_same<T, double>::value ? rev_grid6(rt, tan) : (ffma ? rev_grid7(rt, tan) : rev_grid5(rt, tan)))
+	const int full = recon ? (std::is_same<T, double>::value ? rev_grid6(rt, tan) : (ffma ? rev_grid7(rt, tan) : rev_grid5(rt, tan)))
 	                       : rev_grid<T>(rt, tan);
+	// no more blocks (and partials to clear and sum) than tiles
+	const int64_t most_tiles = (N >> std::min(MAXNB, L)) * (C / CW);
+	const int nblk = (int)std::min<int64_t>(full, most_tiles);
 	// blocks of the forward launches that sum f (one FP64 partial each)
-	const int nfb = std::is_same<T, double>::value ? nblk : 2 * rt.num_sms;
+	const int nfb = std::is_same<T, double>::value ? nblk : (int)std::min<int64_t>(2 * rt.num_sms, most_tiles);
 	const int nps = std::is_same<T, double>::value ? NPART3 : (ffma ? NPART2 : NRAW4);   // partial doubles per gate and block
 	const size_t part_doubles = (size_t)G * nblk * nps + 2 * (size_t)nfb;
 	if ((ret = ensure_device(rt.partials, part_doubles * sizeof(double)))) return ret;
@@ -2646,6 +2625,15 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 			rt.launches++;
 			if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 			if ((ret = RQC_CUDA(cudaStreamSynchronize(rt.stream)))) return ret;
+		} else if (t.dense) {
+			ColumnSource s;
+			s.tab = c.columns;
+			s.b0 = b0;
+			s.end = cend;
+			s.pair_half = rt.real_pairs ? N / 2 : 0;
+			k2_target_dense<T><<<rt.num_sms * 8, 256, 0, rt.stream>>>(t.dense, L, s, PHI, C);
+			rt.launches++;
+			if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 		} else {
 			for (int p = 0; p < Pt; p++) {
 				PassGeom g = geom(tpasses[p]);
@@ -2757,11 +2745,11 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 	}
 
 	if (std::is_same<T, double>::value)
-		k3_reduce<<<G + 1, NPART3, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
+		k3_reduce<<<G + 1, RED_GROUPS * NPART3, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
 	else if (ffma)
-		k2_reduce<<<G + 1, NPART2, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
+		k2_reduce<<<G + 1, RED_GROUPS * NPART2, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
 	else
-		k4_reduce<<<G + 1, NRAW4, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
+		k4_reduce<<<G + 1, RED_GROUPS * NRAW4, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
 	rt.launches++;
 	return RQC_CUDA(cudaGetLastError());
 }

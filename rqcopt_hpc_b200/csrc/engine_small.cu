@@ -1,0 +1,520 @@
+// Small evaluations: f, gradient and Hessian-vector product of a circuit whose basis
+// columns fit a block's shared memory, in two launches.
+//
+// An evaluation of a few qubits is bound by latency: as passes (engine_fused.cu) it is a
+// dozen or more launches of which each does a microsecond of work (L = 6, depth 5: 13
+// launches, 165 us on the device, 207 us a call; here 2 launches).  k_small runs the whole
+// evaluation of a column in one block: phi = -conj(U e_b) (target gates, or a column of a
+// dense U), the forward sweep of psi and dpsi, f, and the reverse sweep, with the four states
+// in shared memory throughout.  Four threads share an amplitude group; thread q computes
+// component q of every product and owns row q of the outer sums, so that a group's exchange
+// stays inside a warp and each gate costs one block barrier.
+//
+// The forward sweep leaves the state entering each gate in a scratch array (L2-resident for
+// the sizes this path is for); the reverse sweep brings the next gate's by cp.async into a
+// second pair of tiles while it works on the current one, so that a gate's outer sums
+//   dG += phi (x) psi,   HZ += phi (x) dpsi + dphi (x) psi
+// and its moves phi <- G^T phi, dphi <- G^T dphi + Z^T phi are all independent.  (Rebuilding
+// the states with adjoint gates instead, 12 more products per group and gate, measured the
+// same time at L = 6 and 2.5 times the rounding error.)  The gates of a brickwall layer are
+// copies of one, so the sums add up over the layer.  Sums per block go to fixed slots that
+// k_small_post adds in block order (compensated), so results are deterministic.
+#include "engine_small.h"
+
+#include <string.h>
+#include <algorithm>
+
+#include "rqc_common.cuh"
+
+namespace rqc {
+
+namespace {
+
+constexpr int SMALL_THREADS = 256;     // most threads per block
+constexpr int SMALL_MAX_L = 10;        // six tiles of a column: 96 KB
+constexpr int SMALL_MAX_UNITS = 128;   // gate tables in shared memory: 512 B per unit
+constexpr size_t SMALL_SMEM = 200 * 1024;
+// Amplitude x gate updates up to which an evaluation runs here (512 MB of scratch); beyond,
+// the pass engine has enough work per launch.
+constexpr double SMALL_MAX_WORK = 1 << 24;
+constexpr int SLOT = 64;               // doubles per unit and block: row q of dG (8), of HZ (8)
+
+struct SmallArgs
+{
+	int L, G, per, nunits, Gt;
+	int cb;                  // columns per block
+	int real;                // paired real columns: clear the imaginary parts of the sums
+	int64_t ncols;
+	ColumnSource src;
+	const double2* ug;       // [nunits][16]
+	const double2* uz;
+	const int* bits;         // [2 G] state bits of the gates' wires
+	const double2* tg;       // [Gt][16]
+	const int* tbits;
+	const double2* dense;    // U row-major, or null
+	double* part;            // [blocks][2 + SLOT nunits]
+	double2* states;         // [blocks][G - 1][psi, dpsi][cb 2^L]: the states entering gates 1 .. G-1
+};
+
+// place of amplitude i in shared memory: 16-byte words of a 128-byte line permuted so that
+// group members at strides of 4 and 8 amplitudes fall into different banks
+__device__ __forceinline__ int swz(int i) { return i ^ ((i >> 3) & 7); }
+
+// amplitude (unswizzled) of member m of group gg for wire bits (bi, bj)
+struct Group
+{
+	int lo, hi, bi, bj;
+	__device__ __forceinline__ Group(int i, int j) : lo(min(i, j)), hi(max(i, j)), bi(i), bj(j) {}
+	__device__ __forceinline__ int base(int gg) const
+	{
+		gg = ((gg >> lo) << (lo + 1)) | (gg & ((1 << lo) - 1));
+		return ((gg >> hi) << (hi + 1)) | (gg & ((1 << hi) - 1));
+	}
+	__device__ __forceinline__ int member(int m) const { return ((m >> 1) << bi) | ((m & 1) << bj); }
+};
+
+__device__ __forceinline__ double2 dot4(const double2 a[4], const double2 x[4])
+{
+	double2 s = cmul(a[0], x[0]);
+#pragma unroll
+	for (int m = 1; m < 4; m++) s = cfma(a[m], x[m], s);
+	return s;
+}
+
+__device__ __forceinline__ double2 dot4_acc(const double2 a[4], const double2 x[4], double2 s)
+{
+#pragma unroll
+	for (int m = 0; m < 4; m++) s = cfma(a[m], x[m], s);
+	return s;
+}
+
+// sums of v[k] over the lanes that share q = lane & 3: lane l gets those of entries e, e + 1,
+// e = 8 (l >> 4 & 1) + 4 (l >> 3 & 1) + 2 (l >> 2 & 1), in v[0], v[1]
+__device__ __forceinline__ void row_sums(double (&v)[16], int lane)
+{
+#pragma unroll
+	for (int o = 16, h = 8; o >= 4; o >>= 1, h >>= 1) {
+		const bool up = (lane & o) != 0;
+#pragma unroll
+		for (int k = 0; k < h; k++) {
+			const double send = up ? v[k] : v[k + h];
+			const double keep = up ? v[k + h] : v[k];
+			v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+		}
+	}
+}
+
+__device__ __forceinline__ void copy16(double2* smem, const double2* gmem)
+{
+	const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem) : "memory");
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
+{
+	constexpr bool TAN = MODE == EVAL_HVP;
+	extern __shared__ __align__(16) double2 sm[];
+	__shared__ double red[2][SMALL_THREADS / 32][SLOT];
+	__shared__ double fred[2][SMALL_THREADS / 32];
+	const int L = a.L, N = 1 << L, T = a.cb << L;
+	double2* Psi = sm;                       // [2]: the reverse sweep alternates
+	double2* Phi = sm + 2 * T;
+	double2* dPsi = TAN ? sm + 3 * T : nullptr;
+	double2* dPhi = TAN ? sm + 5 * T : nullptr;
+	double2* tab = sm + (TAN ? 6 : 3) * T;   // per unit: G, and for HVPs Z
+	constexpr int US = TAN ? 32 : 16;
+	constexpr int NS = TAN ? 2 : 1;
+	double2* states = MODE == EVAL_F ? nullptr : a.states + (size_t)blockIdx.x * (a.G - 1) * NS * T;
+	const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
+	const int q = tid & 3;
+	const int lg = L - 2, ntasks = a.cb << L;   // four threads per group: one task per amplitude
+	const int64_t col0 = (int64_t)blockIdx.x * a.cb;
+	double* part = a.part + (size_t)blockIdx.x * (2 + SLOT * (size_t)a.nunits);
+
+	for (int e = tid; e < 16 * a.nunits; e += nt) {
+		const int u = e >> 4, w = e & 15;
+		tab[u * US + w] = a.ug[e];
+		if (TAN) tab[u * US + 16 + w] = a.uz[e];
+	}
+	ColumnSource wsrc = a.src;
+	wsrc.weighted = 1;
+	for (int e = tid; e < T; e += nt) {
+		const int c = e >> L, row = e & (N - 1), p = swz(e);
+		Psi[p] = basis_amp<double>(a.src, row, col0 + c);
+		if (TAN) {
+			dPsi[p] = make_double2(0, 0);
+			dPhi[p] = make_double2(0, 0);
+		}
+		if (a.dense) {
+			Phi[p] = cneg_conj(dense_amp(a.dense, L, a.src, row, col0 + c));
+		} else {
+			Phi[p] = cneg_conj(basis_amp<double>(wsrc, row, col0 + c));
+		}
+	}
+	__syncthreads();
+	// phi = -conj(U e): the conjugate gates on the negated conjugate column
+	if (!a.dense) {
+		for (int k = 0; k < a.Gt; k++) {
+			const Group gr(a.tbits[2 * k], a.tbits[2 * k + 1]);
+			double2 g[4];
+#pragma unroll
+			for (int m = 0; m < 4; m++) {
+				g[m] = a.tg[16 * k + 4 * q + m];
+				g[m].y = -g[m].y;
+			}
+			for (int t = tid; t < ntasks; t += nt) {
+				const int gi = t >> 2, at = ((gi >> lg) << L) + gr.base(gi & ((1 << lg) - 1));
+				double2 x[4];
+#pragma unroll
+				for (int m = 0; m < 4; m++) x[m] = Phi[swz(at | gr.member(m))];
+				const double2 y = dot4(g, x);
+				__syncwarp();
+				Phi[swz(at | gr.member(q))] = y;
+			}
+			__syncthreads();
+		}
+	}
+	__syncthreads();
+
+	// forward
+	for (int k = 0; k < a.G; k++) {
+		const Group gr(a.bits[2 * k], a.bits[2 * k + 1]);
+		const double2* gt = tab + (k / a.per) * US;
+		if (MODE != EVAL_F && k > 0) {
+			double2* st = states + (size_t)(k - 1) * NS * T;
+			for (int e = tid; e < T; e += nt) {
+				st[e] = Psi[e];
+				if (TAN) st[T + e] = dPsi[e];
+			}
+		}
+		double2 g[4], z[4];
+#pragma unroll
+		for (int m = 0; m < 4; m++) {
+			g[m] = gt[4 * q + m];
+			if (TAN) z[m] = gt[16 + 4 * q + m];
+		}
+		for (int t = tid; t < ntasks; t += nt) {
+			const int gi = t >> 2, at = ((gi >> lg) << L) + gr.base(gi & ((1 << lg) - 1));
+			double2 x[4], dx[4];
+#pragma unroll
+			for (int m = 0; m < 4; m++) {
+				const int p = swz(at | gr.member(m));
+				x[m] = Psi[p];
+				if (TAN) dx[m] = dPsi[p];
+			}
+			const double2 y = dot4(g, x);
+			double2 dy;
+			if (TAN) dy = dot4_acc(z, x, dot4(g, dx));
+			__syncwarp();
+			const int p = swz(at | gr.member(q));
+			Psi[p] = y;
+			if (TAN) dPsi[p] = dy;
+		}
+		__syncthreads();
+	}
+
+	// f = phi . psi
+	{
+		double fx = 0, fy = 0;
+		for (int e = tid; e < T; e += nt) {
+			const double2 p = Phi[e], v = Psi[e];
+			fx += p.x * v.x - p.y * v.y;
+			fy += p.x * v.y + p.y * v.x;
+		}
+		fx = warp_sum(fx);
+		fy = warp_sum(fy);
+		if (lane == 0) { fred[0][warp] = fx; fred[1][warp] = fy; }
+		__syncthreads();
+		if (tid < 2) {
+			double s = 0;
+			for (int w = 0; w < nwarps; w++) s += fred[tid][w];
+			part[tid] = s;
+		}
+	}
+	if (MODE == EVAL_F) return;
+
+	// the state entering gate k into pair b of the psi tiles
+	auto fetch = [&](int k, int b) {
+		double2* p = Psi + b * T;
+		double2* d = TAN ? dPsi + b * T : nullptr;
+		if (k > 0) {
+			const double2* st = states + (size_t)(k - 1) * NS * T;
+			for (int e = tid; e < T; e += nt) {
+				copy16(p + e, st + e);
+				if (TAN) copy16(d + e, st + T + e);
+			}
+		} else if (k == 0) {
+			for (int e = tid; e < T; e += nt) {
+				p[swz(e)] = basis_amp<double>(a.src, e & (N - 1), col0 + (e >> L));
+				if (TAN) d[e] = make_double2(0, 0);
+			}
+		}
+		asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
+	auto arrived = [] { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); };
+
+	// reverse
+	double acc[16];
+#pragma unroll
+	for (int e = 0; e < 16; e++) acc[e] = 0;
+	fetch(a.G - 1, 1);
+	arrived();
+	__syncthreads();
+	for (int k = a.G - 1, b = 1; k >= 0; k--, b ^= 1) {
+		fetch(k - 1, b ^ 1);   // that pair's last readers are behind the barrier
+		const double2* X = Psi + b * T;
+		const double2* dX = TAN ? dPsi + b * T : nullptr;
+		const Group gr(a.bits[2 * k], a.bits[2 * k + 1]);
+		const int u = k / a.per;
+		const double2* gt = tab + u * US;
+		double2 g[4], z[4];   // column q of G and Z
+#pragma unroll
+		for (int m = 0; m < 4; m++) {
+			g[m] = gt[4 * m + q];
+			if (TAN) z[m] = gt[16 + 4 * m + q];
+		}
+		for (int t = tid; t < ntasks; t += nt) {
+			const int gi = t >> 2, at = ((gi >> lg) << L) + gr.base(gi & ((1 << lg) - 1));
+			const int own = swz(at | gr.member(q));
+			double2 x[4], p[4], dx[4], dp[4];
+#pragma unroll
+			for (int m = 0; m < 4; m++) {
+				const int s = swz(at | gr.member(m));
+				x[m] = X[s];
+				p[m] = Phi[s];
+				if (TAN) {
+					dx[m] = dX[s];
+					dp[m] = dPhi[s];
+				}
+			}
+			const double2 pq = Phi[own];
+			double2 dpq;
+			if (TAN) dpq = dPhi[own];
+#pragma unroll
+			for (int c = 0; c < 4; c++) {
+				const double2 v = cfma(pq, x[c], make_double2(acc[2 * c], acc[2 * c + 1]));
+				acc[2 * c] = v.x;
+				acc[2 * c + 1] = v.y;
+				if (TAN) {
+					double2 h = make_double2(acc[8 + 2 * c], acc[9 + 2 * c]);
+					h = cfma(pq, dx[c], h);
+					h = cfma(dpq, x[c], h);
+					acc[8 + 2 * c] = h.x;
+					acc[9 + 2 * c] = h.y;
+				}
+			}
+			const double2 yp = dot4(g, p);
+			double2 ydp;
+			if (TAN) ydp = dot4_acc(z, p, dot4(g, dp));
+			__syncwarp();
+			Phi[own] = yp;
+			if (TAN) dPhi[own] = ydp;
+		}
+		const bool done = k % a.per == 0;   // the unit's last gate of the sweep
+		if (done) {
+			row_sums(acc, lane);
+			const int e = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2;
+			red[u & 1][warp][16 * q + e] = acc[0];
+			red[u & 1][warp][16 * q + e + 1] = acc[1];
+#pragma unroll
+			for (int i = 0; i < 16; i++) acc[i] = 0;
+		}
+		arrived();
+		__syncthreads();
+		// the other buffer of red is written before the next barrier at the earliest
+		if (done && tid < 32) {
+			for (int e = tid; e < SLOT; e += 32) {
+				double s = 0;
+				for (int v = 0; v < nwarps; v++) s += red[u & 1][v][e];
+				part[2 + SLOT * (size_t)u + e] = s;
+			}
+		}
+	}
+}
+
+// Unit u (one block each): the sums dG, HZ over blocks and their projection (src/target.c:410-430),
+// a thread per matrix entry; the last block sums f.
+__global__ void __launch_bounds__(RED_GROUPS * SLOT) k_small_post(SmallArgs a, int nblk, int mode, SmallOut out)
+{
+	__shared__ double red[RED_GROUPS][SLOT];
+	__shared__ double raw[SLOT];
+	__shared__ double2 V[16], Z[16], D[16], H[16], A[16], B[16], X[16];
+	const int u = blockIdx.x, t = threadIdx.x;
+	const size_t stride = 2 + SLOT * (size_t)a.nunits;
+	if (u == a.nunits) {
+		const double s = block_column_sum<SLOT>(a.part + (t & 1), nblk, stride, red);
+		if (t < 2 && out.f) reinterpret_cast<double*>(out.f)[t] = a.real && t == 1 ? 0.0 : s;
+		return;
+	}
+	if (mode == EVAL_F) return;
+	const bool tan = mode == EVAL_HVP;
+	const double s = block_column_sum<SLOT>(a.part + 2 + SLOT * (size_t)u + (t % SLOT), nblk, stride, red);
+	if (t < SLOT) raw[t] = a.real && (t & 1) ? 0.0 : s;
+	if (t < 16) {
+		V[t] = a.ug[16 * u + t];
+		Z[t] = tan ? a.uz[16 * u + t] : make_double2(0, 0);
+	}
+	__syncthreads();
+	if (t >= 16) return;
+	const unsigned mask = 0xffffu;
+	const int r = t >> 2, c = t & 3;
+	auto conj = [](double2 v) { return make_double2(v.x, -v.y); };
+	const double2 dg = make_double2(raw[16 * r + 2 * c], raw[16 * r + 2 * c + 1]);
+	const double2 hz = make_double2(raw[16 * r + 8 + 2 * c], raw[16 * r + 9 + 2 * c]);
+	if (out.dunits) out.dunits[16 * u + t] = dg;
+	if (out.hunits && tan) out.hunits[16 * u + t] = hz;
+	D[t] = conj(dg);
+	__syncwarp(mask);
+	// x = Re + Im of the anti-Hermitian part of V^+ M
+	auto tangent = [&](const double2* M, double* x) {
+		double2 w = make_double2(0, 0);
+		for (int m = 0; m < 4; m++) w = cfma(conj(V[4 * m + r]), M[4 * m + c], w);
+		X[t] = w;
+		__syncwarp(mask);
+		const double2 wt = X[4 * c + r];
+		if (x) x[16 * u + t] = 0.5 * (w.x - wt.x) + 0.5 * (w.y + wt.y);
+		__syncwarp(mask);
+	};
+	if (out.grad) tangent(D, out.grad);
+	if (!tan || !out.hvp) return;
+	// minus (Z D^+ V + V D^+ Z) / 2
+	double2 av = make_double2(0, 0), bz = make_double2(0, 0);
+	for (int m = 0; m < 4; m++) {
+		av = cfma(conj(D[4 * m + r]), V[4 * m + c], av);
+		bz = cfma(conj(D[4 * m + r]), Z[4 * m + c], bz);
+	}
+	A[t] = av;
+	B[t] = bz;
+	__syncwarp(mask);
+	double2 pd = make_double2(0, 0);
+	for (int i = 0; i < 4; i++) {
+		pd = cfma(Z[4 * r + i], A[4 * i + c], pd);
+		pd = cfma(V[4 * r + i], B[4 * i + c], pd);
+	}
+	H[t] = make_double2(hz.x - 0.5 * pd.x, -hz.y - 0.5 * pd.y);
+	__syncwarp(mask);
+	tangent(H, out.hvp);
+}
+
+// columns per block: enough groups to fill a warp
+int columns_per_block(int L) { return L >= 5 ? 1 : 32 >> L; }
+
+size_t small_smem(int L, int nunits, bool tan)
+{
+	return ((tan ? 6 : 3) * ((size_t)columns_per_block(L) << L) + (size_t)nunits * (tan ? 32 : 16)) * sizeof(double2);
+}
+
+template <int MODE>
+int launch_small(Runtime& rt, const SmallArgs& a, int blocks)
+{
+	static bool ready = false;
+	if (!ready) {
+		if (int e = RQC_CUDA(cudaFuncSetAttribute(k_small<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM)))
+			return e;
+		ready = true;
+	}
+	const int threads = std::max(32, std::min(SMALL_THREADS, a.cb << a.L));
+	cudaEvent_t ev;
+	launch_begin(rt, KC_FUSED, &ev);
+	k_small<MODE><<<blocks, threads, small_smem(a.L, a.nunits, MODE == EVAL_HVP), rt.stream>>>(a);
+	launch_end(rt, KC_FUSED, ev);
+	return RQC_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+bool SmallEval::fits(const Runtime& rt, const Problem& pb, const TargetHolder& th, int64_t ncols)
+{
+	if (rt.pin_gpp || rt.pin_chunk || rt.pin_recon || rt.col_begin != 0 || rt.col_end != 0) return false;
+	if (pb.L < 2 || pb.L > SMALL_MAX_L || pb.nunits > SMALL_MAX_UNITS || ncols < 1) return false;
+	if (th.spec.ufunc || (!th.spec.dense && th.spec.ngates < 1)) return false;
+	if ((double)ncols * (double)(1 << pb.L) * (pb.G + th.spec.ngates) >= SMALL_MAX_WORK) return false;
+	return small_smem(pb.L, pb.nunits, true) <= SMALL_SMEM;
+}
+
+int SmallEval::prepare(Runtime& rt, const Problem& pb, const TargetHolder& th, const std::vector<BasisCol>& cols,
+                       const double2* ugates, const double2* udirs)
+{
+	const int64_t N = (int64_t)1 << pb.L;
+	L_ = pb.L;
+	G_ = pb.G;
+	nunits_ = pb.nunits;
+	per_ = pb.per;
+	Gt_ = th.spec.dense ? 0 : th.spec.ngates;
+	src_ = ColumnSource{};
+	if (cols.empty()) {
+		const int64_t all = rt.real_pairs ? N / 2 : N;
+		src_.end = all;
+		src_.pair_half = rt.real_pairs ? N / 2 : 0;
+	} else {
+		src_.end = (int64_t)cols.size();
+	}
+	ncols_ = src_.end - src_.b0;
+	// one staged copy: unit gates | directions | target gates | columns | wire bits
+	const size_t nug = ugates ? 16 * (size_t)nunits_ : 0, nuz = udirs ? 16 * (size_t)nunits_ : 0, ntg = 16 * (size_t)Gt_;
+	const size_t gates_b = (nug + nuz + ntg) * sizeof(double2), cols_b = cols.size() * sizeof(BasisCol);
+	const size_t bytes = gates_b + cols_b + 2 * (size_t)(G_ + Gt_) * sizeof(int);
+	int ret = ensure_host_pinned(rt.small_host, bytes);
+	if (!ret) ret = ensure_device(rt.small_dev, bytes);
+	if (ret) return ret;
+	char* h = static_cast<char*>(rt.small_host.ptr);
+	double2* hg = reinterpret_cast<double2*>(h);
+	if (nug) memcpy(hg, ugates, nug * sizeof(double2));
+	if (nuz) memcpy(hg + nug, udirs, nuz * sizeof(double2));
+	if (ntg) memcpy(hg + nug + nuz, th.spec.gates, ntg * sizeof(double2));
+	if (cols_b) memcpy(h + gates_b, cols.data(), cols_b);
+	int* hb = reinterpret_cast<int*>(h + gates_b + cols_b);
+	for (int k = 0; k < 2 * G_; k++) hb[k] = L_ - 1 - pb.wires[k];
+	for (int k = 0; k < 2 * Gt_; k++) hb[2 * G_ + k] = L_ - 1 - th.wires[k];
+	if ((ret = RQC_CUDA(cudaMemcpyAsync(rt.small_dev.ptr, h, bytes, cudaMemcpyHostToDevice, rt.stream)))) return ret;
+	const char* d = static_cast<const char*>(rt.small_dev.ptr);
+	const double2* dg = reinterpret_cast<const double2*>(d);
+	ug_ = nug ? dg : nullptr;
+	uz_ = nuz ? dg + nug : nullptr;
+	tg_ = dg + nug + nuz;
+	if (!cols.empty()) src_.tab = reinterpret_cast<const BasisCol*>(d + gates_b);
+	bits_ = reinterpret_cast<const int*>(d + gates_b + cols_b);
+	tbits_ = bits_ + 2 * G_;
+	dense_ = th.spec.dense;
+	return OK;
+}
+
+int SmallEval::eval(Runtime& rt, int mode, const double2* ugates, const double2* udirs, const SmallOut& out)
+{
+	SmallArgs a;
+	a.L = L_;
+	a.G = G_;
+	a.per = per_;
+	a.nunits = nunits_;
+	a.Gt = Gt_;
+	a.cb = columns_per_block(L_);
+	a.real = rt.real_pairs;
+	a.ncols = ncols_;
+	a.src = src_;
+	a.ug = ugates ? ugates : ug_;
+	a.uz = udirs ? udirs : uz_;
+	a.bits = bits_;
+	a.tg = tg_;
+	a.tbits = tbits_;
+	a.dense = dense_;
+	const int blocks = (int)((ncols_ + a.cb - 1) / a.cb);
+	int ret = ensure_device(rt.partials, (size_t)blocks * (2 + SLOT * (size_t)nunits_) * sizeof(double));
+	if (ret) return ret;
+	a.part = static_cast<double*>(rt.partials.ptr);
+	if (mode != EVAL_F) {
+		const size_t states = (size_t)blocks * (G_ - 1) * (mode == EVAL_HVP ? 2 : 1) * ((size_t)a.cb << L_);
+		if ((ret = ensure_device(rt.work, states * sizeof(double2)))) return ret;
+	}
+	a.states = static_cast<double2*>(rt.work.ptr);
+	if (mode == EVAL_HVP) ret = launch_small<EVAL_HVP>(rt, a, blocks);
+	else if (mode == EVAL_GRAD) ret = launch_small<EVAL_GRAD>(rt, a, blocks);
+	else ret = launch_small<EVAL_F>(rt, a, blocks);
+	if (ret) return ret;
+	k_small_post<<<nunits_ + 1, RED_GROUPS * SLOT, 0, rt.stream>>>(a, blocks, mode, out);
+	rt.launches++;
+	rt.last_choice = {rt.gates_per_pass, rt.column_chunk, rt.recon_c128, rt.c64_ffma, 0.0, 0};
+	return RQC_CUDA(cudaGetLastError());
+}
+
+}  // namespace rqc

@@ -587,20 +587,19 @@ __global__ void k_hmirror(int m, double* __restrict__ H)
 }
 
 // Truncated CG with a dense Hessian (src/trust_region.c:83-141): the matrix-vector
-// product by rows in parallel, every other step by thread 0 with sequential FP64
-// arithmetic (trust_region.cuh).
+// product by rows in parallel, the other steps with dot products in index order
+// (trust_region.cuh).
 __global__ void __launch_bounds__(HT) k_tcg_hmat(int n, const double* __restrict__ grad, const double* __restrict__ hess,
                                                  double radius, int maxiter, double abstol, double reltol, double* r,
                                                  double* d, double* hd, double* z, int* status)
 {
 	__shared__ TcgState st;
-	if (threadIdx.x == 0) tcg_init_dev(n, grad, r, d, z, &st, radius, abstol, reltol);
-	__syncthreads();
+	__shared__ BlockDots dots;
+	tcg_init_blk(n, grad, r, d, z, &st, radius, abstol, reltol, dots);
 	for (int it = 0; it < maxiter; it++) {
 		for (int row = threadIdx.x; row < n; row += blockDim.x) hd[row] = dot_seq(n, hess + (size_t)row * n, d);
 		__syncthreads();
-		if (threadIdx.x == 0) tcg_step_dev(n, d, hd, z, r, &st);
-		__syncthreads();
+		tcg_step_blk(n, d, hd, z, r, &st, dots);
 		if (st.status != TCG_CONTINUE) break;
 	}
 	if (threadIdx.x == 0) status[0] = st.status == TCG_BOUNDARY ? 1 : 0;

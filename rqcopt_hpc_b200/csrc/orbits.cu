@@ -73,13 +73,13 @@ std::vector<BasisCol> orbit_columns(int L, const std::vector<int>& sym)
 	// image of a basis state under relabelling g, a byte of it at a time (wire q is bit L-1-q)
 	std::vector<int32_t> table((size_t)ng * nbytes * 256, 0);
 	for (int g = 0; g < ng; g++)
-		for (int k = 0; k < nbytes; k++)
-			for (int v = 0; v < 256; v++) {
-				int32_t r = 0;
-				for (int b = 0; b < 8 && 8 * k + b < L; b++)
-					if ((v >> b) & 1) r |= (int32_t)1 << (L - 1 - sym[(size_t)g * L + (L - 1 - (8 * k + b))]);
-				table[((size_t)g * nbytes + k) * 256 + v] = r;
+		for (int k = 0; k < nbytes; k++) {
+			int32_t* t = &table[((size_t)g * nbytes + k) * 256];
+			for (int b = 0; b < 8 && 8 * k + b < L; b++) {
+				const int32_t image = (int32_t)1 << (L - 1 - sym[(size_t)g * L + (L - 1 - (8 * k + b))]);
+				for (int v = 0; v < 1 << b; v++) t[(1 << b) + v] = t[v] | image;
 			}
+		}
 	std::vector<BasisCol> out;
 	for (int32_t b = 0; b < (int32_t)1 << L; b++) {
 		int fixed = 1;

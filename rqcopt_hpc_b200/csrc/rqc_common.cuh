@@ -78,6 +78,27 @@ __device__ __forceinline__ cplx<T> basis_amp(const ColumnSource& s, int64_t row,
 	return v;
 }
 
+// amplitude `row` of U applied to (weighted) column c of the chunk, U a dense row-major 2^L x 2^L
+// matrix
+__device__ __forceinline__ double2 dense_amp(const double2* __restrict__ u, int L, const ColumnSource& s, int64_t row,
+                                             int64_t c)
+{
+	const int64_t k = s.b0 + c;
+	double2 v = make_double2(0, 0);
+	if (k >= s.end) return v;
+	const int64_t re = s.tab ? s.tab[k].re : k;
+	const int64_t im = s.tab ? s.tab[k].im : (s.pair_half ? k + s.pair_half : -1);
+	const double wre = s.tab ? s.tab[k].wre : 1.0, wim = s.tab ? s.tab[k].wim : 1.0;
+	const double2 x = u[(row << L) + re];
+	v = make_double2(wre * x.x, wre * x.y);
+	if (im >= 0) {
+		const double2 y = u[(row << L) + im];
+		v.x -= wim * y.y;
+		v.y += wim * y.x;
+	}
+	return v;
+}
+
 // ---------------------------------------------------------------- amplitude groups
 
 // Wire pair of a gate acting on an L-qubit register: bit positions of the two
@@ -196,6 +217,37 @@ __device__ __forceinline__ double warp_sum(double v)
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
 	return v;
+}
+
+// Compensated sum of p[b * stride], b = 0 .. n-1, by the threads of a block: the block's
+// RED_GROUPS groups of NV threads take every RED_GROUPS-th term each (a serial chain over a
+// few hundred blocks' partials took 50-60 us; eight chains an eighth of it), then thread v < NV
+// of group 0 adds the groups' sums in order and gets the result of its own p.
+constexpr int RED_GROUPS = 8;
+
+template <int NV>
+__device__ __forceinline__ double block_column_sum(const double* __restrict__ p, int n, size_t stride,
+                                                   double (*red)[NV])
+{
+	const int v = threadIdx.x % NV, g = threadIdx.x / NV;
+	double sum = 0, comp = 0;
+	for (int b = g; b < n; b += RED_GROUPS) {
+		const double y = p[(size_t)b * stride] - comp;
+		const double u = sum + y;
+		comp = (u - sum) - y;
+		sum = u;
+	}
+	red[g][v] = sum;
+	__syncthreads();
+	if (g != 0) return 0;
+	comp = 0;
+	for (int k = 1; k < RED_GROUPS; k++) {
+		const double y = red[k][v] - comp;
+		const double u = sum + y;
+		comp = (u - sum) - y;
+		sum = u;
+	}
+	return sum;
 }
 
 }  // namespace rqc

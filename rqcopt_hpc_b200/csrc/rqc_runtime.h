@@ -39,6 +39,10 @@ struct Runtime
 	Buffer stage[4];      // staging of host statevectors
 	Buffer arrays;        // statevector arrays and gate-input caches of the full-Hessian calls
 	Buffer columns;       // column list of the current call (orbits.h)
+	Buffer dense;         // dense target of the current call
+	Buffer small_dev;     // inputs of the current call's small evaluations (engine_small.cu), and
+	Buffer small_host;    // their pinned staging
+	Buffer out_host;      // pinned results of the current call
 	Buffer hpin;          // pinned host scratch
 	Buffer status;        // device status word of kernels with bounded waits (non-zero: a wait gave up)
 

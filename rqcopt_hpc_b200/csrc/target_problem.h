@@ -34,13 +34,22 @@ struct TargetHolder
 	std::vector<double2> gates;
 	std::vector<int> wires;
 	TargetSpec spec;
+	// dense target (rqcopt_dense_ufunc): host matrix, to be laid out on the device
+	const double2* dense_host = nullptr;
+	int dense_L = 0;
 	bool set(linear_func ufunc, void* udata, int L);
+	// Copies a dense target to the device for the evaluations of this call (up to 1 GiB; larger
+	// ones stay a host callback, one column at a time).
+	int to_device(Runtime& rt);
 };
 
 // Sum over the orbits of the wire relabellings that circuit and target share, instead of
 // over all basis states (orbits.h): a brickwall against a device-native brickwall whose
 // results are per-layer sums, over all columns.  Sets *columns and *ncolumns where there is
-// such a symmetry; the list lies in rt.columns (held until the next call).
+// such a symmetry; the list lies in rt.columns (held until the next call).  orbits_of: the list
+// itself, empty where there is none.
+int upload_columns(Runtime& rt, const std::vector<BasisCol>& cols, const BasisCol** columns, int64_t* ncolumns);
+std::vector<BasisCol> orbits_of(const Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th);
 int use_orbits(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th, const BasisCol** columns,
                int64_t* ncolumns);
 // The same for the block encoding of a brickwall on L/2 qubits (the target) by one on L: the
@@ -52,7 +61,7 @@ int use_orbits_blockenc(Runtime& rt, int L, int nlayers, const int* wires, const
 int post_launch(Runtime& rt, const double2* d_res, const Problem& pb, const double2* d_ugates, const double2* d_udirs,
                 int with_hvp, double2* d_dunits, double2* d_hunits, double* d_grad, double* d_hvp);
 
-int run_target(const Problem& pb, const TargetHolder& th, int mode, numeric* fval, struct mat4x4* dunits,
+int run_target(const Problem& pb, TargetHolder& th, int mode, numeric* fval, struct mat4x4* dunits,
                struct mat4x4* hunits, double* grad_vec, double* hvp_vec);
 
 }  // namespace rqc
