@@ -82,15 +82,16 @@ __device__ __forceinline__ double2 shfl2(double2 v, int src)
 	return c_(__shfl_sync(0xffffffffu, v.x, src, 16), __shfl_sync(0xffffffffu, v.y, src, 16));
 }
 
-// inverse of the 4x4 matrix whose entry (r, c) lane 4 r + c of a 16-lane group holds: m4_inverse
-// (manifold.cuh), an entry per lane
+// inverse of the 4x4 matrix whose entry (r, c) lane 4 r + c of a 16-lane group holds: the
+// Gauss-Jordan steps of m4_inverse (manifold.cuh), an entry per lane, with one reciprocal per
+// pivot in place of three quotients and the pivot chosen by the squared modulus
 __device__ inline double2 group_inverse(double2 m, int r, int c)
 {
 	double2 v = c_(r == c ? 1.0 : 0.0, 0);
 #pragma unroll
 	for (int k = 0; k < 4; k++) {
 		// pivot row: the first largest entry of column k at or below row k
-		const double mine = c_abs(m);
+		const double mine = m.x * m.x + m.y * m.y;
 		int piv = k;
 		double best = __shfl_sync(0xffffffffu, mine, 5 * k, 16);
 #pragma unroll
@@ -102,10 +103,12 @@ __device__ inline double2 group_inverse(double2 m, int r, int c)
 		m = shfl2(m, from);
 		v = shfl2(v, from);
 		const double2 d = shfl2(m, 5 * k), mk = shfl2(m, 4 * k + c), vk = shfl2(v, 4 * k + c);
-		const double2 s = c_div(shfl2(m, 4 * r + k), d);
+		const double scale = 1.0 / (d.x * d.x + d.y * d.y);
+		const double2 inv = c_(d.x * scale, -d.y * scale);
+		const double2 s = c_mul(shfl2(m, 4 * r + k), inv);
 		if (r == k) {
-			m = c == k ? c_(1, 0) : c > k ? c_div(m, d) : m;
-			v = c_div(v, d);
+			m = c == k ? c_(1, 0) : c > k ? c_mul(m, inv) : m;
+			v = c_mul(v, inv);
 		} else {
 			m = c == k ? c_(0, 0) : c > k ? c_sub(m, c_mul(s, mk)) : m;
 			v = c_sub(v, c_mul(s, vk));
@@ -136,11 +139,12 @@ __global__ void k_retract(int nunits, const double2* x, const double* eta, doubl
 		const double2 inv = group_inverse(y, r, c);
 		const double2 t = c_conj(shfl2(inv, 4 * c + r));
 		const double2 next = c_scale(c_add(y, t), 0.5);
-		double d = c_abs(c_sub(next, t));
+		const double2 diff = c_sub(next, t);
+		double d = diff.x * diff.x + diff.y * diff.y;
 #pragma unroll
 		for (int o = 8; o > 0; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o, 16));
 		if (!done) y = next;
-		done = done || (k >= 4 && d < 1e-14);
+		done = done || (k >= 4 && d < 1e-28);
 		if (__all_sync(0xffffffffu, done)) break;
 	}
 	if ((i >> 4) < nunits) xs[i] = y;

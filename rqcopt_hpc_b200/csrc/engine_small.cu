@@ -48,9 +48,8 @@ struct SmallArgs
 	ColumnSource src;
 	const double2* ug;       // [nunits][16]
 	const double2* uz;
-	const int* bits;         // [2 G] state bits of the gates' wires
+	const int* bits;         // [2 (G + Gt)] state bits of the gates' wires, circuit then target
 	const double2* tg;       // [Gt][16]
-	const int* tbits;
 	const double2* dense;    // U row-major, or null
 	double* part;            // [blocks][2 + SLOT nunits]
 	double2* states;         // [blocks][G - 1][psi, dpsi][cb 2^L]: the states entering gates 1 .. G-1
@@ -60,32 +59,41 @@ struct SmallArgs
 // group members at strides of 4 and 8 amplitudes fall into different banks
 __device__ __forceinline__ int swz(int i) { return i ^ ((i >> 3) & 7); }
 
-// amplitude (unswizzled) of member m of group gg for wire bits (bi, bj)
+// The groups of one gate.  swz is linear over XOR, so a member's place is the group's base
+// place XOR the member's own, both fixed per gate and per task.
 struct Group
 {
-	int lo, hi, bi, bj;
-	__device__ __forceinline__ Group(int i, int j) : lo(min(i, j)), hi(max(i, j)), bi(i), bj(j) {}
-	__device__ __forceinline__ int base(int gg) const
+	int lo, hi, m[4];
+	__device__ __forceinline__ explicit Group(int2 w) : lo(min(w.x, w.y)), hi(max(w.x, w.y))
 	{
-		gg = ((gg >> lo) << (lo + 1)) | (gg & ((1 << lo) - 1));
-		return ((gg >> hi) << (hi + 1)) | (gg & ((1 << hi) - 1));
+		m[0] = 0;
+		m[1] = swz(1 << w.y);
+		m[2] = swz(1 << w.x);
+		m[3] = m[1] ^ m[2];
 	}
-	__device__ __forceinline__ int member(int m) const { return ((m >> 1) << bi) | ((m & 1) << bj); }
+	// place of member 0 of group gi (over all columns of the block)
+	__device__ __forceinline__ int base(int gi, int lg, int L) const
+	{
+		int g = gi & ((1 << lg) - 1);
+		g = ((g >> lo) << (lo + 1)) | (g & ((1 << lo) - 1));
+		g = ((g >> hi) << (hi + 1)) | (g & ((1 << hi) - 1));
+		return swz(((gi >> lg) << L) | g);
+	}
 };
 
+// sum of a[m] x[m]: the two products of each component in chains of their own (a single warp
+// waits for each dependent FMA)
 __device__ __forceinline__ double2 dot4(const double2 a[4], const double2 x[4])
 {
-	double2 s = cmul(a[0], x[0]);
+	double rr = a[0].x * x[0].x, ii = a[0].y * x[0].y, ri = a[0].x * x[0].y, ir = a[0].y * x[0].x;
 #pragma unroll
-	for (int m = 1; m < 4; m++) s = cfma(a[m], x[m], s);
-	return s;
-}
-
-__device__ __forceinline__ double2 dot4_acc(const double2 a[4], const double2 x[4], double2 s)
-{
-#pragma unroll
-	for (int m = 0; m < 4; m++) s = cfma(a[m], x[m], s);
-	return s;
+	for (int m = 1; m < 4; m++) {
+		rr = fma(a[m].x, x[m].x, rr);
+		ii = fma(a[m].y, x[m].y, ii);
+		ri = fma(a[m].x, x[m].y, ri);
+		ir = fma(a[m].y, x[m].x, ir);
+	}
+	return make_double2(rr - ii, ri + ir);
 }
 
 // sums of v[k] over the lanes that share q = lane & 3: lane l gets those of entries e, e + 1,
@@ -124,6 +132,9 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 	double2* dPhi = TAN ? sm + 5 * T : nullptr;
 	double2* tab = sm + (TAN ? 6 : 3) * T;   // per unit: G, and for HVPs Z
 	constexpr int US = TAN ? 32 : 16;
+	double2* ttab = tab + US * a.nunits;     // the target's gates, conjugated
+	int2* bits = reinterpret_cast<int2*>(ttab + 16 * a.Gt);
+	int2* tbits = bits + a.G;
 	constexpr int NS = TAN ? 2 : 1;
 	double2* states = MODE == EVAL_F ? nullptr : a.states + (size_t)blockIdx.x * (a.G - 1) * NS * T;
 	const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
@@ -137,6 +148,8 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 		tab[u * US + w] = a.ug[e];
 		if (TAN) tab[u * US + 16 + w] = a.uz[e];
 	}
+	for (int e = tid; e < 16 * a.Gt; e += nt) ttab[e] = make_double2(a.tg[e].x, -a.tg[e].y);
+	for (int e = tid; e < a.G + a.Gt; e += nt) bits[e] = make_int2(a.bits[2 * e], a.bits[2 * e + 1]);
 	ColumnSource wsrc = a.src;
 	wsrc.weighted = 1;
 	for (int e = tid; e < T; e += nt) {
@@ -156,21 +169,21 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 	// phi = -conj(U e): the conjugate gates on the negated conjugate column
 	if (!a.dense) {
 		for (int k = 0; k < a.Gt; k++) {
-			const Group gr(a.tbits[2 * k], a.tbits[2 * k + 1]);
+			const Group gr(tbits[k]);
+			const int mq = q == 0 ? 0 : q == 1 ? gr.m[1] : q == 2 ? gr.m[2] : gr.m[3];
 			double2 g[4];
 #pragma unroll
 			for (int m = 0; m < 4; m++) {
-				g[m] = a.tg[16 * k + 4 * q + m];
-				g[m].y = -g[m].y;
+				g[m] = ttab[16 * k + 4 * q + m];   // conjugated
 			}
 			for (int t = tid; t < ntasks; t += nt) {
-				const int gi = t >> 2, at = ((gi >> lg) << L) + gr.base(gi & ((1 << lg) - 1));
+				const int at = gr.base(t >> 2, lg, L);
 				double2 x[4];
 #pragma unroll
-				for (int m = 0; m < 4; m++) x[m] = Phi[swz(at | gr.member(m))];
+				for (int m = 0; m < 4; m++) x[m] = Phi[at ^ gr.m[m]];
 				const double2 y = dot4(g, x);
 				__syncwarp();
-				Phi[swz(at | gr.member(q))] = y;
+				Phi[at ^ mq] = y;
 			}
 			__syncthreads();
 		}
@@ -179,7 +192,8 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 
 	// forward
 	for (int k = 0; k < a.G; k++) {
-		const Group gr(a.bits[2 * k], a.bits[2 * k + 1]);
+		const Group gr(bits[k]);
+		const int mq = q == 0 ? 0 : q == 1 ? gr.m[1] : q == 2 ? gr.m[2] : gr.m[3];
 		const double2* gt = tab + (k / a.per) * US;
 		if (MODE != EVAL_F && k > 0) {
 			double2* st = states + (size_t)(k - 1) * NS * T;
@@ -195,19 +209,19 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 			if (TAN) z[m] = gt[16 + 4 * q + m];
 		}
 		for (int t = tid; t < ntasks; t += nt) {
-			const int gi = t >> 2, at = ((gi >> lg) << L) + gr.base(gi & ((1 << lg) - 1));
+			const int at = gr.base(t >> 2, lg, L);
 			double2 x[4], dx[4];
 #pragma unroll
 			for (int m = 0; m < 4; m++) {
-				const int p = swz(at | gr.member(m));
+				const int p = at ^ gr.m[m];
 				x[m] = Psi[p];
 				if (TAN) dx[m] = dPsi[p];
 			}
 			const double2 y = dot4(g, x);
 			double2 dy;
-			if (TAN) dy = dot4_acc(z, x, dot4(g, dx));
+			if (TAN) dy = cadd(dot4(z, x), dot4(g, dx));
 			__syncwarp();
-			const int p = swz(at | gr.member(q));
+			const int p = at ^ mq;
 			Psi[p] = y;
 			if (TAN) dPsi[p] = dy;
 		}
@@ -265,7 +279,8 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 		fetch(k - 1, b ^ 1);   // that pair's last readers are behind the barrier
 		const double2* X = Psi + b * T;
 		const double2* dX = TAN ? dPsi + b * T : nullptr;
-		const Group gr(a.bits[2 * k], a.bits[2 * k + 1]);
+		const Group gr(bits[k]);
+		const int mq = q == 0 ? 0 : q == 1 ? gr.m[1] : q == 2 ? gr.m[2] : gr.m[3];
 		const int u = k / a.per;
 		const double2* gt = tab + u * US;
 		double2 g[4], z[4];   // column q of G and Z
@@ -275,12 +290,12 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 			if (TAN) z[m] = gt[16 + 4 * m + q];
 		}
 		for (int t = tid; t < ntasks; t += nt) {
-			const int gi = t >> 2, at = ((gi >> lg) << L) + gr.base(gi & ((1 << lg) - 1));
-			const int own = swz(at | gr.member(q));
+			const int at = gr.base(t >> 2, lg, L);
+			const int own = at ^ mq;
 			double2 x[4], p[4], dx[4], dp[4];
 #pragma unroll
 			for (int m = 0; m < 4; m++) {
-				const int s = swz(at | gr.member(m));
+				const int s = at ^ gr.m[m];
 				x[m] = X[s];
 				p[m] = Phi[s];
 				if (TAN) {
@@ -306,7 +321,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 			}
 			const double2 yp = dot4(g, p);
 			double2 ydp;
-			if (TAN) ydp = dot4_acc(z, p, dot4(g, dp));
+			if (TAN) ydp = cadd(dot4(z, p), dot4(g, dp));
 			__syncwarp();
 			Phi[own] = yp;
 			if (TAN) dPhi[own] = ydp;
@@ -400,9 +415,10 @@ __global__ void __launch_bounds__(RED_GROUPS * SLOT) k_small_post(SmallArgs a, i
 // columns per block: enough groups to fill a warp
 int columns_per_block(int L) { return L >= 5 ? 1 : 32 >> L; }
 
-size_t small_smem(int L, int nunits, bool tan)
+size_t small_smem(int L, int nunits, int G, int Gt, bool tan)
 {
-	return ((tan ? 6 : 3) * ((size_t)columns_per_block(L) << L) + (size_t)nunits * (tan ? 32 : 16)) * sizeof(double2);
+	return ((tan ? 6 : 3) * ((size_t)columns_per_block(L) << L) + (size_t)nunits * (tan ? 32 : 16) + 16 * (size_t)Gt) * sizeof(double2) +
+	       (size_t)(G + Gt) * sizeof(int2);
 }
 
 template <int MODE>
@@ -417,7 +433,7 @@ int launch_small(Runtime& rt, const SmallArgs& a, int blocks)
 	const int threads = std::max(32, std::min(SMALL_THREADS, a.cb << a.L));
 	cudaEvent_t ev;
 	launch_begin(rt, KC_FUSED, &ev);
-	k_small<MODE><<<blocks, threads, small_smem(a.L, a.nunits, MODE == EVAL_HVP), rt.stream>>>(a);
+	k_small<MODE><<<blocks, threads, small_smem(a.L, a.nunits, a.G, a.Gt, MODE == EVAL_HVP), rt.stream>>>(a);
 	launch_end(rt, KC_FUSED, ev);
 	return RQC_CUDA(cudaGetLastError());
 }
@@ -430,7 +446,7 @@ bool SmallEval::fits(const Runtime& rt, const Problem& pb, const TargetHolder& t
 	if (pb.L < 2 || pb.L > SMALL_MAX_L || pb.nunits > SMALL_MAX_UNITS || ncols < 1) return false;
 	if (th.spec.ufunc || (!th.spec.dense && th.spec.ngates < 1)) return false;
 	if ((double)ncols * (double)(1 << pb.L) * (pb.G + th.spec.ngates) >= SMALL_MAX_WORK) return false;
-	return small_smem(pb.L, pb.nunits, true) <= SMALL_SMEM;
+	return small_smem(pb.L, pb.nunits, pb.G, th.spec.ngates, true) <= SMALL_SMEM;
 }
 
 int SmallEval::prepare(Runtime& rt, const Problem& pb, const TargetHolder& th, const std::vector<BasisCol>& cols,
@@ -475,7 +491,6 @@ int SmallEval::prepare(Runtime& rt, const Problem& pb, const TargetHolder& th, c
 	tg_ = dg + nug + nuz;
 	if (!cols.empty()) src_.tab = reinterpret_cast<const BasisCol*>(d + gates_b);
 	bits_ = reinterpret_cast<const int*>(d + gates_b + cols_b);
-	tbits_ = bits_ + 2 * G_;
 	dense_ = th.spec.dense;
 	return OK;
 }
@@ -496,7 +511,6 @@ int SmallEval::eval(Runtime& rt, int mode, const double2* ugates, const double2*
 	a.uz = udirs ? udirs : uz_;
 	a.bits = bits_;
 	a.tg = tg_;
-	a.tbits = tbits_;
 	a.dense = dense_;
 	const int blocks = (int)((ncols_ + a.cb - 1) / a.cb);
 	int ret = ensure_device(rt.partials, (size_t)blocks * (2 + SLOT * (size_t)nunits_) * sizeof(double));

@@ -41,7 +41,7 @@ private:
 	int64_t ncols_ = 0;
 	ColumnSource src_;
 	const double2 *ug_ = nullptr, *uz_ = nullptr, *tg_ = nullptr, *dense_ = nullptr;
-	const int *bits_ = nullptr, *tbits_ = nullptr;
+	const int* bits_ = nullptr;
 };
 
 }  // namespace rqc
