@@ -30,8 +30,8 @@ namespace rqc {
 
 namespace {
 
-constexpr int SMALL_THREADS = 256;     // most threads per block
-constexpr int SMALL_MAX_L = 10;        // six tiles of a column: 96 KB
+constexpr int SMALL_THREADS = 384;     // most threads per block (three roles of 128)
+constexpr int SMALL_MAX_L = 10;        // eight tiles of a column: 128 KB
 constexpr int SMALL_MAX_UNITS = 128;   // gate tables in shared memory: 512 B per unit
 constexpr size_t SMALL_SMEM = 200 * 1024;
 // Amplitude x gate updates up to which an evaluation runs here (512 MB of scratch); beyond,
@@ -96,12 +96,12 @@ __device__ __forceinline__ double2 dot4(const double2 a[4], const double2 x[4])
 	return make_double2(rr - ii, ri + ir);
 }
 
-// sums of v[k] over the lanes that share q = lane & 3: lane l gets those of entries e, e + 1,
-// e = 8 (l >> 4 & 1) + 4 (l >> 3 & 1) + 2 (l >> 2 & 1), in v[0], v[1]
-__device__ __forceinline__ void row_sums(double (&v)[16], int lane)
+// sums of v[k] over the lanes that share q = lane & 3: lane l gets that of entry
+// 4 (l >> 4 & 1) + 2 (l >> 3 & 1) + (l >> 2 & 1)
+__device__ __forceinline__ double row_sums(double (&v)[8], int lane)
 {
 #pragma unroll
-	for (int o = 16, h = 8; o >= 4; o >>= 1, h >>= 1) {
+	for (int o = 16, h = 4; o >= 4; o >>= 1, h >>= 1) {
 		const bool up = (lane & o) != 0;
 #pragma unroll
 		for (int k = 0; k < h; k++) {
@@ -109,6 +109,18 @@ __device__ __forceinline__ void row_sums(double (&v)[16], int lane)
 			const double keep = up ? v[k + h] : v[k];
 			v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
 		}
+	}
+	return v[0];
+}
+
+// acc[c] += p x[c] (complex, c < 4)
+__device__ __forceinline__ void outer_row(double (&acc)[8], double2 p, const double2 x[4])
+{
+#pragma unroll
+	for (int c = 0; c < 4; c++) {
+		const double2 v = cfma(p, x[c], make_double2(acc[2 * c], acc[2 * c + 1]));
+		acc[2 * c] = v.x;
+		acc[2 * c + 1] = v.y;
 	}
 }
 
@@ -118,19 +130,24 @@ __device__ __forceinline__ void copy16(double2* smem, const double2* gmem)
 	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem) : "memory");
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
+// Threads: `nb` per role.  With one role every thread does all of a gate's work on its groups;
+// with ROLES = 3 (columns too small to fill a block) the warps of role 0 take the value part
+// (psi, dG, phi), those of role 1 the tangent of psi and HZ, those of role 2 the copies of
+// forward states and the tangent of phi.  All states have two tiles, read and written in turn,
+// so that a gate costs one barrier whatever the roles.
+template <int MODE, int ROLES>
+__global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a, int nb)
 {
 	constexpr bool TAN = MODE == EVAL_HVP;
 	extern __shared__ __align__(16) double2 sm[];
-	__shared__ double red[2][SMALL_THREADS / 32][SLOT];
+	__shared__ double red[2][2][SMALL_THREADS / 32][32];   // units in turn: dG, HZ: per warp
 	__shared__ double fred[2][SMALL_THREADS / 32];
 	const int L = a.L, N = 1 << L, T = a.cb << L;
-	double2* Psi = sm;                       // [2]: the reverse sweep alternates
-	double2* Phi = sm + 2 * T;
-	double2* dPsi = TAN ? sm + 3 * T : nullptr;
-	double2* dPhi = TAN ? sm + 5 * T : nullptr;
-	double2* tab = sm + (TAN ? 6 : 3) * T;   // per unit: G, and for HVPs Z
+	double2* Psi = sm;                       // [2]
+	double2* Phi = sm + 2 * T;               // [2]
+	double2* dPsi = TAN ? sm + 4 * T : nullptr;
+	double2* dPhi = TAN ? sm + 6 * T : nullptr;
+	double2* tab = sm + (TAN ? 8 : 4) * T;   // per unit: G, and for HVPs Z
 	constexpr int US = TAN ? 32 : 16;
 	double2* ttab = tab + US * a.nunits;     // the target's gates, conjugated
 	int2* bits = reinterpret_cast<int2*>(ttab + 16 * a.Gt);
@@ -138,6 +155,9 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 	constexpr int NS = TAN ? 2 : 1;
 	double2* states = MODE == EVAL_F ? nullptr : a.states + (size_t)blockIdx.x * (a.G - 1) * NS * T;
 	const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
+	const int role = ROLES == 1 ? 0 : tid / nb, rt = ROLES == 1 ? tid : tid - role * nb;
+	const bool value = ROLES == 1 || role == 0, tanp = TAN && (ROLES == 1 || role == 1);
+	const bool third = ROLES == 1 || role == 2;
 	const int q = tid & 3;
 	const int lg = L - 2, ntasks = a.cb << L;   // four threads per group: one task per amplitude
 	const int64_t col0 = (int64_t)blockIdx.x * a.cb;
@@ -152,79 +172,78 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 	for (int e = tid; e < a.G + a.Gt; e += nt) bits[e] = make_int2(a.bits[2 * e], a.bits[2 * e + 1]);
 	ColumnSource wsrc = a.src;
 	wsrc.weighted = 1;
+	int ph = a.dense ? 0 : a.Gt & 1;   // the tile that holds phi once the target is done
 	for (int e = tid; e < T; e += nt) {
 		const int c = e >> L, row = e & (N - 1), p = swz(e);
 		Psi[p] = basis_amp<double>(a.src, row, col0 + c);
 		if (TAN) {
 			dPsi[p] = make_double2(0, 0);
 			dPhi[p] = make_double2(0, 0);
+			dPhi[T + p] = make_double2(0, 0);
 		}
-		if (a.dense) {
-			Phi[p] = cneg_conj(dense_amp(a.dense, L, a.src, row, col0 + c));
-		} else {
-			Phi[p] = cneg_conj(basis_amp<double>(wsrc, row, col0 + c));
-		}
+		if (a.dense) Phi[p] = cneg_conj(dense_amp(a.dense, L, a.src, row, col0 + c));
+		else Phi[p] = cneg_conj(basis_amp<double>(wsrc, row, col0 + c));
 	}
 	__syncthreads();
+
 	// phi = -conj(U e): the conjugate gates on the negated conjugate column
 	if (!a.dense) {
 		for (int k = 0; k < a.Gt; k++) {
 			const Group gr(tbits[k]);
 			const int mq = q == 0 ? 0 : q == 1 ? gr.m[1] : q == 2 ? gr.m[2] : gr.m[3];
+			const double2* in = Phi + (k & 1) * T;
+			double2* out = Phi + (~k & 1) * T;
 			double2 g[4];
 #pragma unroll
-			for (int m = 0; m < 4; m++) {
-				g[m] = ttab[16 * k + 4 * q + m];   // conjugated
-			}
+			for (int m = 0; m < 4; m++) g[m] = ttab[16 * k + 4 * q + m];
 			for (int t = tid; t < ntasks; t += nt) {
 				const int at = gr.base(t >> 2, lg, L);
 				double2 x[4];
 #pragma unroll
-				for (int m = 0; m < 4; m++) x[m] = Phi[at ^ gr.m[m]];
-				const double2 y = dot4(g, x);
-				__syncwarp();
-				Phi[at ^ mq] = y;
+				for (int m = 0; m < 4; m++) x[m] = in[at ^ gr.m[m]];
+				out[at ^ mq] = dot4(g, x);
 			}
 			__syncthreads();
 		}
 	}
-	__syncthreads();
 
 	// forward
-	for (int k = 0; k < a.G; k++) {
+	int cur = 0;   // the tile that holds psi, dpsi
+	for (int k = 0, u = 0, r = 0; k < a.G; k++, cur ^= 1) {
 		const Group gr(bits[k]);
 		const int mq = q == 0 ? 0 : q == 1 ? gr.m[1] : q == 2 ? gr.m[2] : gr.m[3];
-		const double2* gt = tab + (k / a.per) * US;
-		if (MODE != EVAL_F && k > 0) {
+		const double2* gt = tab + u * US + 4 * q;
+		const double2* in = Psi + cur * T;
+		const double2* din = TAN ? dPsi + cur * T : nullptr;
+		double2* out = Psi + (cur ^ 1) * T;
+		double2* dout = TAN ? dPsi + (cur ^ 1) * T : nullptr;
+		if (MODE != EVAL_F && k > 0 && third) {
 			double2* st = states + (size_t)(k - 1) * NS * T;
-			for (int e = tid; e < T; e += nt) {
-				st[e] = Psi[e];
-				if (TAN) st[T + e] = dPsi[e];
+			for (int e = rt; e < T; e += nb) {
+				st[e] = in[e];
+				if (TAN) st[T + e] = din[e];
 			}
 		}
-		double2 g[4], z[4];
-#pragma unroll
-		for (int m = 0; m < 4; m++) {
-			g[m] = gt[4 * q + m];
-			if (TAN) z[m] = gt[16 + 4 * q + m];
-		}
-		for (int t = tid; t < ntasks; t += nt) {
-			const int at = gr.base(t >> 2, lg, L);
-			double2 x[4], dx[4];
+		if (value || tanp) {
+			double2 g[4], z[4];
 #pragma unroll
 			for (int m = 0; m < 4; m++) {
-				const int p = at ^ gr.m[m];
-				x[m] = Psi[p];
-				if (TAN) dx[m] = dPsi[p];
+				g[m] = gt[m];
+				if (tanp) z[m] = gt[16 + m];
 			}
-			const double2 y = dot4(g, x);
-			double2 dy;
-			if (TAN) dy = cadd(dot4(z, x), dot4(g, dx));
-			__syncwarp();
-			const int p = at ^ mq;
-			Psi[p] = y;
-			if (TAN) dPsi[p] = dy;
+			for (int t = rt; t < ntasks; t += nb) {
+				const int at = gr.base(t >> 2, lg, L);
+				double2 x[4], dx[4];
+#pragma unroll
+				for (int m = 0; m < 4; m++) {
+					x[m] = in[at ^ gr.m[m]];
+					if (tanp) dx[m] = din[at ^ gr.m[m]];
+				}
+				if (value) out[at ^ mq] = dot4(g, x);
+				if (tanp) dout[at ^ mq] = cadd(dot4(z, x), dot4(g, dx));
+			}
 		}
+		if (++r == a.per) { r = 0; u++; }
 		__syncthreads();
 	}
 
@@ -232,7 +251,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 	{
 		double fx = 0, fy = 0;
 		for (int e = tid; e < T; e += nt) {
-			const double2 p = Phi[e], v = Psi[e];
+			const double2 p = Phi[ph * T + e], v = Psi[cur * T + e];
 			fx += p.x * v.x - p.y * v.y;
 			fy += p.x * v.y + p.y * v.x;
 		}
@@ -248,18 +267,18 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 	}
 	if (MODE == EVAL_F) return;
 
-	// the state entering gate k into pair b of the psi tiles
-	auto fetch = [&](int k, int b) {
+	// the state entering gate k into tile b of psi, dpsi
+	auto fetch = [&](int k, int b, int from, int step) {
 		double2* p = Psi + b * T;
 		double2* d = TAN ? dPsi + b * T : nullptr;
 		if (k > 0) {
 			const double2* st = states + (size_t)(k - 1) * NS * T;
-			for (int e = tid; e < T; e += nt) {
+			for (int e = from; e < T; e += step) {
 				copy16(p + e, st + e);
 				if (TAN) copy16(d + e, st + T + e);
 			}
 		} else if (k == 0) {
-			for (int e = tid; e < T; e += nt) {
+			for (int e = from; e < T; e += step) {
 				p[swz(e)] = basis_amp<double>(a.src, e & (N - 1), col0 + (e >> L));
 				if (TAN) d[e] = make_double2(0, 0);
 			}
@@ -269,82 +288,89 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(SmallArgs a)
 	auto arrived = [] { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); };
 
 	// reverse
-	double acc[16];
+	double ag[8], ah[8];
 #pragma unroll
-	for (int e = 0; e < 16; e++) acc[e] = 0;
-	fetch(a.G - 1, 1);
+	for (int e = 0; e < 8; e++) ag[e] = ah[e] = 0;
+	fetch(a.G - 1, cur ^ 1, tid, nt);   // psi at the output (tile cur) is still being read for f
 	arrived();
 	__syncthreads();
-	for (int k = a.G - 1, b = 1; k >= 0; k--, b ^= 1) {
-		fetch(k - 1, b ^ 1);   // that pair's last readers are behind the barrier
-		const double2* X = Psi + b * T;
-		const double2* dX = TAN ? dPsi + b * T : nullptr;
+	cur ^= 1;
+	for (int k = a.G - 1, u = a.nunits - 1, r = a.per - 1; k >= 0; k--, cur ^= 1, ph ^= 1) {
+		if (third) fetch(k - 1, cur ^ 1, rt, nb);   // that tile's last readers are behind the barrier
+		const double2* X = Psi + cur * T;
+		const double2* dX = TAN ? dPsi + cur * T : nullptr;
+		const double2* P = Phi + ph * T;
+		const double2* dP = TAN ? dPhi + ph * T : nullptr;
+		double2* Po = Phi + (ph ^ 1) * T;
+		double2* dPo = TAN ? dPhi + (ph ^ 1) * T : nullptr;
 		const Group gr(bits[k]);
 		const int mq = q == 0 ? 0 : q == 1 ? gr.m[1] : q == 2 ? gr.m[2] : gr.m[3];
-		const int u = k / a.per;
-		const double2* gt = tab + u * US;
+		const double2* gt = tab + u * US + q;
 		double2 g[4], z[4];   // column q of G and Z
 #pragma unroll
 		for (int m = 0; m < 4; m++) {
-			g[m] = gt[4 * m + q];
-			if (TAN) z[m] = gt[16 + 4 * m + q];
+			if (value || third) g[m] = gt[4 * m];
+			if (TAN && third) z[m] = gt[16 + 4 * m];
 		}
-		for (int t = tid; t < ntasks; t += nt) {
-			const int at = gr.base(t >> 2, lg, L);
-			const int own = at ^ mq;
-			double2 x[4], p[4], dx[4], dp[4];
+		for (int t = rt; t < ntasks; t += nb) {
+			const int at = gr.base(t >> 2, lg, L), own = at ^ mq;
+			double2 x[4], p[4], dp[4];
+			if (value || tanp) {
 #pragma unroll
-			for (int m = 0; m < 4; m++) {
-				const int s = at ^ gr.m[m];
-				x[m] = X[s];
-				p[m] = Phi[s];
-				if (TAN) {
-					dx[m] = dX[s];
-					dp[m] = dPhi[s];
-				}
+				for (int m = 0; m < 4; m++) x[m] = X[at ^ gr.m[m]];
 			}
-			const double2 pq = Phi[own];
-			double2 dpq;
-			if (TAN) dpq = dPhi[own];
+			if (value || (TAN && third)) {
 #pragma unroll
-			for (int c = 0; c < 4; c++) {
-				const double2 v = cfma(pq, x[c], make_double2(acc[2 * c], acc[2 * c + 1]));
-				acc[2 * c] = v.x;
-				acc[2 * c + 1] = v.y;
-				if (TAN) {
-					double2 h = make_double2(acc[8 + 2 * c], acc[9 + 2 * c]);
-					h = cfma(pq, dx[c], h);
-					h = cfma(dpq, x[c], h);
-					acc[8 + 2 * c] = h.x;
-					acc[9 + 2 * c] = h.y;
-				}
+				for (int m = 0; m < 4; m++) p[m] = P[at ^ gr.m[m]];
 			}
-			const double2 yp = dot4(g, p);
-			double2 ydp;
-			if (TAN) ydp = cadd(dot4(z, p), dot4(g, dp));
-			__syncwarp();
-			Phi[own] = yp;
-			if (TAN) dPhi[own] = ydp;
+			if (value) {
+				outer_row(ag, P[own], x);
+				Po[own] = dot4(g, p);
+			}
+			if (tanp) {
+				double2 dx[4];
+#pragma unroll
+				for (int m = 0; m < 4; m++) dx[m] = dX[at ^ gr.m[m]];
+				outer_row(ah, P[own], dx);
+				outer_row(ah, dP[own], x);
+			}
+			if (TAN && third) {
+#pragma unroll
+				for (int m = 0; m < 4; m++) dp[m] = dP[at ^ gr.m[m]];
+				dPo[own] = cadd(dot4(z, p), dot4(g, dp));
+			}
 		}
-		const bool done = k % a.per == 0;   // the unit's last gate of the sweep
+		const bool done = r == 0;   // the unit's last gate of the sweep
 		if (done) {
-			row_sums(acc, lane);
-			const int e = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2;
-			red[u & 1][warp][16 * q + e] = acc[0];
-			red[u & 1][warp][16 * q + e + 1] = acc[1];
+			const int e = 8 * q + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+			if (value) red[u & 1][0][warp][e] = row_sums(ag, lane);
+			if (tanp) red[u & 1][1][warp][e] = row_sums(ah, lane);
 #pragma unroll
-			for (int i = 0; i < 16; i++) acc[i] = 0;
+			for (int i = 0; i < 8; i++) ag[i] = ah[i] = 0;
 		}
 		arrived();
 		__syncthreads();
-		// the other buffer of red is written before the next barrier at the earliest
-		if (done && tid < 32) {
-			for (int e = tid; e < SLOT; e += 32) {
+		if (done) {
+			// warp 0 adds up dG, warp 1 (or 0) HZ, over the warps that hold them; this half of red is
+			// written again two units on, behind the next barrier
+			const int nw = nb >> 5;
+			double* o = part + 2 + SLOT * (size_t)u;
+			const int row = lane >> 3, v = lane & 7;
+			if (warp == 0) {
 				double s = 0;
-				for (int v = 0; v < nwarps; v++) s += red[u & 1][v][e];
-				part[2 + SLOT * (size_t)u + e] = s;
+				for (int w = 0; w < nw; w++) s += red[u & 1][0][w][lane];
+				o[16 * row + v] = s;
 			}
+			if (TAN && warp == (nwarps > 1 ? 1 : 0)) {
+				double s = 0;
+				for (int w = 0; w < nw; w++) s += red[u & 1][1][(ROLES == 1 ? 0 : nw) + w][lane];
+				o[16 * row + 8 + v] = s;
+			}
+			if (!TAN && warp == 0) o[16 * row + 8 + v] = 0;
+			r = a.per;
+			u--;
 		}
+		r--;
 	}
 }
 
@@ -417,25 +443,35 @@ int columns_per_block(int L) { return L >= 5 ? 1 : 32 >> L; }
 
 size_t small_smem(int L, int nunits, int G, int Gt, bool tan)
 {
-	return ((tan ? 6 : 3) * ((size_t)columns_per_block(L) << L) + (size_t)nunits * (tan ? 32 : 16) + 16 * (size_t)Gt) * sizeof(double2) +
+	return ((tan ? 8 : 4) * ((size_t)columns_per_block(L) << L) + (size_t)nunits * (tan ? 32 : 16) + 16 * (size_t)Gt) * sizeof(double2) +
 	       (size_t)(G + Gt) * sizeof(int2);
 }
 
-template <int MODE>
-int launch_small(Runtime& rt, const SmallArgs& a, int blocks)
+template <int MODE, int ROLES>
+int launch_small_as(Runtime& rt, const SmallArgs& a, int blocks, int nb)
 {
 	static bool ready = false;
 	if (!ready) {
-		if (int e = RQC_CUDA(cudaFuncSetAttribute(k_small<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM)))
+		if (int e = RQC_CUDA(cudaFuncSetAttribute(k_small<MODE, ROLES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                          (int)SMALL_SMEM)))
 			return e;
 		ready = true;
 	}
-	const int threads = std::max(32, std::min(SMALL_THREADS, a.cb << a.L));
 	cudaEvent_t ev;
 	launch_begin(rt, KC_FUSED, &ev);
-	k_small<MODE><<<blocks, threads, small_smem(a.L, a.nunits, a.G, a.Gt, MODE == EVAL_HVP), rt.stream>>>(a);
+	k_small<MODE, ROLES><<<blocks, ROLES * nb, small_smem(a.L, a.nunits, a.G, a.Gt, MODE == EVAL_HVP), rt.stream>>>(a, nb);
 	launch_end(rt, KC_FUSED, ev);
 	return RQC_CUDA(cudaGetLastError());
+}
+
+// A thread per amplitude of the block's columns, up to 256.  Up to 128 (L <= 7) three roles share
+// a gate's work: a warp or two per SM sub-partition wait out every latency in turn.
+template <int MODE>
+int launch_small(Runtime& rt, const SmallArgs& a, int blocks)
+{
+	const int nb = std::max(32, std::min(256, a.cb << a.L));
+	if (MODE == EVAL_HVP && nb <= 128) return launch_small_as<MODE, 3>(rt, a, blocks, nb);
+	return launch_small_as<MODE, 1>(rt, a, blocks, nb);
 }
 
 }  // namespace
