@@ -27,6 +27,9 @@
 // each gate moves 16 (a + 1) + 1 states instead of 16 times the number of
 // earlier occurrences.
 //
+// That is the general sweep (any gates; one state; k_hsweep, k_hlayer).  For unitary gates the
+// column sums take the layer sweep (below, "layer sweep"), which moves whole layers.
+//
 // Sums: each block reduces its 16 complex products per state (warp transpose
 // reduction, then over warps) and adds them to its own slot of a partial-sum
 // array, [layer][state][32 doubles][block]; the launches of a layer and the
@@ -34,11 +37,13 @@
 // sums the slots over blocks in index order, so results are deterministic.
 #include "hess.h"
 
+#include <math.h>
 #include <stdio.h>
 #include <string.h>
 #include <algorithm>
 #include <vector>
 
+#include "layer_pass.h"
 #include "manifold.cuh"
 #include "rqc_common.cuh"
 #include "rqcopt_gpu.h"
@@ -611,6 +616,231 @@ __global__ void k_gemv(int n, const double* __restrict__ a, const double* __rest
 	if (row < n) y[row] = dot_seq(n, a + (size_t)row * n, x);
 }
 
+// ------------------------------------------------------------------ layer sweep
+//
+// The gates of a layer commute, so everything the sweep needs can be taken at the layer's OUTPUT.
+// With psi, phi the state and cotangent there and T any tangent carried through the whole layer,
+// the contraction at gate q is the raw sum R_q[i][j] = sum phi[.. i at q ..] T[.. j at q ..] times
+// conj(G) (G unitary).  Summed over the layer's gates that is ONE inner product with states made
+// from phi,
+//     R[i][j] = sum_q R_q[i][j] = <Phi_{ij}, T>,   Phi_{ij}[a] = sum over q with bits_q(a) = j of phi[a, i at q],
+// so the layer's Hessian blocks are a complex matrix product of 16 cotangent states with the
+// 16 (a + 1) tangents over all amplitudes and columns (k_hgemm): 16 multiply-adds per amplitude
+// and tangent whatever the layer's length, in FP64 MMAs whose operands come straight from memory.
+// The layer's own tangents at its output are T_{rc}[a] = sum over q with bits_q(a) = r of
+// (row c of G_q^+ psi at q)[a], and the pairs p = q that the product with them contains are
+//     dV[i][yc] conj(G[yr][xc])          (x = (i, xc), y = (yr, yc))
+// with dV the layer's gradient, taken off in k_hrecord.  What is left per layer: carry the
+// earlier tangents (layer_pass.cu), 32 new states (k_hstates) and the product.  Against the
+// general layer kernel this is a third of the flops at L = 12, 1-2 memory round trips a layer
+// instead of two tiles' worth of shared-memory traffic per gate; L = 10, depth 7, one column
+// per orbit: 3.8 -> 1.5 ms (see the figures at k_hgemm).
+
+// T_{rc} (own tangents) and Phi_{ij} at a layer's output, 16 states each, from psi and phi
+struct LayerWires
+{
+	int n;
+	int8_t bi[16], bj[16];   // state bits of the pairs
+	Gate4<double> g;
+};
+
+// a thread per amplitude and column; own: write the tangents (not where only the gradient is wanted)
+__global__ void __launch_bounds__(256) k_hstates(const double2* __restrict__ psi, const double2* __restrict__ phi,
+                                                 const __grid_constant__ LayerWires w, int64_t n,
+                                                 double2* __restrict__ own, double2* __restrict__ cot)
+{
+	for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
+		double2 t[16];
+		if (own) {
+#pragma unroll
+			for (int e = 0; e < 16; e++) t[e] = make_double2(0, 0);
+			for (int q = 0; q < w.n; q++) {
+				const int64_t si = (int64_t)1 << w.bi[q], sj = (int64_t)1 << w.bj[q];
+				const int r = ((a & si) ? 2 : 0) | ((a & sj) ? 1 : 0);
+				const int64_t b = a & ~(si | sj);
+				const double2 x[4] = {psi[b], psi[b | sj], psi[b | si], psi[b | si | sj]};
+#pragma unroll
+				for (int c = 0; c < 4; c++) {
+					double2 v = make_double2(0, 0);
+#pragma unroll
+					for (int m = 0; m < 4; m++) v = cfma(make_double2(w.g.m[4 * m + c].x, -w.g.m[4 * m + c].y), x[m], v);
+#pragma unroll
+					for (int k = 0; k < 4; k++)
+						if (k == r) t[4 * k + c] = cadd(t[4 * k + c], v);
+				}
+			}
+#pragma unroll
+			for (int e = 0; e < 16; e++) own[e * n + a] = t[e];
+		}
+#pragma unroll
+		for (int e = 0; e < 16; e++) t[e] = make_double2(0, 0);
+		for (int q = 0; q < w.n; q++) {
+			const int64_t si = (int64_t)1 << w.bi[q], sj = (int64_t)1 << w.bj[q];
+			const int j = ((a & si) ? 2 : 0) | ((a & sj) ? 1 : 0);
+			const int64_t b = a & ~(si | sj);
+			const double2 x[4] = {phi[b], phi[b | sj], phi[b | si], phi[b | si | sj]};
+#pragma unroll
+			for (int k = 0; k < 4; k++)
+				if (k == j)
+#pragma unroll
+					for (int i = 0; i < 4; i++) t[4 * i + k] = cadd(t[4 * i + k], x[i]);
+		}
+#pragma unroll
+		for (int e = 0; e < 16; e++) cot[e * n + a] = t[e];
+	}
+}
+
+__device__ __forceinline__ void hdmma(double (&d)[2], double a, double b)
+{
+	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+	    : "+d"(d[0]), "+d"(d[1])
+	    : "d"(a), "d"(b));
+}
+
+constexpr int GW = 4;               // warps per block of the product
+constexpr int GN = 32;              // tangents per block: two layers
+constexpr int GSLOT = 16 * GN;      // complex sums per block
+
+// R[m][n] += sum_k A[m][k] B[n][k] (no conjugation) for 16 cotangent states A and tangents B, n =
+// 32 blockIdx.x ..: the last blockIdx.x takes psi as its only column.  K amplitudes per state;
+// blockIdx.y and the block's warps split them in runs of 16.  FP64 MMAs m8n8k4 on the real and
+// imaginary parts (four per complex 8 x 8 x 4 product): a lane's operand is the complex number it
+// loads, rows of four consecutive amplitudes (64 B), so the fragments come from memory as they
+// are, six 16-byte loads for 32 MMAs; no shared memory until the block's final sum.  Bound: the
+// tangents' one read from HBM at small 16 (a + 1), the FP64 pipe beyond.
+__global__ void __launch_bounds__(32 * GW, 3)
+k_hgemm(const double2* __restrict__ A, const double2* __restrict__ B, const double2* __restrict__ psi, int64_t K, int ntan,
+        double2* __restrict__ part, int add)
+{
+	__shared__ double2 red[GW][GSLOT];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int row = lane >> 2, kk = lane & 3;
+	const bool grad = blockIdx.x == gridDim.x - 1;
+	const int n0 = blockIdx.x * GN;
+	const int nf = grad ? 1 : min(4, (ntan - n0) / 8);   // fragments of 8 tangents
+	const double2* pa[2] = {A + row * K + kk, A + (row + 8) * K + kk};
+	const double2* pb[4];
+#pragma unroll
+	for (int f = 0; f < 4; f++) pb[f] = grad ? psi + kk : B + (int64_t)(n0 + (f < nf ? 8 * f : 0) + row) * K + kk;
+	const bool live = !grad || row == 0;   // the gradient tile has one column
+	double re[2][4][2], im[2][4][2];
+#pragma unroll
+	for (int m = 0; m < 2; m++)
+#pragma unroll
+		for (int f = 0; f < 4; f++) re[m][f][0] = re[m][f][1] = im[m][f][0] = im[m][f][1] = 0;
+	const int64_t nrun = (K + 15) / 16, step = (int64_t)gridDim.y * GW;
+	for (int64_t run = (int64_t)blockIdx.y * GW + warp; run < nrun; run += step) {
+#pragma unroll
+		for (int s = 0; s < 4; s++) {
+			const int64_t k = run * 16 + 4 * s;
+			const bool in = k + kk < K;
+			const double2 zero = make_double2(0, 0);
+			double2 x[2], y[4];
+#pragma unroll
+			for (int m = 0; m < 2; m++) x[m] = in ? pa[m][k] : zero;
+#pragma unroll
+			for (int f = 0; f < 4; f++) y[f] = f < nf && in && live ? pb[f][k] : zero;
+#pragma unroll
+			for (int f = 0; f < 4; f++) {
+				if (f >= nf) break;
+#pragma unroll
+				for (int m = 0; m < 2; m++) {
+					hdmma(re[m][f], x[m].x, y[f].x);
+					hdmma(im[m][f], x[m].x, y[f].y);
+					hdmma(re[m][f], -x[m].y, y[f].y);
+					hdmma(im[m][f], x[m].y, y[f].x);
+				}
+			}
+		}
+	}
+	// lane: rows row (+ 8 m), columns 8 f + 2 kk, + 1
+#pragma unroll
+	for (int m = 0; m < 2; m++)
+#pragma unroll
+		for (int f = 0; f < 4; f++)
+#pragma unroll
+			for (int c = 0; c < 2; c++)
+				red[warp][(row + 8 * m) * GN + 8 * f + 2 * kk + c] = make_double2(re[m][f][c], im[m][f][c]);
+	__syncthreads();
+	double2* o = part + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * GSLOT;
+	for (int e = threadIdx.x; e < GSLOT; e += blockDim.x) {
+		double2 v = red[0][e];
+#pragma unroll
+		for (int w = 1; w < GW; w++) v = cadd(v, red[w][e]);
+		o[e] = add ? cadd(o[e], v) : v;
+	}
+}
+
+// where a layer's partial sums lie: tile x of split s at off + (x * nsplit + s) * GSLOT
+struct LayerParts
+{
+	int64_t off;
+	int nsplit, ntile;   // tiles with the gradient's last
+};
+
+// raw sum e of tile x over the splits
+__device__ __forceinline__ double2 part_sum(const double2* __restrict__ part, const LayerParts& p, int x, int e)
+{
+	const double2* q = part + p.off + (int64_t)x * p.nsplit * GSLOT + e;
+	double2 s = make_double2(0, 0);
+	for (int k = 0; k < p.nsplit; k++) s = cadd(s, q[(int64_t)k * GSLOT]);
+	return s;
+}
+
+// Record of the layer sweep: block b handles the layer pair (a, l <= a) in row-major order of the
+// lower triangle; with_f: f from the last layer's gradient sums, sum_i R[i][i] = (gates per layer) phi.psi
+__global__ void __launch_bounds__(256) k_hrecord(const double2* __restrict__ part, const LayerParts* __restrict__ parts,
+                                                 const double2* __restrict__ ug, int nl, int per, int with_f, int hess,
+                                                 double2* __restrict__ rec)
+{
+	__shared__ double2 R[256], V[16], D[16], H[256];
+	int a = 0, l = blockIdx.x;
+	if (hess) while (l > a) l -= ++a;
+	else { a = l; }
+	const int t = threadIdx.x, m = 16 * nl;
+	const LayerParts p = parts[a];
+	if (t < 16) {
+		V[t] = ug[16 * a + t];
+		if (l == a) R[t] = part_sum(part, p, p.ntile - 1, t * GN);
+	}
+	__syncthreads();
+	auto times_conj = [&](const double2* r, int stride, int i, int c) {   // sum_j r[(i, j)] conj(G[j][c])
+		double2 s = make_double2(0, 0);
+		for (int j = 0; j < 4; j++) s = cfma(r[(4 * i + j) * stride], make_double2(V[4 * j + c].x, -V[4 * j + c].y), s);
+		return s;
+	};
+	if (l == a) {
+		if (t < 16) {
+			D[t] = times_conj(R, 1, t >> 2, t & 3);
+			rec[1 + 16 * a + t] = D[t];
+		}
+		if (t == 0 && with_f && a == nl - 1) {
+			const double2 s = cadd(cadd(R[0], R[5]), cadd(R[10], R[15]));
+			rec[0] = make_double2(s.x / per, s.y / per);
+		}
+		__syncthreads();
+	}
+	if (!hess) return;
+	const int x = t >> 4, y = t & 15;
+	R[t] = part_sum(part, p, l / 2, x * GN + 16 * (l & 1) + y);   // column y of layer l in its tile
+	__syncthreads();
+	double2 h = times_conj(R + y, 16, x >> 2, x & 3);
+	double2* out = rec + 1 + 16 * nl;
+	if (l == a) {
+		// the pairs p = q: dV[i][yc] conj(G[yr][xc])
+		const double2 g = V[4 * (y >> 2) + (x & 3)];
+		h = csub(h, cmul(D[4 * (x >> 2) + (y & 3)], make_double2(g.x, -g.y)));
+		H[t] = h;
+		__syncthreads();
+		const double2 ht = H[16 * y + x];
+		h = make_double2(0.5 * (h.x + ht.x), 0.5 * (h.y + ht.y));
+		out[(int64_t)(16 * a + x) * m + 16 * a + y] = h;
+	} else {
+		out[(int64_t)(16 * a + x) * m + 16 * l + y] = h;
+		out[(int64_t)(16 * l + y) * m + 16 * a + x] = h;
+	}
+}
+
 // ------------------------------------------------------------------ interleaved arrays
 
 __global__ void __launch_bounds__(HT) k_gate_array(const double2* __restrict__ in, double2* __restrict__ out,
@@ -827,6 +1057,188 @@ struct Sweep
 	}
 };
 
+// every layer gate unitary to 1e-14 and every layer's pairs on wires of their own
+bool layer_sweep_ok(const HessCircuit& c)
+{
+	const int per = c.L / 2;
+	if (per > 16) return false;
+	for (int l = 0; l < c.nlayers; l++) {
+		const double2* g = c.ugates + 16 * l;
+		for (int r = 0; r < 4; r++)
+			for (int k = 0; k < 4; k++) {
+				double re = 0, im = 0;
+				for (int q = 0; q < 4; q++) {
+					const double2 x = g[4 * q + r], y = g[4 * q + k];
+					re += x.x * y.x + x.y * y.y;
+					im += x.x * y.y - x.y * y.x;
+				}
+				if (!(fabs(re - (r == k ? 1.0 : 0.0)) <= 1e-14 && fabs(im) <= 1e-14)) return false;
+			}
+		std::vector<LayerGate> gates;
+		for (int p = 0; p < per; p++)
+			gates.push_back({g, c.wires[2 * (l * per + p)], c.wires[2 * (l * per + p) + 1]});
+		if (!gates_disjoint(c.L, gates)) return false;
+	}
+	return true;
+}
+
+struct LayerSweep
+{
+	Runtime& rt;
+	const HessCircuit& c;
+	int L, nl, per;
+	bool hess = true;
+	std::vector<std::vector<LayerGate>> layers;
+	std::vector<LayerParts> parts;
+	double2* d_part = nullptr;
+	const double2* d_ug = nullptr;
+	const LayerParts* d_parts = nullptr;
+
+	LayerSweep(Runtime& r, const HessCircuit& hc, bool with_hess)
+		: rt(r), c(hc), L(hc.L), nl(hc.nlayers), per(hc.L / 2), hess(with_hess), layers(hc.nlayers)
+	{
+		for (int l = 0; l < nl; l++)
+			for (int p = 0; p < per; p++)
+				layers[l].push_back({c.ugates + 16 * l, c.wires[2 * (l * per + p)], c.wires[2 * (l * per + p) + 1]});
+	}
+
+	// partial-sum slots for chunks of up to K amplitudes per state: enough splits to fill the
+	// GPU (three blocks of four warps per SM), none shorter than eight runs per warp
+	int init(int64_t K)
+	{
+		int64_t off = 0;
+		parts.resize(nl);
+		for (int a = 0; a < nl; a++) {
+			const int ntile = hess ? (16 * (a + 1) + GN - 1) / GN + 1 : 1;
+			const int64_t fill = (3 * (int64_t)rt.num_sms + ntile - 1) / ntile, most = K / (16 * GW * 8);
+			parts[a] = {off, (int)std::max<int64_t>(1, std::min(fill, most)), ntile};
+			off += (int64_t)ntile * parts[a].nsplit * GSLOT;
+		}
+		// sums | unit gates | slots
+		const size_t bytes = ((size_t)off + 16 * (size_t)nl) * sizeof(double2) + nl * sizeof(LayerParts);
+		int ret = ensure_device(rt.partials, bytes);
+		if (ret) return ret;
+		d_part = static_cast<double2*>(rt.partials.ptr);
+		double2* ug = d_part + off;
+		LayerParts* lp = reinterpret_cast<LayerParts*>(ug + 16 * nl);
+		d_ug = ug;
+		d_parts = lp;
+		if ((ret = RQC_CUDA(cudaMemcpyAsync(ug, c.ugates, 16 * (size_t)nl * sizeof(double2), cudaMemcpyHostToDevice, rt.stream))))
+			return ret;
+		return RQC_CUDA(cudaMemcpyAsync(lp, parts.data(), nl * sizeof(LayerParts), cudaMemcpyHostToDevice, rt.stream));
+	}
+
+	// psi at every layer's output (psi + a K); psi_0 in `in`, or the basis columns of *src
+	int forward(const double2* in, const ColumnSource* src, double2* psi, int64_t ncols)
+	{
+		const int64_t K = ncols << L;
+		for (int a = 0; a < nl; a++)
+			if (int e = layer_apply(rt, L, layers[a], false, a == 0 ? in : psi + (a - 1) * K, psi + a * K, ncols,
+			                        a == 0 ? src : nullptr))
+				return e;
+		return OK;
+	}
+
+	// phi at every layer's output from that of the last
+	int reverse(double2* phi, int64_t ncols)
+	{
+		const int64_t K = ncols << L;
+		for (int a = nl - 1; a >= 1; a--)
+			if (int e = layer_apply(rt, L, layers[a], true, phi + a * K, phi + (a - 1) * K, ncols)) return e;
+		return OK;
+	}
+
+	// tangents and sums of one chunk; tan: 16 states per layer, cot: 16 states.  At the end the
+	// tangents are at the circuit's output.
+	int sweep(const double2* psi, const double2* phi, double2* tan, double2* cot, int64_t ncols, bool add)
+	{
+		const int64_t K = ncols << L;
+		for (int a = 0; a < nl; a++) {
+			if (hess && a > 0)
+				if (int e = layer_apply(rt, L, layers[a], false, tan, tan, 16 * a * ncols)) return e;
+			LayerWires w;
+			w.n = per;
+			for (int q = 0; q < per; q++) {
+				w.bi[q] = (int8_t)(L - 1 - layers[a][q].i);
+				w.bj[q] = (int8_t)(L - 1 - layers[a][q].j);
+			}
+			w.g = gate_of(c.ugates + 16 * a, false);
+			k_hstates<<<grid_of(rt, K, 8), 256, 0, rt.stream>>>(psi + a * K, phi + a * K, w, K, hess ? tan + 16 * a * K : nullptr, cot);
+			if (int e = checked(rt)) return e;
+			cudaEvent_t ev;
+			launch_begin(rt, KC_HESS, &ev);
+			k_hgemm<<<dim3(parts[a].ntile, parts[a].nsplit), 32 * GW, 0, rt.stream>>>(
+				cot, tan, psi + a * K, K, hess ? 16 * (a + 1) : 0, d_part + parts[a].off, add ? 1 : 0);
+			launch_end(rt, KC_HESS, ev);
+			if (int e = RQC_CUDA(cudaGetLastError())) return e;
+		}
+		return OK;
+	}
+
+	int record(double2* d_rec, bool with_f)
+	{
+		const int blocks = hess ? nl * (nl + 1) / 2 : nl;
+		k_hrecord<<<blocks, 256, 0, rt.stream>>>(d_part, d_parts, d_ug, nl, per, with_f ? 1 : 0, hess ? 1 : 0, d_rec);
+		return checked(rt);
+	}
+};
+
+// hessian_target_device for unitary gates: the layer sweep over column chunks
+int hessian_layers(Runtime& rt, const HessCircuit& c, const TargetSpec& t, double2* d_rec, const SampleSpec* samp)
+{
+	const int L = c.L, nl = c.nlayers;
+	const int64_t N = (int64_t)1 << L;
+	const int64_t ncols = samp ? samp->nsamples : (c.columns ? c.ncolumns : N);
+	// states per column: psi and phi at every layer's output, 16 tangents per layer (before
+	// that two scratch states of the target), 16 cotangent states, the sample states
+	const int64_t nstates = 2 * nl + 16 * (int64_t)nl + 16 + (samp ? 1 : 0);
+	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
+	int64_t C = ncols;
+	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
+	if (t.ufunc) C = std::min<int64_t>(C, std::max<int64_t>(1, ((int64_t)256 << 20) / (N * 16)));
+	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
+	if (C < 1) {
+		fprintf(stderr, "rqcopt_gpu: one basis column of the Hessian sweep needs %zu bytes of workspace, more than the limit\n",
+		        col_bytes);
+		return E_ALLOC;
+	}
+	int ret = ensure_device(rt.work, (size_t)C * col_bytes);
+	if (ret) return ret;
+	LayerSweep sw(rt, c, true);
+	if ((ret = sw.init(C * N))) return ret;
+	for (int64_t b0 = 0; b0 < ncols; b0 += C) {
+		const int64_t Cc = std::min(C, ncols - b0), K = Cc * N;
+		double2* psi = static_cast<double2*>(rt.work.ptr);
+		double2* phi = psi + nl * K;
+		double2* tan = phi + nl * K;
+		double2* cot = tan + 16 * nl * K;
+		double2* states = cot + 16 * K;
+		double2* last = phi + (nl - 1) * K;
+		ColumnSource src;
+		src.tab = c.columns;
+		src.b0 = b0;
+		src.end = ncols;
+		if (samp) {
+			if ((ret = haar_states_device(rt, *samp, L, b0, Cc, states))) return ret;
+			if ((ret = target_states_device(rt, t, L, states, Cc, last, tan, tan + K))) return ret;
+		} else {
+			ColumnSource tsrc = src;
+			tsrc.weighted = 1;
+			if ((ret = target_columns_device(rt, t, L, tsrc, Cc, last, tan, tan + K))) return ret;
+		}
+		if ((ret = sw.forward(samp ? states : nullptr, samp ? nullptr : &src, psi, Cc))) return ret;
+		if ((ret = sw.reverse(phi, Cc))) return ret;
+		if ((ret = sw.sweep(psi, phi, tan, cot, Cc, b0 > 0))) return ret;
+	}
+	if ((ret = sw.record(d_rec, true))) return ret;
+	if (samp) {
+		const int64_t n = (int64_t)hess_record_count(nl);
+		k_scale_rec<<<grid_of(rt, n, 4), HT, 0, rt.stream>>>(d_rec, n, (double)N / (double)samp->nsamples);
+		ret = checked(rt);
+	}
+	return ret;
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ engine entry points
@@ -836,6 +1248,7 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	const int L = c.L, nl = c.nlayers;
 	if (L < 2 || L % 2 || nl < 1) return E_ARG;
 	if (samp && samp->nsamples < 1) return E_ARG;
+	if (layer_sweep_ok(c)) return hessian_layers(rt, c, t, d_rec, samp);
 	const int per = L / 2, G = nl * per;
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ncols = samp ? samp->nsamples : (c.columns ? c.ncolumns : N);   // basis columns, or sample states
@@ -944,9 +1357,13 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	const int64_t N = (int64_t)1 << L, s = (int64_t)1 << half;
 	const bool hess = mode == 2;
 	const bool layered = L <= 12 && per <= HMAXPER;
-	// states per column: phi_q of every gate; psi_q of every gate (layered) or two psi
-	// buffers and the input states; W P e_b; the tangents (Hessian only)
-	const int64_t nstates = G + (layered ? G : 3) + 1 + (hess ? 16 * (int64_t)nl : 0);
+	const bool sweep = layer_sweep_ok(c);
+	// layer sweep, states per column: the input states, psi and phi at every layer's output, 16
+	// cotangent states, the tangents (Hessian only).
+	// General sweep: phi_q of every gate; psi_q of every gate (layered) or two psi buffers and
+	// the input states; W P e_b; the tangents (Hessian only)
+	const int64_t nstates = sweep ? 1 + 2 * nl + 16 + (hess ? 16 * (int64_t)nl : 0)
+	                              : G + (layered ? G : 3) + 1 + (hess ? 16 * (int64_t)nl : 0);
 	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
 	const int64_t ncols = c.columns ? c.ncolumns : s;
 	int64_t C = ncols;
@@ -977,6 +1394,40 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	if ((ret = RQC_CUDA(cudaMemsetAsync(fres, 0, nres * sizeof(double2), rt.stream)))) return ret;
 	if (hess && (ret = RQC_CUDA(cudaMemsetAsync(part2, 0, (size_t)m * m * sizeof(double2), rt.stream)))) return ret;
 	if ((ret = target_columns_device(rt, t, half, ColumnSource{}, s, hneg, sc0, sc1))) return ret;
+
+	if (sweep) {
+		LayerSweep ls(rt, c, hess);
+		if ((ret = ls.init(C * N))) return ret;
+		for (int64_t b0 = 0; b0 < ncols; b0 += C) {
+			const int64_t Cc = std::min(C, ncols - b0), K = Cc * N;
+			double2* in = phi;
+			double2* psi_l = in + K;
+			double2* phi_l = psi_l + nl * K;
+			double2* cot = phi_l + nl * K;
+			double2* tan_l = cot + 16 * K;
+			double2* chi = phi_l + (nl - 1) * K;
+			k_benc_init<<<grid_of(rt, K, 8), HT, 0, rt.stream>>>(in, L, c.columns, b0, Cc);
+			if ((ret = checked(rt))) return ret;
+			if ((ret = ls.forward(in, nullptr, psi_l, Cc))) return ret;
+			if (mode >= 1 && (ret = RQC_CUDA(cudaMemsetAsync(chi, 0, (size_t)K * sizeof(double2), rt.stream)))) return ret;
+			k_benc_residual<<<nres, HT, 0, rt.stream>>>(psi_l + (nl - 1) * K, hneg, L, c.columns, b0, Cc,
+			                                            mode >= 1 ? chi : nullptr, fres);
+			if ((ret = checked(rt))) return ret;
+			if (mode == 0) continue;
+			if ((ret = ls.reverse(phi_l, Cc))) return ret;
+			if ((ret = ls.sweep(psi_l, phi_l, tan_l, cot, Cc, b0 > 0))) return ret;
+			if (hess) {
+				k_benc_gather<<<grid_of(rt, (int64_t)m * Cc * s, 8), HT, 0, rt.stream>>>(tan_l, L, Cc, K, m, jac);
+				if ((ret = checked(rt))) return ret;
+				k_benc_gram<<<m * m, HT, 0, rt.stream>>>(jac, Cc * s, nl, c.columns, b0, half, part2);
+				if ((ret = checked(rt))) return ret;
+			}
+		}
+		if (mode >= 1 && (ret = ls.record(d_rec, false))) return ret;
+		k_benc_finish<<<grid_of(rt, (int64_t)m * m, 4), HT, 0, rt.stream>>>(part2, nl, fres, nres, d_rec,
+		                                                                     hess ? d_hess2 : nullptr);
+		return checked(rt);
+	}
 
 	Sweep sw(rt, c);
 	sw.keep_final = hess;

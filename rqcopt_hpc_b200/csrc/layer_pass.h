@@ -1,0 +1,27 @@
+// Gates on disjoint wires applied to many states in one pass (see layer_pass.cu).
+#pragma once
+
+#include <vector>
+
+#include "rqc_common.cuh"
+#include "rqc_runtime.h"
+
+namespace rqc {
+
+struct LayerGate
+{
+	const double2* m;   // 16 entries, row-major (host)
+	int i, j;           // wires
+};
+
+// Whether the gates act on wires of their own.
+bool gates_disjoint(int L, const std::vector<LayerGate>& gates);
+
+// out = (the gates) in for ncols complex128 states of 2^L amplitudes one after another (device;
+// in place where in == out).  The gates act on disjoint wires; transposed: their transposes.
+//   columns: non-null: in is ignored, state c is (weighted) column c of *columns
+//   neg_conj: out = -conj(...)
+int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool transposed, const double2* in, double2* out,
+                int64_t ncols, const ColumnSource* columns = nullptr, bool neg_conj = false);
+
+}  // namespace rqc

@@ -11,6 +11,12 @@ from helpers import brickwall_instance, crandn, haar_unitary, random_tangent_dir
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _no_fixed_settings(gpu):
+    gpu.set_precision(gpu.PRECISION_C128)
+    gpu.set_autotune(True)   # settings that another test fixed keep evaluations on the pass engine
+
+
 def _check(got, ref, L):
     # f may nearly cancel: bound it by the size of its terms
     assert abs(got[0] - ref[0]) <= 1e-12 * 2 ** (L / 2)
