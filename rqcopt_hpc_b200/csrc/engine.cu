@@ -21,6 +21,7 @@
 // FP64), then per block, then over blocks with compensated summation.
 #include "engine.h"
 #include "engine_fused.h"
+#include "layer_pass.h"
 
 #include <stdio.h>
 #include <string.h>
@@ -787,15 +788,7 @@ int target_columns_device(Runtime& rt, const TargetSpec& t, int L, const ColumnS
 		// the pinned buffer is reused by the next chunk
 		return RQC_CUDA(cudaStreamSynchronize(rt.stream));
 	}
-	double2* P[2] = { p0, p1 };
-	for (int k = 0; k < t.ngates; k++) {
-		const bool first = k == 0, last = k == t.ngates - 1;
-		if ((ret = launch_apply<double>(rt, first ? 1 : 0, last ? 1 : 0, first ? nullptr : P[(k - 1) & 1],
-		                                last ? phi : P[k & 1], nullptr, to_gate<double>(t.gates + 16 * k),
-		                                make_pair_(L, t.wires[2 * k], t.wires[2 * k + 1]), L, ngroups, src, nullptr, 0)))
-			return ret;
-	}
-	return OK;
+	return circuit_apply(rt, L, t.ngates, t.gates, t.wires, nullptr, phi, p0, ncols, &src, true);
 }
 
 int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2* states, int64_t ncols, double2* phi,
@@ -834,15 +827,7 @@ int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2*
 		if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 		return RQC_CUDA(cudaStreamSynchronize(rt.stream));
 	}
-	double2* P[2] = { p0, p1 };
-	for (int k = 0; k < t.ngates; k++) {
-		const bool first = k == 0, last = k == t.ngates - 1;
-		if ((ret = launch_apply<double>(rt, 0, last ? 1 : 0, first ? states : P[(k - 1) & 1], last ? phi : P[k & 1],
-		                                nullptr, to_gate<double>(t.gates + 16 * k),
-		                                make_pair_(L, t.wires[2 * k], t.wires[2 * k + 1]), L, ngroups, ColumnSource{}, nullptr, 0)))
-			return ret;
-	}
-	return OK;
+	return circuit_apply(rt, L, t.ngates, t.gates, t.wires, states, phi, p0, ncols, nullptr, true);
 }
 
 int add_device(Runtime& rt, const double2* a, const double2* b, double2* c, long n)

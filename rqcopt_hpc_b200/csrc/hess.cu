@@ -644,11 +644,14 @@ struct LayerWires
 	Gate4<double> g;
 };
 
-// a thread per amplitude and column; own: write the tangents (not where only the gradient is wanted)
+// a thread per amplitude and column; own: write the tangents (not where only the gradient is
+// wanted); fpart (the circuit's last layer): f = phi . psi, per block
 __global__ void __launch_bounds__(256) k_hstates(const double2* __restrict__ psi, const double2* __restrict__ phi,
                                                  const __grid_constant__ LayerWires w, int64_t n,
-                                                 double2* __restrict__ own, double2* __restrict__ cot)
+                                                 double2* __restrict__ own, double2* __restrict__ cot,
+                                                 double2* __restrict__ fpart)
 {
+	double fx = 0, fy = 0;
 	for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
 		double2 t[16];
 		if (own) {
@@ -687,6 +690,24 @@ __global__ void __launch_bounds__(256) k_hstates(const double2* __restrict__ psi
 		}
 #pragma unroll
 		for (int e = 0; e < 16; e++) cot[e * n + a] = t[e];
+		if (fpart) {
+			const double2 p = phi[a], v = psi[a];
+			fx += p.x * v.x - p.y * v.y;
+			fy += p.x * v.y + p.y * v.x;
+		}
+	}
+	if (fpart) {
+		__shared__ double fr[2][8];
+		fx = warp_sum(fx);
+		fy = warp_sum(fy);
+		if ((threadIdx.x & 31) == 0) { fr[0][threadIdx.x >> 5] = fx; fr[1][threadIdx.x >> 5] = fy; }
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			double sx = 0, sy = 0;
+			for (int k = 0; k < 8; k++) { sx += fr[0][k]; sy += fr[1][k]; }
+			fpart[blockIdx.x].x += sx;
+			fpart[blockIdx.x].y += sy;
+		}
 	}
 }
 
@@ -778,20 +799,29 @@ struct LayerParts
 	int nsplit, ntile;   // tiles with the gradient's last
 };
 
-// raw sum e of tile x over the splits
-__device__ __forceinline__ double2 part_sum(const double2* __restrict__ part, const LayerParts& p, int x, int e)
+// Sums of tile blockIdx.x of layer blockIdx.y over the splits, into the tile's first split: 32
+// complex entries a block at a time, eight groups of threads sharing the splits.
+__global__ void __launch_bounds__(256) k_hsum(double2* __restrict__ part, const LayerParts* __restrict__ parts)
 {
-	const double2* q = part + p.off + (int64_t)x * p.nsplit * GSLOT + e;
+	__shared__ double2 red[8][32];
+	const LayerParts p = parts[blockIdx.y];
+	if ((int)blockIdx.x >= p.ntile) return;
+	const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+	double2* q = part + p.off + (int64_t)blockIdx.x * p.nsplit * GSLOT + 32 * blockIdx.z + lane;
 	double2 s = make_double2(0, 0);
-	for (int k = 0; k < p.nsplit; k++) s = cadd(s, q[(int64_t)k * GSLOT]);
-	return s;
+	for (int k = g; k < p.nsplit; k += 8) s = cadd(s, q[(int64_t)k * GSLOT]);
+	red[g][lane] = s;
+	__syncthreads();
+	if (g != 0) return;
+	for (int k = 1; k < 8; k++) s = cadd(s, red[k][lane]);
+	q[0] = s;
 }
 
-// Record of the layer sweep: block b handles the layer pair (a, l <= a) in row-major order of the
-// lower triangle; with_f: f from the last layer's gradient sums, sum_i R[i][i] = (gates per layer) phi.psi
+// Record of the layer sweep from k_hsum's sums: block b handles the layer pair (a, l <= a) in
+// row-major order of the lower triangle; fpart: partial sums of f, or null
 __global__ void __launch_bounds__(256) k_hrecord(const double2* __restrict__ part, const LayerParts* __restrict__ parts,
-                                                 const double2* __restrict__ ug, int nl, int per, int with_f, int hess,
-                                                 double2* __restrict__ rec)
+                                                 const double2* __restrict__ ug, int nl, const double2* __restrict__ fpart,
+                                                 int nfpart, int hess, double2* __restrict__ rec)
 {
 	__shared__ double2 R[256], V[16], D[16], H[256];
 	int a = 0, l = blockIdx.x;
@@ -799,9 +829,24 @@ __global__ void __launch_bounds__(256) k_hrecord(const double2* __restrict__ par
 	else { a = l; }
 	const int t = threadIdx.x, m = 16 * nl;
 	const LayerParts p = parts[a];
+	auto sum_at = [&](int x, int e) { return part[p.off + (int64_t)x * p.nsplit * GSLOT + e]; };
 	if (t < 16) {
 		V[t] = ug[16 * a + t];
-		if (l == a) R[t] = part_sum(part, p, p.ntile - 1, t * GN);
+		if (l == a) R[t] = sum_at(p.ntile - 1, t * GN);
+	}
+	if (blockIdx.x == 0 && fpart) {
+		double fx = 0, fy = 0;
+		for (int k = t; k < nfpart; k += 256) { fx += fpart[k].x; fy += fpart[k].y; }
+		__shared__ double fr[2][8];
+		fx = warp_sum(fx);
+		fy = warp_sum(fy);
+		if ((t & 31) == 0) { fr[0][t >> 5] = fx; fr[1][t >> 5] = fy; }
+		__syncthreads();
+		if (t < 2) {
+			double s = 0;
+			for (int k = 0; k < 8; k++) s += fr[t][k];
+			reinterpret_cast<double*>(rec)[t] = s;
+		}
 	}
 	__syncthreads();
 	auto times_conj = [&](const double2* r, int stride, int i, int c) {   // sum_j r[(i, j)] conj(G[j][c])
@@ -814,15 +859,11 @@ __global__ void __launch_bounds__(256) k_hrecord(const double2* __restrict__ par
 			D[t] = times_conj(R, 1, t >> 2, t & 3);
 			rec[1 + 16 * a + t] = D[t];
 		}
-		if (t == 0 && with_f && a == nl - 1) {
-			const double2 s = cadd(cadd(R[0], R[5]), cadd(R[10], R[15]));
-			rec[0] = make_double2(s.x / per, s.y / per);
-		}
 		__syncthreads();
 	}
 	if (!hess) return;
 	const int x = t >> 4, y = t & 15;
-	R[t] = part_sum(part, p, l / 2, x * GN + 16 * (l & 1) + y);   // column y of layer l in its tile
+	R[t] = sum_at(l / 2, x * GN + 16 * (l & 1) + y);   // column y of layer l in its tile
 	__syncthreads();
 	double2 h = times_conj(R + y, 16, x >> 2, x & 3);
 	double2* out = rec + 1 + 16 * nl;
@@ -1092,6 +1133,8 @@ struct LayerSweep
 	std::vector<LayerParts> parts;
 	double2* d_part = nullptr;
 	const double2* d_ug = nullptr;
+	double2* d_f = nullptr;
+	int nf = 0, most_tiles = 1;
 	const LayerParts* d_parts = nullptr;
 
 	LayerSweep(Runtime& r, const HessCircuit& hc, bool with_hess)
@@ -1111,16 +1154,20 @@ struct LayerSweep
 		for (int a = 0; a < nl; a++) {
 			const int ntile = hess ? (16 * (a + 1) + GN - 1) / GN + 1 : 1;
 			const int64_t fill = (3 * (int64_t)rt.num_sms + ntile - 1) / ntile, most = K / (16 * GW * 8);
+			most_tiles = std::max(most_tiles, ntile);
 			parts[a] = {off, (int)std::max<int64_t>(1, std::min(fill, most)), ntile};
 			off += (int64_t)ntile * parts[a].nsplit * GSLOT;
 		}
-		// sums | unit gates | slots
-		const size_t bytes = ((size_t)off + 16 * (size_t)nl) * sizeof(double2) + nl * sizeof(LayerParts);
+		// sums | unit gates | parts of f | slots
+		nf = grid_of(rt, K, 8);
+		const size_t bytes = ((size_t)off + 16 * (size_t)nl + nf) * sizeof(double2) + nl * sizeof(LayerParts);
 		int ret = ensure_device(rt.partials, bytes);
 		if (ret) return ret;
 		d_part = static_cast<double2*>(rt.partials.ptr);
 		double2* ug = d_part + off;
-		LayerParts* lp = reinterpret_cast<LayerParts*>(ug + 16 * nl);
+		d_f = ug + 16 * nl;
+		LayerParts* lp = reinterpret_cast<LayerParts*>(d_f + nf);
+		if ((ret = RQC_CUDA(cudaMemsetAsync(d_f, 0, nf * sizeof(double2), rt.stream)))) return ret;
 		d_ug = ug;
 		d_parts = lp;
 		if ((ret = RQC_CUDA(cudaMemcpyAsync(ug, c.ugates, 16 * (size_t)nl * sizeof(double2), cudaMemcpyHostToDevice, rt.stream))))
@@ -1163,7 +1210,8 @@ struct LayerSweep
 				w.bj[q] = (int8_t)(L - 1 - layers[a][q].j);
 			}
 			w.g = gate_of(c.ugates + 16 * a, false);
-			k_hstates<<<grid_of(rt, K, 8), 256, 0, rt.stream>>>(psi + a * K, phi + a * K, w, K, hess ? tan + 16 * a * K : nullptr, cot);
+			k_hstates<<<std::min(nf, grid_of(rt, K, 8)), 256, 0, rt.stream>>>(psi + a * K, phi + a * K, w, K, hess ? tan + 16 * a * K : nullptr, cot,
+			                                                    a == nl - 1 ? d_f : nullptr);
 			if (int e = checked(rt)) return e;
 			cudaEvent_t ev;
 			launch_begin(rt, KC_HESS, &ev);
@@ -1178,7 +1226,9 @@ struct LayerSweep
 	int record(double2* d_rec, bool with_f)
 	{
 		const int blocks = hess ? nl * (nl + 1) / 2 : nl;
-		k_hrecord<<<blocks, 256, 0, rt.stream>>>(d_part, d_parts, d_ug, nl, per, with_f ? 1 : 0, hess ? 1 : 0, d_rec);
+		k_hsum<<<dim3(most_tiles, nl, GSLOT / 32), 256, 0, rt.stream>>>(d_part, d_parts);
+		if (int e = checked(rt)) return e;
+		k_hrecord<<<blocks, 256, 0, rt.stream>>>(d_part, d_parts, d_ug, nl, with_f ? d_f : nullptr, nf, hess ? 1 : 0, d_rec);
 		return checked(rt);
 	}
 };

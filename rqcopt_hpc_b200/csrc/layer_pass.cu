@@ -64,12 +64,16 @@ __device__ __forceinline__ void apply4(const Gate4<double>& g, double2* x)
 	for (int r = 0; r < 4; r++) x[r * S] = y[r];
 }
 
+// Tiles of 2^11 amplitudes are double-buffered: three blocks per SM, each with the next tile's
+// loads (32 KB) in flight while it works on the current one; 2^12 ones alternate between two
+// blocks per SM.
 template <int TB, int IN, int OUT>
-__global__ void __launch_bounds__(1 << (TB - 4), TB == 11 ? 4 : 2)
+__global__ void __launch_bounds__(1 << (TB - 4), TB == 11 ? 3 : 2)
 k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 {
-	constexpr int NT = 1 << (TB - 4), A = 1 << TB;
-	extern __shared__ __align__(16) double2 tile[];
+	constexpr int NT = 1 << (TB - 4);
+	constexpr int NBUF = TB == 11 ? 2 : 1;
+	extern __shared__ __align__(16) double2 tiles[];
 	__shared__ uint32_t lo[64], hi[64];
 	const int tid = threadIdx.x;
 	if (tid < 64) {
@@ -94,21 +98,37 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 	}
 	__syncthreads();
 	const int64_t mask = ((int64_t)1 << a.L) - 1;
-	for (int64_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-		const int64_t at = deposit64(t, a.rest);
+	// tile t into buffer `tile`
+	auto fetch = [&](int64_t t, double2* tile) {
+		if (t < a.ntiles) {
+			const int64_t at = deposit64(t, a.rest);
 #pragma unroll
-		for (int k = 0; k < 16; k++) {
-			const int i = tid + k * NT;
-			const int64_t e = at + lo[i & 63] + hi[i >> 6];
-			if (IN == 0) {
-				const unsigned d = (unsigned)__cvta_generic_to_shared(tile + swz(i));
-				if (e < a.total) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(in + e) : "memory");
-			} else {
-				tile[swz(i)] = basis_amp<double>(a.src, e & mask, e >> a.L);
+			for (int k = 0; k < 16; k++) {
+				const int i = tid + k * NT;
+				const int64_t e = at + lo[i & 63] + hi[i >> 6];
+				if (IN == 0) {
+					const unsigned d = (unsigned)__cvta_generic_to_shared(tile + swz(i));
+					if (e < a.total) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(in + e) : "memory");
+				} else {
+					tile[swz(i)] = basis_amp<double>(a.src, e & mask, e >> a.L);
+				}
 			}
 		}
-		if (IN == 0) asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+		if (IN == 0) asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
+	if (NBUF == 2) fetch(blockIdx.x, tiles);
+	int buf = 0;
+	for (int64_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+		double2* tile = tiles + ((size_t)buf << TB);
+		if (NBUF == 1) fetch(t, tile);
+		if (IN == 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+		// this tile has landed, and every thread is done with the other buffer
 		__syncthreads();
+		if (NBUF == 2) {
+			buf ^= 1;
+			fetch(t + gridDim.x, tiles + ((size_t)buf << TB));
+		}
+		const int64_t at = deposit64(t, a.rest);
 #pragma unroll
 		for (int r = 0; r < ROUNDS; r++) {
 			if (2 * r < a.K) {
@@ -135,14 +155,14 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 			const int64_t e = at + lo[i & 63] + hi[i >> 6];
 			if (e < a.total) out[e] = OUT == 1 ? cneg_conj(tile[swz(i)]) : tile[swz(i)];
 		}
-		__syncthreads();
+		if (NBUF == 1) __syncthreads();
 	}
 }
 
 template <int TB, int IN, int OUT>
 int launch(Runtime& rt, const double2* in, double2* out, const PassArgs& a)
 {
-	constexpr int smem = (1 << TB) * (int)sizeof(double2);
+	constexpr int smem = (TB == 11 ? 2 : 1) * (1 << TB) * (int)sizeof(double2);
 	static int per_sm = 0;
 	if (!per_sm) {
 		if (int e = RQC_CUDA(cudaFuncSetAttribute(k_lpass<TB, IN, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
@@ -255,6 +275,33 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 		const int ret = TB == 12 ? launch_any<12>(rt, in_mode, out_mode, src, out, a) : launch_any<11>(rt, in_mode, out_mode, src, out, a);
 		if (ret) return ret;
 		first += K;
+	}
+	return OK;
+}
+
+int circuit_apply(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, const double2* in, double2* out,
+                  double2* scratch, int64_t ncols, const ColumnSource* columns, bool neg_conj)
+{
+	// runs of gates on wires of their own
+	std::vector<std::vector<LayerGate>> runs;
+	uint64_t used = 0;
+	for (int k = 0; k < ngates; k++) {
+		const int i = wires[2 * k], j = wires[2 * k + 1];
+		const uint64_t w = ((uint64_t)1 << i) | ((uint64_t)1 << j);
+		if (runs.empty() || (used & w)) {
+			runs.emplace_back();
+			used = 0;
+		}
+		runs.back().push_back({gates + 16 * (size_t)k, i, j});
+		used |= w;
+	}
+	const int n = (int)runs.size();
+	const double2* src = in;
+	for (int r = 0; r < n; r++) {
+		double2* dst = (n - 1 - r) % 2 == 0 ? out : scratch;
+		const bool last = r == n - 1;
+		if (int e = layer_apply(rt, L, runs[r], false, src, dst, ncols, r == 0 ? columns : nullptr, last && neg_conj)) return e;
+		src = dst;
 	}
 	return OK;
 }
