@@ -721,48 +721,93 @@ __device__ __forceinline__ void hdmma(double (&d)[2], double a, double b)
 constexpr int GW = 4;               // warps per block of the product
 constexpr int GN = 32;              // tangents per block: two layers
 constexpr int GSLOT = 16 * GN;      // complex sums per block
+constexpr int GRUN = 64;            // amplitudes a warp takes in a row: 1 KB of each state
+constexpr int GDEPTH = 5;           // steps of four amplitudes in a warp's queue
+constexpr int GSMEM = GW * (GDEPTH * 6 * 32 > GSLOT ? GDEPTH * 6 * 32 : GSLOT) * (int)sizeof(double2);
 
-// R[m][n] += sum_k A[m][k] B[n][k] (no conjugation) for 16 cotangent states A and tangents B, n =
-// 32 blockIdx.x ..: the last blockIdx.x takes psi as its only column.  K amplitudes per state;
-// blockIdx.y and the block's warps split them in runs of 16.  FP64 MMAs m8n8k4 on the real and
-// imaginary parts (four per complex 8 x 8 x 4 product): a lane's operand is the complex number it
-// loads, rows of four consecutive amplitudes (64 B), so the fragments come from memory as they
-// are, six 16-byte loads for 32 MMAs; no shared memory until the block's final sum.  Bound: the
-// tangents' one read from HBM at small 16 (a + 1), the FP64 pipe beyond.
+// R[m][n] += sum_k A[m][k] B[n][k] (no conjugation) for 16 cotangent states A and the ntan tangents
+// B, then psi as column ntan.  Block x takes four fragments of eight columns, K amplitudes per
+// state; blockIdx.y and the block's warps split them in runs of GRUN.  FP64 MMAs m8n8k4 on the real
+// and imaginary parts (four per complex 8 x 8 x 4 product): a lane's operand is the complex number
+// it loads, rows of four consecutive amplitudes (64 B), so the fragments come from memory as they
+// are, six 16-byte loads for 32 MMAs.  Bound: the FP64 pipe (32 MMAs per 3 KB), at few tangents the read from HBM.
+//
+// The operands wait in shared memory only as a queue: each lane copies its own six numbers of a
+// step (cp.async, GDEPTH - 1 steps ahead) and reads them back itself.  With the next step's in
+// registers instead, the warps waited for memory half the time (FP64 MMA pipe 47 % busy).
 __global__ void __launch_bounds__(32 * GW, 3)
 k_hgemm(const double2* __restrict__ A, const double2* __restrict__ B, const double2* __restrict__ psi, int64_t K, int ntan,
         double2* __restrict__ part, int add)
 {
-	__shared__ double2 red[GW][GSLOT];
+	extern __shared__ __align__(16) double2 hsm[];   // queue [GW][GDEPTH][6][32], then the block's sums [GW][GSLOT]
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int row = lane >> 2, kk = lane & 3;
-	const bool grad = blockIdx.x == gridDim.x - 1;
-	const int n0 = blockIdx.x * GN;
-	const int nf = grad ? 1 : min(4, (ntan - n0) / 8);   // fragments of 8 tangents
-	const double2* pa[2] = {A + row * K + kk, A + (row + 8) * K + kk};
-	const double2* pb[4];
+	const int nt = ntan / 8, f0 = 4 * blockIdx.x;   // fragments of tangents; this block's first
+	const int nf = min(4, nt + 1 - f0);
+	const double2* p[6] = {A + row * K + kk, A + (row + 8) * K + kk};
+	bool live[6] = {true, true};
 #pragma unroll
-	for (int f = 0; f < 4; f++) pb[f] = grad ? psi + kk : B + (int64_t)(n0 + (f < nf ? 8 * f : 0) + row) * K + kk;
-	const bool live = !grad || row == 0;   // the gradient tile has one column
+	for (int f = 0; f < 4; f++) {
+		const bool tangent = f0 + f < nt;
+		p[2 + f] = tangent ? B + (int64_t)(8 * (f0 + f) + row) * K + kk : psi + kk;
+		live[2 + f] = tangent || (f0 + f == nt && row == 0);
+	}
 	double re[2][4][2], im[2][4][2];
 #pragma unroll
 	for (int m = 0; m < 2; m++)
 #pragma unroll
 		for (int f = 0; f < 4; f++) re[m][f][0] = re[m][f][1] = im[m][f][0] = im[m][f][1] = 0;
-	const int64_t nrun = (K + 15) / 16, step = (int64_t)gridDim.y * GW;
-	for (int64_t run = (int64_t)blockIdx.y * GW + warp; run < nrun; run += step) {
+	const int64_t nrun = (K + GRUN - 1) / GRUN, stride = (int64_t)gridDim.y * GW;
+	const int64_t first = (int64_t)blockIdx.y * GW + warp;
+	const int nstep = first < nrun ? (int)((nrun - first + stride - 1) / stride) * (GRUN / 4) : 0;
+	double2* queue = hsm + (size_t)warp * GDEPTH * 6 * 32 + lane;
+	const unsigned qaddr = (unsigned)__cvta_generic_to_shared(queue);
+	int64_t knext = first * GRUN;   // amplitude of the next step to copy
+	auto fetch = [&](int n) {
+		if (n < nstep) {
+			const bool in = knext + kk < K;
+			const unsigned d = qaddr + (n % GDEPTH) * 6 * 32 * 16;
 #pragma unroll
-		for (int s = 0; s < 4; s++) {
-			const int64_t k = run * 16 + 4 * s;
-			const bool in = k + kk < K;
-			const double2 zero = make_double2(0, 0);
-			double2 x[2], y[4];
+			for (int f = 0; f < 6; f++) {
+				if (f - 2 >= nf) break;
+				const bool on = in && live[f];
+				const double2* src = on ? p[f] + knext : A;
+				asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d + f * 32 * 16), "l"(src), "r"(on ? 16 : 0)
+				             : "memory");
+			}
+			knext += (n % (GRUN / 4)) == GRUN / 4 - 1 ? (stride - 1) * GRUN + 4 : 4;
+		}
+		asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
 #pragma unroll
-			for (int m = 0; m < 2; m++) x[m] = in ? pa[m][k] : zero;
+	for (int n = 0; n < GDEPTH - 1; n++) fetch(n);
+	for (int n = 0; n < nstep; n++) {
+		asm volatile("cp.async.wait_group %0;\n" ::"n"(GDEPTH - 2) : "memory");
+		const double2* q = queue + (n % GDEPTH) * 6 * 32;
+		const double2 x[2] = {q[0], q[32]};
+		double2 y[4];
 #pragma unroll
-			for (int f = 0; f < 4; f++) y[f] = f < nf && in && live ? pb[f][k] : zero;
+		for (int f = 0; f < 4; f++) y[f] = f < nf ? q[(2 + f) * 32] : make_double2(0, 0);
+		fetch(n + GDEPTH - 1);   // into the slot read one step ago
+		// the two products into one accumulator sixteen MMAs apart
+		if (nf == 4) {
 #pragma unroll
-			for (int f = 0; f < 4; f++) {
+			for (int f = 0; f < 4; f++)
+#pragma unroll
+				for (int m = 0; m < 2; m++) {
+					hdmma(re[m][f], x[m].x, y[f].x);
+					hdmma(im[m][f], x[m].x, y[f].y);
+				}
+#pragma unroll
+			for (int f = 0; f < 4; f++)
+#pragma unroll
+				for (int m = 0; m < 2; m++) {
+					hdmma(re[m][f], -x[m].y, y[f].y);
+					hdmma(im[m][f], x[m].y, y[f].x);
+				}
+		} else {
+#pragma unroll
+			for (int f = 0; f < 3; f++) {
 				if (f >= nf) break;
 #pragma unroll
 				for (int m = 0; m < 2; m++) {
@@ -774,6 +819,9 @@ k_hgemm(const double2* __restrict__ A, const double2* __restrict__ B, const doub
 			}
 		}
 	}
+	asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+	__syncthreads();
+	double2 (*red)[GSLOT] = reinterpret_cast<double2 (*)[GSLOT]>(hsm);
 	// lane: rows row (+ 8 m), columns 8 f + 2 kk, + 1
 #pragma unroll
 	for (int m = 0; m < 2; m++)
@@ -796,7 +844,7 @@ k_hgemm(const double2* __restrict__ A, const double2* __restrict__ B, const doub
 struct LayerParts
 {
 	int64_t off;
-	int nsplit, ntile;   // tiles with the gradient's last
+	int nsplit, ntile;   // 16 (a + 1) tangents (none without a Hessian), then psi, 32 columns a tile
 };
 
 // Sums of tile blockIdx.x of layer blockIdx.y over the splits, into the tile's first split: 32
@@ -832,7 +880,10 @@ __global__ void __launch_bounds__(256) k_hrecord(const double2* __restrict__ par
 	auto sum_at = [&](int x, int e) { return part[p.off + (int64_t)x * p.nsplit * GSLOT + e]; };
 	if (t < 16) {
 		V[t] = ug[16 * a + t];
-		if (l == a) R[t] = sum_at(p.ntile - 1, t * GN);
+		if (l == a) {
+			const int n = hess ? 16 * (a + 1) : 0;   // psi's column
+			R[t] = sum_at(n / GN, t * GN + n % GN);
+		}
 	}
 	if (blockIdx.x == 0 && fpart) {
 		double fx = 0, fy = 0;
@@ -1146,14 +1197,19 @@ struct LayerSweep
 	}
 
 	// partial-sum slots for chunks of up to K amplitudes per state: enough splits to fill the
-	// GPU (three blocks of four warps per SM), none shorter than eight runs per warp
+	// GPU (three blocks of four warps per SM), none shorter than two runs per warp
 	int init(int64_t K)
 	{
+		static bool smem_set = false;
+		if (!smem_set) {
+			if (int e = RQC_CUDA(cudaFuncSetAttribute(k_hgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, GSMEM))) return e;
+			smem_set = true;
+		}
 		int64_t off = 0;
 		parts.resize(nl);
 		for (int a = 0; a < nl; a++) {
-			const int ntile = hess ? (16 * (a + 1) + GN - 1) / GN + 1 : 1;
-			const int64_t fill = (3 * (int64_t)rt.num_sms + ntile - 1) / ntile, most = K / (16 * GW * 8);
+			const int ntile = hess ? (16 * (a + 1) + 1 + GN - 1) / GN : 1;
+			const int64_t fill = (3 * (int64_t)rt.num_sms + ntile - 1) / ntile, most = K / (GRUN * GW * 2);
 			most_tiles = std::max(most_tiles, ntile);
 			parts[a] = {off, (int)std::max<int64_t>(1, std::min(fill, most)), ntile};
 			off += (int64_t)ntile * parts[a].nsplit * GSLOT;
@@ -1215,7 +1271,7 @@ struct LayerSweep
 			if (int e = checked(rt)) return e;
 			cudaEvent_t ev;
 			launch_begin(rt, KC_HESS, &ev);
-			k_hgemm<<<dim3(parts[a].ntile, parts[a].nsplit), 32 * GW, 0, rt.stream>>>(
+			k_hgemm<<<dim3(parts[a].ntile, parts[a].nsplit), 32 * GW, GSMEM, rt.stream>>>(
 				cot, tan, psi + a * K, K, hess ? 16 * (a + 1) : 0, d_part + parts[a].off, add ? 1 : 0);
 			launch_end(rt, KC_HESS, ev);
 			if (int e = RQC_CUDA(cudaGetLastError())) return e;
