@@ -26,26 +26,26 @@ struct PassArgs
 {
 	Gate4<double> g[MAXG];
 	int K, L;
-	int8_t bit[ROUNDS][4];      // tile bits of wires i, j of the round's first and second gate (or fillers)
+	int step[ROUNDS][4];        // places (bytes) of the tile bits of wires i, j of a round's first and second gate (or fillers)
 	int8_t pos[ROUNDS][8];      // tile bits of a thread's index bits
 	int8_t tbit[12];            // index bit of tile bit b
-	uint64_t rest;              // index bits that are not tile bits
+	uint32_t koff[16];          // index bits of the tile's top four bits
+	// tile number to index bits outside the tile: nseg runs of consecutive bits, bits seg_from ..
+	// of the number to bits seg_to .. of the index, seg_mask wide
+	int nseg;
+	int8_t seg_from[13], seg_to[13];
+	uint64_t seg_mask[13];
 	int64_t total, ntiles;      // amplitudes, tiles
 	ColumnSource src;
 };
 
 // place of tile amplitude i: its 16-byte word within a 128-byte line XORed with the bits above
-__device__ __forceinline__ int swz(int i) { return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9)) & 7); }
+__host__ __device__ __forceinline__ constexpr int swz(int i) { return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9)) & 7); }
 
-__device__ __forceinline__ int64_t deposit64(int64_t v, uint64_t mask)
+__device__ __forceinline__ int64_t tile_base(const PassArgs& a, int64_t t)
 {
 	int64_t r = 0;
-	while (v && mask) {
-		const uint64_t low = mask & (0 - mask);
-		if (v & 1) r |= (int64_t)low;
-		v >>= 1;
-		mask ^= low;
-	}
+	for (int k = 0; k < a.nseg; k++) r |= (int64_t)(((uint64_t)t >> a.seg_from[k]) & a.seg_mask[k]) << a.seg_to[k];
 	return r;
 }
 
@@ -53,40 +53,53 @@ __device__ __forceinline__ int64_t deposit64(int64_t v, uint64_t mask)
 template <int S>
 __device__ __forceinline__ void apply4(const Gate4<double>& g, double2* x)
 {
+	// eight sums side by side, each touched every eighth FMA
 	double2 y[4];
 #pragma unroll
-	for (int r = 0; r < 4; r++) {
-		y[r] = cmul(g.m[4 * r], x[0]);
+	for (int r = 0; r < 4; r++) y[r] = make_double2(g.m[4 * r].x * x[0].x, g.m[4 * r].x * x[0].y);
 #pragma unroll
-		for (int c = 1; c < 4; c++) y[r] = cfma(g.m[4 * r + c], x[c * S], y[r]);
+	for (int r = 0; r < 4; r++) {
+		y[r].x = fma(-g.m[4 * r].y, x[0].y, y[r].x);
+		y[r].y = fma(g.m[4 * r].y, x[0].x, y[r].y);
+	}
+#pragma unroll
+	for (int c = 1; c < 4; c++) {
+#pragma unroll
+		for (int r = 0; r < 4; r++) {
+			y[r].x = fma(g.m[4 * r + c].x, x[c * S].x, y[r].x);
+			y[r].y = fma(g.m[4 * r + c].x, x[c * S].y, y[r].y);
+		}
+#pragma unroll
+		for (int r = 0; r < 4; r++) {
+			y[r].x = fma(-g.m[4 * r + c].y, x[c * S].y, y[r].x);
+			y[r].y = fma(g.m[4 * r + c].y, x[c * S].x, y[r].y);
+		}
 	}
 #pragma unroll
 	for (int r = 0; r < 4; r++) x[r * S] = y[r];
 }
 
-// Tiles of 2^11 amplitudes are double-buffered: three blocks per SM, each with the next tile's
-// loads (32 KB) in flight while it works on the current one; 2^12 ones alternate between two
-// blocks per SM.
+// Shared-memory addresses are byte offsets into the tile (places * 16), so that a member's is one
+// XOR away from its neighbour's.  An FP64 instruction holds the issue port for two cycles, so every other instruction counts: with
+// 64-bit index arithmetic per access there were as many of those as FMAs (18 TFLOP/s at any
+// occupancy, with one or two tiles per block; 19-20 now).  Measured on 2^26 amplitudes, 2 GB a pass
+// (read and write): one or two gates 6.2 TB/s, the copy bandwidth; four 4.8 TB/s, 19 TFLOP/s; five at
+// L = 10 4.1 TB/s, 21 TFLOP/s.  Four blocks per SM at 128 registers: five or six spill and lose 5-30 %,
+// three with the next tile prefetched lose 4 %.
 template <int TB, int IN, int OUT>
-__global__ void __launch_bounds__(1 << (TB - 4), TB == 11 ? 3 : 2)
+__global__ void __launch_bounds__(1 << (TB - 4), TB == 11 ? 4 : 2)
 k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 {
 	constexpr int NT = 1 << (TB - 4);
-	constexpr int NBUF = TB == 11 ? 2 : 1;
-	extern __shared__ __align__(16) double2 tiles[];
-	__shared__ uint32_t lo[64], hi[64];
+	extern __shared__ __align__(16) char tile[];
 	const int tid = threadIdx.x;
-	if (tid < 64) {
-		uint32_t o = 0, p = 0;
-		for (int b = 0; b < 6; b++)
-			if ((tid >> b) & 1) {
-				o |= 1u << a.tbit[b];
-				if (6 + b < TB) p |= 1u << a.tbit[6 + b];
-			}
-		lo[tid] = o;
-		hi[tid] = p;
-	}
-	// first amplitude (place) of this thread's set in each round
+	auto at_smem = [&](int byte) -> double2& { return *reinterpret_cast<double2*>(tile + byte); };
+	// this thread's amplitudes of a tile are tid + k NT: index offset own + a.koff[k], place swz(tid) ^ swz(k NT)
+	uint32_t own = 0;
+#pragma unroll
+	for (int b = 0; b < TB - 4; b++) own |= (uint32_t)((tid >> b) & 1) << a.tbit[b];
+	const int place = swz(tid) << 4;
+	// first amplitude of this thread's set in each round
 	int base[ROUNDS];
 #pragma unroll
 	for (int r = 0; r < ROUNDS; r++) {
@@ -94,75 +107,62 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 		if (2 * r < a.K)
 #pragma unroll
 			for (int b = 0; b < TB - 4; b++) v |= ((tid >> b) & 1) << a.pos[r][b];
-		base[r] = swz(v);
+		base[r] = swz(v) << 4;
 	}
-	__syncthreads();
-	const int64_t mask = ((int64_t)1 << a.L) - 1;
-	// tile t into buffer `tile`
-	auto fetch = [&](int64_t t, double2* tile) {
-		if (t < a.ntiles) {
-			const int64_t at = deposit64(t, a.rest);
+	for (int64_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+		const int64_t at = tile_base(a, t) + own;
+		const bool whole = at + a.koff[15] < a.total;   // only tiles of contiguous columns can be cut off
+		if (IN == 0) {
+			const double2* src = in + at;
+			const unsigned dst = (unsigned)__cvta_generic_to_shared(tile);
+#pragma unroll
+			for (int k = 0; k < 16; k++)
+				if (whole || at + a.koff[k] < a.total)
+					asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (place ^ (swz(k * NT) << 4))),
+					             "l"(src + a.koff[k])
+					             : "memory");
+			asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+		} else {
+			const int64_t mask = ((int64_t)1 << a.L) - 1;
 #pragma unroll
 			for (int k = 0; k < 16; k++) {
-				const int i = tid + k * NT;
-				const int64_t e = at + lo[i & 63] + hi[i >> 6];
-				if (IN == 0) {
-					const unsigned d = (unsigned)__cvta_generic_to_shared(tile + swz(i));
-					if (e < a.total) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(in + e) : "memory");
-				} else {
-					tile[swz(i)] = basis_amp<double>(a.src, e & mask, e >> a.L);
-				}
+				const int64_t e = at + a.koff[k];
+				at_smem(place ^ (swz(k * NT) << 4)) = basis_amp<double>(a.src, e & mask, e >> a.L);
 			}
 		}
-		if (IN == 0) asm volatile("cp.async.commit_group;\n" ::: "memory");
-	};
-	if (NBUF == 2) fetch(blockIdx.x, tiles);
-	int buf = 0;
-	for (int64_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-		double2* tile = tiles + ((size_t)buf << TB);
-		if (NBUF == 1) fetch(t, tile);
-		if (IN == 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-		// this tile has landed, and every thread is done with the other buffer
 		__syncthreads();
-		if (NBUF == 2) {
-			buf ^= 1;
-			fetch(t + gridDim.x, tiles + ((size_t)buf << TB));
-		}
-		const int64_t at = deposit64(t, a.rest);
 #pragma unroll
 		for (int r = 0; r < ROUNDS; r++) {
 			if (2 * r < a.K) {
-				const int i0 = swz(1 << a.bit[r][0]), j0 = swz(1 << a.bit[r][1]);
-				const int i1 = swz(1 << a.bit[r][2]), j1 = swz(1 << a.bit[r][3]);
-				double2 x[16];   // [member of the first gate][member of the second]
+				const int s0 = a.step[r][0], s1 = a.step[r][1], s2 = a.step[r][2], s3 = a.step[r][3];
+				auto mem = [&](int k) { return base[r] ^ (k & 8 ? s0 : 0) ^ (k & 4 ? s1 : 0) ^ (k & 2 ? s2 : 0) ^ (k & 1 ? s3 : 0); };
+				double2 x[16];
 #pragma unroll
-				for (int m = 0; m < 16; m++)
-					x[m] = tile[base[r] ^ (m & 8 ? i0 : 0) ^ (m & 4 ? j0 : 0) ^ (m & 2 ? i1 : 0) ^ (m & 1 ? j1 : 0)];
+				for (int k = 0; k < 16; k++) x[k] = at_smem(mem(k));
 #pragma unroll
-				for (int m = 0; m < 4; m++) apply4<4>(a.g[2 * r], x + m);
+				for (int k = 0; k < 4; k++) apply4<4>(a.g[2 * r], x + k);
 				if (2 * r + 1 < a.K)
 #pragma unroll
-					for (int m = 0; m < 4; m++) apply4<1>(a.g[2 * r + 1], x + 4 * m);
+					for (int k = 0; k < 4; k++) apply4<1>(a.g[2 * r + 1], x + 4 * k);
 #pragma unroll
-				for (int m = 0; m < 16; m++)
-					tile[base[r] ^ (m & 8 ? i0 : 0) ^ (m & 4 ? j0 : 0) ^ (m & 2 ? i1 : 0) ^ (m & 1 ? j1 : 0)] = x[m];
+				for (int k = 0; k < 16; k++) at_smem(mem(k)) = x[k];
 				__syncthreads();
 			}
 		}
+		double2* dst = out + at;
 #pragma unroll
 		for (int k = 0; k < 16; k++) {
-			const int i = tid + k * NT;
-			const int64_t e = at + lo[i & 63] + hi[i >> 6];
-			if (e < a.total) out[e] = OUT == 1 ? cneg_conj(tile[swz(i)]) : tile[swz(i)];
+			const double2 v = at_smem(place ^ (swz(k * NT) << 4));
+			if (whole || at + a.koff[k] < a.total) dst[a.koff[k]] = OUT == 1 ? cneg_conj(v) : v;
 		}
-		if (NBUF == 1) __syncthreads();
+		__syncthreads();
 	}
 }
 
 template <int TB, int IN, int OUT>
 int launch(Runtime& rt, const double2* in, double2* out, const PassArgs& a)
 {
-	constexpr int smem = (TB == 11 ? 2 : 1) * (1 << TB) * (int)sizeof(double2);
+	constexpr int smem = (1 << TB) * (int)sizeof(double2);
 	static int per_sm = 0;
 	if (!per_sm) {
 		if (int e = RQC_CUDA(cudaFuncSetAttribute(k_lpass<TB, IN, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
@@ -230,14 +230,33 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 				local[b] = nb;
 				a.tbit[nb++] = (int8_t)b;
 			}
-		a.rest = ~bits;
+		for (int k = 0; k < 16; k++) {
+			a.koff[k] = 0;
+			for (int b = 0; b < 4; b++)
+				if ((k >> b) & 1) a.koff[k] |= 1u << a.tbit[TB - 4 + b];
+		}
+		a.nseg = 0;
+		for (int b = 0, from = 0; b < 64;) {
+			if ((bits >> b) & 1) {
+				b++;
+				continue;
+			}
+			int e = b;
+			while (e < 64 && !((bits >> e) & 1)) e++;
+			a.seg_from[a.nseg] = (int8_t)from;
+			a.seg_to[a.nseg] = (int8_t)b;
+			a.seg_mask[a.nseg++] = e - b >= 64 ? ~(uint64_t)0 : ((uint64_t)1 << (e - b)) - 1;
+			from += e - b;
+			b = e;
+		}
 		const int64_t tile = (int64_t)1 << TB;
 		a.ntiles = (a.total + tile - 1) / tile;
 		for (int r = 0; 2 * r < K; r++) {
 			uint32_t used = 0;
 			auto take = [&](int slot, int wire) {
-				a.bit[r][slot] = (int8_t)local[L - 1 - wire];
-				used |= 1u << a.bit[r][slot];
+				const int b = local[L - 1 - wire];
+				a.step[r][slot] = swz(1 << b) << 4;
+				used |= 1u << b;
 			};
 			take(0, gates[first + 2 * r].i);
 			take(1, gates[first + 2 * r].j);
@@ -247,7 +266,7 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 			} else {   // a gate alone: the set takes the two highest other bits
 				for (int s = 2, b = TB - 1; s < 4; b--)
 					if (!((used >> b) & 1)) {
-						a.bit[r][s++] = (int8_t)b;
+						a.step[r][s++] = swz(1 << b) << 4;
 						used |= 1u << b;
 					}
 			}
@@ -275,6 +294,33 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 		const int ret = TB == 12 ? launch_any<12>(rt, in_mode, out_mode, src, out, a) : launch_any<11>(rt, in_mode, out_mode, src, out, a);
 		if (ret) return ret;
 		first += K;
+	}
+	return OK;
+}
+
+int circuit_apply_reordered(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, int most,
+                            const double2* in, double2* out)
+{
+	// Each pass takes, in order, the gates whose wires no gate left behind shares (they commute with
+	// those) and no gate of the pass, up to `most`.
+	std::vector<char> done(ngates, 0);
+	const double2* src = in;
+	for (int left = ngates; left > 0;) {
+		std::vector<LayerGate> pass;
+		uint64_t taken = 0;   // wires of the pass and of the gates left behind
+		for (int k = 0; k < ngates && (int)pass.size() < most; k++) {
+			if (done[k]) continue;
+			const int i = wires[2 * k], j = wires[2 * k + 1];
+			const uint64_t w = ((uint64_t)1 << i) | ((uint64_t)1 << j);
+			if (!(taken & w)) {
+				pass.push_back({gates + 16 * (size_t)k, i, j});
+				done[k] = 1;
+				left--;
+			}
+			taken |= w;
+		}
+		if (int e = layer_apply(rt, L, pass, false, src, out, 1)) return e;
+		src = out;
 	}
 	return OK;
 }

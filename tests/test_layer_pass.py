@@ -1,0 +1,55 @@
+"""Passes over complex128 states with gates on wires of their own (csrc/layer_pass.cu): tiles larger
+and smaller than the state, passes of one to six gates, reordering where gates commute and not
+where they do not.  Each gate adds at most a few units of 1.1e-16 of the state's norm: the bar of
+1e-13 holds for the at most 40 gates here with two orders to spare."""
+import numpy as np
+import pytest
+
+from helpers import brickwall_instance, crandn, haar_unitary, periodic_perms
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _no_fixed_settings(gpu):
+    gpu.set_autotune(True)
+    yield
+    gpu.set_autotune(True)
+
+
+@pytest.mark.parametrize("L", [10, 11, 12, 13, 14])
+@pytest.mark.parametrize("G,near", [(1, False), (2, False), (17, False), (40, False), (23, True)])
+@pytest.mark.parametrize("per_pass", [0, 2, 3])
+def test_circuits_match_the_oracle(gpu, oracle, L, G, near, per_pass):
+    rng = np.random.default_rng(100 * L + G)
+    gates = np.stack([haar_unitary(rng) for _ in range(G)])
+    pool = 4 if near else L   # near: every gate shares wires with its neighbours in the sequence
+    wires = np.array([rng.choice(pool, 2, replace=False) for _ in range(G)], np.int32)
+    psi = crandn(1 << L, rng)
+    if per_pass:
+        gpu.set_gates_per_pass(per_pass)
+    got = gpu.apply_quantum_circuit(gates, wires, psi)
+    ref = oracle.apply_quantum_circuit(gates, wires, psi)
+    assert np.linalg.norm(got - ref) <= 1e-13 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("L", [2, 4, 6, 8, 10, 12, 14])
+@pytest.mark.parametrize("ns", [1, 3])
+def test_sampled_sums_take_layers_of_every_length(gpu, oracle, L, ns):
+    vlist, perms, tvlist, tperms = brickwall_instance(L, 2, L, 2, L + 1)
+    got = gpu.brickwall_unitary_target_gradient_hessian_sampling(gpu.Target(brickwall=(tvlist, tperms)), vlist, perms, L, ns,
+                                                                 gpu.seed_rng_state(3))
+    ref = oracle.brickwall_unitary_target_gradient_hessian_sampling(oracle.target("brickwall", (tvlist, tperms)), vlist, perms,
+                                                                    L, ns, oracle.seed_rng_state(3))
+    assert abs(got[0] - ref[0]) <= 1e-12 * 2 ** L
+    for a, b in zip(got[1:], ref[1:]):
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
+
+
+def test_hessians_of_gates_that_are_not_unitary(gpu, oracle):
+    rng = np.random.default_rng(1)
+    v, tv, perms = crandn((3, 4, 4), rng), crandn((2, 4, 4), rng), periodic_perms(6, 3)
+    got = gpu.brickwall_unitary_target_gradient_hessian(gpu.Target(brickwall=(tv, perms[:2])), v, perms, 6)
+    ref = oracle.brickwall_unitary_target_gradient_hessian(oracle.target("brickwall", (tv, perms[:2])), v, perms, 6)
+    for a, b in zip(got, ref):
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
