@@ -301,23 +301,38 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 int circuit_apply_reordered(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, int most,
                             const double2* in, double2* out)
 {
-	// Each pass takes, in order, the gates whose wires no gate left behind shares (they commute with
-	// those) and no gate of the pass, up to `most`.
-	std::vector<char> done(ngates, 0);
-	const double2* src = in;
-	for (int left = ngates; left > 0;) {
-		std::vector<LayerGate> pass;
-		uint64_t taken = 0;   // wires of the pass and of the gates left behind
-		for (int k = 0; k < ngates && (int)pass.size() < most; k++) {
-			if (done[k]) continue;
-			const int i = wires[2 * k], j = wires[2 * k + 1];
-			const uint64_t w = ((uint64_t)1 << i) | ((uint64_t)1 << j);
-			if (!(taken & w)) {
-				pass.push_back({gates + 16 * (size_t)k, i, j});
-				done[k] = 1;
-				left--;
+	// A gate waits for the last gates before it on its two wires; gates that wait for none commute
+	// and act on wires of their own.  Each pass takes the `most` of them with the longest chains of
+	// gates behind them: taken in the order of the circuit, chains are left over at the end that
+	// cost a pass per gate or two (64 gates on random pairs of 27 wires: 16 passes of four instead
+	// of 16-19).
+	std::vector<int> waits(ngates, 0), height(ngates, 1), last(L, -1);
+	std::vector<std::vector<int>> next(ngates);
+	for (int k = 0; k < ngates; k++)
+		for (int e = 0; e < 2; e++) {
+			const int w = wires[2 * k + e];
+			if (last[w] >= 0) {
+				next[last[w]].push_back(k);
+				waits[k]++;
 			}
-			taken |= w;
+			last[w] = k;
+		}
+	for (int k = ngates - 1; k >= 0; k--)
+		for (int m : next[k]) height[k] = std::max(height[k], height[m] + 1);
+	std::vector<int> ready;
+	for (int k = 0; k < ngates; k++)
+		if (!waits[k]) ready.push_back(k);
+	const double2* src = in;
+	while (!ready.empty()) {
+		std::stable_sort(ready.begin(), ready.end(), [&](int x, int y) { return height[x] > height[y]; });
+		const int n = std::min<int>(most, (int)ready.size());
+		std::vector<LayerGate> pass;
+		std::vector<int> taken(ready.begin(), ready.begin() + n);
+		ready.erase(ready.begin(), ready.begin() + n);
+		for (int k : taken) {
+			pass.push_back({gates + 16 * (size_t)k, wires[2 * k], wires[2 * k + 1]});
+			for (int m : next[k])
+				if (--waits[m] == 0) ready.push_back(m);
 		}
 		if (int e = layer_apply(rt, L, pass, false, src, out, 1)) return e;
 		src = out;

@@ -390,14 +390,13 @@ int apply_circuit_fused_t(Runtime& rt, int L, int ngates, const double2* gates, 
 
 // out = C in for one statevector (complex128), maxk gates per pass.  16-byte aligned states take
 // the passes of layer_pass.cu with the gates reordered where they commute: L = 27, 64 gates on
-// random pairs 14.9 ms against 22.5 ms of 64 KiB bulk-copied tiles with four consecutive gates
-// (256 copies of 256 B a tile each way, and a shared-memory round trip per gate).  Five gates a
-// pass, as a tile's bits allow, unless the caller fixed their number.
+// random pairs 16.1 ms against 21.4 ms of 64 KiB bulk-copied tiles with four consecutive gates
+// (256 copies of 256 B a tile each way, and a shared-memory round trip per gate).
 int apply_circuit_fused_device(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
                                const double2* d_in, double2* d_out, int maxk)
 {
 	if (((uintptr_t)d_in % 16) == 0 && ((uintptr_t)d_out % 16) == 0)
-		return circuit_apply_reordered(rt, L, ngates, gates, wires, rt.pin_gpp ? std::min(maxk, 5) : 5, d_in, d_out);
+		return circuit_apply_reordered(rt, L, ngates, gates, wires, maxk, d_in, d_out);
 	return apply_circuit_fused_t<double>(rt, L, ngates, gates, wires, d_in, d_out, maxk);
 }
 
