@@ -62,6 +62,10 @@ struct PassGeom
 	int64_t ntiles;        // row tiles (2^(L-NB)) x column groups
 	ColumnSource src;      // the chunk's columns
 	uint32_t rest_mask;    // state row bits that are not tile bits
+	// complex128: groups of gates on wires of their own, in the order of application: group l is
+	// gates group[l] .. group[l + 1] - 1
+	int ngroups;
+	int group[MAXK + 1];
 };
 
 template <typename T> struct PassGates { Gate4<T> g[MAXK]; Gate4<T> z[MAXK]; };
@@ -657,27 +661,45 @@ __global__ void __launch_bounds__(NTR, 1) k3_rev(const double2* __restrict__ psi
 	}
 }
 
-// Sum raw 8x8 partials over blocks (compensated) and fold them into complex dG, HZ:
+// The gate that a slot of partial sums belongs to, with conj(G) and -W, W = G^+ Z G^+, for sums taken
+// at the gate's output.
+struct SlotGate
+{
+	double2 gc[16], wn[16];
+	int gate, pad[3];
+};
+
+// Sum raw 8x8 partials over blocks (compensated) and fold them into complex sums; at_output: these
+// are R1, R2 at the gate's output, dG = R1 conj(G) and HZ = R2 conj(G) - R1 W^T.  Folding:
 // X[r][c] = (R[2r][2c] - R[2r+1][2c+1]) + i (R[2r][2c+1] + R[2r+1][2c]).
 __global__ void __launch_bounds__(RED_GROUPS * NPART3)
 k3_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* __restrict__ fpart, int nblk_f,
-          int with_hvp, double2* __restrict__ out)
+          int with_hvp, const SlotGate* __restrict__ slots, int at_output, double2* __restrict__ out)
 {
 	__shared__ double red[RED_GROUPS][NPART3];
 	__shared__ double raw[NPART3];
+	__shared__ double2 sums[32];
 	const int s = blockIdx.x, t = threadIdx.x % NPART3;
 	const bool first = threadIdx.x < NPART3;
 	if (s < nslots) {
 		const double sum = block_column_sum<NPART3>(part + (size_t)s * nblk * NPART3 + t, nblk, NPART3, red);
 		if (first) raw[t] = sum;
 		__syncthreads();
-		if (first && t < 32) {
-			const int which = t >> 4, e = t & 15, r = e >> 2, c = e & 3;
-			if (which == 1 && !with_hvp) return;
+		if (threadIdx.x < 32) {
+			const int which = t >> 4, e = t & 15, r = e >> 2, c = e & 3, g = slots[s].gate;
 			const double* R = raw + 64 * which;
-			const double re = R[(2 * r) * 8 + 2 * c] - R[(2 * r + 1) * 8 + 2 * c + 1];
-			const double im = R[(2 * r) * 8 + 2 * c + 1] + R[(2 * r + 1) * 8 + 2 * c];
-			out[1 + 16 * (size_t)(which ? nslots + s : s) + e] = make_double2(re, im);
+			double2 v = make_double2(R[(2 * r) * 8 + 2 * c] - R[(2 * r + 1) * 8 + 2 * c + 1],
+			                         R[(2 * r) * 8 + 2 * c + 1] + R[(2 * r + 1) * 8 + 2 * c]);
+			if (at_output) {
+				sums[t] = v;
+				__syncwarp();
+				v = make_double2(0, 0);
+				for (int j = 0; j < 4; j++) {
+					v = cfma(sums[16 * which + 4 * r + j], slots[s].gc[4 * j + c], v);
+					if (which) v = cfma(sums[4 * r + j], slots[s].wn[4 * c + j], v);
+				}
+			}
+			if (which == 0 || with_hvp) out[1 + 16 * (size_t)(which ? nslots + g : g) + e] = v;
 		}
 	} else {
 		const double sum = block_column_sum<NPART3>(reinterpret_cast<const double*>(fpart) + (t & 1), nblk_f, 2, red);
@@ -1449,87 +1471,42 @@ __global__ void __launch_bounds__(NT5, 2) k5_rev(const float2* __restrict__ psi,
 	}
 }
 
-// ------------------------------------------------------------------------------ complex128 reverse pass, adjoint reconstruction
+// ------------------------------------------------------------------------------ complex128 reverse pass, sums at the output
 
-// Per-gate operands of the reconstructing complex128 reverse pass, formed on the host in
-// FP64: gc = conj(G) (as a row-vector operand it applies G^+) and wn = -W, W = G^+ Z G^+.
-struct PassAdj { Gate4<double> gc[MAXK]; Gate4<double> wn[MAXK]; };
-
-// Operands of one gate of the reconstructing reverse pass: B fragments of conj(G) (the
-// adjoint gate as a row-vector operand), -W, G and Z, from the gate block of shared memory
-// ([G, Z, conj(G), -W], 16 complex each).
+// Units u0 and u1 of a gate's outer sums over eight groups each (two group bases times four
+// columns): R1 += phi (x) psi, R2 += phi (x) dpsi + dphi (x) psi, raw 8x8 sums.
 template <bool TAN>
-struct RevGate
+__device__ __forceinline__ void outer_unit(const double* Psi, const double* dPsi, const double* Phi, const double* dPhi,
+                                           int u, const StepLane& sl, int lane, double (&g)[2], double (&h)[2])
 {
-	StepLane sl;
-	double bc[2], bw[2] = {0, 0}, bg[2], bz[2] = {0, 0};
-	bool first_gate, last_gate;
-	__device__ __forceinline__ RevGate(const double2* sg, int k, int K, bool first, bool last, const PassGeom& pg,
-	                                   int lane)
-		: sl(pg.gi[k], pg.gj[k], lane), first_gate(first && k == K - 1), last_gate(last && k == 0)
-	{
-		bfrag(sg + 64 * k + 32, false, lane, bc);
-		if (TAN) bfrag(sg + 64 * k + 48, true, lane, bw);
-		bfrag(sg + 64 * k, false, lane, bg);
-		if (TAN) bfrag(sg + 64 * k + 16, false, lane, bz);
-	}
-};
-
-// One gate of the reconstructing reverse pass on two units (the second unless has1 is
-// false): rebuild the state (and tangent) entering the gate, in place; add the outer
-// sums dG += phi (x) psi, HZ += phi (x) dpsi + dphi (x) psi over the units' groups, into
-// fresh partials first (short MMA chains); move phi, dphi through the gate in place.
-template <bool TAN>
-__device__ __forceinline__ void rev_gate6(const RevGate<TAN>& g, const UnitBases& ub, bool has1, double2* Psi,
-                                          double2* dPsi, double2* Phi, double2* dPhi, double& g0, double& g1,
-                                          double& h0, double& h1, int lane)
-{
-	const double* fPsi = reinterpret_cast<const double*>(Psi);
-	const double* fPhi = reinterpret_cast<const double*>(Phi);
-	const double* fdPsi = reinterpret_cast<const double*>(dPsi);
-	const double* fdPhi = reinterpret_cast<const double*>(dPhi);
-	const int hs = lane >> 4;
-	const int bs0 = hs ? ub.b01 : ub.b00, bs1 = hs ? ub.b11 : ub.b10;
-	const StepLane& sl = g.sl;
-	if (TAN && !g.last_gate)
-		apply_bases2<true>(fPsi, fdPsi, Psi, dPsi, bs0, bs1, has1, sl, g.bc, g.bw, false, lane);
-	else
-		apply_bases2<false>(fPsi, nullptr, Psi, nullptr, bs0, bs1, has1, sl, g.bc, g.bw, false, lane);
-	__syncwarp();
-	double tg[2][2] = {{0, 0}, {0, 0}}, th[2][2] = {{0, 0}, {0, 0}};
-#pragma unroll
-	for (int q = 0; q < 2; q++) {
-		if (q == 1 && !has1) break;
-		const int base0 = q ? ub.b10 : ub.b00, base1 = q ? ub.b11 : ub.b01;
-		const int i0 = sidx(base0 | sl.m_outer, lane & 3) * 2 + sl.part_outer;
-		const int i1 = sidx(base1 | sl.m_outer, lane & 3) * 2 + sl.part_outer;
-		const double p0 = fPhi[i0], x0 = fPsi[i0], p1 = fPhi[i1], x1 = fPsi[i1];
-		double dx0 = 0, dx1 = 0, dp0 = 0, dp1 = 0;
-		if (TAN && !g.last_gate) { dx0 = fdPsi[i0]; dx1 = fdPsi[i1]; }
-		if (TAN && !g.first_gate) { dp0 = fdPhi[i0]; dp1 = fdPhi[i1]; }
-		dmma(tg[q][0], tg[q][1], p0, x0);
-		if (TAN && !g.last_gate) dmma(th[q][0], th[q][1], p0, dx0);
-		dmma(tg[q][0], tg[q][1], p1, x1);
-		if (TAN && !g.last_gate) dmma(th[q][0], th[q][1], p1, dx1);
-		if (TAN && !g.first_gate) {
-			dmma(th[q][0], th[q][1], dp0, x0);
-			dmma(th[q][0], th[q][1], dp1, x1);
-		}
-	}
-	g0 += tg[0][0] + tg[1][0];
-	g1 += tg[0][1] + tg[1][1];
+	const int i0 = sidx(insert2(2 * u, sl.lo, sl.hi) | sl.m_outer, lane & 3) * 2 + sl.part_outer;
+	const int i1 = sidx(insert2(2 * u + 1, sl.lo, sl.hi) | sl.m_outer, lane & 3) * 2 + sl.part_outer;
+	const double p0 = Phi[i0], x0 = Psi[i0], p1 = Phi[i1], x1 = Psi[i1];
+	double dx0 = 0, dx1 = 0, dp0 = 0, dp1 = 0;
 	if (TAN) {
-		h0 += th[0][0] + th[1][0];
-		h1 += th[0][1] + th[1][1];
+		dx0 = dPsi[i0];
+		dx1 = dPsi[i1];
+		dp0 = dPhi[i0];
+		dp1 = dPhi[i1];
 	}
-	if (g.last_gate) return;
-	apply_bases2<TAN>(fPhi, fdPhi, Phi, dPhi, bs0, bs1, has1, sl, g.bg, g.bz, g.first_gate, lane);
+	dmma(g[0], g[1], p0, x0);
+	if (TAN) dmma(h[0], h[1], p0, dx0);
+	dmma(g[0], g[1], p1, x1);
+	if (TAN) {
+		dmma(h[0], h[1], p1, dx1);
+		dmma(h[0], h[1], dp0, x0);
+		dmma(h[0], h[1], dp1, x1);
+	}
 }
 
-constexpr int NT6 = 128;   // threads of the reconstructing complex128 reverse kernel (three blocks per SM)
+// The gates' operands of a reverse pass that rebuilds states between groups: conj(G) (as a
+// row-vector operand it applies G^+) and -W, W = G^+ Z G^+.
+struct PassAdj { Gate4<double> gc[MAXK]; Gate4<double> wn[MAXK]; };
+
+constexpr int NT6 = 128;   // threads of the complex128 reverse kernel (three blocks per SM)
 constexpr int EPT6 = (1 << MAXNB) * 4 / NT6;   // tile elements per thread and state
 
-inline size_t k6_rev_smem(bool tan)
+inline size_t k8_rev_smem(bool tan)
 {
 	const size_t A = (size_t)(1 << MAXNB) * 4;
 	const size_t tiles = (tan ? 4 : 2) * A * sizeof(double2);
@@ -1537,21 +1514,26 @@ inline size_t k6_rev_smem(bool tan)
 	return 64 * MAXK * sizeof(double2) + (1 << MAXNB) * sizeof(int) + std::max(tiles, red);
 }
 
-// Reverse pass (complex128) for unitary gates.  It starts from the state at the OUTPUT
-// of the pass (psi, dpsi: the next pass's checkpoint, or the circuit's final state) and
-// walks back through the pass, rebuilding the state entering each gate with the adjoint
-// gate on the FP64 tensor pipe,
-//   psi_k = G^+ psi_{k+1},  dpsi_k = G^+ dpsi_{k+1} - W psi_{k+1},  W = G^+ Z G^+,
-// so that no state inside the pass is recomputed or kept: four tiles (psi, dpsi, phi,
-// dphi), updated in place, and two blocks per SM whose load, compute and store phases
-// overlap.  For each gate, per unit of eight amplitude groups: rebuild psi_k, dpsi_k;
-// add the outer sums dG_k += phi (x) psi_k, HZ_k += phi (x) dpsi_k + dphi (x) psi_k; move
-// phi, dphi through gate k.  Partials and contract as in k3_rev.
+// Reverse pass (complex128) for unitary gates.  psi, dpsi are the state
+// and tangent at the pass OUTPUT (the next pass's checkpoint, or the circuit's final state),
+// phi, dphi the cotangents there.  The gates of the last group commute, so each may count as the
+// pass's last gate, and its sums follow from those at the output, with W = G^+ Z G^+:
+//   R1 = sum phi (x) psi,  R2 = sum phi (x) dpsi + dphi (x) psi,
+//   dG = R1 conj(G),       HZ = R2 conj(G) - R1 W^T          (formed once, by k3_reduce).
+// So the states entering the gates are not needed: 12 FP64 MMAs per unit of eight groups and gate
+// instead of the 18 of a kernel that rebuilds them (L = 12, depth 9, one column per orbit: 3.41 ->
+// 2.97 ms an evaluation), and a group's sums need no barrier between gates; then phi, dphi move
+// through the group in place, two gates per barrier.  The layers of a brickwall make passes of
+// one group.  Where a pass has more (gates that share wires), psi and dpsi move back through a
+// group too, psi <- G^+ psi, dpsi <- G^+ dpsi - W psi, and the group before it is done the same
+// way.  Four tiles (64 KB), three blocks of 128 threads per SM.  Bound by the FP64 pipe (12 flop
+// per byte).  Partials: raw 8x8 sums R1, R2 (part + k * nblk * 128 + blockIdx.x * 128).
 template <bool TAN, bool FIRST, bool LAST>
-__global__ void __launch_bounds__(NT6, 3) k6_rev(const double2* __restrict__ psi, const double2* __restrict__ dpsi,
+__global__ void __launch_bounds__(NT6, 3) k8_rev(const double2* __restrict__ psi, const double2* __restrict__ dpsi,
                                                  const double2* __restrict__ phi, const double2* __restrict__ dphi,
                                                  double2* __restrict__ phi_o, double2* __restrict__ dphi_o, PassGeom pg,
-                                                 PassGates<double> gates, PassAdj adj, double* __restrict__ part, int nblk)
+                                                 PassGates<double> gates, const __grid_constant__ PassAdj adj,
+                                                 double* __restrict__ part, int nblk)
 {
 	constexpr int CW = 4;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1563,14 +1545,18 @@ __global__ void __launch_bounds__(NT6, 3) k6_rev(const double2* __restrict__ psi
 	double2* Phi = tiles + A;
 	double2* dPsi = TAN ? tiles + 2 * A : nullptr;
 	double2* dPhi = TAN ? tiles + 3 * A : nullptr;
+	const double* fPsi = reinterpret_cast<const double*>(Psi);
+	const double* fPhi = reinterpret_cast<const double*>(Phi);
+	const double* fdPsi = reinterpret_cast<const double*>(dPsi);
+	const double* fdPhi = reinterpret_cast<const double*>(dPhi);
 	for (int e = threadIdx.x; e < 64 * MAXK; e += blockDim.x) {
 		const int k = e / 64, w = e % 64;
 		if (k >= K) continue;
 		double2 v = make_double2(0, 0);
 		if (w < 16) v = gates.g[k].m[w];
-		else if (w < 32) v = TAN ? gates.z[k].m[w - 16] : make_double2(0, 0);
+		else if (w < 32) v = TAN ? gates.z[k].m[w - 16] : v;
 		else if (w < 48) v = adj.gc[k].m[w - 32];
-		else v = TAN ? adj.wn[k].m[w - 48] : make_double2(0, 0);
+		else v = TAN ? adj.wn[k].m[w - 48] : v;
 		sg[e] = v;
 	}
 	row_offsets(pg, rowoff);
@@ -1580,6 +1566,18 @@ __global__ void __launch_bounds__(NT6, 3) k6_rev(const double2* __restrict__ psi
 #pragma unroll
 	for (int k = 0; k < MAXK; k++) { cg0[k] = cg1[k] = ch0[k] = ch1[k] = 0; }
 	const int units = R / 8;
+
+	// X, dX through gate k on this lane's bases of two units, by the matrices at m (and mt for the
+	// tangent's term), in the embedding that tr and tt select
+	auto move = [&](double2* X, double2* dX, int k, const double2* m, bool tr, const double2* mt, bool tt, bool dzero,
+	                int bs0, int bs1, bool has1) {
+		const StepLane sl(pg.gi[k], pg.gj[k], lane);
+		double bg[2], bz[2] = {0, 0};
+		bfrag(m, tr, lane, bg);
+		if (TAN) bfrag(mt, tt, lane, bz);
+		apply_bases2<TAN>(reinterpret_cast<const double*>(X), reinterpret_cast<const double*>(dX), X, dX, bs0, bs1, has1, sl, bg,
+		                  bz, dzero, lane);
+	};
 
 	for (int64_t tile = blockIdx.x; tile < pg.ntiles; tile += gridDim.x) {
 		const int64_t rt = tile / pg.ncg, cgp = tile - rt * pg.ncg;
@@ -1603,39 +1601,57 @@ __global__ void __launch_bounds__(NT6, 3) k6_rev(const double2* __restrict__ psi
 		cp_async_commit();
 		cp_async_wait_all();
 		__syncthreads();
-		bool skip = false;   // gate k was done with gate k+1
+		for (int l = pg.ngroups - 1; l >= 0; l--) {
+			const int lo = pg.group[l], hi = pg.group[l + 1];
+			// the sums of every gate of the group, two units' MMA chains at a time
 #pragma unroll
-		for (int k = MAXK - 1; k >= 0; k--) {
-			if (k >= K) continue;
-			if (skip) { skip = false; continue; }
-			const int k2 = k >= 1 ? k - 1 : 0;
-			if (k >= 1 && pg.NB >= 4 && gates_disjoint(pg, k, k2)) {
-				// gates k and k-1 on this warp's row sets, one block barrier for both (each
-				// gate's operands are loaded per set, which keeps registers for one gate)
-				const int m = (1 << pg.gi[k]) | (1 << pg.gj[k]) | (1 << pg.gi[k2]) | (1 << pg.gj[k2]);
-				for (int s = warp; s < (R >> 4); s += nwarps) {
-					const int S0 = set_base(s, m);
-					{
-						const RevGate<TAN> ga(sg, k, K, FIRST, LAST, pg, lane);
-						rev_gate6<TAN>(ga, set_units(S0, pg.gi[k2], pg.gj[k2]), true, Psi, dPsi, Phi, dPhi, cg0[k],
-						               cg1[k], ch0[k], ch1[k], lane);
-					}
-					__syncwarp();
-					const RevGate<TAN> gb(sg, k2, K, FIRST, LAST, pg, lane);
-					rev_gate6<TAN>(gb, set_units(S0, pg.gi[k], pg.gj[k]), true, Psi, dPsi, Phi, dPhi, cg0[k2], cg1[k2],
-					               ch0[k2], ch1[k2], lane);
-				}
-				skip = true;
-			} else {
-				const RevGate<TAN> ga(sg, k, K, FIRST, LAST, pg, lane);
+			for (int k = 0; k < MAXK; k++) {
+				if (k < lo || k >= hi) continue;
+				const StepLane sl(pg.gi[k], pg.gj[k], lane);
+				double ga[2] = {0, 0}, gb[2] = {0, 0}, ha[2] = {0, 0}, hb[2] = {0, 0};
 				for (int u = warp; u < units; u += 2 * nwarps) {
-					const int u1 = u + nwarps;
-					const bool has1 = u1 < units;   // the same for the whole warp
-					rev_gate6<TAN>(ga, unit_pair(u, has1 ? u1 : u, ga.sl.lo, ga.sl.hi), has1, Psi, dPsi, Phi, dPhi,
-					               cg0[k], cg1[k], ch0[k], ch1[k], lane);
+					outer_unit<TAN>(fPsi, fdPsi, fPhi, fdPhi, u, sl, lane, ga, ha);
+					if (u + nwarps < units) outer_unit<TAN>(fPsi, fdPsi, fPhi, fdPhi, u + nwarps, sl, lane, gb, hb);
+				}
+				cg0[k] += ga[0] + gb[0];
+				cg1[k] += ga[1] + gb[1];
+				if (TAN) {
+					ch0[k] += ha[0] + hb[0];
+					ch1[k] += ha[1] + hb[1];
 				}
 			}
+			if (LAST && l == 0) break;
 			__syncthreads();
+			// phi, dphi (and psi, dpsi where a group comes before) through gates k and k + 1 on this
+			// warp's row sets, one block barrier for both
+			for (int k = lo; k < hi; k += 2) {
+				const double2 *ma = sg + 64 * k, *mb = sg + 64 * (k + 1);
+				const bool dz = FIRST && l == pg.ngroups - 1 && k == lo;
+				const int hs = lane >> 4;
+				if (k + 1 < hi) {
+					const int m = (1 << pg.gi[k]) | (1 << pg.gj[k]) | (1 << pg.gi[k + 1]) | (1 << pg.gj[k + 1]);
+					for (int s = warp; s < (R >> 4); s += nwarps) {
+						const int S0 = set_base(s, m);
+						const UnitBases ua = set_units(S0, pg.gi[k + 1], pg.gj[k + 1]), ub = set_units(S0, pg.gi[k], pg.gj[k]);
+						const int a0 = hs ? ua.b01 : ua.b00, a1 = hs ? ua.b11 : ua.b10;
+						const int b0 = hs ? ub.b01 : ub.b00, b1 = hs ? ub.b11 : ub.b10;
+						move(Phi, dPhi, k, ma, false, ma + 16, false, dz, a0, a1, true);
+						if (l > 0) move(Psi, dPsi, k, ma + 32, false, ma + 48, true, false, a0, a1, true);
+						__syncwarp();
+						move(Phi, dPhi, k + 1, mb, false, mb + 16, false, false, b0, b1, true);
+						if (l > 0) move(Psi, dPsi, k + 1, mb + 32, false, mb + 48, true, false, b0, b1, true);
+					}
+				} else {
+					const StepLane sl(pg.gi[k], pg.gj[k], lane);
+					for (int u = warp; u < units; u += 2 * nwarps) {
+						const bool has1 = u + nwarps < units;
+						const int b0 = insert2(2 * u + hs, sl.lo, sl.hi), b1 = insert2(2 * (has1 ? u + nwarps : u) + hs, sl.lo, sl.hi);
+						move(Phi, dPhi, k, ma, false, ma + 16, false, dz, b0, b1, has1);
+						if (l > 0) move(Psi, dPsi, k, ma + 32, false, ma + 48, true, false, b0, b1, has1);
+					}
+				}
+				__syncthreads();
+			}
 		}
 		if (!LAST) {
 #pragma unroll
@@ -2097,21 +2113,69 @@ k2_reduce(const double* __restrict__ part, int nslots, int nblk, const double2* 
 struct Pass
 {
 	int first, K;
+	int gate[MAXK];  // the pass's gates; their partial sums are slots first, first + 1, ...
 	PassGeom geom;   // chunk fields filled per launch
 };
 
-// Group consecutive gates into passes of up to MAXK gates; tile bits = the union of
-// their wires (state bits), padded with the lowest other bits to min(8, L).
-std::vector<Pass> schedule(int L, int G, const int* wires, int maxk)
+// The gates of the passes, up to maxk each.  Consecutive gates; or reordered where they commute,
+// so that a pass has as few groups as possible: a gate is ready when the last gates before it on
+// its two wires are done, and a pass takes the gates ready at its start with the longest chains
+// of gates behind them, and only if these are too few those that became ready within the pass.
+std::vector<std::vector<int>> pass_lists(int L, int G, const int* wires, int maxk, bool reorder)
+{
+	std::vector<std::vector<int>> out;
+	if (!reorder) {
+		for (int i = 0; i < G; i += maxk) {
+			out.emplace_back();
+			for (int k = i; k < std::min(G, i + maxk); k++) out.back().push_back(k);
+		}
+		return out;
+	}
+	std::vector<int> waits(G, 0), height(G, 1), last(L, -1), ready;
+	std::vector<std::vector<int>> next(G);
+	for (int k = 0; k < G; k++)
+		for (int e = 0; e < 2; e++) {
+			int& l = last[wires[2 * k + e]];
+			if (l >= 0) {
+				next[l].push_back(k);
+				waits[k]++;
+			}
+			l = k;
+		}
+	for (int k = G - 1; k >= 0; k--)
+		for (int m : next[k]) height[k] = std::max(height[k], height[m] + 1);
+	for (int k = 0; k < G; k++)
+		if (!waits[k]) ready.push_back(k);
+	while (!ready.empty()) {
+		out.emplace_back();
+		while ((int)out.back().size() < maxk && !ready.empty()) {
+			std::stable_sort(ready.begin(), ready.end(), [&](int x, int y) { return height[x] > height[y]; });
+			const int n = std::min<int>(maxk - (int)out.back().size(), (int)ready.size());
+			const std::vector<int> taken(ready.begin(), ready.begin() + n);
+			ready.erase(ready.begin(), ready.begin() + n);
+			for (int k : taken) {
+				out.back().push_back(k);
+				for (int m : next[k])
+					if (--waits[m] == 0) ready.push_back(m);
+			}
+		}
+	}
+	return out;
+}
+
+// Passes of up to MAXK gates; tile bits = the union of their wires (state bits), padded with the
+// lowest other bits to min(8, L).
+std::vector<Pass> schedule(int L, int G, const int* wires, int maxk, bool reorder)
 {
 	std::vector<Pass> out;
 	const int NB = std::min(MAXNB, L);
-	for (int i = 0; i < G;) {
-		const int K = std::min(maxk, G - i);
+	int i = 0;
+	for (const std::vector<int>& list : pass_lists(L, G, wires, maxk, reorder)) {
+		const int K = (int)list.size();
 		uint32_t bits = 0;
-		for (int k = 0; k < K; k++) {
-			bits |= 1u << (L - 1 - wires[2 * (i + k)]);
-			bits |= 1u << (L - 1 - wires[2 * (i + k) + 1]);
+		for (int k : list) {
+			bits |= 1u << (L - 1 - wires[2 * k]);
+			bits |= 1u << (L - 1 - wires[2 * k + 1]);
 		}
 		for (int b = 0; __builtin_popcount(bits) < NB && b < L; b++) bits |= 1u << b;
 		Pass p;
@@ -2126,9 +2190,21 @@ std::vector<Pass> schedule(int L, int G, const int* wires, int maxk)
 		for (int b = 0; b < L; b++)
 			if ((bits >> b) & 1) { local[b] = n; p.geom.tbit[n++] = b; }
 		for (int k = 0; k < K; k++) {
-			p.geom.gi[k] = local[L - 1 - wires[2 * (i + k)]];
-			p.geom.gj[k] = local[L - 1 - wires[2 * (i + k) + 1]];
+			p.gate[k] = list[k];
+			p.geom.gi[k] = local[L - 1 - wires[2 * list[k]]];
+			p.geom.gj[k] = local[L - 1 - wires[2 * list[k] + 1]];
 		}
+		// groups: a gate that shares a wire with its group begins the next one
+		uint32_t group = 0;
+		for (int k = 0; k < K; k++) {
+			const uint32_t w = (1u << p.geom.gi[k]) | (1u << p.geom.gj[k]);
+			if (k == 0 || (group & w)) {
+				p.geom.group[p.geom.ngroups++] = k;
+				group = 0;
+			}
+			group |= w;
+		}
+		p.geom.group[p.geom.ngroups] = K;
 		const uint32_t all = L >= 32 ? 0xffffffffu : ((1u << L) - 1);
 		p.geom.rest_mask = all & ~bits;
 		out.push_back(p);
@@ -2144,10 +2220,10 @@ PassGates<T> pass_gates(const Pass& p, const double2* gates, const double2* dirs
 	memset(&pg, 0, sizeof(pg));
 	for (int k = 0; k < p.K; k++)
 		for (int e = 0; e < 16; e++) {
-			const double2 g = gates[16 * (p.first + k) + e];
+			const double2 g = gates[16 * (size_t)p.gate[k] + e];
 			pg.g[k].m[e] = mk<T>((T)g.x, (T)g.y);
 			if (dirs) {
-				const double2 z = dirs[16 * (p.first + k) + e];
+				const double2 z = dirs[16 * (size_t)p.gate[k] + e];
 				pg.z[k].m[e] = mk<T>((T)z.x, (T)z.y);
 			}
 		}
@@ -2316,41 +2392,41 @@ int launch_rev5_any(Runtime& rt, bool first, bool last, const float2* psi, const
 }
 
 template <bool TAN, bool FIRST, bool LAST>
-int launch_rev6(Runtime& rt, const double2* psi, const double2* dpsi, const double2* phi, const double2* dphi,
-                double2* phi_o, double2* dphi_o, const PassGeom& pg, const PassGates<double>& gates, const PassAdj& adj,
-                double* part, int nblk)
+int launch_rev8(Runtime& rt, const double2* psi, const double2* dpsi, const double2* phi, const double2* dphi,
+                double2* phi_o, double2* dphi_o, const PassGeom& pg, const PassGates<double>& gates, const PassAdj& adj, double* part,
+                int nblk)
 {
 	static bool ready = false;
 	if (!ready) {
 		int per_sm;
-		int ret = prepare(k6_rev<TAN, FIRST, LAST>, k6_rev_smem(TAN), &per_sm, NT6);
+		int ret = prepare(k8_rev<TAN, FIRST, LAST>, k8_rev_smem(TAN), &per_sm, NT6);
 		if (ret) return ret;
 		ready = true;
 	}
-	RQC_LAUNCH3(rt, KC_REVERSE, (k6_rev<TAN, FIRST, LAST>), nblk, NT6, k6_rev_smem(TAN), psi, dpsi, phi, dphi, phi_o,
+	RQC_LAUNCH3(rt, KC_REVERSE, (k8_rev<TAN, FIRST, LAST>), nblk, NT6, k8_rev_smem(TAN), psi, dpsi, phi, dphi, phi_o,
 	            dphi_o, pg, gates, adj, part, nblk);
 	return OK;
 }
 
 template <bool TAN>
-int launch_rev6_any(Runtime& rt, bool first, bool last, const double2* psi, const double2* dpsi, const double2* phi,
+int launch_rev8_any(Runtime& rt, bool first, bool last, const double2* psi, const double2* dpsi, const double2* phi,
                     const double2* dphi, double2* phi_o, double2* dphi_o, const PassGeom& pg,
                     const PassGates<double>& gates, const PassAdj& adj, double* part, int nblk)
 {
 	if (first && last)
-		return launch_rev6<TAN, true, true>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
+		return launch_rev8<TAN, true, true>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
 	if (first)
-		return launch_rev6<TAN, true, false>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
+		return launch_rev8<TAN, true, false>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
 	if (last)
-		return launch_rev6<TAN, false, true>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
-	return launch_rev6<TAN, false, false>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
+		return launch_rev8<TAN, false, true>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
+	return launch_rev8<TAN, false, false>(rt, psi, dpsi, phi, dphi, phi_o, dphi_o, pg, gates, adj, part, nblk);
 }
 
-int rev_grid6(Runtime& rt, bool tan)
+int rev_grid8(Runtime& rt, bool tan)
 {
 	int per_sm = 1;
-	const int ret = tan ? prepare(k6_rev<true, false, false>, k6_rev_smem(true), &per_sm, NT6)
-	                    : prepare(k6_rev<false, false, false>, k6_rev_smem(false), &per_sm, NT6);
+	const int ret = tan ? prepare(k8_rev<true, false, false>, k8_rev_smem(true), &per_sm, NT6)
+	                    : prepare(k8_rev<false, false, false>, k8_rev_smem(false), &per_sm, NT6);
 	if (ret) per_sm = 1;
 	return rt.num_sms * per_sm;
 }
@@ -2425,35 +2501,48 @@ bool gates_unitary(const double2* gates, int G, double tol = 1e-10)
 	return true;
 }
 
-// conj(G) and -W = -G^+ Z G^+ of every gate of a pass, in FP64 (complex128 reconstruction)
-PassAdj pass_adj(const Pass& p, const double2* gates, const double2* dirs)
+// slots of partial sums in pass order
+std::vector<SlotGate> slot_gates(const std::vector<Pass>& passes, const double2* gates, const double2* dirs)
+{
+	std::vector<SlotGate> out;
+	for (const Pass& p : passes)
+		for (int k = 0; k < p.K; k++) {
+			SlotGate s;
+			memset(&s, 0, sizeof(s));
+			s.gate = p.gate[k];
+			const double2* g = gates + 16 * (size_t)s.gate;
+			for (int e = 0; e < 16; e++) s.gc[e] = make_double2(g[e].x, -g[e].y);
+			if (dirs) {
+				const double2* z = dirs + 16 * (size_t)s.gate;
+				double2 t[16];   // Z G^+
+				for (int r = 0; r < 4; r++)
+					for (int c = 0; c < 4; c++) {
+						double2 v = make_double2(0, 0);
+						for (int q = 0; q < 4; q++) v = cadd(v, cmul(z[4 * r + q], s.gc[4 * c + q]));
+						t[4 * r + c] = v;
+					}
+				for (int r = 0; r < 4; r++)
+					for (int c = 0; c < 4; c++) {
+						double2 v = make_double2(0, 0);
+						for (int q = 0; q < 4; q++) v = cadd(v, cmul(s.gc[4 * q + r], t[4 * q + c]));
+						s.wn[4 * r + c] = make_double2(-v.x, -v.y);
+					}
+			}
+			out.push_back(s);
+		}
+	return out;
+}
+
+// conj(G) and -W of a pass whose slots begin at sg
+PassAdj pass_adj(const Pass& p, const SlotGate* sg)
 {
 	PassAdj pa;
 	memset(&pa, 0, sizeof(pa));
-	for (int k = 0; k < p.K; k++) {
-		const double2* g = gates + 16 * (size_t)(p.first + k);
-		for (int e = 0; e < 16; e++) pa.gc[k].m[e] = make_double2(g[e].x, -g[e].y);
-		if (!dirs) continue;
-		const double2* z = dirs + 16 * (size_t)(p.first + k);
-		double2 gh[16], t[16], w[16];
-		for (int r = 0; r < 4; r++)
-			for (int c = 0; c < 4; c++) gh[4 * r + c] = make_double2(g[4 * c + r].x, -g[4 * c + r].y);
-		auto mul = [](const double2* a, const double2* b, double2* o) {
-			for (int r = 0; r < 4; r++)
-				for (int c = 0; c < 4; c++) {
-					double re = 0, im = 0;
-					for (int q = 0; q < 4; q++) {
-						const double2 x = a[4 * r + q], y = b[4 * q + c];
-						re += x.x * y.x - x.y * y.y;
-						im += x.x * y.y + x.y * y.x;
-					}
-					o[4 * r + c] = make_double2(re, im);
-				}
-		};
-		mul(gh, z, t);
-		mul(t, gh, w);
-		for (int e = 0; e < 16; e++) pa.wn[k].m[e] = make_double2(-w[e].x, -w[e].y);
-	}
+	for (int k = 0; k < p.K; k++)
+		for (int e = 0; e < 16; e++) {
+			pa.gc[k].m[e] = sg[k].gc[e];
+			pa.wn[k].m[e] = sg[k].wn[e];
+		}
 	return pa;
 }
 
@@ -2515,22 +2604,24 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 	const int64_t ncols = column_count(rt, c);
 	const bool tan = mode == EVAL_HVP;
 	const bool host_target = t.ufunc != nullptr;
-	std::vector<Pass> passes = schedule(L, G, c.wires, maxk);
-	std::vector<Pass> tpasses = host_target ? std::vector<Pass>() : schedule(L, t.ngates, t.wires, maxk);   // none of a dense one
+	// complex64 keeps the order of the circuit (its results depend on it to 1e-6)
+	constexpr bool reorder = std::is_same<T, double>::value;
+	std::vector<Pass> passes = schedule(L, G, c.wires, maxk, reorder);
+	// none of a dense target
+	std::vector<Pass> tpasses = host_target ? std::vector<Pass>() : schedule(L, t.ngates, t.wires, maxk, reorder);
 	const int P = (int)passes.size(), Pt = (int)tpasses.size();
 	std::vector<PassGates<T>> pgates(P), tgates(Pt);
 	for (int p = 0; p < P; p++) pgates[p] = pass_gates<T>(passes[p], c.gates, tan ? c.dirs : nullptr);
 	for (int p = 0; p < Pt; p++) tgates[p] = pass_gates<T>(tpasses[p], t.gates, nullptr);
 
-	// complex64 with unitary gates: the reverse passes start from each pass's output
-	// (the next checkpoint, or the final state) and rebuild states with adjoint gates
+	// unitary gates: the reverse passes start from each pass's output (the next checkpoint, or
+	// the final state); complex64 ones rebuild the states inside a pass with adjoint gates
 	bool recon = false;
 	if constexpr (!std::is_same<T, double>::value) recon = mode != EVAL_F && gates_unitary(c.gates, G);
-	else recon = mode != EVAL_F && rt.recon_c128 && gates_unitary(c.gates, G, 1e-14);
+	// (one gate: its second derivative is exactly zero, which a difference of sums is not)
+	else recon = mode != EVAL_F && rt.recon_c128 && G > 1 && gates_unitary(c.gates, G, 1e-14);
 	std::vector<PassW<float>> pw(recon && tan && !std::is_same<T, double>::value ? P : 0);
 	for (int p = 0; p < (int)pw.size(); p++) pw[p] = pass_w(passes[p], c.gates, c.dirs);
-	std::vector<PassAdj> padj(recon && std::is_same<T, double>::value ? P : 0);
-	for (int p = 0; p < (int)padj.size(); p++) padj[p] = pass_adj(passes[p], c.gates, tan ? c.dirs : nullptr);
 	const int64_t nck = recon ? P : P - 1;   // checkpoints (recon: also the final state)
 
 	// states per column: PHI, P0, P1 (+ D0, D1) and the pass checkpoints
@@ -2559,7 +2650,7 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 
 	// complex64 reverse passes on the FP32 pipe (k7_rev) or on the TF32 MMA (k5_rev)
 	const bool ffma = !std::is_same<T, double>::value && recon && rt.c64_ffma;
-	const int full = recon ? (std::is_same<T, double>::value ? rev_grid6(rt, tan) : (ffma ? rev_grid7(rt, tan) : rev_grid5(rt, tan)))
+	const int full = recon ? (std::is_same<T, double>::value ? rev_grid8(rt, tan) : (ffma ? rev_grid7(rt, tan) : rev_grid5(rt, tan)))
 	                       : rev_grid<T>(rt, tan);
 	// no more blocks (and partials to clear and sum) than tiles
 	const int64_t most_tiles = (N >> std::min(MAXNB, L)) * (C / CW);
@@ -2572,6 +2663,14 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 	double* part = reinterpret_cast<double*>(rt.partials.ptr);
 	double2* fpart = reinterpret_cast<double2*>(part + (size_t)G * nblk * nps);
 	if ((ret = RQC_CUDA(cudaMemsetAsync(part, 0, part_doubles * sizeof(double), rt.stream)))) return ret;
+	std::vector<SlotGate> sg;
+	if (std::is_same<T, double>::value) {
+		sg = slot_gates(passes, c.gates, recon && tan ? c.dirs : nullptr);
+		if ((ret = ensure_device(rt.slots, sg.size() * sizeof(SlotGate)))) return ret;
+		if ((ret = RQC_CUDA(cudaMemcpyAsync(rt.slots.ptr, sg.data(), sg.size() * sizeof(SlotGate), cudaMemcpyHostToDevice,
+		                                    rt.stream))))
+			return ret;
+	}
 	double* scratch = nullptr;
 	if (!std::is_same<T, double>::value) {
 		if ((ret = ensure_device(rt.scratch, (size_t)nblk * (NT4R / 32) * 32 * MAXK * 4 * sizeof(double)))) return ret;
@@ -2698,12 +2797,13 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 			if constexpr (std::is_same<T, double>::value) {
 				if (recon) {
 					if (tan)
-						ret = launch_rev6_any<true>(rt, first, last, ck_at(p + 1), dck_at(p + 1), ph, dph,
-						                            last ? nullptr : Pb[nxt], last ? nullptr : Db[nxt], g, pgates[p], padj[p],
-						                            pp, nblk);
+						ret = launch_rev8_any<true>(rt, first, last, ck_at(p + 1), dck_at(p + 1), ph, dph,
+						                            last ? nullptr : Pb[nxt], last ? nullptr : Db[nxt], g, pgates[p],
+						                            pass_adj(passes[p], &sg[passes[p].first]), pp, nblk);
 					else
-						ret = launch_rev6_any<false>(rt, first, last, ck_at(p + 1), nullptr, ph, nullptr,
-						                             last ? nullptr : Pb[nxt], nullptr, g, pgates[p], padj[p], pp, nblk);
+						ret = launch_rev8_any<false>(rt, first, last, ck_at(p + 1), nullptr, ph, nullptr,
+						                             last ? nullptr : Pb[nxt], nullptr, g, pgates[p],
+						                             pass_adj(passes[p], &sg[passes[p].first]), pp, nblk);
 					if (ret) return ret;
 					continue;
 				}
@@ -2745,7 +2845,8 @@ int evaluate_fused_t(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, int
 	}
 
 	if (std::is_same<T, double>::value)
-		k3_reduce<<<G + 1, RED_GROUPS * NPART3, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
+		k3_reduce<<<G + 1, RED_GROUPS * NPART3, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, static_cast<const SlotGate*>(rt.slots.ptr),
+		                                                              recon ? 1 : 0, d_out);
 	else if (ffma)
 		k2_reduce<<<G + 1, RED_GROUPS * NPART2, 0, rt.stream>>>(part, G, nblk, fpart, nfb, tan ? 1 : 0, d_out);
 	else

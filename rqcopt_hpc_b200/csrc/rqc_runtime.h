@@ -39,6 +39,7 @@ struct Runtime
 	Buffer stage[4];      // staging of host statevectors
 	Buffer arrays;        // statevector arrays and gate-input caches of the full-Hessian calls
 	Buffer columns;       // column list of the current call (orbits.h)
+	Buffer slots;         // gates of the complex128 passes' partial sums
 	Buffer dense;         // dense target of the current call
 	Buffer small_dev;     // inputs of the current call's small evaluations (engine_small.cu), and
 	Buffer small_host;    // their pinned staging

@@ -53,3 +53,29 @@ def test_hessians_of_gates_that_are_not_unitary(gpu, oracle):
     ref = oracle.brickwall_unitary_target_gradient_hessian(oracle.target("brickwall", (tv, perms[:2])), v, perms, 6)
     for a, b in zip(got, ref):
         assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("L,G", [(11, 9), (11, 40), (12, 17), (13, 6)])
+@pytest.mark.parametrize("near", [False, True])
+@pytest.mark.parametrize("per_pass", [4, 3, 2])
+def test_circuit_sums_in_passes_of_several_groups(gpu, L, G, near, per_pass):
+    """Reordered passes, with gates that share wires in one pass, against one gate per pass.  Column
+    sums of the same products in another order: 1e-12, the bar between the engines."""
+    rng = np.random.default_rng(10 * L + G)
+    gates = np.stack([haar_unitary(rng) for _ in range(G)])
+    pool = 5 if near else L
+    wires = np.array([rng.choice(pool, 2, replace=False) for _ in range(G)], np.int32)
+    dirs = crandn((G, 4, 4), rng)
+    t = gpu.Target(circuit=(gates[:3], wires[:3][:, ::-1].copy()))
+    run = lambda: gpu.circuit_unitary_target_hessian_vector_product(t, gates, dirs, wires, L)   # noqa: E731
+    try:
+        gpu.set_column_range(3, 40)
+        gpu.set_gates_per_pass(per_pass)
+        got, grad = run(), gpu.circuit_unitary_target_and_gradient(t, gates, wires, L)
+        gpu.set_gates_per_pass(1)
+        ref = run()
+    finally:
+        gpu.set_column_range(0, 0)
+    for a, b in zip(got, ref):
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
+    assert np.linalg.norm(grad[1] - ref[1]) <= 1e-12 * np.linalg.norm(ref[1])
