@@ -3,14 +3,23 @@
 // The full-Hessian sweep carries 16 tangent states per layer and column through every later
 // layer; a layer's gates act on disjoint wires.  A block holds a tile of 2^11 (or 2^12)
 // amplitudes over the gates' bits and the lowest others in shared memory and takes two gates
-// per round: a thread's 16 amplitudes are closed under both, so they pass through registers
-// once for 512 FMAs, with the gate entries as constant operands.  What bounds it is close to
-// balanced: at four gates a tile moves 2 x 16 B per amplitude to and from memory and does 64
-// complex multiply-adds (8 flop per byte; 6.5 TB/s against 34 TFLOP/s of DFMA is 5.2), and
-// shared memory moves a quarter-warp per cycle for two thirds of the FMA time.  One gate per
-// launch (k_happly) needs 1.3 flop per byte.  The tile's words are permuted within 128-byte
-// lines (swz) and the lanes' bits chosen per round so that a quarter-warp's 16-byte accesses
-// fall into different banks.
+// per round, so that the amplitudes pass through registers once for both.  The first gate runs on
+// the FP64 MMA (m8n8k4) with the amplitude's real and imaginary parts as two operands: a lane's
+// operand is then one amplitude of its group, and the result comes back as the same amplitude of
+// the same group, so nothing is exchanged.  The second gate's four amplitudes lie in the thread's
+// own 16 and take FMAs with the gate's entries as constant operands.  Both run on the one FP64
+// pipe; the MMAs are there because an FP64 FMA holds the issue port for two cycles.
+//
+// What bounds it is close to balanced: at four gates a tile moves 2 x 16 B per amplitude to and
+// from memory and does 64 complex multiply-adds (8 flop per byte; 6.5 TB/s against 36 TFLOP/s is
+// 5.5).  One gate per launch (k_happly) needs 1.3 flop per byte.  Measured on 2^26 amplitudes (2 GB
+// read and written a pass): one or two gates 5.7 TB/s; four 5.3 TB/s, 21 TFLOP/s; five at L = 10
+// 4.7 TB/s, 23 TFLOP/s.  Both gates in FMAs: 4.8 TB/s and 4.1 TB/s; with 64-bit index arithmetic per
+// shared-memory access besides, 18 TFLOP/s.  Four blocks per SM at 128 registers; five spill and
+// lose 12 %, three with the next tile prefetched gain 2 % at four gates and lose 5 % at five.
+//
+// The tile's words are permuted within 128-byte lines (swz) and the lanes' bits chosen per round
+// so that a quarter-warp's 16-byte accesses fall into different banks.
 #include "layer_pass.h"
 
 #include <algorithm>
@@ -26,8 +35,9 @@ struct PassArgs
 {
 	Gate4<double> g[MAXG];
 	int K, L;
-	int step[ROUNDS][4];        // places (bytes) of the tile bits of wires i, j of a round's first and second gate (or fillers)
-	int8_t pos[ROUNDS][8];      // tile bits of a thread's index bits
+	int step[ROUNDS][4];        // places (bytes) of the tile bits of a thread's 16 amplitudes: two others, wires i, j of the
+	                            // round's second gate (or two more others)
+	int8_t pos[ROUNDS][8];      // tile bits of a thread's index bits (0, 1: wires j, i of the round's first gate)
 	int8_t tbit[12];            // index bit of tile bit b
 	uint32_t koff[16];          // index bits of the tile's top four bits
 	// tile number to index bits outside the tile: nseg runs of consecutive bits, bits seg_from ..
@@ -47,6 +57,15 @@ __device__ __forceinline__ int64_t tile_base(const PassArgs& a, int64_t t)
 	int64_t r = 0;
 	for (int k = 0; k < a.nseg; k++) r |= (int64_t)(((uint64_t)t >> a.seg_from[k]) & a.seg_mask[k]) << a.seg_to[k];
 	return r;
+}
+
+// D (8 groups x [re, im of 4 amplitudes]) += a (8 groups x 4) b: a lane's a is one part of amplitude
+// lane & 3 of group lane >> 2, and its D are the parts of that same amplitude
+__device__ __forceinline__ void dmma(double2& d, double a, double b)
+{
+	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+	    : "+d"(d.x), "+d"(d.y)
+	    : "d"(a), "d"(b));
 }
 
 // the 4x4 gate on the four amplitudes x[0], x[s], x[2 s], x[3 s]
@@ -80,12 +99,7 @@ __device__ __forceinline__ void apply4(const Gate4<double>& g, double2* x)
 }
 
 // Shared-memory addresses are byte offsets into the tile (places * 16), so that a member's is one
-// XOR away from its neighbour's.  An FP64 instruction holds the issue port for two cycles, so every other instruction counts: with
-// 64-bit index arithmetic per access there were as many of those as FMAs (18 TFLOP/s at any
-// occupancy, with one or two tiles per block; 19-20 now).  Measured on 2^26 amplitudes, 2 GB a pass
-// (read and write): one or two gates 6.2 TB/s, the copy bandwidth; four 4.8 TB/s, 19 TFLOP/s; five at
-// L = 10 4.1 TB/s, 21 TFLOP/s.  Four blocks per SM at 128 registers: five or six spill and lose 5-30 %,
-// three with the next tile prefetched lose 4 %.
+// XOR away from its neighbour's.
 template <int TB, int IN, int OUT>
 __global__ void __launch_bounds__(1 << (TB - 4), TB == 11 ? 4 : 2)
 k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
@@ -109,10 +123,19 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 			for (int b = 0; b < TB - 4; b++) v |= ((tid >> b) & 1) << a.pos[r][b];
 		base[r] = swz(v) << 4;
 	}
-	for (int64_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+	// operand of the rounds' first gates: for input amplitude k = lane & 3 and output part n = lane >> 2
+	double bre[ROUNDS], bim[ROUNDS];
+#pragma unroll
+	for (int r = 0; r < ROUNDS; r++) {
+		const int lane = tid & 31;
+		const double2 g = 2 * r < a.K ? a.g[2 * r].m[4 * (lane >> 3) + (lane & 3)] : make_double2(0, 0);
+		bre[r] = lane & 4 ? g.y : g.x;
+		bim[r] = lane & 4 ? g.x : -g.y;
+	}
+	auto load = [&](int64_t t) {
 		const int64_t at = tile_base(a, t) + own;
-		const bool whole = at + a.koff[15] < a.total;   // only tiles of contiguous columns can be cut off
 		if (IN == 0) {
+			const bool whole = at + a.koff[15] < a.total;   // only tiles of contiguous columns can be cut off
 			const double2* src = in + at;
 			const unsigned dst = (unsigned)__cvta_generic_to_shared(tile);
 #pragma unroll
@@ -130,6 +153,9 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 				at_smem(place ^ (swz(k * NT) << 4)) = basis_amp<double>(a.src, e & mask, e >> a.L);
 			}
 		}
+	};
+	for (int64_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+		load(t);
 		__syncthreads();
 #pragma unroll
 		for (int r = 0; r < ROUNDS; r++) {
@@ -140,7 +166,12 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 #pragma unroll
 				for (int k = 0; k < 16; k++) x[k] = at_smem(mem(k));
 #pragma unroll
-				for (int k = 0; k < 4; k++) apply4<4>(a.g[2 * r], x + k);
+				for (int k = 0; k < 16; k++) {
+					double2 y = make_double2(0, 0);
+					dmma(y, x[k].x, bre[r]);
+					dmma(y, x[k].y, bim[r]);
+					x[k] = y;
+				}
 				if (2 * r + 1 < a.K)
 #pragma unroll
 					for (int k = 0; k < 4; k++) apply4<1>(a.g[2 * r + 1], x + 4 * k);
@@ -149,6 +180,9 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 				__syncthreads();
 			}
 		}
+		// (the tile's base again: held through the rounds it costs spills)
+		const int64_t at = tile_base(a, t) + own;
+		const bool whole = at + a.koff[15] < a.total;
 		double2* dst = out + at;
 #pragma unroll
 		for (int k = 0; k < 16; k++) {
@@ -252,36 +286,43 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 		const int64_t tile = (int64_t)1 << TB;
 		a.ntiles = (a.total + tile - 1) / tile;
 		for (int r = 0; 2 * r < K; r++) {
+			// thread index bits 0 and 1: the first gate's wires j and i (the lanes of an MMA's amplitude);
+			// 16 amplitudes per thread: the second gate's wires and two other bits
 			uint32_t used = 0;
-			auto take = [&](int slot, int wire) {
+			auto bit_of = [&](int wire) {
 				const int b = local[L - 1 - wire];
-				a.step[r][slot] = swz(1 << b) << 4;
 				used |= 1u << b;
+				return b;
 			};
-			take(0, gates[first + 2 * r].i);
-			take(1, gates[first + 2 * r].j);
+			const LayerGate& g0 = gates[first + 2 * r];
+			a.pos[r][0] = (int8_t)bit_of(g0.j);
+			a.pos[r][1] = (int8_t)bit_of(g0.i);
+			int slot = 2;
 			if (2 * r + 1 < K) {
-				take(2, gates[first + 2 * r + 1].i);
-				take(3, gates[first + 2 * r + 1].j);
-			} else {   // a gate alone: the set takes the two highest other bits
-				for (int s = 2, b = TB - 1; s < 4; b--)
-					if (!((used >> b) & 1)) {
-						a.step[r][s++] = swz(1 << b) << 4;
-						used |= 1u << b;
-					}
+				const LayerGate& g1 = gates[first + 2 * r + 1];
+				a.step[r][2] = swz(1 << bit_of(g1.i)) << 4;
+				a.step[r][3] = swz(1 << bit_of(g1.j)) << 4;
+			} else {
+				slot = 4;
 			}
-			// thread index bits: first three of different residues mod 3 (different lines of swz), then the rest
-			int m = 0;
-			uint32_t left = ((1u << TB) - 1) & ~used;
-			for (int c = 0; c < 3; c++)
-				for (int b = c; b < TB; b += 3)
-					if ((left >> b) & 1) {
-						a.pos[r][m++] = (int8_t)b;
-						left &= ~(1u << b);
-						break;
-					}
+			// thread bit 2: of the residue mod 3 that the gate's two bits leave (a quarter-warp's accesses
+			// then fall into different banks), if there is one
+			int third = -1;
+			for (int b = 0; b < TB && third < 0; b++)
+				if (!((used >> b) & 1) && b % 3 != a.pos[r][0] % 3 && b % 3 != a.pos[r][1] % 3) third = b;
+			for (int b = 0; b < TB && third < 0; b++)
+				if (!((used >> b) & 1)) third = b;
+			a.pos[r][2] = (int8_t)third;
+			used |= 1u << third;
+			// the remaining bits: the highest to the thread's own amplitudes, the others to the thread index
+			for (int b = TB - 1, s = 0; s < slot; b--)
+				if (!((used >> b) & 1)) {
+					a.step[r][s++] = swz(1 << b) << 4;
+					used |= 1u << b;
+				}
+			int m = 3;
 			for (int b = 0; b < TB; b++)
-				if ((left >> b) & 1) a.pos[r][m++] = (int8_t)b;
+				if (!((used >> b) & 1)) a.pos[r][m++] = (int8_t)b;
 		}
 		const bool first_pass = p == 0, last_pass = p == npass - 1;
 		int in_mode = 0;
