@@ -33,6 +33,7 @@
 
 #include "engine.h"
 #include "engine_fused.h"
+#include "pass_tile.cuh"
 #include "rqc_common.cuh"
 #include "rqcopt_gpu.h"
 
@@ -165,7 +166,6 @@ __device__ __forceinline__ double embed(const double2* m, int rowk, int coln, bo
 	return a == 0 ? (b == 0 ? v.x : v.y) : (b == 0 ? -v.y : v.x);
 }
 
-constexpr int NTF = 128;   // threads of the complex128 forward kernel (three blocks per SM)
 constexpr int NTR = 512;   // threads of the complex128 reverse kernel
 constexpr int NPART3 = 128;   // raw 8x8 sums per gate and block: dG then HZ
 
@@ -240,10 +240,6 @@ __device__ __forceinline__ void apply_unit(const double* in, const double* din, 
 // closed under both gates (the rows that agree outside the four bits), so a warp can
 // apply a then b to its sets with warp-level synchronisation only, and the block
 // barrier between the two gates goes away.
-__device__ __forceinline__ bool gates_disjoint(const PassGeom& pg, int a, int b)
-{
-	return (((1 << pg.gi[a]) | (1 << pg.gj[a])) & ((1 << pg.gi[b]) | (1 << pg.gj[b]))) == 0;
-}
 
 // first row of set s: s with zero bits inserted at the set bits of m (in increasing order)
 __device__ __forceinline__ int set_base(int s, int m)
@@ -264,14 +260,6 @@ struct UnitBases
 {
 	int b00, b01, b10, b11;
 };
-
-// units u0 and u1 of a gate's own enumeration (unit u: group bases 2u, 2u+1 with zero
-// bits inserted at the gate's tile bits)
-__device__ __forceinline__ UnitBases unit_pair(int u0, int u1, int lo, int hi)
-{
-	return {insert2(2 * u0, lo, hi), insert2(2 * u0 + 1, lo, hi), insert2(2 * u1, lo, hi),
-	        insert2(2 * u1 + 1, lo, hi)};
-}
 
 // the two units of the row set with first row S for a gate whose partner gate has tile
 // bits (o1, o2): bases S, S|2^o1 and S|2^o2, S|2^o1|2^o2
@@ -330,18 +318,6 @@ __device__ __forceinline__ void apply_bases2(const double* in, const double* din
 	}
 }
 
-// apply_bases2 for units u0 and u1 of a gate (unit u: the group bases 2u, 2u+1 of the
-// gate's own enumeration)
-template <bool TAN>
-__device__ __forceinline__ void apply_unit2(const double* in, const double* din, double2* out, double2* dout, int u0,
-                                           int u1, bool has1, const StepLane& sl, const double bg[2], const double bz[2],
-                                           bool dzero, int lane)
-{
-	const int bs0 = insert2(2 * u0 + (lane >> 4), sl.lo, sl.hi);
-	const int bs1 = insert2(2 * (has1 ? u1 : u0) + (lane >> 4), sl.lo, sl.hi);
-	apply_bases2<TAN>(in, din, out, dout, bs0, bs1, has1, sl, bg, bz, dzero, lane);
-}
-
 // 16-byte asynchronous copy global -> shared (cp.async, L2 only), and its group fences
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 {
@@ -351,160 +327,325 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// shared memory of k3_fwd: gates, row offsets and two buffers of (state, tangent) tiles
-inline size_t k3_fwd_smem(int NB, bool tan)
+// A forward pass's gates in rounds of one or two, and its tile: 2^TB amplitudes, the lowest tile
+// bits the column's, the others those of the pass's row bits.
+struct FwdArgs
 {
-	return 32 * MAXK * sizeof(double2) + (1 << MAXNB) * sizeof(int) + (tan ? 4 : 2) * ((size_t)1 << NB) * 4 * sizeof(double2);
+	Gate4<double> g[MAXK], z[MAXK];           // first gates of the rounds
+	Gate4<double> g2[MAXK - 1], z2[MAXK - 1];   // second gates (round MAXK - 1 has none)
+	int rounds, pair[MAXK];                     // pair: the round has a second gate
+	int cb;                                     // tile bits of the column
+	int step[MAXK][4];                          // places (bytes) of the tile bits of a thread's amplitudes
+	int8_t pos[MAXK][8];                        // tile bits of a thread's index bits (0, 1: wires j, i of the first gate)
+	int8_t tbit[16];                            // row bit of tile bit b >= cb
+	uint32_t krow[16];                          // row bits of a thread's amplitude k of a tile, and its offset
+	int64_t koff[16];
+	// row tile number to row bits outside the tile: runs of consecutive bits
+	int nseg;
+	int8_t seg_from[MAXNB + 1], seg_to[MAXNB + 1];
+	uint32_t seg_mask[MAXNB + 1];
+	int64_t C, cols;                            // row pitch; columns to take (a multiple of 4)
+	uint32_t ncgt, ntiles;                      // column tiles; all tiles
+	ColumnSource src;
+};
+
+constexpr int NT8F = 128;   // threads of the complex128 forward kernel (four blocks per SM)
+__host__ __device__ constexpr int fwd_tile_bits(bool tan) { return tan ? 10 : 11; }
+constexpr int FWD_TILE_BYTES = 2048 * (int)sizeof(double2);   // one tile of 2^11, or state and tangent of 2^10
+
+// dx <- G dx + Z x, x <- G x on the four amplitudes
+__device__ __forceinline__ void apply4_tan(const Gate4<double>& g, const Gate4<double>& z, double2* x, double2* dx)
+{
+	double2 y[4];
+#pragma unroll
+	for (int r = 0; r < 4; r++) y[r] = make_double2(0, 0);
+#pragma unroll
+	for (int c = 0; c < 4; c++) {
+#pragma unroll
+		for (int r = 0; r < 4; r++) {
+			y[r].x = fma(z.m[4 * r + c].x, x[c].x, y[r].x);
+			y[r].y = fma(z.m[4 * r + c].x, x[c].y, y[r].y);
+		}
+#pragma unroll
+		for (int r = 0; r < 4; r++) {
+			y[r].x = fma(-z.m[4 * r + c].y, x[c].y, y[r].x);
+			y[r].y = fma(z.m[4 * r + c].y, x[c].x, y[r].y);
+		}
+#pragma unroll
+		for (int r = 0; r < 4; r++) {
+			y[r].x = fma(g.m[4 * r + c].x, dx[c].x, y[r].x);
+			y[r].y = fma(g.m[4 * r + c].x, dx[c].y, y[r].y);
+		}
+#pragma unroll
+		for (int r = 0; r < 4; r++) {
+			y[r].x = fma(-g.m[4 * r + c].y, dx[c].y, y[r].x);
+			y[r].y = fma(g.m[4 * r + c].y, dx[c].x, y[r].y);
+		}
+	}
+#pragma unroll
+	for (int r = 0; r < 4; r++) dx[r] = y[r];
+	apply4<1>(g, x);
 }
 
-// One pass forward over tiles (complex128).  IN: 0 read psi/dpsi, 1 basis columns (dpsi = 0).
+// One pass forward over tiles (complex128), two gates per round where consecutive ones act on wires
+// of their own, as in layer_pass.cu: the round's first gate on the FP64 MMA with an amplitude's parts
+// as two operands, the second in FMAs on a thread's own 16 amplitudes (8 with their tangents), so
+// that a round reads and writes the tile in shared memory once.  IN: 0 read psi/dpsi, 1 basis
+// columns (dpsi = 0).
 // OUT: 0 store psi/dpsi, 1 store -conj(psi) (no tangent), 2 f += <phi, psi> (no store),
 // 3 store the pass output and add f, as the last pass does when the reverse pass rebuilds
 // states from it.
-// Tiles are double-buffered in shared memory: the next tile position's state arrives
-// by cp.async while the gates run on the current one.
+// With tangents four gates do 6 flop per byte, the balance of the FP64 pipe and memory; without, 4.
+// A kernel that applied a gate at a time, with 8 x 8 real embeddings as MMA operands and so a read
+// (in 8-byte words) and a write of the tile per gate, took 68 us a pass of four gates with tangents
+// on the L = 12 brickwall's 352 columns and 50 us without on the 2^22 amplitudes of L = 11; this one
+// 54 and 34 us (3.9 TB/s, 16 TFLOP/s).
 template <bool TAN, int IN, int OUT>
-__global__ void __launch_bounds__(NTF, TAN ? 3 : 6) k3_fwd(const double2* __restrict__ psi, const double2* __restrict__ dpsi,
-                                              double2* __restrict__ psi_o, double2* __restrict__ dpsi_o,
-                                              const double2* __restrict__ phi, PassGeom pg, PassGates<double> gates,
-                                              double2* __restrict__ fpart)
+__global__ void __launch_bounds__(NT8F, 4) k8_fwd(const double2* __restrict__ psi, const double2* __restrict__ dpsi,
+                                                  double2* __restrict__ psi_o, double2* __restrict__ dpsi_o,
+                                                  const double2* __restrict__ phi, const __grid_constant__ FwdArgs a,
+                                                  double2* __restrict__ fpart)
 {
-	constexpr int CW = 4;
-	constexpr int EPTF = (1 << MAXNB) * CW / NTF;
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	const int R = 1 << pg.NB, A = R * CW, K = pg.K;
-	double2* sg = reinterpret_cast<double2*>(smem_raw);
-	int* rowoff = reinterpret_cast<int*>(sg + 32 * MAXK);
-	double2* bufs = reinterpret_cast<double2*>(rowoff + (1 << MAXNB));   // [2][state, tangent][A], or [2][state][A] without tangents
-	gates_to_smem<double>(gates, K, TAN, sg);
-	row_offsets(pg, rowoff);
-	__syncthreads();
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-	double fx = 0, fy = 0;
-	const int units = R / 8;
-	// the pass input of a tile position into buffer b (IN 0: read from psi, dpsi)
-	auto fetch = [&](int64_t tile, int b) {
-		if (IN != 0 || tile >= pg.ntiles) return;
-		const int64_t rt = tile / pg.ncg, cg = tile - rt * pg.ncg;
-		const int64_t rowbase = deposit(rt, pg.rest_mask), colbase = cg * CW;
-		double2* dst = bufs + (size_t)b * (TAN ? 2 : 1) * A;
-#pragma unroll
-		for (int i = 0; i < EPTF; i++) {
-			const int e = threadIdx.x + i * NTF;
-			if (e >= A) continue;
-			const int64_t a = (rowbase + rowoff[e >> 2]) * pg.C + colbase + (e & 3);
-			const int pe = sidx(e >> 2, e & 3);
-			cp_async16(dst + pe, psi + a);
-			if (TAN) cp_async16(dst + A + pe, dpsi + a);
+	constexpr int TB = fwd_tile_bits(TAN), PER = 1 << (TB - 7);   // amplitudes per thread
+	constexpr int NP = TAN ? 4 : 2;                               // operands per round
+	extern __shared__ __align__(16) char tile[];
+	constexpr int DT = 16 << TB;                                  // the tangent's tile
+	__shared__ double sb[MAXK][NP][32];
+	const int tid = threadIdx.x, lane = tid & 31;
+	auto at_smem = [&](int byte) -> double2& { return *reinterpret_cast<double2*>(tile + byte); };
+	// operands of the rounds' first gates: for input amplitude k = lane & 3 and output part n = lane >> 2
+	for (int e = tid; e < MAXK * 32; e += NT8F) {
+		const int r = e >> 5, ln = e & 31;
+		if (r >= a.rounds) continue;
+		const double2 g = a.g[r].m[4 * (ln >> 3) + (ln & 3)];
+		sb[r][0][ln] = ln & 4 ? g.y : g.x;
+		sb[r][1][ln] = ln & 4 ? g.x : -g.y;
+		if (TAN) {
+			const double2 z = a.z[r].m[4 * (ln >> 3) + (ln & 3)];
+			sb[r][NP - 2][ln] = ln & 4 ? z.y : z.x;
+			sb[r][NP - 1][ln] = ln & 4 ? z.x : -z.y;
 		}
+	}
+	// this thread's amplitudes of a tile are tid + k 128
+	uint32_t row = 0;
+	int col = 0;
+#pragma unroll
+	for (int b = 0; b < 7; b++)
+		if ((tid >> b) & 1) {
+			if (b < a.cb) col |= 1 << b;
+			else row |= 1u << a.tbit[b];
+		}
+	const int64_t own = (int64_t)row * a.C + col;
+	const int place = swz(tid) << 4;
+	// first amplitude of this thread's set in each round
+	int base[MAXK];
+#pragma unroll
+	for (int r = 0; r < MAXK; r++) {
+		int v = 0;
+		if (r < a.rounds)
+#pragma unroll
+			for (int b = 0; b < 7; b++) v |= ((tid >> b) & 1) << a.pos[r][b];
+		base[r] = swz(v) << 4;
+	}
+	// rows and columns at which tile t begins
+	auto tile_at = [&](uint32_t t, uint32_t& rowbase, int64_t& colbase) {
+		const uint32_t rt = t / a.ncgt;
+		colbase = (int64_t)(t - rt * a.ncgt) << a.cb;
+		rowbase = 0;
+		for (int k = 0; k < a.nseg; k++) rowbase |= ((rt >> a.seg_from[k]) & a.seg_mask[k]) << a.seg_to[k];
 	};
-	fetch(blockIdx.x, 0);
-	cp_async_commit();
-
-	int buf = 0;
-	for (int64_t tile = blockIdx.x; tile < pg.ntiles; tile += gridDim.x, buf ^= 1) {
-		const int64_t rt = tile / pg.ncg, cg = tile - rt * pg.ncg;
-		const int64_t rowbase = deposit(rt, pg.rest_mask);
-		const int64_t colbase = cg * CW;
-		double2* S = bufs + (size_t)buf * (TAN ? 2 : 1) * A;
-		double2* dS = TAN ? S + A : nullptr;
-		if (IN == 0) {
-			cp_async_wait_all();
-		} else {
+	double fx = 0, fy = 0;
+	__syncthreads();
+	for (uint32_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+		{
+			uint32_t rowbase;
+			int64_t colbase;
+			tile_at(t, rowbase, colbase);
+			if (IN == 0) {
+				const int64_t at = (int64_t)rowbase * a.C + colbase + own;
+				const unsigned dst = (unsigned)__cvta_generic_to_shared(tile);
 #pragma unroll
-			for (int i = 0; i < EPTF; i++) {
-				const int e = threadIdx.x + i * NTF;
-				if (e >= A) continue;
-				const int r = e >> 2, cc = e & 3;
-				const int pe = sidx(r, cc);
-				const int64_t row = rowbase + rowoff[r], col = colbase + cc;
-				S[pe] = basis_amp<double>(pg.src, row, col);
-				if (TAN) dS[pe] = make_double2(0, 0);
-			}
-		}
-		// every thread's copies (or writes) of this tile have landed, and every thread is
-		// done with the other buffer (its previous tile), which the next fetch overwrites
-		__syncthreads();
-		fetch(tile + gridDim.x, buf ^ 1);
-		cp_async_commit();
-		const double* fS = reinterpret_cast<const double*>(S);
-		const double* fdS = reinterpret_cast<const double*>(dS);
-		bool skip = false;   // gate k was applied with gate k-1
-#pragma unroll
-		for (int k = 0; k < MAXK; k++) {
-			if (k >= K) break;
-			if (skip) { skip = false; continue; }
-			const bool dzero = IN == 1 && k == 0;
-			const int k2 = k + 1 < MAXK ? k + 1 : k;
-			if (k + 1 < K && pg.NB >= 4 && gates_disjoint(pg, k, k2)) {
-				// gates k and k+1 on this warp's row sets, one block barrier for both (each
-				// gate's operands are loaded per set, which keeps registers for one gate)
-				const int m = (1 << pg.gi[k]) | (1 << pg.gj[k]) | (1 << pg.gi[k2]) | (1 << pg.gj[k2]);
-				const int hs = lane >> 4;
-				for (int s = warp; s < (R >> 4); s += nwarps) {
-					const int S0 = set_base(s, m);
-					{
-						const StepLane sl(pg.gi[k], pg.gj[k], lane);
-						double bg[2], bz[2] = {0, 0};
-						bfrag(sg + 32 * k, true, lane, bg);
-						if (TAN) bfrag(sg + 32 * k + 16, true, lane, bz);
-						const UnitBases ua = set_units(S0, pg.gi[k2], pg.gj[k2]);
-						apply_bases2<TAN>(fS, fdS, S, dS, hs ? ua.b01 : ua.b00, hs ? ua.b11 : ua.b10, true, sl, bg,
-						                  bz, dzero, lane);
+				for (int k = 0; k < PER; k++)
+					if (colbase + col < a.cols) {
+						const unsigned d = dst + (place ^ (swz(k << 7) << 4));
+						asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(psi + at + a.koff[k]) : "memory");
+						if (TAN)
+							asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + DT), "l"(dpsi + at + a.koff[k])
+							             : "memory");
 					}
-					__syncwarp();
-					const StepLane sl2(pg.gi[k2], pg.gj[k2], lane);
-					double bg2[2], bz2[2] = {0, 0};
-					bfrag(sg + 32 * k2, true, lane, bg2);
-					if (TAN) bfrag(sg + 32 * k2 + 16, true, lane, bz2);
-					const UnitBases ub = set_units(S0, pg.gi[k], pg.gj[k]);
-					apply_bases2<TAN>(fS, fdS, S, dS, hs ? ub.b01 : ub.b00, hs ? ub.b11 : ub.b10, true, sl2, bg2, bz2,
-					                  false, lane);
-				}
-				skip = true;
+				cp_async_commit();
+				cp_async_wait_all();
 			} else {
-				const StepLane sl(pg.gi[k], pg.gj[k], lane);
-				double bg[2], bz[2] = {0, 0};
-				bfrag(sg + 32 * k, true, lane, bg);
-				if (TAN) bfrag(sg + 32 * k + 16, true, lane, bz);
-				for (int u = warp; u < units; u += 2 * nwarps)
-					apply_unit2<TAN>(fS, fdS, S, dS, u, u + nwarps, u + nwarps < units, sl, bg, bz, dzero, lane);
+#pragma unroll
+				for (int k = 0; k < PER; k++) {
+					const int d = place ^ (swz(k << 7) << 4);
+					at_smem(d) = basis_amp<double>(a.src, (int64_t)(rowbase | row | a.krow[k]), colbase + col);
+					if (TAN) at_smem(d + DT) = make_double2(0, 0);
+				}
 			}
-			__syncthreads();
 		}
-		for (int i = 0; i < EPTF; i++) {
-			const int e = threadIdx.x + i * NTF;
-			if (e >= A) continue;
-			const int r = e >> 2, cc = e & 3;
-			const int64_t a = (rowbase + rowoff[r]) * pg.C + colbase + cc;
-			const int pe = sidx(r, cc);
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r < MAXK; r++) {
+			if (r < a.rounds) {
+				const int s0 = a.step[r][0], s1 = a.step[r][1], s2 = a.step[r][2], s3 = TAN ? 0 : a.step[r][3];
+				auto mem = [&](int k) {
+					return TAN ? base[r] ^ (k & 4 ? s0 : 0) ^ (k & 2 ? s1 : 0) ^ (k & 1 ? s2 : 0)
+					           : base[r] ^ (k & 8 ? s0 : 0) ^ (k & 4 ? s1 : 0) ^ (k & 2 ? s2 : 0) ^ (k & 1 ? s3 : 0);
+				};
+				double2 x[PER], dx[TAN ? PER : 1];
+#pragma unroll
+				for (int k = 0; k < PER; k++) {
+					x[k] = at_smem(mem(k));
+					if (TAN) dx[k] = at_smem(mem(k) + DT);
+				}
+				const double b0 = sb[r][0][lane], b1 = sb[r][1][lane];
+				const double z0 = TAN ? sb[r][NP - 2][lane] : 0, z1 = TAN ? sb[r][NP - 1][lane] : 0;
+#pragma unroll
+				for (int k = 0; k < PER; k++) {
+					if (TAN) {
+						double2 y = make_double2(0, 0);
+						dmma_amp(y, x[k].x, z0);
+						dmma_amp(y, x[k].y, z1);
+						dmma_amp(y, dx[k].x, b0);
+						dmma_amp(y, dx[k].y, b1);
+						dx[k] = y;
+					}
+					double2 y = make_double2(0, 0);
+					dmma_amp(y, x[k].x, b0);
+					dmma_amp(y, x[k].y, b1);
+					x[k] = y;
+				}
+				if (r < MAXK - 1 && a.pair[r])
+#pragma unroll
+					for (int k = 0; k < PER; k += 4) {
+						if (TAN) apply4_tan(a.g2[r], a.z2[r], x + k, dx + k);
+						else apply4<1>(a.g2[r], x + k);
+					}
+#pragma unroll
+				for (int k = 0; k < PER; k++) {
+					at_smem(mem(k)) = x[k];
+					if (TAN) at_smem(mem(k) + DT) = dx[k];
+				}
+				__syncthreads();
+			}
+		}
+		uint32_t rowbase;
+		int64_t colbase;
+		tile_at(t, rowbase, colbase);
+		const int64_t at = (int64_t)rowbase * a.C + colbase + own;
+#pragma unroll
+		for (int k = 0; k < PER; k++) {
+			if (colbase + col >= a.cols) continue;
+			const int d = place ^ (swz(k << 7) << 4);
+			const double2 v = at_smem(d);
 			if (OUT == 2 || OUT == 3) {
-				const double2 p = phi[a], v = S[pe];
+				const double2 p = phi[at + a.koff[k]];
 				fx += p.x * v.x - p.y * v.y;
 				fy += p.x * v.y + p.y * v.x;
 			}
 			if (OUT == 1) {
-				psi_o[a] = cneg_conj(S[pe]);
+				psi_o[at + a.koff[k]] = cneg_conj(v);
 			} else if (OUT != 2) {
-				psi_o[a] = S[pe];
-				if (TAN) dpsi_o[a] = dS[pe];
+				psi_o[at + a.koff[k]] = v;
+				if (TAN) dpsi_o[at + a.koff[k]] = at_smem(d + DT);
 			}
 		}
+		__syncthreads();
 	}
-	cp_async_wait_all();
 	if (OUT == 2 || OUT == 3) {
-		__shared__ double red[2][NTF / 32];
+		__shared__ double red[2][NT8F / 32];
+		const int warp = tid >> 5;
 		fx = warp_sum(fx);
 		fy = warp_sum(fy);
 		if (lane == 0) { red[0][warp] = fx; red[1][warp] = fy; }
 		__syncthreads();
-		if (threadIdx.x == 0) {
+		if (tid == 0) {
 			double sx = 0, sy = 0;
-			for (int w = 0; w < nwarps; w++) { sx += red[0][w]; sy += red[1][w]; }
+			for (int w = 0; w < NT8F / 32; w++) { sx += red[0][w]; sy += red[1][w]; }
 			fpart[blockIdx.x].x += sx;
 			fpart[blockIdx.x].y += sy;
 		}
 	}
+}
+
+// the arguments of k8_fwd for a pass
+FwdArgs fwd_args(const PassGeom& pg, const PassGates<double>& gates, bool tan)
+{
+	FwdArgs a;
+	const int TB = fwd_tile_bits(tan), cb = TB - pg.NB, own = TB - 7;   // own: bits of a thread's amplitudes
+	a.cb = cb;
+	a.C = pg.C;
+	a.cols = pg.ncg * 4;
+	a.src = pg.src;
+	a.ncgt = (uint32_t)((a.cols + ((int64_t)1 << cb) - 1) >> cb);
+	a.ntiles = a.ncgt << (pg.L - pg.NB);
+	for (int b = 0; b < TB; b++) a.tbit[b] = (int8_t)(b < cb ? 0 : pg.tbit[b - cb]);
+	for (int k = 0; k < 1 << own; k++) {
+		a.krow[k] = 0;   // (L >= 4: the column's bits are thread bits)
+		for (int b = 0; b < own; b++)
+			if ((k >> b) & 1) a.krow[k] |= 1u << a.tbit[7 + b];
+		a.koff[k] = (int64_t)a.krow[k] * a.C;
+	}
+	a.nseg = 0;
+	for (int b = 0, from = 0; b < pg.L;) {
+		if (!((pg.rest_mask >> b) & 1)) {
+			b++;
+			continue;
+		}
+		int e = b;
+		while (e < pg.L && ((pg.rest_mask >> e) & 1)) e++;
+		a.seg_from[a.nseg] = (int8_t)from;
+		a.seg_to[a.nseg] = (int8_t)b;
+		a.seg_mask[a.nseg++] = (1u << (e - b)) - 1;
+		from += e - b;
+		b = e;
+	}
+	// consecutive gates on wires of their own share a round
+	a.rounds = 0;
+	for (int k = 0; k < pg.K;) {
+		const int r = a.rounds++;
+		uint32_t used = 0;
+		auto bit_of = [&](int local) {
+			used |= 1u << (cb + local);
+			return cb + local;
+		};
+		const uint32_t w0 = (1u << pg.gi[k]) | (1u << pg.gj[k]);
+		const bool pair = k + 1 < pg.K && !(w0 & ((1u << pg.gi[k + 1]) | (1u << pg.gj[k + 1])));
+		a.pair[r] = pair;
+		a.g[r] = gates.g[k];
+		a.z[r] = gates.z[k];
+		a.pos[r][0] = (int8_t)bit_of(pg.gj[k]);
+		a.pos[r][1] = (int8_t)bit_of(pg.gi[k]);
+		int slot = own;
+		if (pair) {
+			slot -= 2;
+			a.g2[r] = gates.g[k + 1];
+			a.z2[r] = gates.z[k + 1];
+			a.step[r][slot] = swz(1 << bit_of(pg.gi[k + 1])) << 4;
+			a.step[r][slot + 1] = swz(1 << bit_of(pg.gj[k + 1])) << 4;
+		}
+		k += pair ? 2 : 1;
+		// thread bit 2: of the residue mod 3 that the gate's two bits leave (a quarter-warp's accesses
+		// then fall into different banks), if there is one
+		int third = -1;
+		for (int b = 0; b < TB && third < 0; b++)
+			if (!((used >> b) & 1) && b % 3 != a.pos[r][0] % 3 && b % 3 != a.pos[r][1] % 3) third = b;
+		for (int b = 0; b < TB && third < 0; b++)
+			if (!((used >> b) & 1)) third = b;
+		a.pos[r][2] = (int8_t)third;
+		used |= 1u << third;
+		// the remaining bits: the highest to the thread's own amplitudes, the others to the thread index
+		for (int b = TB - 1, s = 0; s < slot; b--)
+			if (!((used >> b) & 1)) {
+				a.step[r][s++] = swz(1 << b) << 4;
+				used |= 1u << b;
+			}
+		int m = 3;
+		for (int b = 0; b < TB; b++)
+			if (!((used >> b) & 1)) a.pos[r][m++] = (int8_t)b;
+	}
+	return a;
 }
 
 // One pass in reverse (complex128), from the checkpoint psi, dpsi at the pass input and
@@ -899,7 +1040,7 @@ inline size_t k4_fwd_smem(int NB, bool tan, bool with_phi)
 	       MAXK * 32 * sizeof(int) + 2 * ns * A * sizeof(float2);
 }
 
-// Forward pass (complex64).  Same contract as k3_fwd.  The next tile streams into a
+// Forward pass (complex64).  Same contract as k8_fwd.  The next tile streams into a
 // second set of shared-memory buffers with cp.async while the current one is processed.
 template <bool TAN, int IN, int OUT>
 __global__ void __launch_bounds__(NT4F, 3) k4_fwd(const float2* __restrict__ psi, const float2* __restrict__ dpsi,
@@ -2231,12 +2372,6 @@ PassGates<T> pass_gates(const Pass& p, const double2* gates, const double2* dirs
 }
 
 template <typename T>
-size_t fwd_smem(int NB)
-{
-	return 32 * MAXK * sizeof(cplx<T>) + (1 << MAXNB) * sizeof(int) + 2 * ((size_t)1 << NB) * ColsPer<T>::v * sizeof(cplx<T>);
-}
-
-template <typename T>
 size_t rev_smem(int NB, int K, bool tan)
 {
 	if (!std::is_same<T, double>::value) return k4_rev_smem(NB, K, tan);
@@ -2286,16 +2421,15 @@ template <typename T, bool TAN, int IN, int OUT>
 int launch_fwd(Runtime& rt, const cplx<T>* psi, const cplx<T>* dpsi, cplx<T>* psi_o, cplx<T>* dpsi_o, const cplx<T>* phi,
                const PassGeom& pg, const PassGates<T>& gates, double2* fpart, int fgrid)
 {
-	const size_t smem = fwd_smem<T>(pg.NB);
 	static int per_sm = 0;
 	if constexpr (std::is_same<T, double>::value) {
 		if (!per_sm) {
-			int ret = prepare(k3_fwd<TAN, IN, OUT>, k3_fwd_smem(MAXNB, TAN), &per_sm, NTF);
+			int ret = prepare(k8_fwd<TAN, IN, OUT>, FWD_TILE_BYTES, &per_sm, NT8F);
 			if (ret) return ret;
 		}
-		const int grid = OUT >= 2 ? fgrid : (int)std::max<int64_t>(1, std::min<int64_t>(pg.ntiles, (int64_t)rt.num_sms * per_sm));
-		RQC_LAUNCH3(rt, KC_FUSED, (k3_fwd<TAN, IN, OUT>), grid, NTF, k3_fwd_smem(pg.NB, TAN), psi, dpsi, psi_o, dpsi_o, phi,
-		            pg, gates, fpart);
+		const FwdArgs args = fwd_args(pg, gates, TAN);
+		const int grid = OUT >= 2 ? fgrid : (int)std::max<int64_t>(1, std::min<int64_t>(args.ntiles, (int64_t)rt.num_sms * per_sm));
+		RQC_LAUNCH3(rt, KC_FUSED, (k8_fwd<TAN, IN, OUT>), grid, NT8F, FWD_TILE_BYTES, psi, dpsi, psi_o, dpsi_o, phi, args, fpart);
 	} else if (rt.c64_ffma) {
 		static int per_sm7 = 0;
 		if (!per_sm7) {

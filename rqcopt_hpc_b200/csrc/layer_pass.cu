@@ -21,6 +21,7 @@
 // The tile's words are permuted within 128-byte lines (swz) and the lanes' bits chosen per round
 // so that a quarter-warp's 16-byte accesses fall into different banks.
 #include "layer_pass.h"
+#include "pass_tile.cuh"
 
 #include <algorithm>
 
@@ -49,53 +50,11 @@ struct PassArgs
 	ColumnSource src;
 };
 
-// place of tile amplitude i: its 16-byte word within a 128-byte line XORed with the bits above
-__host__ __device__ __forceinline__ constexpr int swz(int i) { return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9)) & 7); }
-
 __device__ __forceinline__ int64_t tile_base(const PassArgs& a, int64_t t)
 {
 	int64_t r = 0;
 	for (int k = 0; k < a.nseg; k++) r |= (int64_t)(((uint64_t)t >> a.seg_from[k]) & a.seg_mask[k]) << a.seg_to[k];
 	return r;
-}
-
-// D (8 groups x [re, im of 4 amplitudes]) += a (8 groups x 4) b: a lane's a is one part of amplitude
-// lane & 3 of group lane >> 2, and its D are the parts of that same amplitude
-__device__ __forceinline__ void dmma(double2& d, double a, double b)
-{
-	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-	    : "+d"(d.x), "+d"(d.y)
-	    : "d"(a), "d"(b));
-}
-
-// the 4x4 gate on the four amplitudes x[0], x[s], x[2 s], x[3 s]
-template <int S>
-__device__ __forceinline__ void apply4(const Gate4<double>& g, double2* x)
-{
-	// eight sums side by side, each touched every eighth FMA
-	double2 y[4];
-#pragma unroll
-	for (int r = 0; r < 4; r++) y[r] = make_double2(g.m[4 * r].x * x[0].x, g.m[4 * r].x * x[0].y);
-#pragma unroll
-	for (int r = 0; r < 4; r++) {
-		y[r].x = fma(-g.m[4 * r].y, x[0].y, y[r].x);
-		y[r].y = fma(g.m[4 * r].y, x[0].x, y[r].y);
-	}
-#pragma unroll
-	for (int c = 1; c < 4; c++) {
-#pragma unroll
-		for (int r = 0; r < 4; r++) {
-			y[r].x = fma(g.m[4 * r + c].x, x[c * S].x, y[r].x);
-			y[r].y = fma(g.m[4 * r + c].x, x[c * S].y, y[r].y);
-		}
-#pragma unroll
-		for (int r = 0; r < 4; r++) {
-			y[r].x = fma(-g.m[4 * r + c].y, x[c * S].y, y[r].x);
-			y[r].y = fma(g.m[4 * r + c].y, x[c * S].x, y[r].y);
-		}
-	}
-#pragma unroll
-	for (int r = 0; r < 4; r++) x[r * S] = y[r];
 }
 
 // Shared-memory addresses are byte offsets into the tile (places * 16), so that a member's is one
@@ -168,8 +127,8 @@ k_lpass(const double2* in, double2* out, const __grid_constant__ PassArgs a)
 #pragma unroll
 				for (int k = 0; k < 16; k++) {
 					double2 y = make_double2(0, 0);
-					dmma(y, x[k].x, bre[r]);
-					dmma(y, x[k].y, bim[r]);
+					dmma_amp(y, x[k].x, bre[r]);
+					dmma_amp(y, x[k].y, bim[r]);
 					x[k] = y;
 				}
 				if (2 * r + 1 < a.K)

@@ -79,3 +79,33 @@ def test_circuit_sums_in_passes_of_several_groups(gpu, L, G, near, per_pass):
     for a, b in zip(got, ref):
         assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
     assert np.linalg.norm(grad[1] - ref[1]) <= 1e-12 * np.linalg.norm(ref[1])
+
+
+@pytest.mark.parametrize("L", [4, 5, 7, 8, 9, 11])
+@pytest.mark.parametrize("near", [False, True])
+@pytest.mark.parametrize("unitary", [False, True])
+@pytest.mark.parametrize("first,last", [(0, 0), (1, 2), (3, 14)])
+def test_forward_passes_on_ragged_columns(gpu, L, near, unitary, first, last):
+    """Forward passes with and without tangents, column ranges that end inside a tile, gates that
+    share wires: against one kernel per gate, 1e-12 as between the engines."""
+    rng = np.random.default_rng(L)
+    make = (lambda: haar_unitary(rng)) if unitary else (lambda: crandn((4, 4), rng) / 4)
+    gates, target = (np.stack([make() for _ in range(n)]) for n in (9, 5))
+    pool = 4 if near else L
+    wires, twires = (np.array([rng.choice(pool, 2, replace=False) for _ in range(n)], np.int32) for n in (9, 5))
+    dirs = crandn((9, 4, 4), rng)
+    t = gpu.Target(circuit=(target, twires))
+
+    def run(per_pass):
+        gpu.set_gates_per_pass(per_pass)
+        return (*gpu.circuit_unitary_target_hessian_vector_product(t, gates, dirs, wires, L),
+                *gpu.circuit_unitary_target_and_gradient(t, gates, wires, L))
+
+    try:
+        gpu.set_column_range(first, last)
+        ref = run(1)
+        for per_pass in (4, 3):
+            for a, b in zip(run(per_pass), ref):
+                assert np.linalg.norm(a - b) <= 1e-12 * (np.linalg.norm(b) + np.linalg.norm(ref[1]))
+    finally:
+        gpu.set_column_range(0, 0)
