@@ -235,89 +235,6 @@ __device__ __forceinline__ void apply_unit(const double* in, const double* din, 
 	if (TAN) dout[st] = make_double2(z0, z1);
 }
 
-// Rows owned by one warp across two gates.  When gates a and b of a pass act on
-// disjoint tile bits, the 2^NB tile rows split into 2^(NB-4) sets of 16 rows that are
-// closed under both gates (the rows that agree outside the four bits), so a warp can
-// apply a then b to its sets with warp-level synchronisation only, and the block
-// barrier between the two gates goes away.
-
-// first row of set s: s with zero bits inserted at the set bits of m (in increasing order)
-__device__ __forceinline__ int set_base(int s, int m)
-{
-#pragma unroll
-	for (int i = 0; i < 4; i++) {
-		const int p = __ffs(m) - 1;
-		s = ((s >> p) << (p + 1)) | (s & ((1 << p) - 1));
-		m &= m - 1;
-	}
-	return s;
-}
-
-// The group bases of the two units a warp works on at once: unit 0 holds the groups at
-// bases b00 and b01, unit 1 those at b10 and b11 (the group base of a unit is selected by
-// lane >> 4, as in apply_unit).
-struct UnitBases
-{
-	int b00, b01, b10, b11;
-};
-
-// the two units of the row set with first row S for a gate whose partner gate has tile
-// bits (o1, o2): bases S, S|2^o1 and S|2^o2, S|2^o1|2^o2
-__device__ __forceinline__ UnitBases set_units(int S, int o1, int o2)
-{
-	return {S, S | (1 << o1), S | (1 << o2), S | (1 << o1) | (1 << o2)};
-}
-
-// apply_unit for two units of a warp at once; bs0 and bs1 are this lane's group bases of
-// the two units (the second is ignored unless has1, which is the same for all lanes).
-// Both units' operands are loaded before either is stored, so the two independent MMA
-// chains overlap; in place like apply_unit(..., inplace = true).
-template <bool TAN>
-__device__ __forceinline__ void apply_bases2(const double* in, const double* din, double2* out, double2* dout,
-                                            int bs0, int bs1, bool has1, const StepLane& sl, const double bg[2],
-                                            const double bz[2], bool dzero, int lane)
-{
-	const int cc = (lane >> 2) & 3;
-	if (!has1) bs1 = bs0;
-	const int j00 = sidx(bs0 | sl.m_k0, cc) * 2 + sl.part_out, j01 = sidx(bs0 | sl.m_k1, cc) * 2 + sl.part_out;
-	const int j10 = sidx(bs1 | sl.m_k0, cc) * 2 + sl.part_out, j11 = sidx(bs1 | sl.m_k1, cc) * 2 + sl.part_out;
-	const double a00 = in[j00], a01 = in[j01], a10 = in[j10], a11 = in[j11];
-	double d00 = 0, d01 = 0, d10 = 0, d11 = 0;
-	if (TAN && !dzero) {
-		d00 = din[j00];
-		d01 = din[j01];
-		d10 = din[j10];
-		d11 = din[j11];
-	}
-	double y0a = 0, y1a = 0, y0b = 0, y1b = 0, z0a = 0, z1a = 0, z0b = 0, z1b = 0;
-	dmma(y0a, y1a, a00, bg[0]);
-	dmma(y0b, y1b, a10, bg[0]);
-	if (TAN) {
-		dmma(z0a, z1a, a00, bz[0]);
-		dmma(z0b, z1b, a10, bz[0]);
-	}
-	dmma(y0a, y1a, a01, bg[1]);
-	dmma(y0b, y1b, a11, bg[1]);
-	if (TAN) {
-		dmma(z0a, z1a, a01, bz[1]);
-		dmma(z0b, z1b, a11, bz[1]);
-		if (!dzero) {
-			dmma(z0a, z1a, d00, bg[0]);
-			dmma(z0b, z1b, d10, bg[0]);
-			dmma(z0a, z1a, d01, bg[1]);
-			dmma(z0b, z1b, d11, bg[1]);
-		}
-	}
-	__syncwarp();
-	const int st0 = sidx(bs0 | sl.m_st, cc), st1 = sidx(bs1 | sl.m_st, cc);
-	out[st0] = make_double2(y0a, y1a);
-	if (TAN) dout[st0] = make_double2(z0a, z1a);
-	if (has1) {
-		out[st1] = make_double2(y0b, y1b);
-		if (TAN) dout[st1] = make_double2(z0b, z1b);
-	}
-}
-
 // 16-byte asynchronous copy global -> shared (cp.async, L2 only), and its group fences
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 {
@@ -327,15 +244,13 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// A forward pass's gates in rounds of one or two, and its tile: 2^TB amplitudes, the lowest tile
-// bits the column's, the others those of the pass's row bits.
-struct FwdArgs
+// The tile of a complex128 pass, 2^TB amplitudes, the lowest tile bits the column's, the others those
+// of the pass's row bits; and its gates in rounds of one or two on wires of their own.
+struct PassTile
 {
-	Gate4<double> g[MAXK], z[MAXK];           // first gates of the rounds
-	Gate4<double> g2[MAXK - 1], z2[MAXK - 1];   // second gates (round MAXK - 1 has none)
 	int rounds, pair[MAXK];                     // pair: the round has a second gate
 	int cb;                                     // tile bits of the column
-	int step[MAXK][4];                          // places (bytes) of the tile bits of a thread's amplitudes
+	int step[MAXK][4];                          // places (bytes) of the tile bits of a thread's amplitudes in a round
 	int8_t pos[MAXK][8];                        // tile bits of a thread's index bits (0, 1: wires j, i of the first gate)
 	int8_t tbit[16];                            // row bit of tile bit b >= cb
 	uint32_t krow[16];                          // row bits of a thread's amplitude k of a tile, and its offset
@@ -346,8 +261,78 @@ struct FwdArgs
 	uint32_t seg_mask[MAXNB + 1];
 	int64_t C, cols;                            // row pitch; columns to take (a multiple of 4)
 	uint32_t ncgt, ntiles;                      // column tiles; all tiles
+};
+
+// The rounds' matrices: X <- g X, dX <- g dX + z X by the first gate, by g2, z2 the second
+// (round MAXK - 1 has none)
+struct RoundGates
+{
+	Gate4<double> g[MAXK], z[MAXK], g2[MAXK - 1], z2[MAXK - 1];
+};
+
+struct FwdArgs : PassTile
+{
+	RoundGates m;
 	ColumnSource src;
 };
+
+// row and column at which tile t begins
+__device__ __forceinline__ void tile_at(const PassTile& a, uint32_t t, uint32_t& rowbase, int64_t& colbase)
+{
+	const uint32_t rt = t / a.ncgt;
+	colbase = (int64_t)(t - rt * a.ncgt) << a.cb;
+	rowbase = 0;
+	for (int k = 0; k < a.nseg; k++) rowbase |= ((rt >> a.seg_from[k]) & a.seg_mask[k]) << a.seg_to[k];
+}
+
+// row bits and column of this thread's first amplitude of a tile (NTB thread bits)
+template <int NTB>
+__device__ __forceinline__ void tile_own(const PassTile& a, uint32_t& row, int& col)
+{
+	row = 0;
+	col = 0;
+#pragma unroll
+	for (int b = 0; b < NTB; b++)
+		if ((threadIdx.x >> b) & 1) {
+			if (b < a.cb) col |= 1 << b;
+			else row |= 1u << a.tbit[b];
+		}
+}
+
+// place (bytes) of the first amplitude of this thread's set in round r
+template <int NTB>
+__device__ __forceinline__ int round_base(const PassTile& a, int r)
+{
+	int v = 0;
+	if (r < a.rounds)
+#pragma unroll
+		for (int b = 0; b < NTB; b++) v |= ((threadIdx.x >> b) & 1) << a.pos[r][b];
+	return swz(v) << 4;
+}
+
+// operands of the rounds' first gates: for input amplitude k = lane & 3 and output part n = lane >> 2
+template <bool TAN, int NT>
+__device__ __forceinline__ void round_operands(const RoundGates& m, int rounds, double (*sb)[TAN ? 4 : 2][32])
+{
+	constexpr int NP = TAN ? 4 : 2;
+	for (int e = threadIdx.x; e < MAXK * 32; e += NT) {
+		const int r = e >> 5, ln = e & 31;
+		if (r >= rounds) continue;
+		const double2 g = m.g[r].m[4 * (ln >> 3) + (ln & 3)];
+		sb[r][0][ln] = ln & 4 ? g.y : g.x;
+		sb[r][1][ln] = ln & 4 ? g.x : -g.y;
+		if (TAN) {
+			const double2 z = m.z[r].m[4 * (ln >> 3) + (ln & 3)];
+			sb[r][NP - 2][ln] = ln & 4 ? z.y : z.x;
+			sb[r][NP - 1][ln] = ln & 4 ? z.x : -z.y;
+		}
+	}
+}
+
+__device__ __forceinline__ void cp_async_to(unsigned smem_dst, const void* gmem_src)
+{
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_dst), "l"(gmem_src) : "memory");
+}
 
 constexpr int NT8F = 128;   // threads of the complex128 forward kernel (four blocks per SM)
 __host__ __device__ constexpr int fwd_tile_bits(bool tan) { return tan ? 10 : 11; }
@@ -387,6 +372,56 @@ __device__ __forceinline__ void apply4_tan(const Gate4<double>& g, const Gate4<d
 	apply4<1>(g, x);
 }
 
+// One round on a tile: the first gate on the FP64 MMA with an amplitude's parts as two operands, the
+// second in FMAs on the thread's own amplitudes.  X at byte `x` of the tile, its tangent at `dx`.
+template <bool TAN, int PER>
+__device__ __forceinline__ void tile_round(char* tile, int x, int dx, int base, const int (&step)[4], const double (*sb)[32],
+                                           bool pair, const Gate4<double>& g2, const Gate4<double>& z2)
+{
+	constexpr int NP = TAN ? 4 : 2;
+	const int lane = threadIdx.x & 31;
+	auto at = [&](int k, int o) -> double2& {
+		int m = base;
+		if (PER == 16) m ^= (k & 8 ? step[0] : 0) ^ (k & 4 ? step[1] : 0) ^ (k & 2 ? step[2] : 0) ^ (k & 1 ? step[3] : 0);
+		else m ^= (k & 4 ? step[0] : 0) ^ (k & 2 ? step[1] : 0) ^ (k & 1 ? step[2] : 0);
+		return *reinterpret_cast<double2*>(tile + m + o);
+	};
+	double2 v[PER], d[TAN ? PER : 1];
+#pragma unroll
+	for (int k = 0; k < PER; k++) {
+		v[k] = at(k, x);
+		if (TAN) d[k] = at(k, dx);
+	}
+	const double b0 = sb[0][lane], b1 = sb[1][lane];
+	const double z0 = TAN ? sb[NP - 2][lane] : 0, z1 = TAN ? sb[NP - 1][lane] : 0;
+#pragma unroll
+	for (int k = 0; k < PER; k++) {
+		if (TAN) {
+			double2 y = make_double2(0, 0);
+			dmma_amp(y, v[k].x, z0);
+			dmma_amp(y, v[k].y, z1);
+			dmma_amp(y, d[k].x, b0);
+			dmma_amp(y, d[k].y, b1);
+			d[k] = y;
+		}
+		double2 y = make_double2(0, 0);
+		dmma_amp(y, v[k].x, b0);
+		dmma_amp(y, v[k].y, b1);
+		v[k] = y;
+	}
+	if (pair)
+#pragma unroll
+		for (int k = 0; k < PER; k += 4) {
+			if (TAN) apply4_tan(g2, z2, v + k, d + k);
+			else apply4<1>(g2, v + k);
+		}
+#pragma unroll
+	for (int k = 0; k < PER; k++) {
+		at(k, x) = v[k];
+		if (TAN) at(k, dx) = d[k];
+	}
+}
+
 // One pass forward over tiles (complex128), two gates per round where consecutive ones act on wires
 // of their own, as in layer_pass.cu: the round's first gate on the FP64 MMA with an amplitude's parts
 // as two operands, the second in FMAs on a thread's own 16 amplitudes (8 with their tangents), so
@@ -398,7 +433,7 @@ __device__ __forceinline__ void apply4_tan(const Gate4<double>& g, const Gate4<d
 // With tangents four gates do 6 flop per byte, the balance of the FP64 pipe and memory; without, 4.
 // A kernel that applied a gate at a time, with 8 x 8 real embeddings as MMA operands and so a read
 // (in 8-byte words) and a write of the tile per gate, took 68 us a pass of four gates with tangents
-// on the L = 12 brickwall's 352 columns and 50 us without on the 2^22 amplitudes of L = 11; this one
+// on the L = 12 brickwall's 700 columns and 50 us without on the 2^22 amplitudes of L = 11; this one
 // 54 and 34 us (3.9 TB/s, 16 TFLOP/s).
 template <bool TAN, int IN, int OUT>
 __global__ void __launch_bounds__(NT8F, 4) k8_fwd(const double2* __restrict__ psi, const double2* __restrict__ dpsi,
@@ -407,60 +442,28 @@ __global__ void __launch_bounds__(NT8F, 4) k8_fwd(const double2* __restrict__ ps
                                                   double2* __restrict__ fpart)
 {
 	constexpr int TB = fwd_tile_bits(TAN), PER = 1 << (TB - 7);   // amplitudes per thread
-	constexpr int NP = TAN ? 4 : 2;                               // operands per round
 	extern __shared__ __align__(16) char tile[];
 	constexpr int DT = 16 << TB;                                  // the tangent's tile
-	__shared__ double sb[MAXK][NP][32];
+	__shared__ double sb[MAXK][TAN ? 4 : 2][32];
 	const int tid = threadIdx.x, lane = tid & 31;
 	auto at_smem = [&](int byte) -> double2& { return *reinterpret_cast<double2*>(tile + byte); };
-	// operands of the rounds' first gates: for input amplitude k = lane & 3 and output part n = lane >> 2
-	for (int e = tid; e < MAXK * 32; e += NT8F) {
-		const int r = e >> 5, ln = e & 31;
-		if (r >= a.rounds) continue;
-		const double2 g = a.g[r].m[4 * (ln >> 3) + (ln & 3)];
-		sb[r][0][ln] = ln & 4 ? g.y : g.x;
-		sb[r][1][ln] = ln & 4 ? g.x : -g.y;
-		if (TAN) {
-			const double2 z = a.z[r].m[4 * (ln >> 3) + (ln & 3)];
-			sb[r][NP - 2][ln] = ln & 4 ? z.y : z.x;
-			sb[r][NP - 1][ln] = ln & 4 ? z.x : -z.y;
-		}
-	}
+	round_operands<TAN, NT8F>(a.m, a.rounds, sb);
 	// this thread's amplitudes of a tile are tid + k 128
-	uint32_t row = 0;
-	int col = 0;
-#pragma unroll
-	for (int b = 0; b < 7; b++)
-		if ((tid >> b) & 1) {
-			if (b < a.cb) col |= 1 << b;
-			else row |= 1u << a.tbit[b];
-		}
+	uint32_t row;
+	int col;
+	tile_own<7>(a, row, col);
 	const int64_t own = (int64_t)row * a.C + col;
 	const int place = swz(tid) << 4;
-	// first amplitude of this thread's set in each round
 	int base[MAXK];
 #pragma unroll
-	for (int r = 0; r < MAXK; r++) {
-		int v = 0;
-		if (r < a.rounds)
-#pragma unroll
-			for (int b = 0; b < 7; b++) v |= ((tid >> b) & 1) << a.pos[r][b];
-		base[r] = swz(v) << 4;
-	}
-	// rows and columns at which tile t begins
-	auto tile_at = [&](uint32_t t, uint32_t& rowbase, int64_t& colbase) {
-		const uint32_t rt = t / a.ncgt;
-		colbase = (int64_t)(t - rt * a.ncgt) << a.cb;
-		rowbase = 0;
-		for (int k = 0; k < a.nseg; k++) rowbase |= ((rt >> a.seg_from[k]) & a.seg_mask[k]) << a.seg_to[k];
-	};
+	for (int r = 0; r < MAXK; r++) base[r] = round_base<7>(a, r);
 	double fx = 0, fy = 0;
 	__syncthreads();
 	for (uint32_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
 		{
 			uint32_t rowbase;
 			int64_t colbase;
-			tile_at(t, rowbase, colbase);
+			tile_at(a, t, rowbase, colbase);
 			if (IN == 0) {
 				const int64_t at = (int64_t)rowbase * a.C + colbase + own;
 				const unsigned dst = (unsigned)__cvta_generic_to_shared(tile);
@@ -468,10 +471,8 @@ __global__ void __launch_bounds__(NT8F, 4) k8_fwd(const double2* __restrict__ ps
 				for (int k = 0; k < PER; k++)
 					if (colbase + col < a.cols) {
 						const unsigned d = dst + (place ^ (swz(k << 7) << 4));
-						asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(psi + at + a.koff[k]) : "memory");
-						if (TAN)
-							asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + DT), "l"(dpsi + at + a.koff[k])
-							             : "memory");
+						cp_async_to(d, psi + at + a.koff[k]);
+						if (TAN) cp_async_to(d + DT, dpsi + at + a.koff[k]);
 					}
 				cp_async_commit();
 				cp_async_wait_all();
@@ -486,53 +487,16 @@ __global__ void __launch_bounds__(NT8F, 4) k8_fwd(const double2* __restrict__ ps
 		}
 		__syncthreads();
 #pragma unroll
-		for (int r = 0; r < MAXK; r++) {
+		for (int r = 0; r < MAXK; r++)
 			if (r < a.rounds) {
-				const int s0 = a.step[r][0], s1 = a.step[r][1], s2 = a.step[r][2], s3 = TAN ? 0 : a.step[r][3];
-				auto mem = [&](int k) {
-					return TAN ? base[r] ^ (k & 4 ? s0 : 0) ^ (k & 2 ? s1 : 0) ^ (k & 1 ? s2 : 0)
-					           : base[r] ^ (k & 8 ? s0 : 0) ^ (k & 4 ? s1 : 0) ^ (k & 2 ? s2 : 0) ^ (k & 1 ? s3 : 0);
-				};
-				double2 x[PER], dx[TAN ? PER : 1];
-#pragma unroll
-				for (int k = 0; k < PER; k++) {
-					x[k] = at_smem(mem(k));
-					if (TAN) dx[k] = at_smem(mem(k) + DT);
-				}
-				const double b0 = sb[r][0][lane], b1 = sb[r][1][lane];
-				const double z0 = TAN ? sb[r][NP - 2][lane] : 0, z1 = TAN ? sb[r][NP - 1][lane] : 0;
-#pragma unroll
-				for (int k = 0; k < PER; k++) {
-					if (TAN) {
-						double2 y = make_double2(0, 0);
-						dmma_amp(y, x[k].x, z0);
-						dmma_amp(y, x[k].y, z1);
-						dmma_amp(y, dx[k].x, b0);
-						dmma_amp(y, dx[k].y, b1);
-						dx[k] = y;
-					}
-					double2 y = make_double2(0, 0);
-					dmma_amp(y, x[k].x, b0);
-					dmma_amp(y, x[k].y, b1);
-					x[k] = y;
-				}
-				if (r < MAXK - 1 && a.pair[r])
-#pragma unroll
-					for (int k = 0; k < PER; k += 4) {
-						if (TAN) apply4_tan(a.g2[r], a.z2[r], x + k, dx + k);
-						else apply4<1>(a.g2[r], x + k);
-					}
-#pragma unroll
-				for (int k = 0; k < PER; k++) {
-					at_smem(mem(k)) = x[k];
-					if (TAN) at_smem(mem(k) + DT) = dx[k];
-				}
+				constexpr int last = MAXK - 2;
+				tile_round<TAN, PER>(tile, 0, DT, base[r], a.step[r], sb[r], r <= last && a.pair[r], a.m.g2[r <= last ? r : last],
+				                     a.m.z2[r <= last ? r : last]);
 				__syncthreads();
 			}
-		}
 		uint32_t rowbase;
 		int64_t colbase;
-		tile_at(t, rowbase, colbase);
+		tile_at(a, t, rowbase, colbase);
 		const int64_t at = (int64_t)rowbase * a.C + colbase + own;
 #pragma unroll
 		for (int k = 0; k < PER; k++) {
@@ -569,22 +533,22 @@ __global__ void __launch_bounds__(NT8F, 4) k8_fwd(const double2* __restrict__ ps
 	}
 }
 
-// the arguments of k8_fwd for a pass
-FwdArgs fwd_args(const PassGeom& pg, const PassGates<double>& gates, bool tan)
+// The tile of a pass, 2^TB amplitudes and 2^NTB threads, and its rounds: consecutive gates on wires
+// of their own share one (in_group: only those of one group).  set(r, k, first) takes round r's gates.
+template <typename Set>
+void tile_rounds(PassTile& a, const PassGeom& pg, int TB, int NTB, bool in_group, Set set)
 {
-	FwdArgs a;
-	const int TB = fwd_tile_bits(tan), cb = TB - pg.NB, own = TB - 7;   // own: bits of a thread's amplitudes
+	const int cb = TB - pg.NB, own = TB - NTB;   // own: bits of a thread's amplitudes
 	a.cb = cb;
 	a.C = pg.C;
 	a.cols = pg.ncg * 4;
-	a.src = pg.src;
 	a.ncgt = (uint32_t)((a.cols + ((int64_t)1 << cb) - 1) >> cb);
 	a.ntiles = a.ncgt << (pg.L - pg.NB);
 	for (int b = 0; b < TB; b++) a.tbit[b] = (int8_t)(b < cb ? 0 : pg.tbit[b - cb]);
 	for (int k = 0; k < 1 << own; k++) {
 		a.krow[k] = 0;   // (L >= 4: the column's bits are thread bits)
 		for (int b = 0; b < own; b++)
-			if ((k >> b) & 1) a.krow[k] |= 1u << a.tbit[7 + b];
+			if ((k >> b) & 1) a.krow[k] |= 1u << a.tbit[NTB + b];
 		a.koff[k] = (int64_t)a.krow[k] * a.C;
 	}
 	a.nseg = 0;
@@ -601,27 +565,26 @@ FwdArgs fwd_args(const PassGeom& pg, const PassGates<double>& gates, bool tan)
 		from += e - b;
 		b = e;
 	}
-	// consecutive gates on wires of their own share a round
 	a.rounds = 0;
-	for (int k = 0; k < pg.K;) {
+	for (int k = 0, l = 0; k < pg.K;) {
 		const int r = a.rounds++;
+		while (k >= pg.group[l + 1]) l++;
 		uint32_t used = 0;
 		auto bit_of = [&](int local) {
 			used |= 1u << (cb + local);
 			return cb + local;
 		};
 		const uint32_t w0 = (1u << pg.gi[k]) | (1u << pg.gj[k]);
-		const bool pair = k + 1 < pg.K && !(w0 & ((1u << pg.gi[k + 1]) | (1u << pg.gj[k + 1])));
+		const bool pair = k + 1 < pg.K && (!in_group || k + 1 < pg.group[l + 1]) &&
+		                  !(w0 & ((1u << pg.gi[k + 1]) | (1u << pg.gj[k + 1])));
 		a.pair[r] = pair;
-		a.g[r] = gates.g[k];
-		a.z[r] = gates.z[k];
+		set(r, k, true);
 		a.pos[r][0] = (int8_t)bit_of(pg.gj[k]);
 		a.pos[r][1] = (int8_t)bit_of(pg.gi[k]);
 		int slot = own;
 		if (pair) {
 			slot -= 2;
-			a.g2[r] = gates.g[k + 1];
-			a.z2[r] = gates.z[k + 1];
+			set(r, k + 1, false);
 			a.step[r][slot] = swz(1 << bit_of(pg.gi[k + 1])) << 4;
 			a.step[r][slot + 1] = swz(1 << bit_of(pg.gj[k + 1])) << 4;
 		}
@@ -645,6 +608,17 @@ FwdArgs fwd_args(const PassGeom& pg, const PassGates<double>& gates, bool tan)
 		for (int b = 0; b < TB; b++)
 			if (!((used >> b) & 1)) a.pos[r][m++] = (int8_t)b;
 	}
+}
+
+// the arguments of k8_fwd for a pass
+FwdArgs fwd_args(const PassGeom& pg, const PassGates<double>& gates, bool tan)
+{
+	FwdArgs a;
+	a.src = pg.src;
+	tile_rounds(a, pg, fwd_tile_bits(tan), 7, false, [&](int r, int k, bool first) {
+		(first ? a.m.g[r] : a.m.g2[r]) = gates.g[k];
+		(first ? a.m.z[r] : a.m.z2[r]) = gates.z[k];
+	});
 	return a;
 }
 
@@ -1614,46 +1588,25 @@ __global__ void __launch_bounds__(NT5, 2) k5_rev(const float2* __restrict__ psi,
 
 // ------------------------------------------------------------------------------ complex128 reverse pass, sums at the output
 
-// Units u0 and u1 of a gate's outer sums over eight groups each (two group bases times four
-// columns): R1 += phi (x) psi, R2 += phi (x) dpsi + dphi (x) psi, raw 8x8 sums.
-template <bool TAN>
-__device__ __forceinline__ void outer_unit(const double* Psi, const double* dPsi, const double* Phi, const double* dPhi,
-                                           int u, const StepLane& sl, int lane, double (&g)[2], double (&h)[2])
-{
-	const int i0 = sidx(insert2(2 * u, sl.lo, sl.hi) | sl.m_outer, lane & 3) * 2 + sl.part_outer;
-	const int i1 = sidx(insert2(2 * u + 1, sl.lo, sl.hi) | sl.m_outer, lane & 3) * 2 + sl.part_outer;
-	const double p0 = Phi[i0], x0 = Psi[i0], p1 = Phi[i1], x1 = Psi[i1];
-	double dx0 = 0, dx1 = 0, dp0 = 0, dp1 = 0;
-	if (TAN) {
-		dx0 = dPsi[i0];
-		dx1 = dPsi[i1];
-		dp0 = dPhi[i0];
-		dp1 = dPhi[i1];
-	}
-	dmma(g[0], g[1], p0, x0);
-	if (TAN) dmma(h[0], h[1], p0, dx0);
-	dmma(g[0], g[1], p1, x1);
-	if (TAN) {
-		dmma(h[0], h[1], p1, dx1);
-		dmma(h[0], h[1], dp0, x0);
-		dmma(h[0], h[1], dp1, x1);
-	}
-}
-
 // The gates' operands of a reverse pass that rebuilds states between groups: conj(G) (as a
 // row-vector operand it applies G^+) and -W, W = G^+ Z G^+.
 struct PassAdj { Gate4<double> gc[MAXK]; Gate4<double> wn[MAXK]; };
 
-constexpr int NT6 = 128;   // threads of the complex128 reverse kernel (three blocks per SM)
-constexpr int EPT6 = (1 << MAXNB) * 4 / NT6;   // tile elements per thread and state
-
-inline size_t k8_rev_smem(bool tan)
+struct RevArgs : PassTile
 {
-	const size_t A = (size_t)(1 << MAXNB) * 4;
-	const size_t tiles = (tan ? 4 : 2) * A * sizeof(double2);
-	const size_t red = (size_t)(NT6 / 32) * MAXK * NPART3 * sizeof(double);
-	return 64 * MAXK * sizeof(double2) + (1 << MAXNB) * sizeof(int) + std::max(tiles, red);
-}
+	RoundGates back;                // phi through a gate: G^T, Z^T
+	RoundGates undo;                // psi: G^+, -W
+	int K, ngroups;
+	int gate_end[MAXK], round_end[MAXK];   // group l: gates and rounds up to these
+	int ostep[MAXK][4];             // outer sums of gate k: places (bytes) of the tile bits of a thread's 16 steps
+	int8_t opos[MAXK][8];           // tile bits of a thread's index bits: 0, 1 columns of the sum, 3, 4 wires j, i (2 selects
+	                                // an amplitude's part), the rest from 5 on
+};
+
+constexpr int NTB8 = 7, NT8R = 1 << NTB8;   // threads of the complex128 reverse kernel
+constexpr int TB8R = NTB8 + 3;             // bits of its tiles
+constexpr int rev_tile_bytes(bool tan) { return ((tan ? 4 : 2) << TB8R) * (int)sizeof(double2); }
+__host__ __device__ constexpr int rev_blocks(bool tan) { return tan ? 3 : 4; }   // per SM
 
 // Reverse pass (complex128) for unitary gates.  psi, dpsi are the state
 // and tangent at the pass OUTPUT (the next pass's checkpoint, or the circuit's final state),
@@ -1661,159 +1614,152 @@ inline size_t k8_rev_smem(bool tan)
 // pass's last gate, and its sums follow from those at the output, with W = G^+ Z G^+:
 //   R1 = sum phi (x) psi,  R2 = sum phi (x) dpsi + dphi (x) psi,
 //   dG = R1 conj(G),       HZ = R2 conj(G) - R1 W^T          (formed once, by k3_reduce).
-// So the states entering the gates are not needed: 12 FP64 MMAs per unit of eight groups and gate
-// instead of the 18 of a kernel that rebuilds them (L = 12, depth 9, one column per orbit: 3.41 ->
-// 2.97 ms an evaluation), and a group's sums need no barrier between gates; then phi, dphi move
-// through the group in place, two gates per barrier.  The layers of a brickwall make passes of
-// one group.  Where a pass has more (gates that share wires), psi and dpsi move back through a
-// group too, psi <- G^+ psi, dpsi <- G^+ dpsi - W psi, and the group before it is done the same
-// way.  Four tiles (64 KB), three blocks of 128 threads per SM.  Bound by the FP64 pipe (12 flop
-// per byte).  Partials: raw 8x8 sums R1, R2 (part + k * nblk * 128 + blockIdx.x * 128).
+// So the states entering the gates are not needed, and a group's sums need no barrier between
+// gates; then phi, dphi move through the group in rounds of two gates.  The layers of a brickwall
+// make passes of one group.  Where a pass has more (gates that share wires), psi and dpsi move back
+// through a group too, psi <- G^+ psi, dpsi <- G^+ dpsi - W psi, and the group before it is done the
+// same way.
+// The sums are MMAs over four amplitude groups at a time, their operands (one part of an amplitude a
+// lane) read from the tile in 8-byte words; the words of a half warp lie in different banks.
+// Four gates do 8 flop per byte with tangents (FP64 pipe) and 5 without.  A kernel that moved phi a gate
+// at a time, with 8 x 8 real embeddings as MMA operands fetched per row set, took 127 us a pass on the
+// L = 12 brickwall's 700 columns and 111 us without tangents on the 2^22 amplitudes of L = 11; this
+// one 105 us (21 TFLOP/s) and 70 us (15 TFLOP/s, 2.9 TB/s), what is left being the latency of MMA
+// chains and tile copies in 12 to 16 warps per SM.  Without tangents, five blocks at 96 registers
+// measured 1 % better but with spills in the last pass, tiles of 2^11 and 256 threads 5 % worse.
+// Three blocks per SM (64 KB of tiles each), four without tangents (32 KB).  Partials: raw 8x8 sums R1, R2 (part + k * nblk * 128 +
+// blockIdx.x * 128).
 template <bool TAN, bool FIRST, bool LAST>
-__global__ void __launch_bounds__(NT6, 3) k8_rev(const double2* __restrict__ psi, const double2* __restrict__ dpsi,
-                                                 const double2* __restrict__ phi, const double2* __restrict__ dphi,
-                                                 double2* __restrict__ phi_o, double2* __restrict__ dphi_o, PassGeom pg,
-                                                 PassGates<double> gates, const __grid_constant__ PassAdj adj,
-                                                 double* __restrict__ part, int nblk)
+__global__ void __launch_bounds__(NT8R, rev_blocks(TAN))
+k8_rev(const double2* __restrict__ psi, const double2* __restrict__ dpsi, const double2* __restrict__ phi,
+       const double2* __restrict__ dphi, double2* __restrict__ phi_o, double2* __restrict__ dphi_o,
+       const __grid_constant__ RevArgs a, double* __restrict__ part, int nblk)
 {
-	constexpr int CW = 4;
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	const int R = 1 << pg.NB, A = R * CW, K = pg.K;
-	double2* sg = reinterpret_cast<double2*>(smem_raw);           // [MAXK][64]: G, Z, conj(G), -W
-	int* rowoff = reinterpret_cast<int*>(sg + 64 * MAXK);
-	double2* tiles = reinterpret_cast<double2*>(rowoff + (1 << MAXNB));
-	double2* Psi = tiles;
-	double2* Phi = tiles + A;
-	double2* dPsi = TAN ? tiles + 2 * A : nullptr;
-	double2* dPhi = TAN ? tiles + 3 * A : nullptr;
-	const double* fPsi = reinterpret_cast<const double*>(Psi);
-	const double* fPhi = reinterpret_cast<const double*>(Phi);
-	const double* fdPsi = reinterpret_cast<const double*>(dPsi);
-	const double* fdPhi = reinterpret_cast<const double*>(dPhi);
-	for (int e = threadIdx.x; e < 64 * MAXK; e += blockDim.x) {
-		const int k = e / 64, w = e % 64;
-		if (k >= K) continue;
-		double2 v = make_double2(0, 0);
-		if (w < 16) v = gates.g[k].m[w];
-		else if (w < 32) v = TAN ? gates.z[k].m[w - 16] : v;
-		else if (w < 48) v = adj.gc[k].m[w - 32];
-		else v = TAN ? adj.wn[k].m[w - 48] : v;
-		sg[e] = v;
+	constexpr int NTB = NTB8, NT = NT8R, PER = 8;
+	constexpr int DT = 16 << TB8R;                            // bytes of a tile
+	constexpr int PSI = 0, PHI = DT, DPSI = 2 * DT, DPHI = 3 * DT;
+	extern __shared__ __align__(16) char tile[];
+	__shared__ double sb[MAXK][TAN ? 4 : 2][32], su[MAXK][TAN ? 4 : 2][32];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	round_operands<TAN, NT>(a.back, a.rounds, sb);
+	if (a.ngroups > 1) round_operands<TAN, NT>(a.undo, a.rounds, su);
+	uint32_t row;
+	int col;
+	tile_own<NTB>(a, row, col);
+	const int64_t own = (int64_t)row * a.C + col;
+	const int place = swz(tid) << 4;
+	int base[MAXK], obase[MAXK];
+#pragma unroll
+	for (int r = 0; r < MAXK; r++) {
+		base[r] = round_base<NTB>(a, r);
+		int v = 0;
+		if (r < a.K)
+#pragma unroll
+			for (int b = 0; b < NTB; b++)
+				if (b != 2) v |= ((tid >> b) & 1) << a.opos[r][b];
+		obase[r] = swz(v) << 4 | (lane & 4) << 1;
 	}
-	row_offsets(pg, rowoff);
-	__syncthreads();
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
 	double cg0[MAXK], cg1[MAXK], ch0[MAXK], ch1[MAXK];
 #pragma unroll
 	for (int k = 0; k < MAXK; k++) { cg0[k] = cg1[k] = ch0[k] = ch1[k] = 0; }
-	const int units = R / 8;
+	__syncthreads();
 
-	// X, dX through gate k on this lane's bases of two units, by the matrices at m (and mt for the
-	// tangent's term), in the embedding that tr and tt select
-	auto move = [&](double2* X, double2* dX, int k, const double2* m, bool tr, const double2* mt, bool tt, bool dzero,
-	                int bs0, int bs1, bool has1) {
-		const StepLane sl(pg.gi[k], pg.gj[k], lane);
-		double bg[2], bz[2] = {0, 0};
-		bfrag(m, tr, lane, bg);
-		if (TAN) bfrag(mt, tt, lane, bz);
-		apply_bases2<TAN>(reinterpret_cast<const double*>(X), reinterpret_cast<const double*>(dX), X, dX, bs0, bs1, has1, sl, bg,
-		                  bz, dzero, lane);
-	};
-
-	for (int64_t tile = blockIdx.x; tile < pg.ntiles; tile += gridDim.x) {
-		const int64_t rt = tile / pg.ncg, cgp = tile - rt * pg.ncg;
-		const int64_t rowbase = deposit(rt, pg.rest_mask);
-		const int64_t colbase = cgp * CW;
+	for (uint32_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+		{
+			uint32_t rowbase;
+			int64_t colbase;
+			tile_at(a, t, rowbase, colbase);
+			const int64_t at = (int64_t)rowbase * a.C + colbase + own;
+			const unsigned dst = (unsigned)__cvta_generic_to_shared(tile);
+			const bool in = colbase + col < a.cols;
 #pragma unroll
-		for (int i = 0; i < EPT6; i++) {
-			const int e = threadIdx.x + i * NT6;
-			if (e >= A) continue;
-			const int r = e >> 2, cc = e & 3;
-			const int64_t a = (rowbase + rowoff[r]) * pg.C + colbase + cc;
-			const int pe = sidx(r, cc);
-			cp_async16(Psi + pe, psi + a);
-			cp_async16(Phi + pe, phi + a);
-			if (TAN) {
-				cp_async16(dPsi + pe, dpsi + a);
-				if (FIRST) dPhi[pe] = make_double2(0, 0);
-				else cp_async16(dPhi + pe, dphi + a);
+			for (int k = 0; k < PER; k++) {
+				const int o = place ^ (swz(k << NTB) << 4);
+				if (in) {
+					const int64_t e = at + a.koff[k];
+					cp_async_to(dst + o + PSI, psi + e);
+					cp_async_to(dst + o + PHI, phi + e);
+					if (TAN) {
+						cp_async_to(dst + o + DPSI, dpsi + e);
+						if (!FIRST) cp_async_to(dst + o + DPHI, dphi + e);
+					}
+				} else {   // columns that are not there add nothing
+					const double2 zero = make_double2(0, 0);
+					*reinterpret_cast<double2*>(tile + o + PSI) = zero;
+					*reinterpret_cast<double2*>(tile + o + PHI) = zero;
+					if (TAN) *reinterpret_cast<double2*>(tile + o + DPSI) = zero;
+					if (TAN && !FIRST) *reinterpret_cast<double2*>(tile + o + DPHI) = zero;
+				}
+				if (TAN && FIRST) *reinterpret_cast<double2*>(tile + o + DPHI) = make_double2(0, 0);
 			}
+			cp_async_commit();
+			cp_async_wait_all();
 		}
-		cp_async_commit();
-		cp_async_wait_all();
 		__syncthreads();
-		for (int l = pg.ngroups - 1; l >= 0; l--) {
-			const int lo = pg.group[l], hi = pg.group[l + 1];
-			// the sums of every gate of the group, two units' MMA chains at a time
+		for (int l = a.ngroups - 1; l >= 0; l--) {
+			const int glo = l ? a.gate_end[l - 1] : 0, ghi = a.gate_end[l], rlo = l ? a.round_end[l - 1] : 0, rhi = a.round_end[l];
+			// the sums of every gate of the group, two MMA chains at a time
 #pragma unroll
 			for (int k = 0; k < MAXK; k++) {
-				if (k < lo || k >= hi) continue;
-				const StepLane sl(pg.gi[k], pg.gj[k], lane);
-				double ga[2] = {0, 0}, gb[2] = {0, 0}, ha[2] = {0, 0}, hb[2] = {0, 0};
-				for (int u = warp; u < units; u += 2 * nwarps) {
-					outer_unit<TAN>(fPsi, fdPsi, fPhi, fdPhi, u, sl, lane, ga, ha);
-					if (u + nwarps < units) outer_unit<TAN>(fPsi, fdPsi, fPhi, fdPhi, u + nwarps, sl, lane, gb, hb);
+				if (k < glo || k >= ghi) continue;
+				const int s0 = a.ostep[k][0], s1 = a.ostep[k][1], s2 = a.ostep[k][2], s3 = a.ostep[k][3];
+				double g[2][2] = {{0, 0}, {0, 0}}, h[2][2] = {{0, 0}, {0, 0}};
+#pragma unroll
+				for (int u = 0; u < 16; u++) {
+					const char* w = tile + (obase[k] ^ (u & 8 ? s0 : 0) ^ (u & 4 ? s1 : 0) ^ (u & 2 ? s2 : 0) ^ (u & 1 ? s3 : 0));
+					const double p = *reinterpret_cast<const double*>(w + PHI), x = *reinterpret_cast<const double*>(w + PSI);
+					dmma(g[u & 1][0], g[u & 1][1], p, x);
+					if (TAN) {
+						const double dp = *reinterpret_cast<const double*>(w + DPHI), dx = *reinterpret_cast<const double*>(w + DPSI);
+						dmma(h[u & 1][0], h[u & 1][1], p, dx);
+						dmma(h[u & 1][0], h[u & 1][1], dp, x);
+					}
 				}
-				cg0[k] += ga[0] + gb[0];
-				cg1[k] += ga[1] + gb[1];
+				cg0[k] += g[0][0] + g[1][0];
+				cg1[k] += g[0][1] + g[1][1];
 				if (TAN) {
-					ch0[k] += ha[0] + hb[0];
-					ch1[k] += ha[1] + hb[1];
+					ch0[k] += h[0][0] + h[1][0];
+					ch1[k] += h[0][1] + h[1][1];
 				}
 			}
 			if (LAST && l == 0) break;
 			__syncthreads();
-			// phi, dphi (and psi, dpsi where a group comes before) through gates k and k + 1 on this
-			// warp's row sets, one block barrier for both
-			for (int k = lo; k < hi; k += 2) {
-				const double2 *ma = sg + 64 * k, *mb = sg + 64 * (k + 1);
-				const bool dz = FIRST && l == pg.ngroups - 1 && k == lo;
-				const int hs = lane >> 4;
-				if (k + 1 < hi) {
-					const int m = (1 << pg.gi[k]) | (1 << pg.gj[k]) | (1 << pg.gi[k + 1]) | (1 << pg.gj[k + 1]);
-					for (int s = warp; s < (R >> 4); s += nwarps) {
-						const int S0 = set_base(s, m);
-						const UnitBases ua = set_units(S0, pg.gi[k + 1], pg.gj[k + 1]), ub = set_units(S0, pg.gi[k], pg.gj[k]);
-						const int a0 = hs ? ua.b01 : ua.b00, a1 = hs ? ua.b11 : ua.b10;
-						const int b0 = hs ? ub.b01 : ub.b00, b1 = hs ? ub.b11 : ub.b10;
-						move(Phi, dPhi, k, ma, false, ma + 16, false, dz, a0, a1, true);
-						if (l > 0) move(Psi, dPsi, k, ma + 32, false, ma + 48, true, false, a0, a1, true);
-						__syncwarp();
-						move(Phi, dPhi, k + 1, mb, false, mb + 16, false, false, b0, b1, true);
-						if (l > 0) move(Psi, dPsi, k + 1, mb + 32, false, mb + 48, true, false, b0, b1, true);
-					}
-				} else {
-					const StepLane sl(pg.gi[k], pg.gj[k], lane);
-					for (int u = warp; u < units; u += 2 * nwarps) {
-						const bool has1 = u + nwarps < units;
-						const int b0 = insert2(2 * u + hs, sl.lo, sl.hi), b1 = insert2(2 * (has1 ? u + nwarps : u) + hs, sl.lo, sl.hi);
-						move(Phi, dPhi, k, ma, false, ma + 16, false, dz, b0, b1, has1);
-						if (l > 0) move(Psi, dPsi, k, ma + 32, false, ma + 48, true, false, b0, b1, has1);
-					}
-				}
+			// phi, dphi (and psi, dpsi where a group comes before) through the group
+#pragma unroll
+			for (int r = 0; r < MAXK; r++) {
+				if (r < rlo || r >= rhi) continue;
+				constexpr int last = MAXK - 2;
+				const bool pair = r <= last && a.pair[r];
+				tile_round<TAN, PER>(tile, PHI, DPHI, base[r], a.step[r], sb[r], pair, a.back.g2[r <= last ? r : last],
+				                     a.back.z2[r <= last ? r : last]);
+				if (l > 0)
+					tile_round<TAN, PER>(tile, PSI, DPSI, base[r], a.step[r], su[r], pair, a.undo.g2[r <= last ? r : last],
+					                     a.undo.z2[r <= last ? r : last]);
 				__syncthreads();
 			}
 		}
 		if (!LAST) {
+			uint32_t rowbase;
+			int64_t colbase;
+			tile_at(a, t, rowbase, colbase);
+			const int64_t at = (int64_t)rowbase * a.C + colbase + own;
+			if (colbase + col < a.cols)
 #pragma unroll
-			for (int i = 0; i < EPT6; i++) {
-				const int e = threadIdx.x + i * NT6;
-				if (e >= A) continue;
-				const int r = e >> 2, cc = e & 3;
-				const int64_t a = (rowbase + rowoff[r]) * pg.C + colbase + cc;
-				const int pe = sidx(r, cc);
-				phi_o[a] = Phi[pe];
-				if (TAN) dphi_o[a] = dPhi[pe];
-			}
+				for (int k = 0; k < PER; k++) {
+					const int o = place ^ (swz(k << NTB) << 4);
+					phi_o[at + a.koff[k]] = *reinterpret_cast<const double2*>(tile + o + PHI);
+					if (TAN) dphi_o[at + a.koff[k]] = *reinterpret_cast<const double2*>(tile + o + DPHI);
+				}
 		}
 		__syncthreads();
 	}
 
 	// sum the warps' raw 8x8 accumulators; lane l holds entries 2l, 2l+1
-	double* red = reinterpret_cast<double*>(tiles);   // [warps][MAXK][128]
+	constexpr int nwarps = NT / 32;
+	double* red = reinterpret_cast<double*>(tile);   // [warps][MAXK][128]
 #pragma unroll
 	for (int k = 0; k < MAXK; k++) {
-		if (k >= K) break;
+		if (k >= a.K) break;
 		double* w = red + ((size_t)warp * MAXK + k) * NPART3;
 		w[2 * lane] = cg0[k];
 		w[2 * lane + 1] = cg1[k];
@@ -1821,12 +1767,63 @@ __global__ void __launch_bounds__(NT6, 3) k8_rev(const double2* __restrict__ psi
 		w[64 + 2 * lane + 1] = TAN ? ch1[k] : 0.0;
 	}
 	__syncthreads();
-	for (int idx = threadIdx.x; idx < K * NPART3; idx += blockDim.x) {
+	for (int idx = tid; idx < a.K * NPART3; idx += NT) {
 		const int k = idx / NPART3, v = idx % NPART3;
 		double s = 0;
 		for (int w = 0; w < nwarps; w++) s += red[((size_t)w * MAXK + k) * NPART3 + v];
 		part[(size_t)k * nblk * NPART3 + (size_t)blockIdx.x * NPART3 + v] += s;
 	}
+}
+
+// the arguments of k8_rev for a pass
+RevArgs rev_args(const PassGeom& pg, const PassGates<double>& gates, const PassAdj& adj)
+{
+	RevArgs a;
+	const int TB = TB8R, cb = TB - pg.NB;
+	auto transposed = [](const Gate4<double>& m) {
+		Gate4<double> t;
+		for (int e = 0; e < 16; e++) t.m[e] = m.m[4 * (e & 3) + (e >> 2)];
+		return t;
+	};
+	tile_rounds(a, pg, TB, NTB8, true, [&](int r, int k, bool first) {
+		(first ? a.back.g[r] : a.back.g2[r]) = transposed(gates.g[k]);
+		(first ? a.back.z[r] : a.back.z2[r]) = transposed(gates.z[k]);
+		(first ? a.undo.g[r] : a.undo.g2[r]) = transposed(adj.gc[k]);
+		(first ? a.undo.z[r] : a.undo.z2[r]) = adj.wn[k];
+	});
+	a.K = pg.K;
+	a.ngroups = pg.ngroups;
+	for (int l = 0, r = 0, k = 0; l < pg.ngroups; l++) {
+		a.gate_end[l] = pg.group[l + 1];
+		while (k < a.gate_end[l]) k += a.pair[r++] ? 2 : 1;
+		a.round_end[l] = r;
+	}
+	for (int k = 0; k < pg.K; k++) {
+		const int j = cb + pg.gj[k], i = cb + pg.gi[k];
+		uint32_t used = (1u << i) | (1u << j);
+		// the sum's columns: bits of the two residues mod 3 that wire j leaves (the words of a half warp
+		// then lie in different banks; of the 10 bits each residue has three or more)
+		for (int q = 0; q < 2; q++)
+			for (int b = 0; b < TB; b++)
+				if (!((used >> b) & 1) && b % 3 == (j + 1 + q) % 3) {
+					a.opos[k][q] = (int8_t)b;
+					used |= 1u << b;
+					break;
+				}
+		a.opos[k][2] = 0;
+		a.opos[k][3] = (int8_t)j;
+		a.opos[k][4] = (int8_t)i;
+		int n = 0;
+		for (int b = TB - 1; n < 4; b--)
+			if (!((used >> b) & 1)) {
+				a.ostep[k][n++] = swz(1 << b) << 4;
+				used |= 1u << b;
+			}
+		n = 5;
+		for (int b = 0; b < TB; b++)
+			if (!((used >> b) & 1)) a.opos[k][n++] = (int8_t)b;
+	}
+	return a;
 }
 
 // ------------------------------------------------------------------------------ complex64 passes on the FP32 pipe
@@ -2533,12 +2530,12 @@ int launch_rev8(Runtime& rt, const double2* psi, const double2* dpsi, const doub
 	static bool ready = false;
 	if (!ready) {
 		int per_sm;
-		int ret = prepare(k8_rev<TAN, FIRST, LAST>, k8_rev_smem(TAN), &per_sm, NT6);
+		int ret = prepare(k8_rev<TAN, FIRST, LAST>, rev_tile_bytes(TAN), &per_sm, NT8R);
 		if (ret) return ret;
 		ready = true;
 	}
-	RQC_LAUNCH3(rt, KC_REVERSE, (k8_rev<TAN, FIRST, LAST>), nblk, NT6, k8_rev_smem(TAN), psi, dpsi, phi, dphi, phi_o,
-	            dphi_o, pg, gates, adj, part, nblk);
+	RQC_LAUNCH3(rt, KC_REVERSE, (k8_rev<TAN, FIRST, LAST>), nblk, NT8R, rev_tile_bytes(TAN), psi, dpsi, phi, dphi,
+	            phi_o, dphi_o, rev_args(pg, gates, adj), part, nblk);
 	return OK;
 }
 
@@ -2559,8 +2556,8 @@ int launch_rev8_any(Runtime& rt, bool first, bool last, const double2* psi, cons
 int rev_grid8(Runtime& rt, bool tan)
 {
 	int per_sm = 1;
-	const int ret = tan ? prepare(k8_rev<true, false, false>, k8_rev_smem(true), &per_sm, NT6)
-	                    : prepare(k8_rev<false, false, false>, k8_rev_smem(false), &per_sm, NT6);
+	const int ret = tan ? prepare(k8_rev<true, false, false>, rev_tile_bytes(true), &per_sm, NT8R)
+	                    : prepare(k8_rev<false, false, false>, rev_tile_bytes(false), &per_sm, NT8R);
 	if (ret) per_sm = 1;
 	return rt.num_sms * per_sm;
 }
