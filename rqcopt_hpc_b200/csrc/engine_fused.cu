@@ -498,21 +498,25 @@ __global__ void __launch_bounds__(NT8F, 4) k8_fwd(const double2* __restrict__ ps
 		int64_t colbase;
 		tile_at(a, t, rowbase, colbase);
 		const int64_t at = (int64_t)rowbase * a.C + colbase + own;
+		if (colbase + col < a.cols) {
+			double2 p[OUT >= 2 ? PER : 1];
+			if (OUT >= 2)
 #pragma unroll
-		for (int k = 0; k < PER; k++) {
-			if (colbase + col >= a.cols) continue;
-			const int d = place ^ (swz(k << 7) << 4);
-			const double2 v = at_smem(d);
-			if (OUT == 2 || OUT == 3) {
-				const double2 p = phi[at + a.koff[k]];
-				fx += p.x * v.x - p.y * v.y;
-				fy += p.x * v.y + p.y * v.x;
-			}
-			if (OUT == 1) {
-				psi_o[at + a.koff[k]] = cneg_conj(v);
-			} else if (OUT != 2) {
-				psi_o[at + a.koff[k]] = v;
-				if (TAN) dpsi_o[at + a.koff[k]] = at_smem(d + DT);
+				for (int k = 0; k < PER; k++) p[k] = phi[at + a.koff[k]];
+#pragma unroll
+			for (int k = 0; k < PER; k++) {
+				const int d = place ^ (swz(k << 7) << 4);
+				const double2 v = at_smem(d);
+				if (OUT >= 2) {
+					fx += p[k].x * v.x - p[k].y * v.y;
+					fy += p[k].x * v.y + p[k].y * v.x;
+				}
+				if (OUT == 1) {
+					psi_o[at + a.koff[k]] = cneg_conj(v);
+				} else if (OUT != 2) {
+					psi_o[at + a.koff[k]] = v;
+					if (TAN) dpsi_o[at + a.koff[k]] = at_smem(d + DT);
+				}
 			}
 		}
 		__syncthreads();
@@ -1703,7 +1707,7 @@ k8_rev(const double2* __restrict__ psi, const double2* __restrict__ dpsi, const 
 			for (int k = 0; k < MAXK; k++) {
 				if (k < glo || k >= ghi) continue;
 				const int s0 = a.ostep[k][0], s1 = a.ostep[k][1], s2 = a.ostep[k][2], s3 = a.ostep[k][3];
-				double g[2][2] = {{0, 0}, {0, 0}}, h[2][2] = {{0, 0}, {0, 0}};
+				double g[2][2] = {{0, 0}, {0, 0}}, h[2][2] = {{0, 0}, {0, 0}}, q[2][2] = {{0, 0}, {0, 0}};
 #pragma unroll
 				for (int u = 0; u < 16; u++) {
 					const char* w = tile + (obase[k] ^ (u & 8 ? s0 : 0) ^ (u & 4 ? s1 : 0) ^ (u & 2 ? s2 : 0) ^ (u & 1 ? s3 : 0));
@@ -1712,14 +1716,14 @@ k8_rev(const double2* __restrict__ psi, const double2* __restrict__ dpsi, const 
 					if (TAN) {
 						const double dp = *reinterpret_cast<const double*>(w + DPHI), dx = *reinterpret_cast<const double*>(w + DPSI);
 						dmma(h[u & 1][0], h[u & 1][1], p, dx);
-						dmma(h[u & 1][0], h[u & 1][1], dp, x);
+						dmma(q[u & 1][0], q[u & 1][1], dp, x);
 					}
 				}
 				cg0[k] += g[0][0] + g[1][0];
 				cg1[k] += g[0][1] + g[1][1];
 				if (TAN) {
-					ch0[k] += h[0][0] + h[1][0];
-					ch1[k] += h[0][1] + h[1][1];
+					ch0[k] += (h[0][0] + h[1][0]) + (q[0][0] + q[1][0]);
+					ch1[k] += (h[0][1] + h[1][1]) + (q[0][1] + q[1][1]);
 				}
 			}
 			if (LAST && l == 0) break;
