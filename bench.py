@@ -26,6 +26,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import subprocess
 import sys
@@ -76,24 +77,30 @@ def flops_per_eval(L, G, Gt):
     return float(N) * N * (32 * Gt + 292 * G - 124)
 
 
-def reverse_flops_per_eval(L, G):
-    """Algorithmic flops of the reverse (gradient/HVP) passes of one evaluation as the
-    reference executes them: per gate and amplitude of each of the N = 2^L columns, the
+def orbit_columns(L):
+    """Columns that a complex128 evaluation of a periodic brickwall on L (even) wires takes: one
+    per orbit of the basis states under the relabellings of the wires that keep every layer,
+    which are the shifts by two wires.  So: necklaces of L/2 beads in four colours."""
+    n = L // 2
+    return sum(4 ** math.gcd(k, n) for k in range(n)) // n
+
+
+def reverse_flops_per_eval(L, G, columns):
+    """Flops of the reverse (gradient/HVP) passes of one evaluation on `columns` columns, by the
+    products the reference executes: per gate and amplitude of each column, the
     outer sums dG += phi (x) psi and HZ += phi (x) dpsi + dphi (x) psi and the adjoint
     updates phi' = G^T phi, dphi' = G^T dphi + Z^T phi: six 4x4 complex products of an
     amplitude group, 6 x 32 = 192 flop per amplitude (states rebuilt inside a fused pass
     are not counted)."""
-    N = 1 << L
-    return 192.0 * G * N * N
+    return 192.0 * G * columns * (1 << L)
 
 
-def reverse_bytes_per_eval(L, P, itemsize):
+def reverse_bytes_per_eval(L, P, itemsize, columns):
     """Algorithmic HBM bytes of the reverse (gradient/HVP) passes of one evaluation with P
     passes (one per gate, or one per group of fused gates): per column 6P - 5 statevector
     passes (reads of phi, dphi, psi, dpsi and writes of phi', dphi' per pass; the pass at the
     circuit output has no dphi to read, the pass at its input no psi / outputs)."""
-    N = 1 << L
-    return float(6 * P - 5) * N * N * itemsize
+    return float(6 * P - 5) * columns * (1 << L) * itemsize
 
 
 # ----------------------------------------------------------------------------- clocks
@@ -278,20 +285,21 @@ def gate_throughput(gpu, torch, L=28, G=256, seed=20):
 
 def hess_model(L, nlayers, single):
     """Algorithmic HBM transfers (state-sized reads + writes) and complex multiply-adds
-    per basis column of the full-Hessian sweep kernels of one evaluation.
+    per column of the full-Hessian kernels of one evaluation.
 
-    L <= 12 runs k_hlayer, one launch per layer with the tangents' column tiles in
-    shared memory: per layer a the tangents of the earlier layers (16 a) are read once
-    and all 16 (a + 1) written once (not after the last layer), phi_q and psi_q of the
-    layer's gates are read once (psi_0 of a basis column is generated).  Larger L runs
-    k_hsweep, one launch per gate: per gate q of layer a, phi_q is read, the tangents of
-    the earlier layers are read and written, the 16 tangents of layer a are read (not
-    at the layer's first gate) and written (not at the last gate), and psi_q is read
-    (and, in target sums, the next psi written).  Complex multiply-adds: 16 for the
+    Sums over columns (unitary gates) take the products of k_hgemm, one per layer: the 16
+    cotangent states of layer a with the 16 (a + 1) tangents and psi, 256 (a + 1) + 16
+    multiply-adds per amplitude, each state read once.  One state (single) runs k_hsweep, one
+    launch per gate: per gate q of layer a, phi_q is read, the tangents of the earlier layers
+    are read and written, the 16 tangents of layer a are read (not at the layer's first gate)
+    and written (not at the last gate), and psi_q is read.  Complex multiply-adds: 16 for the
     contraction with phi_q and 16 for G_q per group of 4 amplitudes and active state."""
+    if not single:
+        return {"kernel": "k_hgemm (products of a layer's cotangent states with the tangents, FP64 MMA)",
+                "transfers": sum(16 + 16 * (a + 1) + 1 for a in range(nlayers)),
+                "cmacs": sum(256 * (a + 1) + 16 for a in range(nlayers)) << L, "bound": "tensor"}
     per = L // 2
     G = nlayers * per
-    layered = L <= 12
     transfers = 0
     cmacs = 0
     for q in range(G):
@@ -301,21 +309,12 @@ def hess_model(L, nlayers, single):
         cmacs += 16 + (16 if last else 0)
         cmacs += 16 * a * (16 + (0 if last else 16))
         cmacs += 0 if pos == 0 else 16 * (16 + (0 if last else 16))
-        if layered:
-            continue
         t_read = 16 * a + (0 if pos == 0 else 16)
         t_write = 0 if last else 16 * (a + 1)
-        psi = 1 if single else (1 if q > 0 else 0) + (0 if last else 1)
-        transfers += 1 + psi + t_read + t_write
-    if layered:
-        for a in range(nlayers):
-            transfers += 16 * a + (16 * (a + 1) if a < nlayers - 1 else 0) + per + per
-        if not single:
-            transfers -= 1          # psi_0 is the basis column
+        transfers += 2 + t_read + t_write
     groups = (1 << L) // 4
-    return {"kernel": ("k_hlayer (one brickwall layer of the full-Hessian tangent sweep, column tiles in shared memory)"
-                       if layered else "k_hsweep (one gate of the full-Hessian tangent sweep)"),
-            "launches": nlayers if layered else G, "transfers": transfers, "cmacs": cmacs * groups}
+    return {"kernel": "k_hsweep (one gate of the full-Hessian tangent sweep)", "transfers": transfers,
+            "cmacs": cmacs * groups, "bound": "hbm"}
 
 
 def _ref_hessian_worker(args):
@@ -387,8 +386,8 @@ def hmat_path(gpu, torch, stream, hbm_peak, with_reference=True, steps=3, fp64_p
         return r, wall, e0.elapsed_time(e1) / n, hs_ms / n, hs_n // n, gpu.launch_count() // n
 
     def roofline(model, columns, L, ms, launches):
-        """HBM roofline for the per-gate sweep; the layer kernel moves ~L/2 times fewer
-        bytes and is bound by FP64 arithmetic instead, against the FP64 peak measured in
+        """HBM roofline for the per-gate sweep; the layers' products are bound by FP64
+        arithmetic instead, against the FP64 peak measured in
         this run (cuBLAS DGEMM), or the nominal 37 TFLOP/s of B200 where none was measured."""
         state_bytes = columns * (16 << L)
         per_launch = model["transfers"] * state_bytes / launches
@@ -398,7 +397,7 @@ def hmat_path(gpu, torch, stream, hbm_peak, with_reference=True, steps=3, fp64_p
                "bytes_per_launch": per_launch,
                "bytes_model": "algorithmic state transfers of the sweep (bench.hess_model) x columns x 2^L x 16 B",
                "hbm_gbs": gbs, "hbm_frac": gbs / hbm_peak, "fp64_tflops": tflops}
-        if "k_hlayer" in model["kernel"]:
+        if model["bound"] == "tensor":
             pk = fp64_peak or 37.0
             out.update({"bound": "tensor", "achieved": tflops, "peak": pk, "unit": "TFLOP/s", "frac": tflops / pk,
                         "peak_source": "FP64 peak measured in this run (cuBLAS DGEMM 8192^3)" if fp64_peak
@@ -448,7 +447,7 @@ def hmat_path(gpu, torch, stream, hbm_peak, with_reference=True, steps=3, fp64_p
         r2 = {"workload": f"f + gradient vector + Hessian matrix, brickwall L={L} depth {depth} vs brickwall target "
                           f"depth {tdepth}, all {N} basis columns", "evals_per_s_e2e": 1.0 / wall,
               "evals_per_s_device": 1e3 / dev_ms, "sweep_ms": hs_ms, "gpu_launches": launches,
-              "roofline": roofline(hess_model(L, depth, False), N, L, hs_ms, hs_n)}
+              "roofline": roofline(hess_model(L, depth, False), orbit_columns(L), L, hs_ms, hs_n)}
         out[f"target_L{L}_depth{depth}"] = r2
         target_cases.append((r2, L, depth, tdepth, vlist, perms, tvlist, tperms, g, H, wall))
 
@@ -496,9 +495,8 @@ def hmat_path(gpu, torch, stream, hbm_peak, with_reference=True, steps=3, fp64_p
                       f"L={L} depth {depth}, H a brickwall of depth {hdepth} on {L // 2} qubits, all {1 << (L // 2)} "
                       f"columns", "evals_per_s_e2e": 1.0 / wall, "ms_per_call": wall * 1e3, "sweep_ms": hs_ms,
           "gpu_launches": launches,
-          "roofline": roofline(hess_model(L, depth, False), 1 << (L // 2), L, hs_ms, hs_n)}
-    r5["roofline"]["bytes_model"] += (" (the 2^(L/2) block-encoding columns; the tangents the sweep also carries "
-                                      "through the last gate are not counted)")
+          "roofline": roofline(hess_model(L, depth, False), orbit_columns(L // 2), L, hs_ms, hs_n)}
+    r5["roofline"]["bytes_model"] += " (block-encoding columns, one per orbit of the wire symmetries)"
     out["blockenc_L12"] = r5
     if not have_ref:
         return out
@@ -638,17 +636,18 @@ def real_build_path(gpu, steps=3, L=14, depth=9, tdepth=5, seconds=8.0, with_ref
     cfg = gpu.last_config()
     G = depth * (L // 2)
     npass = G if cfg["gates_per_pass"] == 1 else -(-G // cfg["gates_per_pass"])
-    rbytes = float(6 * npass - 5) * N * (N // 2) * 16   # npass reverse passes per column over N/2 paired columns
+    columns = orbit_columns(L) // 2   # two basis columns in one, one per orbit of the wire symmetries
+    rbytes = float(6 * npass - 5) * N * columns * 16
     achieved = rbytes / (rev_ms * 1e-3) / 1e9 if rev_ms > 0 else None
     out = {"workload": f"real build: f + projected gradient (6 per gate) + projected HVP, real orthogonal brickwall "
                        f"L={L} depth {depth} vs real brickwall target depth {tdepth}, all {N} basis columns as "
-                       f"{N // 2} paired columns, complex128 engine", "evals_per_s_e2e": 1.0 / wall,
+                       f"{columns} paired columns (one per orbit of the wire symmetries), complex128 engine", "evals_per_s_e2e": 1.0 / wall,
            "ms_per_eval": wall * 1e3, "gpu_launches": launches, "f": float(f),
-           "roofline": {"kernel": ("k6_rev" if cfg["reconstruct"] else "k3_rev") + " (complex128 FP64-MMA "
+           "roofline": {"kernel": ("k8_rev" if cfg["reconstruct"] else "k3_rev") + " (complex128 FP64-MMA "
                                   "gradient/HVP pass)", "bound": "hbm",
                         "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                         "frac": achieved / hbm_peak if achieved else None,
-                        "bytes_model": "(6P-5) x 2^L x 2^(L-1) x 16 B per evaluation (P reverse passes over the "
+                        "bytes_model": "(6P-5) x 2^L x C x 16 B per evaluation (P reverse passes over the C "
                                        "paired columns)", "passes_per_column": npass, "launches": rev_n,
                         "reverse_ms": rev_ms,
                         "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if "hbm_gbs" in peaks
@@ -841,7 +840,7 @@ def compare_mixed(gpu, torch, stream, step, res_c128, steps, L, G, Gt, P, hbm_pe
     gpu.set_precision(gpu.PRECISION_C128)
     ms = e0.elapsed_time(e1) / steps
     P = G if cfg["gates_per_pass"] == 1 else -(-G // cfg["gates_per_pass"])
-    rbytes = reverse_bytes_per_eval(L, P, 8) * steps
+    rbytes = reverse_bytes_per_eval(L, P, 8, 1 << L) * steps
     achieved = rbytes / (rev_ms * 1e-3) / 1e9 if rev_ms > 0 else None
     flops = flops_per_eval(L, G, Gt)
     pipe = "FP32 FMA pipe" if cfg["c64_fp32_pipe"] else "3xTF32 MMA"
@@ -1127,28 +1126,31 @@ def main():
         gpp = tuned["gates_per_pass"]
         npass = G if gpp == 1 else -(-G // gpp)
         value = whole_job_rate(world, a.steps, dev_ms)
-        flops = flops_per_eval(L, G, Gt)
-        rbytes = reverse_bytes_per_eval(L, npass, itemsize) * a.steps
+        # complex128 takes one column per orbit of the brickwall's wire symmetries, complex64 all of them
+        columns = orbit_columns(L) if itemsize == 16 else 1 << L
+        flops = flops_per_eval(L, G, Gt) * columns / (1 << L)
+        rbytes = reverse_bytes_per_eval(L, npass, itemsize, columns) * a.steps
         gbs = rbytes / (rev_ms * 1e-3) / 1e9 if rev_ms > 0 else None
         if itemsize == 16:
-            # complex128: the reverse pass does ~11 flop per byte it moves, above the FP64
-            # ridge (~6 flop/B), so its roofline is the FP64 tensor pipe (DMMA) that runs it
-            rflops = reverse_flops_per_eval(L, G) * a.steps
+            # complex128: the reverse pass does 8 flop per byte it moves, above the FP64
+            # ridge (~6 flop/B), so its roofline is the FP64 pipe (DMMA and DFMA)
+            rflops = reverse_flops_per_eval(L, G, columns) * a.steps
             achieved = rflops / (rev_ms * 1e-3) / 1e12 if rev_ms > 0 else None
             fp64 = fp.get("fp64_tflops")
-            roof = {"kernel": (("k6_rev (complex128 reverse pass rebuilding states with adjoint gates"
+            roof = {"kernel": (("k8_rev (complex128 reverse pass, sums at the pass output"
                                 if tuned["reconstruct"] else "k3_rev (complex128 reverse pass recomputing states")
                                + f" on the FP64 tensor pipe, DMMA m8n8k4, {gpp} fused gates over a column chunk)"
                                if gpp > 1 else "k_reverse (complex128 gradient/HVP pass of one gate, FP64)"),
                     "bound": "tensor", "achieved": achieved, "peak": fp64, "unit": "TFLOP/s",
                     "frac": achieved / fp64 if (achieved and fp64) else None,
-                    "flops_model": "192 flop per amplitude, gate and basis column (six 4x4 complex products of an "
-                                   "amplitude group: the outer sums dG, HZ and the adjoint updates phi, dphi); states "
-                                   "rebuilt inside a pass not counted",
+                    "flops_model": f"192 flop per amplitude, gate and column (six 4x4 complex products of an amplitude "
+                                   f"group: the outer sums dG, HZ and the adjoint updates phi, dphi), {columns} columns: "
+                                   "one per orbit of the brickwall's wire symmetries; states rebuilt inside a pass not "
+                                   "counted",
                     "peak_source": "FP64 peak measured in this run (cuBLAS DGEMM 8192^3)",
-                    "traffic": rbytes / max(rev_n, 1) * 0.99,
-                    "traffic_source": "ncu capture of one middle k6_rev pass at L=12 (DRAM bytes / algorithmic = "
-                                      "0.99, profiles/k6_rev_c128_L12_d5.md), scaled to the bytes of an average "
+                    "traffic": rbytes / max(rev_n, 1) * 0.89,
+                    "traffic_source": "ncu capture of one middle k8_rev pass at L=12 (DRAM bytes / algorithmic = "
+                                      "0.89, the rest hits L2; profiles/k8_rev_c128_L12.md), scaled to the bytes of an average "
                                       "launch here",
                     "hbm_view": {"achieved_gbs": gbs, "peak_gbs": hbm_peak, "frac": gbs / hbm_peak if gbs else None,
                                  "peak_source": hbm_src},
@@ -1180,7 +1182,8 @@ def main():
             "eval_flops": {"per_eval": flops, "achieved_tflops": flops * a.steps / (dev_ms * 1e-3) / 1e12,
                            "peak_tflops": peak_eval,
                            "frac": (flops * a.steps / (dev_ms * 1e-3) / 1e12 / peak_eval) if peak_eval else None,
-                           "model": "N^2 (32 G_t + 292 G - 124): the reference's flops of one evaluation",
+                           "model": f"C N (32 G_t + 292 G - 124): the reference's flops of a column, C = {columns} columns "
+                                    "evaluated",
                            "peak_source": ("FP64" if itemsize == 16 else "FP32") + " peak measured in this run"},
             "measured_peaks": fp,
             "tuned": {"gates_per_pass": gpp, "column_chunk": tuned["column_chunk"] or "from workspace",

@@ -1,26 +1,25 @@
 // Fused basis-column evaluation engine: the gates of a circuit are grouped into
-// passes of up to four consecutive gates acting on at most eight qubits (for
-// the periodic brickwall a pass is one half of a layer), and each pass is one
-// HBM round trip over a column chunk.
+// passes of up to four gates acting on at most eight qubits (consecutive ones, or
+// for complex128 reordered where they commute), and each pass is one HBM round trip
+// over a column chunk.
 //
 // Layout: a chunk of C basis columns is stored column-interleaved, [2^L][C]
 // (amplitude row a, column j at a*C + j), so that a tile over ANY eight qubits
-// -- 256 rows -- reads and writes contiguous runs of CW columns (CW*sizeof =
-// 64 B) per row, whatever the qubits' positions.
+// -- 256 rows -- reads and writes contiguous runs of four or eight columns (64 to
+// 128 B) per row, whatever the qubits' positions.
 //
 // Per pass (gates g_0..g_{K-1} of the pass, directions z_k):
 //   forward  : psi, dpsi (pass input) -> pass output, in shared memory,
 //              dpsi <- g dpsi + z psi, psi <- g psi for each gate;
 //              only the pass-boundary states are stored (checkpoints);
-//   reverse  : from the checkpoint (psi, dpsi at the pass input) the K-1
-//              intermediate states are recomputed in shared memory, then for
-//              k = K-1..0, with phi, dphi the adjoint at the output of gate k:
+//   reverse  : with phi, dphi the adjoint at the output of gate k, for k = K-1..0:
 //                dG_k += phi (x) psi_k,   HZ_k += phi (x) dpsi_k + dphi (x) psi_k,
 //                dphi <- g_k^T dphi + z_k^T phi,  phi <- g_k^T phi;
-//              only phi, dphi at the pass input are stored.
-// Inside a gate step four threads share an amplitude group (4 amplitudes);
-// thread q owns gate row q of the outer products and output component q, so
-// each thread keeps 8 complex accumulators per gate of the pass in registers.
+//              only phi, dphi at the pass input are stored.  Unitary gates:
+//              complex128 takes the sums with the states at the pass output
+//              (k8_rev), complex64 rebuilds psi_k with adjoint gates (k5_rev,
+//              k7_rev); otherwise the psi_k are recomputed in shared memory from
+//              the checkpoint at the pass input (k3_rev, k4_rev).
 //
 // These are the same per-column recurrences as the per-gate engine (the
 // scheme of src/quantum_circuit.c:147-236), evaluated in a different order of

@@ -634,7 +634,7 @@ __global__ void k_gemv(int n, const double* __restrict__ a, const double* __rest
 // earlier tangents (layer_pass.cu), 32 new states (k_hstates) and the product.  Against the
 // general layer kernel this is a third of the flops at L = 12, 1-2 memory round trips a layer
 // instead of two tiles' worth of shared-memory traffic per gate; L = 10, depth 7, one column
-// per orbit: 3.8 -> 1.5 ms (see the figures at k_hgemm).
+// per orbit: 3.8 -> 1.7 ms (see the figures at k_hgemm).
 
 // T_{rc} (own tangents) and Phi_{ij} at a layer's output, 16 states each, from psi and phi
 struct LayerWires

@@ -390,7 +390,7 @@ int apply_circuit_fused_t(Runtime& rt, int L, int ngates, const double2* gates, 
 
 // out = C in for one statevector (complex128), maxk gates per pass.  16-byte aligned states take
 // the passes of layer_pass.cu with the gates reordered where they commute: L = 27, 64 gates on
-// random pairs 16.1 ms against 21.4 ms of 64 KiB bulk-copied tiles with four consecutive gates
+// random pairs 15.5 ms against 21.4 ms of 64 KiB bulk-copied tiles with four consecutive gates
 // (256 copies of 256 B a tile each way, and a shared-memory round trip per gate).
 int apply_circuit_fused_device(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
                                const double2* d_in, double2* d_out, int maxk)

@@ -109,3 +109,13 @@ def test_forward_passes_on_ragged_columns(gpu, L, near, unitary, first, last):
                 assert np.linalg.norm(a - b) <= 1e-12 * (np.linalg.norm(b) + np.linalg.norm(ref[1]))
     finally:
         gpu.set_column_range(0, 0)
+
+
+@pytest.mark.parametrize("L,depth", [(4, 1), (6, 2), (8, 3), (6, 4), (8, 5), (4, 9), (6, 13)])
+def test_hessian_products_of_every_last_tile(gpu, oracle, L, depth):
+    """Layers whose last tile of tangents holds one fragment or three, alone or after whole tiles."""
+    vlist, perms, tvlist, tperms = brickwall_instance(L, depth, L, 2, L + depth)
+    got = gpu.brickwall_unitary_target_gradient_hessian(gpu.Target(brickwall=(tvlist, tperms)), vlist, perms, L)
+    ref = oracle.brickwall_unitary_target_gradient_hessian(oracle.target("brickwall", (tvlist, tperms)), vlist, perms, L)
+    for a, b in zip(got[1:], ref[1:]):
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
