@@ -33,6 +33,7 @@
 
 #include "engine.h"
 #include "manifold.cuh"
+#include "orbits.h"
 #include "rqc_common.cuh"
 #include "rqc_runtime.h"
 #include "rqcopt_batch.h"
@@ -80,7 +81,9 @@ struct BInst
 {
 	int L, nl, tnl, per;       // qubits, layers, target layers, gates per layer
 	int mode, prec, active;    // current round: EVAL_* mode, PREC_C64 / PREC_C128, participates
-	int item0, item1;          // this instance's work items
+	int item0, item1;          // this instance's work items, and rows of partial sums
+	int end128;                // complex128 rounds: rows item0 .. end128 - 1
+	int col0;                  // complex128 rounds: first entry of its columns (< 0: all basis columns)
 	int niter, maxiter;        // RTR iterations, tCG iteration limit
 	double radius_init, maxradius, rho_trust, abstol, reltol;
 	double gtol;               // stop once the gradient norm is at most gtol (0: run niter iterations)
@@ -162,10 +165,16 @@ __device__ __forceinline__ void kahan_add(double* s, double* c, double v)
 
 // ------------------------------------------------------------------ evaluation kernel
 
-// One work item: columns item.y .. item.z - 1 of instance item.x, with the four
-// state tiles in shared memory (SMEM) or in this CTA's global scratch.
+// One work item: columns item.y .. item.z - 1 of instance item.x into row item.w of the partial
+// sums, with the four state tiles in shared memory (SMEM) or in this CTA's global scratch.
+//
+// complex128 columns are one per orbit of the instance's wire symmetries, {state, weight} in cols
+// (a periodic brickwall of 8 qubits: 70 of 256, of 12: 700 of 4096); the weight goes with phi.
+// complex64 takes all of them: its sums are held to their last float bits.
+// 16 Hessian products of 6 to 12 qubits in one call 70 -> 15.4 ms.
 template <typename T, bool SMEM>
-__device__ __forceinline__ void beval_item(const BInst& in, const int4& item, int it, const int* __restrict__ wires,
+__device__ __forceinline__ void beval_item(const BInst& in, const int4& item, const int2* __restrict__ cols,
+                                           const int* __restrict__ wires,
                                            const typename BTr<T>::E* __restrict__ tabs, double* __restrict__ partial,
                                            typename BTr<T>::V* __restrict__ gscratch, unsigned char* smem)
 {
@@ -265,12 +274,18 @@ __device__ __forceinline__ void beval_item(const BInst& in, const int4& item, in
 		__syncthreads();
 	};
 
+	// state and weight of a column (of the last tile: none beyond the item's)
+	auto column = [&](int c) {
+		if (sizeof(T) == sizeof(float) || in.col0 < 0) return make_int2(c, 1);
+		return c < item.z ? cols[in.col0 + c] : make_int2(-1, 0);
+	};
 	for (int b0 = item.y; b0 < item.z; b0 += CW) {
 		// phi = -conj(W e_b) for the columns b0 .. b0 + CW - 1
 		for (int e = tid; e < amps; e += BT) {
-			const int row = e >> lcw, c = e & (CW - 1);
+			const int row = e >> lcw;
+			const int2 col = column(b0 + (e & (CW - 1)));
 			P[e] = vzero<V>();
-			if (row == b0 + c) P[e].x = 1;
+			if (row == col.x) P[e].x = (T)col.y;
 		}
 		__syncthreads();
 		for (int l = 0; l < tnl; l++)
@@ -281,9 +296,9 @@ __device__ __forceinline__ void beval_item(const BInst& in, const int4& item, in
 			const V v = P[e];
 			P[e].x = -v.x;
 			P[e].y = v.y;
-			const int row = e >> lcw, c = e & (CW - 1);
+			const int row = e >> lcw;
 			S[e] = vzero<V>();
-			if (row == b0 + c) S[e].x = 1;
+			if (row == column(b0 + (e & (CW - 1))).x) S[e].x = 1;
 			if (tan) dS[e] = vzero<V>();
 		}
 		__syncthreads();
@@ -432,7 +447,7 @@ __device__ __forceinline__ void beval_item(const BInst& in, const int4& item, in
 		cmp[1] = 0;
 	}
 	__syncthreads();
-	double* out = partial + (size_t)it * NACC;
+	double* out = partial + (size_t)item.w * NACC;
 	for (int e = tid; e < nacc; e += BT) out[e] = acc[e] - cmp[e];
 	__syncthreads();
 
@@ -440,8 +455,8 @@ __device__ __forceinline__ void beval_item(const BInst& in, const int4& item, in
 
 template <typename T>
 __global__ void __launch_bounds__(BT, 1)
-k_beval(const BInst* __restrict__ insts, const int4* __restrict__ items, int nitems, int* __restrict__ queue,
-        const int* __restrict__ wires, const typename BTr<T>::E* __restrict__ tabs, double* __restrict__ partial,
+k_beval(const BInst* __restrict__ insts, const int4* __restrict__ items, int nitems, const int2* __restrict__ cols,
+        int* __restrict__ queue, const int* __restrict__ wires, const typename BTr<T>::E* __restrict__ tabs, double* __restrict__ partial,
         typename BTr<T>::V* __restrict__ gscratch, int prec)
 {
 	using V = typename BTr<T>::V;
@@ -460,9 +475,9 @@ k_beval(const BInst* __restrict__ insts, const int4* __restrict__ items, int nit
 		const int N = 1 << in.L;
 		const int amps = N * (N >= BTr<T>::AMP ? 1 : BTr<T>::AMP >> in.L);
 		if ((size_t)4 * amps * sizeof(V) <= STATE_SMEM)
-			beval_item<T, true>(in, item, it, wires, tabs, partial, gscratch, smem);
+			beval_item<T, true>(in, item, cols, wires, tabs, partial, gscratch, smem);
 		else
-			beval_item<T, false>(in, item, it, wires, tabs, partial, gscratch, smem);
+			beval_item<T, false>(in, item, cols, wires, tabs, partial, gscratch, smem);
 	}
 }
 
@@ -560,11 +575,11 @@ __global__ void k_bpost(Slots s, const double* __restrict__ partial)
 	const int i = blockIdx.x, u = threadIdx.x;
 	const BInst in = s.inst[i];
 	if (!in.active) return;
-	const int nl = in.nl;
+	const int nl = in.nl, end = in.prec == PREC_C128 ? in.end128 : in.item1;
 	const BOpt& op = s.opt[i];
 	if (u == MAXU) {
 		double fr = 0, fi = 0, cr = 0, ci = 0;
-		for (int it = in.item0; it < in.item1; it++) {
+		for (int it = in.item0; it < end; it++) {
 			kahan_add(&fr, &cr, partial[(size_t)it * NACC]);
 			kahan_add(&fi, &ci, partial[(size_t)it * NACC + 1]);
 		}
@@ -581,7 +596,7 @@ __global__ void k_bpost(Slots s, const double* __restrict__ partial)
 	M4 dg, hg, g, z;
 	for (int e = 0; e < 16; e++) {
 		double sr = 0, si = 0, cr = 0, ci = 0, hr = 0, hi = 0, chr = 0, chi = 0;
-		for (int it = in.item0; it < in.item1; it++) {
+		for (int it = in.item0; it < end; it++) {
 			const double* p = partial + (size_t)it * NACC;
 			kahan_add(&sr, &cr, p[2 + 32 * u + 2 * e]);
 			kahan_add(&si, &ci, p[2 + 32 * u + 2 * e + 1]);
@@ -683,10 +698,15 @@ struct Batch
 	void* mem = nullptr;
 	std::vector<int> used;                 // slot -> 0 free, 1 in use
 	std::vector<BInst> hinst;
-	std::vector<int4> hitems;
-	std::vector<int> hranges;              // (item0, item1) per slot, staged for the device table
-	int4* ditems = nullptr;
+	std::vector<int4> hitems, hitems64;    // of the complex64 kernel, of the complex128 one
+	std::vector<std::vector<int2>> columns;   // per slot: complex128 columns {state, weight}; none: all basis columns
+	std::vector<int> wants64;              // per slot: has complex128 rounds
+	std::vector<int2> hcols;               // columns of the live slots
+	std::vector<int> hranges;              // (item0, item1, end128, col0) per slot, staged for the device table
+	int4 *ditems = nullptr, *ditems64 = nullptr;
 	size_t items_cap = 0;
+	int2* dcols = nullptr;
+	size_t cols_cap = 0;
 	double* partial = nullptr;
 	size_t partial_cap = 0;
 	float2* gs32 = nullptr;
@@ -748,6 +768,8 @@ int batch_init(Runtime& rt, Batch& b, int cap, int fiter_cap)
 	if (ret) return ret;
 	b.used.assign(cap, 0);
 	b.hinst.assign(cap, BInst{});
+	b.columns.assign(cap, {});
+	b.wants64.assign(cap, 0);
 	b.smem32 = eval_smem(sizeof(float4));
 	b.smem64 = eval_smem(sizeof(double2));
 	if ((ret = RQC_CUDA(cudaFuncSetAttribute(k_beval<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem32)))) return ret;
@@ -778,6 +800,8 @@ int rebuild_items(Runtime& rt, Batch& b)
 	const double target = ITEM_WORK;
 	(void)total;
 	b.hitems.clear();
+	b.hitems64.clear();
+	b.hcols.clear();
 	bool big = false;
 	for (const W& wv : live) {
 		BInst& in = b.hinst[wv.slot];
@@ -785,37 +809,69 @@ int rebuild_items(Runtime& rt, Batch& b)
 		int cols = cw;
 		while (cols < N && (N / cols > MAX_ITEMS || (double)cols * wv.cost < target)) cols *= 2;
 		in.item0 = (int)b.hitems.size();
-		for (int c0 = 0; c0 < N; c0 += cols) b.hitems.push_back(make_int4(wv.slot, c0, std::min(N, c0 + cols), 0));
+		for (int c0 = 0; c0 < N; c0 += cols) b.hitems.push_back(make_int4(wv.slot, c0, std::min(N, c0 + cols), (int)b.hitems.size()));
 		in.item1 = (int)b.hitems.size();
+		// complex128: items of its columns by the same rule, so no more than above; they write the same
+		// rows (an instance is evaluated in one precision a round)
+		const std::vector<int2>& list = b.columns[wv.slot];
+		const int n = list.empty() ? N : (int)list.size();
+		int cols64 = cw;
+		while (cols64 < n && ((n + cols64 - 1) / cols64 > MAX_ITEMS || (double)cols64 * wv.cost < target)) cols64 *= 2;
+		in.end128 = in.item0;
+		if (b.wants64[wv.slot])
+			for (int c0 = 0; c0 < n; c0 += cols64)
+				b.hitems64.push_back(make_int4(wv.slot, c0, std::min(n, c0 + cols64), in.end128++));
+		in.col0 = list.empty() ? -1 : (int)b.hcols.size();
+		b.hcols.insert(b.hcols.end(), list.begin(), list.end());
 		if (in.L >= 12) big = true;
 	}
-	// item ranges live in the device instance table: one strided copy of (item0, item1)
-	// into every slot (free slots get empty ranges)
-	b.hranges.assign(2 * (size_t)b.cap, 0);
+	// item ranges live in the device instance table: one strided copy of (item0, item1, end128,
+	// col0) into every slot (free slots get empty ranges)
+	b.hranges.assign(4 * (size_t)b.cap, 0);
 	for (const W& wv : live) {
-		b.hranges[2 * (size_t)wv.slot] = b.hinst[wv.slot].item0;
-		b.hranges[2 * (size_t)wv.slot + 1] = b.hinst[wv.slot].item1;
+		int* r = &b.hranges[4 * (size_t)wv.slot];
+		r[0] = b.hinst[wv.slot].item0;
+		r[1] = b.hinst[wv.slot].item1;
+		r[2] = b.hinst[wv.slot].end128;
+		r[3] = b.hinst[wv.slot].col0;
 	}
 	{
-		int ret = RQC_CUDA(cudaMemcpy2DAsync(&b.d.inst[0].item0, sizeof(BInst), b.hranges.data(), 2 * sizeof(int),
-		                                     2 * sizeof(int), b.cap, cudaMemcpyHostToDevice, rt.stream));
+		int ret = RQC_CUDA(cudaMemcpy2DAsync(&b.d.inst[0].item0, sizeof(BInst), b.hranges.data(), 4 * sizeof(int),
+		                                     4 * sizeof(int), b.cap, cudaMemcpyHostToDevice, rt.stream));
 		if (ret) return ret;
 	}
 	const size_t ni = std::max<size_t>(b.hitems.size(), 1);
 	if (ni > b.items_cap) {
 		if (b.ditems) cudaFree(b.ditems);
+		if (b.ditems64) cudaFree(b.ditems64);
 		if (b.partial) cudaFree(b.partial);
 		b.items_cap = ni * 2;
+		b.ditems = b.ditems64 = nullptr;
+		b.partial = nullptr;
 		if (cudaMalloc(&b.ditems, b.items_cap * sizeof(int4)) != cudaSuccess ||
+		    cudaMalloc(&b.ditems64, b.items_cap * sizeof(int4)) != cudaSuccess ||
 		    cudaMalloc(&b.partial, b.items_cap * NACC * sizeof(double)) != cudaSuccess) {
 			cudaGetLastError();
+			b.items_cap = 0;
 			return E_ALLOC;
 		}
 	}
-	if (!b.hitems.empty()) {
-		int ret = RQC_CUDA(cudaMemcpyAsync(b.ditems, b.hitems.data(), b.hitems.size() * sizeof(int4), cudaMemcpyHostToDevice, rt.stream));
-		if (ret) return ret;
+	if (b.hcols.size() > b.cols_cap) {
+		if (b.dcols) cudaFree(b.dcols);
+		b.dcols = nullptr;
+		b.cols_cap = b.hcols.size() * 2;
+		if (cudaMalloc(&b.dcols, b.cols_cap * sizeof(int2)) != cudaSuccess) {
+			cudaGetLastError();
+			b.cols_cap = 0;
+			return E_ALLOC;
+		}
 	}
+	auto upload = [&](void* dst, const void* src, size_t bytes) {
+		return bytes ? RQC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, rt.stream)) : 0;
+	};
+	if (int ret = upload(b.ditems, b.hitems.data(), b.hitems.size() * sizeof(int4))) return ret;
+	if (int ret = upload(b.ditems64, b.hitems64.data(), b.hitems64.size() * sizeof(int4))) return ret;
+	if (int ret = upload(b.dcols, b.hcols.data(), b.hcols.size() * sizeof(int2))) return ret;
 	if (big && !b.gs32) {
 		// per-CTA state tiles beyond the shared-memory budget
 		if (cudaMalloc(&b.gs32, (size_t)b.grid * 4 * ((size_t)1 << MAXL) * sizeof(float2)) != cudaSuccess ||
@@ -830,12 +886,12 @@ int rebuild_items(Runtime& rt, Batch& b)
 
 int launch_round(Runtime& rt, Batch& b)
 {
-	const int ni = (int)b.hitems.size();
+	const int ni = (int)b.hitems.size(), ni64 = (int)b.hitems64.size();
 	k_bround<<<1, 1, 0, rt.stream>>>(b.counters);
 	k_bprepare<<<b.cap, 64, 0, rt.stream>>>(b.d, b.counters);
-	k_beval<float><<<b.grid, BT, b.smem32, rt.stream>>>(b.d.inst, b.ditems, ni, b.counters + 0, b.d.wires, b.d.tab32,
+	k_beval<float><<<b.grid, BT, b.smem32, rt.stream>>>(b.d.inst, b.ditems, ni, nullptr, b.counters + 0, b.d.wires, b.d.tab32,
 	                                                     b.partial, b.gs32, PREC_C64);
-	k_beval<double><<<b.grid, BT, b.smem64, rt.stream>>>(b.d.inst, b.ditems, ni, b.counters + 1, b.d.wires, b.d.tab64,
+	k_beval<double><<<b.grid, BT, b.smem64, rt.stream>>>(b.d.inst, b.ditems64, ni64, b.dcols, b.counters + 1, b.d.wires, b.d.tab64,
 	                                                      b.partial, b.gs64, PREC_C128);
 	k_bpost<<<b.cap, MAXU + 1, 0, rt.stream>>>(b.d, b.partial);
 	k_badvance<<<(b.cap + 127) / 128, 128, 0, rt.stream>>>(b.d, b.cap, b.fiter_cap, b.refine_threshold, b.counters,
@@ -919,6 +975,16 @@ int load_slot(Runtime& rt, Batch& b, int i, const struct rqcopt_batch_problem* p
 	for (int l = 0; l < tnl; l++)
 		for (int q = 0; q < L; q++) w[(MAXU + l) * MAXL + q] = p->target_perms[l][q];
 	b.hinst[i] = in;
+	b.wants64[i] = phase == PH_EVAL ? precision == PREC_C128 : precision != PREC_C64;
+	b.columns[i].clear();
+	if (b.wants64[i]) {
+		std::vector<const int*> layers;
+		for (int l = 0; l < nl; l++) layers.push_back(&w[l * MAXL]);
+		for (int l = 0; l < tnl; l++) layers.push_back(&w[(MAXU + l) * MAXL]);
+		const std::vector<int> sym = wire_symmetries(L, layers);
+		if ((int)sym.size() > L)
+			for (const BasisCol& c : orbit_columns(L, sym)) b.columns[i].push_back(make_int2(c.re, (int)c.wre));
+	}
 	int ret = RQC_CUDA(cudaMemcpyAsync(&b.d.inst[i], &in, sizeof(in), cudaMemcpyHostToDevice, rt.stream));
 	if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(&b.d.opt[i], &op, sizeof(op), cudaMemcpyHostToDevice, rt.stream));
 	if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(b.d.wires + (size_t)i * (MAXU + MAXTU) * MAXL, w.data(), w.size() * sizeof(int),
@@ -954,6 +1020,8 @@ void batch_free(Batch* b)
 	if (b->graph) cudaGraphExecDestroy(b->graph);
 	if (b->mem) cudaFree(b->mem);
 	if (b->ditems) cudaFree(b->ditems);
+	if (b->ditems64) cudaFree(b->ditems64);
+	if (b->dcols) cudaFree(b->dcols);
 	if (b->partial) cudaFree(b->partial);
 	if (b->gs32) cudaFree(b->gs32);
 	if (b->gs64) cudaFree(b->gs64);
@@ -997,6 +1065,8 @@ void rqcopt_batch_destroy(struct rqcopt_batch* h)
 	if (h->b.graph) cudaGraphExecDestroy(h->b.graph);
 	if (h->b.mem) cudaFree(h->b.mem);
 	if (h->b.ditems) cudaFree(h->b.ditems);
+	if (h->b.ditems64) cudaFree(h->b.ditems64);
+	if (h->b.dcols) cudaFree(h->b.dcols);
 	if (h->b.partial) cudaFree(h->b.partial);
 	if (h->b.gs32) cudaFree(h->b.gs32);
 	if (h->b.gs64) cudaFree(h->b.gs64);

@@ -192,3 +192,32 @@ def test_orbit_block_encodings_equal_plain_ones(gpu, L, depth, hdepth):
         for a, b in zip(got[1:], ref[1:]):
             assert rel_err(a, b) <= 1e-12
     assert abs(gpu.brickwall_blockenc_target(dev, vlist, perms, L) - ref[0]) <= 1e-12 * abs(ref[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,tol", [("PRECISION_C128", 1e-12), ("PRECISION_MIXED", 1e-4), ("PRECISION_C64", 1e-4)])
+def test_batches_of_problems_with_and_without_symmetries(gpu, precision, tol):
+    """One column per orbit where a problem has wire symmetries and its rounds are complex128, against
+    sums over all columns of one problem at a time; columns that do not fill the last tile."""
+    from rqcopt_hpc_b200 import batch
+    probs, dirs, ref = [], [], []
+    for L, kind, n in [(8, "ring", 4), (6, "any", 3), (10, "renamed", 3), (4, "ring", 3), (12, "ring", 2), (8, "reversed", 4),
+                       (2, "ring", 2), (14, "ring", 2)]:
+        vlist, _, tvlist, _ = brickwall_instance(L, n, L, 2, L + 1)
+        perms = _layers(kind, L, n, L)
+        r = random_tangent_dirs(vlist, 2)
+        z = np.stack([vlist[k] @ real_to_antisymm(r[k]) for k in range(n)])
+        probs.append((L, vlist, perms, tvlist, perms[:2]))
+        dirs.append(z)
+        try:
+            gpu.set_column_range(0, 1 << L)
+            ref.append(gpu.brickwall_unitary_target_projected_hessian_vector_product(gpu.Target(brickwall=(tvlist, perms[:2])),
+                                                                                     vlist, z, perms, L))
+        finally:
+            gpu.set_column_range(0, 0)
+            gpu.set_autotune(True)
+    f, g, h = batch.evaluate(probs, dirs, batch.EVAL_HVP, getattr(gpu, precision))
+    for k, (f0, g0, h0) in enumerate(ref):
+        assert abs(f[k] - f0) <= tol * 2 ** (probs[k][0] / 2)
+        assert rel_err(g[k], g0) <= tol
+        assert rel_err(h[k], h0) <= tol
