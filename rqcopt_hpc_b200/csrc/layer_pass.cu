@@ -304,8 +304,8 @@ int circuit_apply_reordered(Runtime& rt, int L, int ngates, const double2* gates
 	// A gate waits for the last gates before it on its two wires; gates that wait for none commute
 	// and act on wires of their own.  Each pass takes the `most` of them with the longest chains of
 	// gates behind them: taken in the order of the circuit, chains are left over at the end that
-	// cost a pass per gate or two (64 gates on random pairs of 27 wires: 16 passes of four instead
-	// of 16-19).
+	// cost a pass per gate or two (64 gates on random pairs of 27 wires: the least number of passes,
+	// 16 of four gates, for three draws in four).
 	std::vector<int> waits(ngates, 0), height(ngates, 1), last(L, -1);
 	std::vector<std::vector<int>> next(ngates);
 	for (int k = 0; k < ngates; k++)
