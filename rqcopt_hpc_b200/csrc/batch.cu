@@ -843,13 +843,11 @@ int rebuild_items(Runtime& rt, Batch& b)
 	const size_t ni = std::max<size_t>(b.hitems.size(), 1);
 	if (ni > b.items_cap) {
 		if (b.ditems) cudaFree(b.ditems);
-		if (b.ditems64) cudaFree(b.ditems64);
 		if (b.partial) cudaFree(b.partial);
 		b.items_cap = ni * 2;
-		b.ditems = b.ditems64 = nullptr;
+		b.ditems = nullptr;
 		b.partial = nullptr;
-		if (cudaMalloc(&b.ditems, b.items_cap * sizeof(int4)) != cudaSuccess ||
-		    cudaMalloc(&b.ditems64, b.items_cap * sizeof(int4)) != cudaSuccess ||
+		if (cudaMalloc(&b.ditems, 2 * b.items_cap * sizeof(int4)) != cudaSuccess ||
 		    cudaMalloc(&b.partial, b.items_cap * NACC * sizeof(double)) != cudaSuccess) {
 			cudaGetLastError();
 			b.items_cap = 0;
@@ -866,6 +864,7 @@ int rebuild_items(Runtime& rt, Batch& b)
 			return E_ALLOC;
 		}
 	}
+	b.ditems64 = b.ditems + b.items_cap;   // no more than the others
 	auto upload = [&](void* dst, const void* src, size_t bytes) {
 		return bytes ? RQC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, rt.stream)) : 0;
 	};
@@ -1020,7 +1019,6 @@ void batch_free(Batch* b)
 	if (b->graph) cudaGraphExecDestroy(b->graph);
 	if (b->mem) cudaFree(b->mem);
 	if (b->ditems) cudaFree(b->ditems);
-	if (b->ditems64) cudaFree(b->ditems64);
 	if (b->dcols) cudaFree(b->dcols);
 	if (b->partial) cudaFree(b->partial);
 	if (b->gs32) cudaFree(b->gs32);
@@ -1065,7 +1063,6 @@ void rqcopt_batch_destroy(struct rqcopt_batch* h)
 	if (h->b.graph) cudaGraphExecDestroy(h->b.graph);
 	if (h->b.mem) cudaFree(h->b.mem);
 	if (h->b.ditems) cudaFree(h->b.ditems);
-	if (h->b.ditems64) cudaFree(h->b.ditems64);
 	if (h->b.dcols) cudaFree(h->b.dcols);
 	if (h->b.partial) cudaFree(h->b.partial);
 	if (h->b.gs32) cudaFree(h->b.gs32);
