@@ -555,7 +555,7 @@ void* rqcopt_gpu_stream(void);
 
 /* Addition (no counterpart in the reference): apply_quantum_circuit
  * (src/quantum_circuit.h:7, src/quantum_circuit.c:13-35) on complex64 states
- * already in device memory (psi, psi_out: 2^nqubits float2 each, distinct);
+ * already in device memory (psi, psi_out: 2^nqubits float2 each, 8-byte aligned, distinct);
  * gates are complex128 host matrices, rounded to complex64 for the passes.
  * Returns 0, or -5 (CUDA) / -6 (invalid argument, host pointers). */
 int rqcopt_apply_quantum_circuit_c64(const struct mat4x4 gates[], int ngates, const int wires[], const void* psi,
@@ -577,7 +577,7 @@ int rqcopt_apply_quantum_circuit_c64(const struct mat4x4 gates[], int ngates, co
  * of 2 MiB + 256 B that every GPU loading the library keeps until exit.
  *   - psi, dpsi_out and dpsi must hold managed memory or device memory of the
  *     current device (host buffers would need staging, i.e. allocation; memory
- *     of another GPU is refused); dgate may be host or device memory;
+ *     of another GPU is refused), 16-byte aligned; dgate may be host or device memory;
  *   - at most RQCOPT_NOALLOC_MAX_QUBITS qubits; larger states are rejected
  *     with -6 and a message on stderr;
  *   - work is issued on `stream` (a cudaStream_t, NULL for the legacy default

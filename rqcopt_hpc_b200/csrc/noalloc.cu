@@ -158,6 +158,11 @@ extern "C" int rqcopt_apply_gate_backward_noalloc(const struct mat4x4* gate, con
 		        "(no staging without allocation)\n", fn, dev);
 		return -6;
 	}
+	if ((uintptr_t)psi->data % sizeof(double2) || (uintptr_t)dpsi_out->data % sizeof(double2) ||
+	    (uintptr_t)dpsi->data % sizeof(double2)) {
+		fprintf(stderr, "%s: statevector data must be 16-byte aligned (no staging without allocation)\n", fn);
+		return -6;
+	}
 
 	// one-time set-up per device: the device address of the static scratch
 	if (!g_scratch_addr[dev]) {

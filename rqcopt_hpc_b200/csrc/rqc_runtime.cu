@@ -107,10 +107,14 @@ bool is_device_pointer(const void* p)
 	return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// The kernels take amplitudes as 16-byte words: a device state that does not begin at such a
+// boundary (a view into a buffer of doubles) is staged like a host state.
+static bool usable_in_place(const void* p) { return (uintptr_t)p % sizeof(double2) == 0 && is_device_pointer(p); }
+
 int span_in(Runtime& rt, const void* p, size_t bytes, int slot, DeviceSpan& s)
 {
 	s.bytes = bytes;
-	if (is_device_pointer(p)) {
+	if (usable_in_place(p)) {
 		s.dev = const_cast<void*>(p);
 		s.host = nullptr;
 		return OK;
@@ -119,13 +123,13 @@ int span_in(Runtime& rt, const void* p, size_t bytes, int slot, DeviceSpan& s)
 	if (ret) return ret;
 	s.dev = rt.stage[slot].ptr;
 	s.host = const_cast<void*>(p);
-	return RQC_CUDA(cudaMemcpyAsync(s.dev, p, bytes, cudaMemcpyHostToDevice, rt.stream));
+	return RQC_CUDA(cudaMemcpyAsync(s.dev, p, bytes, cudaMemcpyDefault, rt.stream));
 }
 
 int span_out(Runtime& rt, void* p, size_t bytes, int slot, DeviceSpan& s)
 {
 	s.bytes = bytes;
-	if (is_device_pointer(p)) {
+	if (usable_in_place(p)) {
 		s.dev = p;
 		s.host = nullptr;
 		return OK;
@@ -140,7 +144,7 @@ int span_out(Runtime& rt, void* p, size_t bytes, int slot, DeviceSpan& s)
 int span_finish(Runtime& rt, DeviceSpan& s)
 {
 	if (!s.host) return OK;
-	return RQC_CUDA(cudaMemcpyAsync(s.host, s.dev, s.bytes, cudaMemcpyDeviceToHost, rt.stream));
+	return RQC_CUDA(cudaMemcpyAsync(s.host, s.dev, s.bytes, cudaMemcpyDefault, rt.stream));
 }
 
 static cudaEvent_t take_event(Runtime& rt)

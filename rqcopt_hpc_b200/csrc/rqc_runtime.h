@@ -108,8 +108,8 @@ size_t workspace_budget(Runtime& rt, size_t want);
 // true if the pointer is device-accessible memory of this context (device or managed)
 bool is_device_pointer(const void* p);
 
-// A statevector-sized span on the device: either the caller's pointer (device or
-// managed memory) or a staging buffer filled from / written back to host memory.
+// A statevector-sized span on the device: either the caller's pointer (device or managed
+// memory, 16-byte aligned) or a staging buffer filled from / written back to the caller's memory.
 struct DeviceSpan
 {
 	void* dev = nullptr;
