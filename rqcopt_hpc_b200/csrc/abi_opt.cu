@@ -396,7 +396,8 @@ struct DeviceOptimizer
 
 	DeviceOptimizer(Runtime& r, Problem& p, const TargetHolder& t) : rt(r), pb(p), th(t), n(16 * p.nunits) {}
 
-	int init(const double2* x0, bool c128)
+	// hmat: the columns serve the full-Hessian sums too
+	int init(const double2* x0, bool hmat)
 	{
 		const size_t nu = pb.nunits;
 		const size_t nres = result_count(pb.G);
@@ -411,11 +412,10 @@ struct DeviceOptimizer
 		res = dirs + 16 * nu;
 		scratch = reinterpret_cast<double*>(res + nres);
 		hx.assign(x0, x0 + 16 * nu);
-		const std::vector<BasisCol> cols =
-			pb.brickwall ? orbits_of(rt, pb.L, pb.nunits, pb.wires.data(), th) : std::vector<BasisCol>();
+		const std::vector<BasisCol> cols = hmat ? orbits_of(rt, pb.L, pb.nunits, pb.wires.data(), th) : evaluation_columns(rt, pb, th);
 		if (!cols.empty() && (ret = upload_columns(rt, cols, &orbits.columns, &orbits.ncolumns))) return ret;
 		orbits.L = pb.L;
-		small = c128 && SmallEval::fits(rt, pb, th, column_count(rt, orbits));
+		small = (hmat || rt.precision == PREC_C128) && SmallEval::fits(rt, pb, th, column_count(rt, orbits));
 		if (small && (ret = ev.prepare(rt, pb, th, cols))) return ret;
 		return RQC_CUDA(cudaMemcpyAsync(x, x0, 16 * nu * sizeof(double2), cudaMemcpyHostToDevice, rt.stream));
 	}
@@ -658,7 +658,7 @@ void run_optimizer(const char* fn, Problem& pb, linear_func ufunc, void* udata, 
 	params->g_data = NULL;
 	params->g_iter = NULL;
 	DeviceOptimizer opt(*rt, pb, th);
-	int ret = opt.init(reinterpret_cast<const double2*>(start), hmat || rt->precision == PREC_C128);
+	int ret = opt.init(reinterpret_cast<const double2*>(start), hmat);
 	if (!ret)
 		ret = hmat ? opt.run_hmat(params, niter, f_iter, reinterpret_cast<double2*>(out), rng, nsamples)
 		           : opt.run(params, niter, f_iter, reinterpret_cast<double2*>(out), rt->precision);

@@ -203,7 +203,13 @@ std::vector<BasisCol> orbits_of(const Runtime& rt, int L, int nlayers, const int
 	for (int k = 0; k < th.spec.ngates; k += per) layers.push_back(&th.wires[2 * (size_t)k]);
 	const std::vector<int> sym = wire_symmetries(L, layers);
 	if ((int)sym.size() == L) return {};
-	const std::vector<BasisCol> cols = orbit_columns(L, sym);
+	return orbit_columns(L, sym);
+}
+
+std::vector<BasisCol> evaluation_columns(const Runtime& rt, const Problem& pb, const TargetHolder& th)
+{
+	if (!pb.brickwall) return {};
+	const std::vector<BasisCol> cols = orbits_of(rt, pb.L, pb.nunits, pb.wires.data(), th);
 	return rt.real_pairs ? pair_columns(cols) : cols;
 }
 
@@ -338,8 +344,7 @@ int run_target(const Problem& pb, TargetHolder& th, int mode, numeric* fval, str
 	int ret = th.to_device(*rt);
 	if (ret) return ret;
 	if (prec == PREC_C128) {
-		const std::vector<BasisCol> cols =
-			pb.brickwall ? orbits_of(*rt, pb.L, pb.nunits, pb.wires.data(), th) : std::vector<BasisCol>();
+		const std::vector<BasisCol> cols = evaluation_columns(*rt, pb, th);
 		if (SmallEval::fits(*rt, pb, th, cols.empty() ? column_count(*rt, cs) : (int64_t)cols.size()))
 			return run_small(*rt, pb, th, cols, mode, fval, dunits, hunits, grad_vec, hvp_vec);
 		if (!cols.empty() && (ret = upload_columns(*rt, cols, &cs.columns, &cs.ncolumns))) return ret;

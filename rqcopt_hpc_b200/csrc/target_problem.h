@@ -47,9 +47,12 @@ struct TargetHolder
 // over all basis states (orbits.h): a brickwall against a device-native brickwall whose
 // results are per-layer sums, over all columns.  Sets *columns and *ncolumns where there is
 // such a symmetry; the list lies in rt.columns (held until the next call).  orbits_of: the list
-// itself, empty where there is none.
+// itself, empty where there is none.  evaluation_columns: that of f, gradient and Hessian-vector
+// product evaluations, which take the columns of a real problem in pairs (rt.real_pairs); the
+// full-Hessian sums keep imaginary parts and never do.
 int upload_columns(Runtime& rt, const std::vector<BasisCol>& cols, const BasisCol** columns, int64_t* ncolumns);
 std::vector<BasisCol> orbits_of(const Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th);
+std::vector<BasisCol> evaluation_columns(const Runtime& rt, const Problem& pb, const TargetHolder& th);
 int use_orbits(Runtime& rt, int L, int nlayers, const int* wires, const TargetHolder& th, const BasisCol** columns,
                int64_t* ncolumns);
 // The same for the block encoding of a brickwall on L/2 qubits (the target) by one on L: the
