@@ -415,8 +415,12 @@ struct DeviceOptimizer
 		const std::vector<BasisCol> cols = hmat ? orbits_of(rt, pb.L, pb.nunits, pb.wires.data(), th) : evaluation_columns(rt, pb, th);
 		if (!cols.empty() && (ret = upload_columns(rt, cols, &orbits.columns, &orbits.ncolumns))) return ret;
 		orbits.L = pb.L;
-		small = (hmat || rt.precision == PREC_C128) && SmallEval::fits(rt, pb, th, column_count(rt, orbits));
-		if (small && (ret = ev.prepare(rt, pb, th, cols))) return ret;
+		const int most = hmat ? EVAL_F : EVAL_HVP;
+		small = (hmat || rt.precision == PREC_C128) && SmallEval::fits(rt, pb, th, column_count(rt, orbits), most);
+		if (small && (ret = ev.prepare(rt, pb, th, cols, most))) {
+			if (ret != E_ALLOC) return ret;
+			small = false;
+		}
 		return RQC_CUDA(cudaMemcpyAsync(x, x0, 16 * nu * sizeof(double2), cudaMemcpyHostToDevice, rt.stream));
 	}
 

@@ -307,7 +307,7 @@ static int run_small(Runtime& rt, const Problem& pb, const TargetHolder& th, con
 	const size_t nu = 16 * (size_t)pb.nunits;
 	const bool tan = mode == EVAL_HVP;
 	SmallEval ev;
-	int ret = ev.prepare(rt, pb, th, cols, pb.ugates.data(), tan ? pb.udirs.data() : nullptr);
+	int ret = ev.prepare(rt, pb, th, cols, mode, pb.ugates.data(), tan ? pb.udirs.data() : nullptr);
 	if (!ret) ret = ensure_host_pinned(rt.out_host, (1 + 2 * nu) * sizeof(double2) + 2 * nu * sizeof(double));
 	if (ret) return ret;
 	SmallOut out;
@@ -345,8 +345,10 @@ int run_target(const Problem& pb, TargetHolder& th, int mode, numeric* fval, str
 	if (ret) return ret;
 	if (prec == PREC_C128) {
 		const std::vector<BasisCol> cols = evaluation_columns(*rt, pb, th);
-		if (SmallEval::fits(*rt, pb, th, cols.empty() ? column_count(*rt, cs) : (int64_t)cols.size()))
-			return run_small(*rt, pb, th, cols, mode, fval, dunits, hunits, grad_vec, hvp_vec);
+		if (SmallEval::fits(*rt, pb, th, cols.empty() ? column_count(*rt, cs) : (int64_t)cols.size(), mode)) {
+			ret = run_small(*rt, pb, th, cols, mode, fval, dunits, hunits, grad_vec, hvp_vec);
+			if (ret != E_ALLOC) return ret;
+		}
 		if (!cols.empty() && (ret = upload_columns(*rt, cols, &cs.columns, &cs.ncolumns))) return ret;
 	}
 	const size_t nres = result_count(pb.G);

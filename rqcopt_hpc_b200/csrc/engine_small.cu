@@ -10,8 +10,8 @@
 // component q of every product and owns row q of the outer sums, so that a group's exchange
 // stays inside a warp and each gate costs one block barrier.
 //
-// The forward sweep leaves the state entering each gate in a scratch array (L2-resident for
-// the sizes this path is for); the reverse sweep brings the next gate's by cp.async into a
+// The forward sweep leaves the state entering each gate in a scratch array (in L2 up to a
+// quarter of SMALL_MAX_WORK); the reverse sweep brings the next gate's by cp.async into a
 // second pair of tiles while it works on the current one, so that a gate's outer sums
 //   dG += phi (x) psi,   HZ += phi (x) dpsi + dphi (x) psi
 // and its moves phi <- G^T phi, dphi <- G^T dphi + Z^T phi are all independent.  (Rebuilding
@@ -441,6 +441,15 @@ __global__ void __launch_bounds__(RED_GROUPS * SLOT) k_small_post(SmallArgs a, i
 // columns per block: enough groups to fill a warp
 int columns_per_block(int L) { return L >= 5 ? 1 : 32 >> L; }
 
+int block_count(int L, int64_t ncols) { return (int)((ncols + columns_per_block(L) - 1) / columns_per_block(L)); }
+
+// bytes of the states entering gates 1 .. G-1, of all blocks
+size_t states_bytes(int L, int G, int64_t ncols, int mode)
+{
+	if (mode == EVAL_F) return 0;
+	return (size_t)block_count(L, ncols) * (G - 1) * (mode == EVAL_HVP ? 2 : 1) * ((size_t)columns_per_block(L) << L) * sizeof(double2);
+}
+
 size_t small_smem(int L, int nunits, int G, int Gt, bool tan)
 {
 	return ((tan ? 8 : 4) * ((size_t)columns_per_block(L) << L) + (size_t)nunits * (tan ? 32 : 16) + 16 * (size_t)Gt) * sizeof(double2) +
@@ -476,16 +485,26 @@ int launch_small(Runtime& rt, const SmallArgs& a, int blocks)
 
 }  // namespace
 
-bool SmallEval::fits(const Runtime& rt, const Problem& pb, const TargetHolder& th, int64_t ncols)
+bool SmallEval::fits(Runtime& rt, const Problem& pb, const TargetHolder& th, int64_t ncols, int mode)
 {
 	if (rt.pin_gpp || rt.pin_chunk || rt.pin_recon || rt.col_begin != 0 || rt.col_end != 0) return false;
 	if (pb.L < 2 || pb.L > SMALL_MAX_L || pb.nunits > SMALL_MAX_UNITS || ncols < 1) return false;
 	if (th.spec.ufunc || (!th.spec.dense && th.spec.ngates < 1)) return false;
 	if ((double)ncols * (double)(1 << pb.L) * (pb.G + th.spec.ngates) >= SMALL_MAX_WORK) return false;
-	return small_smem(pb.L, pb.nunits, pb.G, th.spec.ngates, true) <= SMALL_SMEM;
+	if (small_smem(pb.L, pb.nunits, pb.G, th.spec.ngates, true) > SMALL_SMEM) return false;
+	// the pass engine splits its columns where the workspace does not hold all of them
+	const size_t states = states_bytes(pb.L, pb.G, ncols, mode);
+	return !states || states <= workspace_budget(rt, states);
 }
 
-int SmallEval::prepare(Runtime& rt, const Problem& pb, const TargetHolder& th, const std::vector<BasisCol>& cols,
+int SmallEval::reserve(Runtime& rt, int mode)
+{
+	int ret = ensure_device(rt.partials, (size_t)block_count(L_, ncols_) * (2 + SLOT * (size_t)nunits_) * sizeof(double));
+	if (!ret) ret = ensure_device(rt.work, states_bytes(L_, G_, ncols_, mode));
+	return ret;
+}
+
+int SmallEval::prepare(Runtime& rt, const Problem& pb, const TargetHolder& th, const std::vector<BasisCol>& cols, int mode,
                        const double2* ugates, const double2* udirs)
 {
 	const int64_t N = (int64_t)1 << pb.L;
@@ -509,6 +528,7 @@ int SmallEval::prepare(Runtime& rt, const Problem& pb, const TargetHolder& th, c
 	const size_t bytes = gates_b + cols_b + 2 * (size_t)(G_ + Gt_) * sizeof(int);
 	int ret = ensure_host_pinned(rt.small_host, bytes);
 	if (!ret) ret = ensure_device(rt.small_dev, bytes);
+	if (!ret) ret = reserve(rt, mode);
 	if (ret) return ret;
 	char* h = static_cast<char*>(rt.small_host.ptr);
 	double2* hg = reinterpret_cast<double2*>(h);
@@ -548,14 +568,10 @@ int SmallEval::eval(Runtime& rt, int mode, const double2* ugates, const double2*
 	a.bits = bits_;
 	a.tg = tg_;
 	a.dense = dense_;
-	const int blocks = (int)((ncols_ + a.cb - 1) / a.cb);
-	int ret = ensure_device(rt.partials, (size_t)blocks * (2 + SLOT * (size_t)nunits_) * sizeof(double));
+	const int blocks = block_count(L_, ncols_);
+	int ret = reserve(rt, mode);   // (other work of an optimiser may have taken the buffers)
 	if (ret) return ret;
 	a.part = static_cast<double*>(rt.partials.ptr);
-	if (mode != EVAL_F) {
-		const size_t states = (size_t)blocks * (G_ - 1) * (mode == EVAL_HVP ? 2 : 1) * ((size_t)a.cb << L_);
-		if ((ret = ensure_device(rt.work, states * sizeof(double2)))) return ret;
-	}
 	a.states = static_cast<double2*>(rt.work.ptr);
 	if (mode == EVAL_HVP) ret = launch_small<EVAL_HVP>(rt, a, blocks);
 	else if (mode == EVAL_GRAD) ret = launch_small<EVAL_GRAD>(rt, a, blocks);
