@@ -1289,25 +1289,26 @@ struct LayerSweep
 	}
 };
 
+// States of the layer sweep per column: psi and phi at every layer's output, 16 tangents per
+// layer (before that two scratch states of the target), 16 cotangent states, the sample states.
+// (The general sweep holds fewer for short circuits: 16 nl + 2 G + 2 up to L = 12.)
+size_t layer_column_bytes(int L, int nl, bool samp)
+{
+	return (size_t)(2 * nl + 16 * nl + 16 + (samp ? 1 : 0)) * sizeof(double2) << L;
+}
+
 // hessian_target_device for unitary gates: the layer sweep over column chunks
 int hessian_layers(Runtime& rt, const HessCircuit& c, const TargetSpec& t, double2* d_rec, const SampleSpec* samp)
 {
 	const int L = c.L, nl = c.nlayers;
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ncols = samp ? samp->nsamples : (c.columns ? c.ncolumns : N);
-	// states per column: psi and phi at every layer's output, 16 tangents per layer (before
-	// that two scratch states of the target), 16 cotangent states, the sample states
-	const int64_t nstates = 2 * nl + 16 * (int64_t)nl + 16 + (samp ? 1 : 0);
-	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
+	const size_t col_bytes = layer_column_bytes(L, nl, samp != nullptr);
 	int64_t C = ncols;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
 	if (t.ufunc) C = std::min<int64_t>(C, std::max<int64_t>(1, ((int64_t)256 << 20) / (N * 16)));
 	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
-	if (C < 1) {
-		fprintf(stderr, "rqcopt_gpu: one basis column of the Hessian sweep needs %zu bytes of workspace, more than the limit\n",
-		        col_bytes);
-		return E_ALLOC;
-	}
+	if (C < 1) return E_ALLOC;   // (the caller has seen that a column fits)
 	int ret = ensure_device(rt.work, (size_t)C * col_bytes);
 	if (ret) return ret;
 	LayerSweep sw(rt, c, true);
@@ -1354,7 +1355,8 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	const int L = c.L, nl = c.nlayers;
 	if (L < 2 || L % 2 || nl < 1) return E_ARG;
 	if (samp && samp->nsamples < 1) return E_ARG;
-	if (layer_sweep_ok(c)) return hessian_layers(rt, c, t, d_rec, samp);
+	const size_t layer_bytes = layer_column_bytes(L, nl, samp != nullptr);
+	if (layer_sweep_ok(c) && layer_bytes <= workspace_budget(rt, layer_bytes)) return hessian_layers(rt, c, t, d_rec, samp);
 	const int per = L / 2, G = nl * per;
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ncols = samp ? samp->nsamples : (c.columns ? c.ncolumns : N);   // basis columns, or sample states
@@ -1463,13 +1465,15 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	const int64_t N = (int64_t)1 << L, s = (int64_t)1 << half;
 	const bool hess = mode == 2;
 	const bool layered = L <= 12 && per <= HMAXPER;
-	const bool sweep = layer_sweep_ok(c);
 	// layer sweep, states per column: the input states, psi and phi at every layer's output, 16
 	// cotangent states, the tangents (Hessian only).
-	// General sweep: phi_q of every gate; psi_q of every gate (layered) or two psi buffers and
-	// the input states; W P e_b; the tangents (Hessian only)
-	const int64_t nstates = sweep ? 1 + 2 * nl + 16 + (hess ? 16 * (int64_t)nl : 0)
-	                              : G + (layered ? G : 3) + 1 + (hess ? 16 * (int64_t)nl : 0);
+	// General sweep (also where the workspace does not hold a column of the layer sweep): phi_q of
+	// every gate; psi_q of every gate (layered) or two psi buffers and the input states; W P e_b;
+	// the tangents (Hessian only)
+	const int64_t layer_states = 1 + 2 * nl + 16 + (hess ? 16 * (int64_t)nl : 0);
+	const size_t layer_bytes = (size_t)layer_states * N * sizeof(double2);
+	const bool sweep = layer_sweep_ok(c) && layer_bytes <= workspace_budget(rt, layer_bytes);
+	const int64_t nstates = sweep ? layer_states : G + (layered ? G : 3) + 1 + (hess ? 16 * (int64_t)nl : 0);
 	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
 	const int64_t ncols = c.columns ? c.ncolumns : s;
 	int64_t C = ncols;
