@@ -1149,11 +1149,12 @@ struct Sweep
 	}
 };
 
-// every layer gate unitary to 1e-14 and every layer's pairs on wires of their own
+// every layer gate unitary to 1e-14 and every layer's pairs on wires of their own; with one pair
+// a layer the diagonal blocks are exactly zero, which the difference in k_hrecord is not
 bool layer_sweep_ok(const HessCircuit& c)
 {
 	const int per = c.L / 2;
-	if (per > 16) return false;
+	if (per < 2 || per > 16) return false;
 	for (int l = 0; l < c.nlayers; l++) {
 		const double2* g = c.ugates + 16 * l;
 		for (int r = 0; r < 4; r++)
