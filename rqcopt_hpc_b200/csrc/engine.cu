@@ -301,11 +301,11 @@ static int dense_columns(Runtime& rt, const double2* u, int L, const ColumnSourc
 }
 
 // phi[s] = -conj(U x[s]) of a dense U for ns states one after another: a warp per row of U and
-// four states
+// four states (the groups of states in grid dimension x: there may be more than 65535)
 __global__ void __launch_bounds__(256) k_dense_states(const double2* __restrict__ u, int L, const double2* __restrict__ x,
                                                       int64_t ns, double2* __restrict__ phi)
 {
-	const int64_t N = (int64_t)1 << L, row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), s0 = (int64_t)blockIdx.y * 4;
+	const int64_t N = (int64_t)1 << L, row = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5), s0 = (int64_t)blockIdx.x * 4;
 	const int lane = threadIdx.x & 31;
 	if (row >= N) return;
 	double2 acc[4];
@@ -800,7 +800,7 @@ int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2*
 	const int64_t ngroups = ncols * (N / 4);
 	int ret;
 	if (t.dense) {
-		k_dense_states<<<dim3((unsigned)((N + 7) / 8), (unsigned)((ncols + 3) / 4)), 256, 0, rt.stream>>>(t.dense, L, states,
+		k_dense_states<<<dim3((unsigned)((ncols + 3) / 4), (unsigned)((N + 7) / 8)), 256, 0, rt.stream>>>(t.dense, L, states,
 		                                                                                                 ncols, phi);
 		rt.launches++;
 		return RQC_CUDA(cudaGetLastError());
