@@ -247,6 +247,7 @@ int TargetHolder::to_device(Runtime& rt)
 {
 	if (!dense_host || dense_L > 13) return OK;
 	const size_t bytes = sizeof(double2) << (2 * dense_L);
+	if (rt.workspace_limit && bytes > rt.workspace_limit) return OK;
 	int ret = ensure_device(rt.dense, bytes);
 	if (ret == E_ALLOC) return OK;   // no room: column by column through the host
 	if (!ret) ret = RQC_CUDA(cudaMemcpyAsync(rt.dense.ptr, dense_host, bytes, cudaMemcpyDefault, rt.stream));

@@ -38,8 +38,8 @@ struct TargetHolder
 	const double2* dense_host = nullptr;
 	int dense_L = 0;
 	bool set(linear_func ufunc, void* udata, int L);
-	// Copies a dense target to the device for the evaluations of this call (up to 1 GiB; larger
-	// ones stay a host callback, one column at a time).
+	// Copies a dense target to the device for the evaluations of this call (up to 1 GiB and within
+	// the workspace limit; others stay a host callback, one column at a time).
 	int to_device(Runtime& rt);
 };
 

@@ -69,3 +69,14 @@ def test_optimisers_keep_within_the_limit(gpu):
     got = gpu.optimize_quantum_circuit(target, gates, wires, L, 3)
     # the same iterates: rounding of f (at most 2^L) through three trust-region iterations
     assert np.all(np.abs(np.asarray(got[0]) - np.asarray(ref[0])) <= 1e-10 * 2 ** L)
+
+
+def test_a_dense_target_is_not_copied_beyond_the_limit(gpu, oracle):
+    L = 8
+    gates, wires, _, u = _circuit(L, 1)
+    target, ot = gpu.Target(dense=u), oracle.target("dense", u)
+    ref = oracle.circuit_unitary_target_and_gradient(ot, gates, wires, L)
+    gpu.set_workspace_limit((STATE << (2 * L)) - 1)
+    gpu.reset_launch_count()
+    _check(gpu.circuit_unitary_target_and_gradient(target, gates, wires, L), ref, L)
+    assert gpu.launch_count() > 2
