@@ -85,7 +85,9 @@ long rqcopt_batch_rounds(const struct rqcopt_batch* batch);
 /* evaluations run so far (one per active problem and round), and of them the
  * Hessian-vector products */
 long rqcopt_batch_evaluations(const struct rqcopt_batch* batch, long* hvp_evaluations);
-/* device bytes held for one problem of this size (admission accounting) */
+/* device bytes one problem of this size needs at most (admission accounting): its slot, its
+ * work items with their partial sums, and its list of columns.  The arrays of all but the slots
+ * are shared by the problems and take twice what is needed when they grow. */
 size_t rqcopt_batch_footprint(int nqubits, int nlayers);
 
 #ifdef __cplusplus

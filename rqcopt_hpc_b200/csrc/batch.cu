@@ -1188,10 +1188,13 @@ size_t rqcopt_batch_footprint(int nqubits, int nlayers)
 	constexpr int NTAB = (MAXU * 3 + MAXTU) * 16;
 	const size_t slot = sizeof(BInst) + sizeof(BOpt) + sizeof(int) * (MAXU + MAXTU) * MAXL + sizeof(double2) * (3 * MAXU + MAXTU) * 16 +
 	                    (sizeof(float4) + sizeof(double2)) * NTAB + sizeof(double) * (7 * MAXN + 2 + 2 * MAXN);
-	// partial sums of its work items (at most MAX_ITEMS, at most one per tile of columns)
+	// its work items (at most MAX_ITEMS, at most one per tile of columns) of both precisions and their
+	// partial sums; its list of columns where it has one, at most one per orbit of two states (a wire
+	// symmetry leaves no wire where it is: at most 2^(L/2) states are their own image)
 	const size_t cols = (size_t)1 << nqubits;
 	const size_t items = std::min<size_t>(MAX_ITEMS, (cols + tile_cols(nqubits) - 1) / tile_cols(nqubits));
-	return slot + items * (sizeof(int4) + NACC * sizeof(double));
+	const size_t listed = (cols + ((size_t)1 << (nqubits / 2))) / 2;
+	return slot + items * (2 * sizeof(int4) + NACC * sizeof(double)) + listed * sizeof(int2);
 }
 
 int rqcopt_brickwall_batch_evaluate(const struct rqcopt_batch_problem* problems, int count,
