@@ -66,8 +66,9 @@ int evaluate_autotuned(Runtime& rt, const CircuitSpec& c, const TargetSpec& t, i
 int apply_circuit_device(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
                          const double2* d_in, double2* d_out, long ncols);
 
-// Same for one complex64 statevector with up to maxk consecutive gates per HBM round trip
-// (shared-memory tiles over the gates' qubits plus the lowest amplitude bits).
+// Same for one statevector with up to maxk gates per HBM round trip (sv_fused.cu).
+int apply_circuit_fused_device(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
+                               const double2* d_in, double2* d_out, int maxk);
 int apply_circuit_fused_device_c64(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
                                    const float2* d_in, float2* d_out, int maxk);
 // out = C in for one complex64 statevector (per-gate passes, or fused passes of

@@ -298,8 +298,7 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 	return OK;
 }
 
-int circuit_apply_reordered(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, int most,
-                            const double2* in, double2* out)
+std::vector<std::vector<int>> reordered_passes(int L, int ngates, const int* wires, int most)
 {
 	// A gate waits for the last gates before it on its two wires; gates that wait for none commute
 	// and act on wires of their own.  Each pass takes the `most` of them with the longest chains of
@@ -322,19 +321,27 @@ int circuit_apply_reordered(Runtime& rt, int L, int ngates, const double2* gates
 	std::vector<int> ready;
 	for (int k = 0; k < ngates; k++)
 		if (!waits[k]) ready.push_back(k);
-	const double2* src = in;
+	std::vector<std::vector<int>> passes;
 	while (!ready.empty()) {
 		std::stable_sort(ready.begin(), ready.end(), [&](int x, int y) { return height[x] > height[y]; });
 		const int n = std::min<int>(most, (int)ready.size());
-		std::vector<LayerGate> pass;
-		std::vector<int> taken(ready.begin(), ready.begin() + n);
+		passes.emplace_back(ready.begin(), ready.begin() + n);
 		ready.erase(ready.begin(), ready.begin() + n);
-		for (int k : taken) {
-			pass.push_back({gates + 16 * (size_t)k, wires[2 * k], wires[2 * k + 1]});
+		for (int k : passes.back())
 			for (int m : next[k])
 				if (--waits[m] == 0) ready.push_back(m);
-		}
-		if (int e = layer_apply(rt, L, pass, false, src, out, 1)) return e;
+	}
+	return passes;
+}
+
+int circuit_apply_passes(Runtime& rt, int L, const std::vector<std::vector<int>>& passes, const double2* gates,
+                         const int* wires, const double2* in, double2* out)
+{
+	const double2* src = in;
+	for (const std::vector<int>& pass : passes) {
+		std::vector<LayerGate> list;
+		for (int k : pass) list.push_back({gates + 16 * (size_t)k, wires[2 * k], wires[2 * k + 1]});
+		if (int e = layer_apply(rt, L, list, false, src, out, 1)) return e;
 		src = out;
 	}
 	return OK;

@@ -29,10 +29,12 @@ int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool tr
 int circuit_apply(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, const double2* in, double2* out,
                   double2* scratch, int64_t ncols, const ColumnSource* columns = nullptr, bool neg_conj = false);
 
-// out = C in for one state (out may be in), gates reordered where they commute so that a pass over
-// the state takes up to `most` (<= 5; 4 measured best: a fifth leaves tiles short runs) on wires of
-// their own.
-int circuit_apply_reordered(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, int most,
-                            const double2* in, double2* out);
+// The gates of a circuit in passes of up to `most` (<= 5; 4 measured best: a fifth leaves tiles short
+// runs) on wires of their own, reordered where they commute.
+std::vector<std::vector<int>> reordered_passes(int L, int ngates, const int* wires, int most);
+
+// out = C in for one state (out may be in), a layer_apply per pass.
+int circuit_apply_passes(Runtime& rt, int L, const std::vector<std::vector<int>>& passes, const double2* gates,
+                         const int* wires, const double2* in, double2* out);
 
 }  // namespace rqc

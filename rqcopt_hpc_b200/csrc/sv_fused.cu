@@ -1,25 +1,28 @@
-// Gate application to single complex64 statevectors with several gates per HBM round trip
-// (complex128 states: layer_pass.cu).
+// Gate application to single statevectors with several gates per HBM round trip.
 //
 // Consecutive gates are grouped into passes of up to four gates (at most eight
 // qubits).  A pass streams the state once: each block stages a tile spanning the
 // pass's qubits plus the lowest amplitude bits in shared memory, applies the pass's
-// gates there, and writes the tile back.  The arithmetic per gate is the one of
-// src/gate.c:10-76.
+// gates there, and writes the tile back.  Used by apply_quantum_circuit /
+// apply_brickwall_unitary for large states; the arithmetic per gate is the one of
+// src/gate.c:10-76.  complex128 circuits that need few passes of gates on wires of their own
+// take those instead (layer_pass.cu; the rule is at apply_circuit_fused_device).
 //
-// Tiles of 64 KiB (8192 amplitudes) take as many of the
+// Tiles of 64 KiB (4096 complex128 or 8192 complex64 amplitudes) take as many of the
 // lowest state bits as fit beside the pass qubits, so a tile is a set of contiguous
-// runs of 2^m amplitudes (m >= 5: runs of 256 B or more), one per combination of the
+// runs of 2^m amplitudes (m >= 4: runs of 256 B or more), one per combination of the
 // pass qubits above the run.  The runs move between HBM and shared memory as TMA bulk
 // copies (cp.async.bulk, completion on an mbarrier for loads, bulk groups for stores),
 // issued by one warp; three blocks per SM overlap their load, gate and store phases.
-// States whose address is not 16-byte aligned take a tile kernel with plain loads.
+// States of fewer than 2^12 amplitudes and complex64 states that are not 16-byte aligned take a
+// tile kernel with plain loads.
 #include <stdio.h>
 #include <string.h>
 #include <algorithm>
 #include <vector>
 
 #include "engine.h"
+#include "layer_pass.h"
 #include "rqc_common.cuh"
 #include "rqcopt_gpu.h"
 
@@ -41,7 +44,7 @@ struct SvPass
 	int first;                     // first gate of the pass
 };
 
-struct SvGates { Gate4<float> g[SV_MAXK]; };
+template <typename T> struct SvGates { Gate4<T> g[SV_MAXK]; };
 
 __device__ __forceinline__ int64_t sv_deposit(int64_t v, uint32_t mask)
 {
@@ -54,10 +57,12 @@ __device__ __forceinline__ int64_t sv_deposit(int64_t v, uint32_t mask)
 	return r;
 }
 
-__global__ void __launch_bounds__(SV_TPB) k_sv_pass(const float2* __restrict__ in, float2* __restrict__ out, SvPass ps,
-                                                    SvGates gates)
+template <typename T>
+__global__ void __launch_bounds__(SV_TPB) k_sv_pass(const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, SvPass ps,
+                                                    SvGates<T> gates)
 {
-	__shared__ float2 S[1 << SV_MAXNB];
+	using V = cplx<T>;
+	__shared__ V S[1 << SV_MAXNB];
 	__shared__ int64_t off[1 << SV_MAXNB];
 	const int A = 1 << ps.NB;
 	for (int r = threadIdx.x; r < A; r += blockDim.x) {
@@ -82,7 +87,7 @@ __global__ void __launch_bounds__(SV_TPB) k_sv_pass(const float2* __restrict__ i
 				b = ((b >> lo) << (lo + 1)) | (b & ((1 << lo) - 1));
 				b = ((b >> hi) << (hi + 1)) | (b & ((1 << hi) - 1));
 				const int r0 = b, r1 = b | (1 << bj), r2 = b | (1 << bi), r3 = b | (1 << bi) | (1 << bj);
-				float2 x[4] = { S[r0], S[r1], S[r2], S[r3] }, y[4];
+				V x[4] = { S[r0], S[r1], S[r2], S[r3] }, y[4];
 				gate_apply(gates.g[k], x, y);
 				S[r0] = y[0];
 				S[r1] = y[1];
@@ -100,9 +105,11 @@ __global__ void __launch_bounds__(SV_TPB) k_sv_pass(const float2* __restrict__ i
 
 constexpr int SVT_TPB = 256;
 constexpr int SVT_TILE_BYTES = 64 * 1024;
-constexpr int SVT_BITS = 13;          // 8192 x 8 B
 constexpr int SVT_MAXRUNS = 256;      // runs per tile: 2^(pass qubits above the run) <= 2^8
 
+template <typename T> struct SvtBits;
+template <> struct SvtBits<double> { static constexpr int v = 12; };   // 4096 x 16 B
+template <> struct SvtBits<float>  { static constexpr int v = 13; };   // 8192 x 8 B
 
 struct SvTile
 {
@@ -139,16 +146,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity)
 	}
 }
 
-__global__ void __launch_bounds__(SVT_TPB, 3) k_sv_tile(const float2* __restrict__ in, float2* __restrict__ out, SvTile ps,
-                                                     SvGates gates, int* __restrict__ err)
+template <typename T>
+__global__ void __launch_bounds__(SVT_TPB, 3) k_sv_tile(const cplx<T>* __restrict__ in, cplx<T>* __restrict__ out, SvTile ps,
+                                                     SvGates<T> gates, int* __restrict__ err)
 {
+	using V = cplx<T>;
 	extern __shared__ __align__(128) unsigned char sm_raw[];
-	float2* S = reinterpret_cast<float2*>(sm_raw);
+	V* S = reinterpret_cast<V*>(sm_raw);
 	int64_t* roff = reinterpret_cast<int64_t*>(sm_raw + SVT_TILE_BYTES);
 	uint64_t* bar = reinterpret_cast<uint64_t*>(roff + SVT_MAXRUNS);
-	Gate4<float>* sgate = reinterpret_cast<Gate4<float>*>(bar + 2);
+	Gate4<T>* sgate = reinterpret_cast<Gate4<T>*>(bar + 2);
 	const int A = 1 << ps.NB, nruns = 1 << (ps.NB - ps.m);
-	const uint32_t run_bytes = (uint32_t)(sizeof(float2) << ps.m);
+	const uint32_t run_bytes = (uint32_t)(sizeof(V) << ps.m);
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	for (int r = threadIdx.x; r < nruns; r += blockDim.x) {
 		int64_t o = 0;
@@ -170,7 +179,7 @@ __global__ void __launch_bounds__(SVT_TPB, 3) k_sv_tile(const float2* __restrict
 			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 			if (lane == 0)
 				asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-				             "r"((uint32_t)(A * sizeof(float2))) : "memory");
+				             "r"((uint32_t)(A * sizeof(V))) : "memory");
 			__syncwarp();
 			for (int r = lane; r < nruns; r += 32)
 				asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -188,13 +197,13 @@ __global__ void __launch_bounds__(SVT_TPB, 3) k_sv_tile(const float2* __restrict
 		for (int k = 0; k < ps.K; k++) {
 			const int bi = ps.gi[k], bj = ps.gj[k];
 			const int lo = bi < bj ? bi : bj, hi = bi < bj ? bj : bi;
-			const Gate4<float>& gk = sgate[k];
+			const Gate4<T>& gk = sgate[k];
 			for (int g = threadIdx.x; g < A / 4; g += blockDim.x) {
 				int b = g;
 				b = ((b >> lo) << (lo + 1)) | (b & ((1 << lo) - 1));
 				b = ((b >> hi) << (hi + 1)) | (b & ((1 << hi) - 1));
 				const int r0 = b, r1 = b | (1 << bj), r2 = b | (1 << bi), r3 = b | (1 << bi) | (1 << bj);
-				float2 x[4] = { S[r0], S[r1], S[r2], S[r3] }, y[4];
+				V x[4] = { S[r0], S[r1], S[r2], S[r3] }, y[4];
 				gate_apply(gk, x, y);
 				S[r0] = y[0];
 				S[r1] = y[1];
@@ -224,10 +233,11 @@ __global__ void __launch_bounds__(SVT_TPB, 3) k_sv_tile(const float2* __restrict
 }
 
 // Tile bits: the pass qubits plus the lowest state bits 0..m-1, m as large as the tile allows.
+template <typename T>
 std::vector<SvTile> sv_tile_schedule(int L, int G, const int* wires, int maxk)
 {
 	std::vector<SvTile> out;
-	const int nbmax = std::min(SVT_BITS, L);
+	const int nbmax = std::min(SvtBits<T>::v, L);
 	for (int i = 0; i < G;) {
 		const int K = std::min(maxk, G - i);
 		uint32_t pass = 0;
@@ -302,36 +312,38 @@ std::vector<SvPass> sv_schedule(int L, int G, const int* wires, int maxk)
 
 }  // namespace
 
-int apply_circuit_fused_device_c64(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
-                                   const float2* d_in, float2* d_out, int maxk)
+template <typename T>
+int apply_circuit_fused_t(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, const cplx<T>* d_in,
+                          cplx<T>* d_out, int maxk)
 {
 	maxk = std::max(1, std::min(SV_MAXK, maxk));
-	const size_t bytes = ((size_t)1 << L) * sizeof(float2);
+	const size_t bytes = ((size_t)1 << L) * sizeof(cplx<T>);
 	int ret;
 	int P;
 	if (ngates > maxk && (ret = ensure_device(rt.stage[3], bytes))) return ret;
-	float2* tmp = reinterpret_cast<float2*>(rt.stage[3].ptr);
+	cplx<T>* tmp = reinterpret_cast<cplx<T>*>(rt.stage[3].ptr);
 	auto gates_of = [&](int first, int K) {
-		SvGates sg;
+		SvGates<T> sg;
 		memset(&sg, 0, sizeof(sg));
 		for (int k = 0; k < K; k++)
 			for (int e = 0; e < 16; e++) {
 				const double2 g = gates[16 * (first + k) + e];
-				sg.g[k].m[e].x = (float)g.x;
-				sg.g[k].m[e].y = (float)g.y;
+				sg.g[k].m[e].x = (T)g.x;
+				sg.g[k].m[e].y = (T)g.y;
 			}
 		return sg;
 	};
 	// TMA bulk tiles for 16-byte aligned states of at least 2^12 amplitudes
-	if (L >= 12 && ((uintptr_t)d_in % 16) == 0 && ((uintptr_t)d_out % 16) == 0) {
-		std::vector<SvTile> passes = sv_tile_schedule(L, ngates, wires, maxk);
+	const bool bulk = L >= 12 && ((uintptr_t)d_in % 16) == 0 && ((uintptr_t)d_out % 16) == 0;
+	if (bulk) {
+		std::vector<SvTile> passes = sv_tile_schedule<T>(L, ngates, wires, maxk);
 		P = (int)passes.size();
 		static int per_sm = 0;
-		const size_t smem = SVT_TILE_BYTES + SVT_MAXRUNS * sizeof(int64_t) + 16 + SV_MAXK * sizeof(Gate4<float>);
+		const size_t smem = SVT_TILE_BYTES + SVT_MAXRUNS * sizeof(int64_t) + 16 + SV_MAXK * sizeof(Gate4<T>);
 		if (!per_sm) {
-			if ((ret = RQC_CUDA(cudaFuncSetAttribute(k_sv_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))))
+			if ((ret = RQC_CUDA(cudaFuncSetAttribute(k_sv_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))))
 				return ret;
-			if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sv_tile, SVT_TPB, smem) != cudaSuccess ||
+			if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sv_tile<T>, SVT_TPB, smem) != cudaSuccess ||
 			    per_sm < 1) {
 				cudaGetLastError();
 				per_sm = 1;
@@ -340,13 +352,13 @@ int apply_circuit_fused_device_c64(Runtime& rt, int L, int ngates, const double2
 		if ((ret = ensure_device(rt.status, sizeof(int)))) return ret;
 		int* d_err = static_cast<int*>(rt.status.ptr);
 		if ((ret = RQC_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), rt.stream)))) return ret;
-		const float2* src = d_in;
+		const cplx<T>* src = d_in;
 		for (int p = 0; p < P; p++) {
-			float2* dst = ((P - 1 - p) % 2 == 0) ? d_out : tmp;
+			cplx<T>* dst = ((P - 1 - p) % 2 == 0) ? d_out : tmp;
 			const int grid = (int)std::min<int64_t>(passes[p].ntiles, (int64_t)rt.num_sms * per_sm);
 			cudaEvent_t ev;
 			launch_begin(rt, KC_FUSED, &ev);
-			k_sv_tile<<<grid, SVT_TPB, smem, rt.stream>>>(src, dst, passes[p], gates_of(passes[p].first, passes[p].K),
+			k_sv_tile<T><<<grid, SVT_TPB, smem, rt.stream>>>(src, dst, passes[p], gates_of(passes[p].first, passes[p].K),
 			                                                 d_err);
 			launch_end(rt, KC_FUSED, ev);
 			if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
@@ -363,18 +375,66 @@ int apply_circuit_fused_device_c64(Runtime& rt, int L, int ngates, const double2
 	}
 	std::vector<SvPass> passes = sv_schedule(L, ngates, wires, maxk);
 	P = (int)passes.size();
-	const float2* src = d_in;
+	const cplx<T>* src = d_in;
 	for (int p = 0; p < P; p++) {
-		float2* dst = ((P - 1 - p) % 2 == 0) ? d_out : tmp;
+		cplx<T>* dst = ((P - 1 - p) % 2 == 0) ? d_out : tmp;
 		const int grid = (int)std::min<int64_t>(passes[p].ntiles, (int64_t)rt.num_sms * 8);
 		cudaEvent_t ev;
 		launch_begin(rt, KC_FUSED, &ev);
-		k_sv_pass<<<grid, SV_TPB, 0, rt.stream>>>(src, dst, passes[p], gates_of(passes[p].first, passes[p].K));
+		k_sv_pass<T><<<grid, SV_TPB, 0, rt.stream>>>(src, dst, passes[p], gates_of(passes[p].first, passes[p].K));
 		launch_end(rt, KC_FUSED, ev);
 		if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 		src = dst;
 	}
 	return OK;
+}
+
+// gates of the longest chain in which each shares a wire with the next
+static int longest_chain(int L, int ngates, const int* wires)
+{
+	std::vector<int> depth(L, 0);
+	int most = 0;
+	for (int k = 0; k < ngates; k++) {
+		int &i = depth[wires[2 * k]], &j = depth[wires[2 * k + 1]];
+		i = j = std::max(i, j) + 1;
+		most = std::max(most, i);
+	}
+	return most;
+}
+
+// out = C in for one statevector (complex128), maxk gates per pass: tiles of consecutive gates, or layer
+// passes of gates on wires of their own, reordered where they commute.  A layer pass is the cheaper one
+// (a tile takes copies of 256 bytes and a shared-memory round trip per gate), but a circuit whose gates share
+// wires needs more of them: never fewer than its longest chain.  Up to 2^22 amplitudes both states lie in L2
+// and a tile pass costs 2 to 2.5 layer passes, and the first one a few more (the status word); beyond, 1.7:
+//   L = 27: 1.19-1.37 ms a tile pass, 0.71-0.92 ms a layer pass.  64 gates on random pairs 21.4 ms in 16 tile
+//   passes, 15.5 ms in 18 layer passes; 16 gates on 8 wires 4.93 ms (4) against 6.04 ms (8);
+//   L = 24, 8 gates on random pairs 0.34 ms (2) against 0.40 ms (4), 16 gates 0.75 ms (4) against 0.53 ms (5);
+//   L = 16: 16 gates on 5 wires 69 us (4) against 89 us (13), on 8 wires 74 us (4) against 59 us (8);
+//   40 gates on 8 wires (10 and 22 passes) L = 12: 126 us against 140 us, L = 14: 141 us against 140 us.
+// States of one or two layer tiles (L = 10, 11) take the small tiles: 40 gates on 11 wires 58 us (10) against
+// 115 us (17).
+int apply_circuit_fused_device(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
+                               const double2* d_in, double2* d_out, int maxk)
+{
+	const int tiles = (ngates + maxk - 1) / maxk;
+	// most layer passes that are as fast as the tiles
+	const int most = L < 12 ? 0 : L < 14 ? 2 * tiles + 1 : L <= 22 ? 2 * tiles + 2 : 17 * tiles / 10;
+	std::vector<std::vector<int>> passes;
+	if (longest_chain(L, ngates, wires) <= most) passes = reordered_passes(L, ngates, wires, maxk);
+	if (passes.empty() || (int)passes.size() > most) {
+		const int ret = apply_circuit_fused_t<double>(rt, L, ngates, gates, wires, d_in, d_out, maxk);
+		if (ret != E_ALLOC) return ret;
+		// (no room for a second state: layer passes need none)
+		if (passes.empty()) passes = reordered_passes(L, ngates, wires, maxk);
+	}
+	return circuit_apply_passes(rt, L, passes, gates, wires, d_in, d_out);
+}
+
+int apply_circuit_fused_device_c64(Runtime& rt, int L, int ngates, const double2* gates, const int* wires,
+                                   const float2* d_in, float2* d_out, int maxk)
+{
+	return apply_circuit_fused_t<float>(rt, L, ngates, gates, wires, d_in, d_out, maxk);
 }
 
 }  // namespace rqc
