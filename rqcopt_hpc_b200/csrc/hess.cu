@@ -1198,7 +1198,7 @@ struct LayerSweep
 	}
 
 	// partial-sum slots for chunks of up to K amplitudes per state: enough splits to fill the
-	// GPU (three blocks of four warps per SM), none shorter than two runs per warp
+	// GPU (three blocks of four warps per SM), of one run per warp at least
 	int init(int64_t K)
 	{
 		static bool smem_set = false;
@@ -1210,7 +1210,7 @@ struct LayerSweep
 		parts.resize(nl);
 		for (int a = 0; a < nl; a++) {
 			const int ntile = hess ? (16 * (a + 1) + 1 + GN - 1) / GN : 1;
-			const int64_t fill = (3 * (int64_t)rt.num_sms + ntile - 1) / ntile, most = K / (GRUN * GW * 2);
+			const int64_t fill = (3 * (int64_t)rt.num_sms + ntile - 1) / ntile, most = (K + GRUN * GW - 1) / (GRUN * GW);
 			most_tiles = std::max(most_tiles, ntile);
 			parts[a] = {off, (int)std::max<int64_t>(1, std::min(fill, most)), ntile};
 			off += (int64_t)ntile * parts[a].nsplit * GSLOT;
@@ -1290,6 +1290,15 @@ struct LayerSweep
 	}
 };
 
+// Hessians of so few amplitudes that either sweep waits for its launches: the layer sweep makes five a layer,
+// of which the product takes longer with every tangent tile, the general sweep two a gate and one a layer, so
+// it is the faster one for long circuits on few wires; with more columns its blocks lose that again.  General
+// against layer sweep: L = 4, 8 layers, all 16 columns 334 us and 388 us, 128 samples 431 us and 422 us; 5
+// layers, all columns 266 us and 265 us.  L = 6, one sample: 8 layers 380 us and 420 us, 6 layers 322 us and
+// 336 us, 5 layers 295 us and 296 us; 8 layers, 8 samples 428 us and 422 us.  L = 8, 10 layers, one sample
+// 530 us and 520 us.
+bool latency_bound(int L, int nl, int64_t ncols) { return nl >= L / 2 + 4 && ncols <= (int64_t)(1 << 14) >> (2 * L); }
+
 // States of the layer sweep per column: psi and phi at every layer's output, 16 tangents per
 // layer (before that two scratch states of the target), 16 cotangent states, the sample states.
 // (The general sweep holds fewer for short circuits: 16 nl + 2 G + 2 up to L = 12.)
@@ -1356,11 +1365,12 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	const int L = c.L, nl = c.nlayers;
 	if (L < 2 || L % 2 || nl < 1) return E_ARG;
 	if (samp && samp->nsamples < 1) return E_ARG;
-	const size_t layer_bytes = layer_column_bytes(L, nl, samp != nullptr);
-	if (layer_sweep_ok(c) && layer_bytes <= workspace_budget(rt, layer_bytes)) return hessian_layers(rt, c, t, d_rec, samp);
 	const int per = L / 2, G = nl * per;
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ncols = samp ? samp->nsamples : (c.columns ? c.ncolumns : N);   // basis columns, or sample states
+	const size_t layer_bytes = layer_column_bytes(L, nl, samp != nullptr);
+	if (layer_sweep_ok(c) && !latency_bound(L, nl, ncols) && layer_bytes <= workspace_budget(rt, layer_bytes))
+		return hessian_layers(rt, c, t, d_rec, samp);
 	// layer kernel (shared-memory tiles) up to L = 12, one kernel per gate beyond
 	const bool layered = L <= 12 && per <= HMAXPER;
 	// states per column: phi_q of every gate, psi_q of every gate (layered) or two psi
@@ -1473,10 +1483,10 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	// the tangents (Hessian only)
 	const int64_t layer_states = 1 + 2 * nl + 16 + (hess ? 16 * (int64_t)nl : 0);
 	const size_t layer_bytes = (size_t)layer_states * N * sizeof(double2);
-	const bool sweep = layer_sweep_ok(c) && layer_bytes <= workspace_budget(rt, layer_bytes);
+	const int64_t ncols = c.columns ? c.ncolumns : s;
+	const bool sweep = layer_sweep_ok(c) && !(hess && latency_bound(L, nl, ncols)) && layer_bytes <= workspace_budget(rt, layer_bytes);
 	const int64_t nstates = sweep ? layer_states : G + (layered ? G : 3) + 1 + (hess ? 16 * (int64_t)nl : 0);
 	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
-	const int64_t ncols = c.columns ? c.ncolumns : s;
 	int64_t C = ncols;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
 	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
