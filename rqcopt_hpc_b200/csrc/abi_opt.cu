@@ -656,7 +656,7 @@ void run_optimizer(const char* fn, Problem& pb, linear_func ufunc, void* udata, 
 	}
 	Runtime* rt = runtime();
 	if (!rt) { set_last_error(E_CUDA); return; }
-	if (int ret = th.to_device(*rt)) { set_last_error(ret); return; }
+	if (int ret = th.to_device(*rt, !hmat)) { set_last_error(ret); return; }
 	// the drivers disable the per-iteration callback (src/brickwall_opt.c:141-143)
 	params->g_func = NULL;
 	params->g_data = NULL;

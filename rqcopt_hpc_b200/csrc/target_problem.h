@@ -39,8 +39,9 @@ struct TargetHolder
 	int dense_L = 0;
 	bool set(linear_func ufunc, void* udata, int L);
 	// Copies a dense target to the device for the evaluations of this call (up to 1 GiB and within
-	// the workspace limit; others stay a host callback, one column at a time).
-	int to_device(Runtime& rt);
+	// the workspace limit; others stay a host callback, one column at a time).  ranged: the call sums
+	// over the column range set by the caller.
+	int to_device(Runtime& rt, bool ranged = false);
 };
 
 // Sum over the orbits of the wire relabellings that circuit and target share, instead of
