@@ -34,8 +34,19 @@ constexpr int SMALL_THREADS = 384;     // most threads per block (three roles of
 constexpr int SMALL_MAX_L = 10;        // eight tiles of a column: 128 KB
 constexpr int SMALL_MAX_UNITS = 128;   // gate tables in shared memory: 512 B per unit
 constexpr size_t SMALL_SMEM = 200 * 1024;
-// Amplitude x gate updates up to which an evaluation runs here (512 MB of scratch); beyond,
-// the pass engine has enough work per launch.
+// Amplitudes of all columns up to which an evaluation runs here: a block takes its column at the rate of its
+// chain of barriers, and beyond a wave or two of blocks the pass engine is the faster one; HVPs, with twice
+// the tiles a block, from half as many.  Small engine against passes: L = 8, 256 columns, 60 gates f 72 and
+// 167 us, gradient 140 and 346 us, HVP 271 and 461 us; L = 9, 512 columns, 40 gates 99 and 146, 235 and 279, 483
+// and 419 us; in 256 paired columns gradient 130 and 263, HVP 260 and 344 us; L = 10, 208 columns, 45 gates 127
+// and 214, 232 and 356, 467 and 496 us; 512 paired columns, 30 gates gradient 275 and 302, HVP 586 and 481 us;
+// 1024 columns, 30 gates 187 and 165, 472 and 386, 1007 and 698 us.
+constexpr int64_t SMALL_MAX_AMPS = 1 << 19, SMALL_MAX_AMPS_HVP = (1 << 18) - 1;
+// Beyond, evaluations of so few gates (the target's included) that launches weigh more: HVP of 12 gates at L = 9
+// 162 and 169 us.  On 1024 columns up to nine gates stay in two launches though the passes are a little faster
+// (seven gates: f 89 and 82 us, gradient 137 and 127 us, HVP 244 and 195 us).
+constexpr int SMALL_FEW_GATES = 15, SMALL_FEW_GATES_1024 = 9;
+// Amplitude x gate updates: 512 MB of states
 constexpr double SMALL_MAX_WORK = 1 << 24;
 constexpr int SLOT = 64;               // doubles per unit and block: row q of dG (8), of HZ (8)
 
@@ -490,7 +501,12 @@ bool SmallEval::fits(Runtime& rt, const Problem& pb, const TargetHolder& th, int
 	if (rt.pin_gpp || rt.pin_chunk || rt.pin_recon || rt.col_begin != 0 || rt.col_end != 0) return false;
 	if (pb.L < 2 || pb.L > SMALL_MAX_L || pb.nunits > SMALL_MAX_UNITS || ncols < 1) return false;
 	if (th.spec.ufunc || (!th.spec.dense && th.spec.ngates < 1)) return false;
-	if ((double)ncols * (double)(1 << pb.L) * (pb.G + th.spec.ngates) >= SMALL_MAX_WORK) return false;
+	const int64_t amps = ncols << pb.L;
+	const int gates = pb.G + th.spec.ngates;
+	if ((double)amps * gates >= SMALL_MAX_WORK) return false;
+	if (amps > (mode == EVAL_HVP ? SMALL_MAX_AMPS_HVP : SMALL_MAX_AMPS) &&
+	    gates > (amps <= SMALL_MAX_AMPS ? SMALL_FEW_GATES : SMALL_FEW_GATES_1024))
+		return false;
 	if (small_smem(pb.L, pb.nunits, pb.G, th.spec.ngates, true) > SMALL_SMEM) return false;
 	// the pass engine splits its columns where the workspace does not hold all of them
 	const size_t states = states_bytes(pb.L, pb.G, ncols, mode);
