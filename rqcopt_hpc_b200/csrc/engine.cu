@@ -455,7 +455,8 @@ static int launch_reverse(Runtime& rt, bool tan, bool first, bool last, const cp
 template <typename T>
 static int partial_grid(const Runtime& rt)
 {
-	static int per_sm = 0;
+	static PerDevice blocks;
+	int& per_sm = blocks[rt];
 	if (per_sm == 0) per_sm = std::max(1, std::min(blocks_per_sm(k_reverse<T, true, false, false>),
 	                                                blocks_per_sm(k_forward<T, false, true>)));
 	return rt.num_sms * per_sm;

@@ -2421,7 +2421,8 @@ template <typename T, bool TAN, int IN, int OUT>
 int launch_fwd(Runtime& rt, const cplx<T>* psi, const cplx<T>* dpsi, cplx<T>* psi_o, cplx<T>* dpsi_o, const cplx<T>* phi,
                const PassGeom& pg, const PassGates<T>& gates, double2* fpart, int fgrid)
 {
-	static int per_sm = 0;
+	static PerDevice blocks;
+	int& per_sm = blocks[rt];
 	if constexpr (std::is_same<T, double>::value) {
 		if (!per_sm) {
 			int ret = prepare(k8_fwd<TAN, IN, OUT>, FWD_TILE_BYTES, &per_sm, NT8F);
@@ -2431,7 +2432,8 @@ int launch_fwd(Runtime& rt, const cplx<T>* psi, const cplx<T>* dpsi, cplx<T>* ps
 		const int grid = OUT >= 2 ? fgrid : (int)std::max<int64_t>(1, std::min<int64_t>(args.ntiles, (int64_t)rt.num_sms * per_sm));
 		RQC_LAUNCH3(rt, KC_FUSED, (k8_fwd<TAN, IN, OUT>), grid, NT8F, FWD_TILE_BYTES, psi, dpsi, psi_o, dpsi_o, phi, args, fpart);
 	} else if (rt.c64_ffma) {
-		static int per_sm7 = 0;
+		static PerDevice blocks7;
+		int& per_sm7 = blocks7[rt];
 		if (!per_sm7) {
 			int ret = prepare(k7_fwd<TAN, IN, OUT>, k7_fwd_smem(), &per_sm7, NT7);
 			if (ret) return ret;
@@ -2457,7 +2459,8 @@ int launch_rev(Runtime& rt, const cplx<T>* psi, const cplx<T>* dpsi, const cplx<
                double* scratch)
 {
 	const size_t smem = rev_smem<T>(pg.NB, pg.K, TAN);
-	static bool ready = false;
+	static PerDevice prepared;
+	int& ready = prepared[rt];
 	if constexpr (std::is_same<T, double>::value) {
 		if (!ready) {
 			int per_sm;
@@ -2499,7 +2502,8 @@ int launch_rev5(Runtime& rt, const float2* psi, const float2* dpsi, const float2
                 float2* dphi_o, const PassGeom& pg, const PassGates<float>& gates, const PassW<float>& wg, double* part,
                 int nblk, double* scratch)
 {
-	static bool ready = false;
+	static PerDevice prepared;
+	int& ready = prepared[rt];
 	if (!ready) {
 		int per_sm;
 		int ret = prepare(k5_rev<TAN, FIRST, LAST>, k5_rev_smem(TAN), &per_sm, NT5);
@@ -2530,7 +2534,8 @@ int launch_rev8(Runtime& rt, const double2* psi, const double2* dpsi, const doub
                 double2* phi_o, double2* dphi_o, const PassGeom& pg, const PassGates<double>& gates, const PassAdj& adj, double* part,
                 int nblk)
 {
-	static bool ready = false;
+	static PerDevice prepared;
+	int& ready = prepared[rt];
 	if (!ready) {
 		int per_sm;
 		int ret = prepare(k8_rev<TAN, FIRST, LAST>, rev_tile_bytes(TAN), &per_sm, NT8R);
@@ -2570,7 +2575,8 @@ int launch_rev7(Runtime& rt, const float2* psi, const float2* dpsi, const float2
                 float2* dphi_o, const PassGeom& pg, const PassGates<float>& gates, const PassW<float>& wg, double* part,
                 int nblk)
 {
-	static bool ready = false;
+	static PerDevice prepared;
+	int& ready = prepared[rt];
 	if (!ready) {
 		int per_sm;
 		int ret = prepare(k7_rev<TAN, FIRST, LAST>, k7_rev_smem(), &per_sm, NT7);

@@ -470,7 +470,8 @@ size_t small_smem(int L, int nunits, int G, int Gt, bool tan)
 template <int MODE, int ROLES>
 int launch_small_as(Runtime& rt, const SmallArgs& a, int blocks, int nb)
 {
-	static bool ready = false;
+	static PerDevice prepared;
+	int& ready = prepared[rt];
 	if (!ready) {
 		if (int e = RQC_CUDA(cudaFuncSetAttribute(k_small<MODE, ROLES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		                                          (int)SMALL_SMEM)))

@@ -1118,7 +1118,8 @@ struct Sweep
 	int layer(int a, const double2* psi, int basis, const double2* phi, double2* tan, int64_t ncols,
 	          int64_t sstride, bool with_f)
 	{
-		static bool smem_set = false;
+		static PerDevice prepared;
+		int& smem_set = prepared[rt];
 		if (!smem_set) {
 			if (int e = RQC_CUDA(cudaFuncSetAttribute(k_hlayer, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			                                          (int)(HTILE * sizeof(double2)))))
@@ -1201,7 +1202,8 @@ struct LayerSweep
 	// GPU (three blocks of four warps per SM), of one run per warp at least
 	int init(int64_t K)
 	{
-		static bool smem_set = false;
+		static PerDevice prepared;
+		int& smem_set = prepared[rt];
 		if (!smem_set) {
 			if (int e = RQC_CUDA(cudaFuncSetAttribute(k_hgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, GSMEM))) return e;
 			smem_set = true;

@@ -156,7 +156,8 @@ template <int TB, int IN, int OUT>
 int launch(Runtime& rt, const double2* in, double2* out, const PassArgs& a)
 {
 	constexpr int smem = (1 << TB) * (int)sizeof(double2);
-	static int per_sm = 0;
+	static PerDevice blocks;
+	int& per_sm = blocks[rt];
 	if (!per_sm) {
 		if (int e = RQC_CUDA(cudaFuncSetAttribute(k_lpass<TB, IN, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
 			return e;

@@ -120,6 +120,14 @@ int span_in(Runtime& rt, const void* p, size_t bytes, int slot, DeviceSpan& s);
 int span_out(Runtime& rt, void* p, size_t bytes, int slot, DeviceSpan& s);
 int span_finish(Runtime& rt, DeviceSpan& s);   // copy back if staged (async on rt.stream)
 
+// What a kernel's first launch finds out or sets (shared memory allowed, blocks per SM; 0 before), for
+// each device of the process: kernel attributes belong to a device.
+struct PerDevice
+{
+	int v[64] = {0};
+	int& operator[](const Runtime& rt) { return v[rt.device & 63]; }
+};
+
 // synchronise the stream and fold pending kernel timings; returns 0 or E_CUDA
 int sync(Runtime& rt);
 

@@ -338,7 +338,8 @@ int apply_circuit_fused_t(Runtime& rt, int L, int ngates, const double2* gates, 
 	if (bulk) {
 		std::vector<SvTile> passes = sv_tile_schedule<T>(L, ngates, wires, maxk);
 		P = (int)passes.size();
-		static int per_sm = 0;
+		static PerDevice blocks;
+		int& per_sm = blocks[rt];
 		const size_t smem = SVT_TILE_BYTES + SVT_MAXRUNS * sizeof(int64_t) + 16 + SV_MAXK * sizeof(Gate4<T>);
 		if (!per_sm) {
 			if ((ret = RQC_CUDA(cudaFuncSetAttribute(k_sv_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))))
