@@ -759,7 +759,7 @@ int gate_backward_device(Runtime& rt, int L, const double2* gate, int i, int j, 
 }
 
 int target_columns_device(Runtime& rt, const TargetSpec& t, int L, const ColumnSource& src, int64_t ncols, double2* phi,
-                          double2* p0, double2* p1)
+                          double2* scratch)
 {
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ngroups = ncols * (N / 4);
@@ -781,19 +781,19 @@ int target_columns_device(Runtime& rt, const TargetSpec& t, int L, const ColumnS
 				return E_UFUNC;
 			}
 		}
-		if ((ret = RQC_CUDA(cudaMemcpyAsync(p0, hcols, ncols * N * sizeof(double2), cudaMemcpyHostToDevice, rt.stream))))
+		if ((ret = RQC_CUDA(cudaMemcpyAsync(scratch, hcols, ncols * N * sizeof(double2), cudaMemcpyHostToDevice, rt.stream))))
 			return ret;
-		k_conj_neg<double><<<grid_for(rt, ncols * N, 8), TPB, 0, rt.stream>>>(p0, phi, ncols * N);
+		k_conj_neg<double><<<grid_for(rt, ncols * N, 8), TPB, 0, rt.stream>>>(scratch, phi, ncols * N);
 		rt.launches++;
 		if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 		// the pinned buffer is reused by the next chunk
 		return RQC_CUDA(cudaStreamSynchronize(rt.stream));
 	}
-	return circuit_apply(rt, L, t.ngates, t.gates, t.wires, nullptr, phi, p0, ncols, &src, true);
+	return circuit_apply(rt, L, t.ngates, t.gates, t.wires, nullptr, phi, scratch, ncols, &src, true);
 }
 
 int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2* states, int64_t ncols, double2* phi,
-                         double2* p0, double2* p1)
+                         double2* scratch)
 {
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ngroups = ncols * (N / 4);
@@ -821,14 +821,14 @@ int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2*
 				return E_UFUNC;
 			}
 		}
-		if ((ret = RQC_CUDA(cudaMemcpyAsync(p0, hout, ncols * N * sizeof(double2), cudaMemcpyHostToDevice, rt.stream))))
+		if ((ret = RQC_CUDA(cudaMemcpyAsync(scratch, hout, ncols * N * sizeof(double2), cudaMemcpyHostToDevice, rt.stream))))
 			return ret;
-		k_conj_neg<double><<<grid_for(rt, ncols * N, 8), TPB, 0, rt.stream>>>(p0, phi, ncols * N);
+		k_conj_neg<double><<<grid_for(rt, ncols * N, 8), TPB, 0, rt.stream>>>(scratch, phi, ncols * N);
 		rt.launches++;
 		if ((ret = RQC_CUDA(cudaGetLastError()))) return ret;
 		return RQC_CUDA(cudaStreamSynchronize(rt.stream));
 	}
-	return circuit_apply(rt, L, t.ngates, t.gates, t.wires, states, phi, p0, ncols, nullptr, true);
+	return circuit_apply(rt, L, t.ngates, t.gates, t.wires, states, phi, scratch, ncols, nullptr, true);
 }
 
 int add_device(Runtime& rt, const double2* a, const double2* b, double2* c, long n)

@@ -91,12 +91,12 @@ int column_passes_device(Runtime& rt, int L, int ngates, const double2* gates, c
                          double2* d_hess);
 // Target columns of one chunk: phi[c] = -conj(U e_c), e_c column c of src, for c < ncols
 // (states of 2^L amplitudes one after another), through the device circuit of t or its host
-// callback (plain basis states only); p0 and p1 are two chunk-sized scratch arrays.
+// callback (plain basis states only); scratch: another array of that size.
 int target_columns_device(Runtime& rt, const TargetSpec& t, int L, const ColumnSource& src, int64_t ncols, double2* phi,
-                          double2* p0, double2* p1);
+                          double2* scratch);
 // The same for given input states: phi[c] = -conj(U states[c]).
 int target_states_device(Runtime& rt, const TargetSpec& t, int L, const double2* states, int64_t ncols, double2* phi,
-                         double2* p0, double2* p1);
+                         double2* scratch);
 // c = a + b elementwise, n complex entries
 int add_device(Runtime& rt, const double2* a, const double2* b, double2* c, long n);
 

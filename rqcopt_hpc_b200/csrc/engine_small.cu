@@ -55,7 +55,6 @@ struct SmallArgs
 	int L, G, per, nunits, Gt;
 	int cb;                  // columns per block
 	int real;                // paired real columns: clear the imaginary parts of the sums
-	int64_t ncols;
 	ColumnSource src;
 	const double2* ug;       // [nunits][16]
 	const double2* uz;
@@ -578,7 +577,6 @@ int SmallEval::eval(Runtime& rt, int mode, const double2* ugates, const double2*
 	a.Gt = Gt_;
 	a.cb = columns_per_block(L_);
 	a.real = rt.real_pairs;
-	a.ncols = ncols_;
 	a.src = src_;
 	a.ug = ugates ? ugates : ug_;
 	a.uz = udirs ? udirs : uz_;

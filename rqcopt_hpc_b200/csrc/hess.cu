@@ -1302,7 +1302,7 @@ struct LayerSweep
 bool latency_bound(int L, int nl, int64_t ncols) { return nl >= L / 2 + 4 && ncols <= (int64_t)(1 << 14) >> (2 * L); }
 
 // States of the layer sweep per column: psi and phi at every layer's output, 16 tangents per
-// layer (before that two scratch states of the target), 16 cotangent states, the sample states.
+// layer (before that a scratch state of the target), 16 cotangent states, the sample states.
 // (The general sweep holds fewer for short circuits: 16 nl + 2 G + 2 up to L = 12.)
 size_t layer_column_bytes(int L, int nl, bool samp)
 {
@@ -1339,11 +1339,11 @@ int hessian_layers(Runtime& rt, const HessCircuit& c, const TargetSpec& t, doubl
 		src.end = ncols;
 		if (samp) {
 			if ((ret = haar_states_device(rt, *samp, L, b0, Cc, states))) return ret;
-			if ((ret = target_states_device(rt, t, L, states, Cc, last, tan, tan + K))) return ret;
+			if ((ret = target_states_device(rt, t, L, states, Cc, last, tan))) return ret;
 		} else {
 			ColumnSource tsrc = src;
 			tsrc.weighted = 1;
-			if ((ret = target_columns_device(rt, t, L, tsrc, Cc, last, tan, tan + K))) return ret;
+			if ((ret = target_columns_device(rt, t, L, tsrc, Cc, last, tan))) return ret;
 		}
 		if ((ret = sw.forward(samp ? states : nullptr, samp ? nullptr : &src, psi, Cc))) return ret;
 		if ((ret = sw.reverse(phi, Cc))) return ret;
@@ -1376,9 +1376,9 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	// layer kernel (shared-memory tiles) up to L = 12, one kernel per gate beyond
 	const bool layered = L <= 12 && per <= HMAXPER;
 	// states per column: phi_q of every gate, psi_q of every gate (layered) or two psi
-	// buffers, 16 tangents per layer; sampled: the sample states and two target scratch
-	// states besides
-	const int64_t nstates = G + (layered ? G : 2) + 16 * (int64_t)nl + (samp ? (layered ? 2 : 3) : 0);
+	// buffers, 16 tangents per layer; sampled: the sample states (layered: psi_0) and a target
+	// scratch state besides
+	const int64_t nstates = G + (layered ? G : 2) + 16 * (int64_t)nl + (samp ? (layered ? 1 : 2) : 0);
 	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
 	int64_t C = ncols;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
@@ -1397,8 +1397,8 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	double2* psi = phi + (int64_t)G * cs;                              // layered: psi_q at psi + q cs
 	double2* tan = phi + (int64_t)(G + (layered ? G : 2)) * cs;
 	double2* extra = tan + 16 * (int64_t)nl * cs;                       // sampled: scratch (and states)
-	double2* states = samp ? (layered ? psi : extra + 2 * cs) : nullptr;
-	double2* tq[2] = { samp ? extra : P[0], samp ? extra + cs : P[1] };   // target scratch
+	double2* states = samp ? (layered ? psi : extra + cs) : nullptr;
+	double2* tscratch = samp ? extra : P[0];                            // target scratch
 	auto phi_at = [&](int q) { return phi + (int64_t)q * cs; };
 	auto psi_at = [&](int q) { return psi + (int64_t)q * cs; };
 
@@ -1415,8 +1415,8 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 		tsrc.weighted = 1;
 		if (samp) {
 			if ((ret = haar_states_device(rt, *samp, L, b0, Cc, states))) return ret;
-			if ((ret = target_states_device(rt, t, L, states, Cc, phi_at(G - 1), tq[0], tq[1]))) return ret;
-		} else if ((ret = target_columns_device(rt, t, L, tsrc, Cc, phi_at(G - 1), tq[0], tq[1]))) {
+			if ((ret = target_states_device(rt, t, L, states, Cc, phi_at(G - 1), tscratch))) return ret;
+		} else if ((ret = target_columns_device(rt, t, L, tsrc, Cc, phi_at(G - 1), tscratch))) {
 			return ret;
 		}
 		if ((ret = sw.reverse_chain(phi_at, ngroups, nullptr))) return ret;
@@ -1506,17 +1506,16 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	auto psi_at = [&](int q) { return psi + (int64_t)q * cs; };
 	// per evaluation: -conj(H e_b) for all b, target scratch, Jacobian rows, Gauss-Newton parts, f parts
 	const int nres = rt.num_sms * 2;
-	const size_t abytes = (3 * (size_t)s * s + (hess ? (size_t)m * C * s + (size_t)m * m : 0) + nres) * sizeof(double2);
+	const size_t abytes = (2 * (size_t)s * s + (hess ? (size_t)m * C * s + (size_t)m * m : 0) + nres) * sizeof(double2);
 	if ((ret = ensure_device(rt.arrays, abytes))) return ret;
 	double2* hneg = static_cast<double2*>(rt.arrays.ptr);
-	double2* sc0 = hneg + s * s;
-	double2* sc1 = sc0 + s * s;
-	double2* jac = sc1 + s * s;
+	double2* scratch = hneg + s * s;
+	double2* jac = scratch + s * s;
 	double2* part2 = hess ? jac + (size_t)m * C * s : jac;
 	double2* fres = hess ? part2 + (size_t)m * m : jac;
 	if ((ret = RQC_CUDA(cudaMemsetAsync(fres, 0, nres * sizeof(double2), rt.stream)))) return ret;
 	if (hess && (ret = RQC_CUDA(cudaMemsetAsync(part2, 0, (size_t)m * m * sizeof(double2), rt.stream)))) return ret;
-	if ((ret = target_columns_device(rt, t, half, ColumnSource{}, s, hneg, sc0, sc1))) return ret;
+	if ((ret = target_columns_device(rt, t, half, ColumnSource{}, s, hneg, scratch))) return ret;
 
 	if (sweep) {
 		LayerSweep ls(rt, c, hess);

@@ -176,20 +176,19 @@ int sampled_f_device(Runtime& rt, int L, int ngates, const double2* gates, const
 {
 	const int64_t N = (int64_t)1 << L;
 	if (sp.nsamples < 1) return E_ARG;
-	// chunk states: samples, target columns, C psi, two target scratch states
-	const size_t col_bytes = 5 * (size_t)N * sizeof(double2);
+	// chunk states: samples, target columns, C psi, a target scratch state
+	const size_t col_bytes = 4 * (size_t)N * sizeof(double2);
 	int64_t C = sp.nsamples;
 	if (rt.column_chunk > 0) C = std::min<int64_t>(C, rt.column_chunk);
 	if (t.ufunc) C = std::min<int64_t>(C, std::max<int64_t>(1, ((int64_t)256 << 20) / (N * 16)));
 	C = std::min<int64_t>(C, (int64_t)(workspace_budget(rt, C * col_bytes) / col_bytes));
 	if (C < 1) return E_ALLOC;
-	int ret = ensure_device(rt.work, 5 * (size_t)C * N * sizeof(double2));
+	int ret = ensure_device(rt.work, (size_t)C * col_bytes);
 	if (ret) return ret;
 	double2* states = reinterpret_cast<double2*>(rt.work.ptr);
 	double2* phi = states + C * N;
 	double2* cpsi = phi + C * N;
-	double2* p0 = cpsi + C * N;
-	double2* p1 = p0 + C * N;
+	double2* scratch = cpsi + C * N;
 	const int nblk = rt.num_sms * 4;
 	if ((ret = ensure_device(rt.partials, (size_t)nblk * sizeof(double2)))) return ret;
 	double2* fpart = reinterpret_cast<double2*>(rt.partials.ptr);
@@ -197,7 +196,7 @@ int sampled_f_device(Runtime& rt, int L, int ngates, const double2* gates, const
 	for (int64_t s0 = 0; s0 < sp.nsamples; s0 += C) {
 		const int64_t Cc = std::min(C, sp.nsamples - s0);
 		if ((ret = haar_states_device(rt, sp, L, s0, Cc, states))) return ret;
-		if ((ret = target_states_device(rt, t, L, states, Cc, phi, p0, p1))) return ret;
+		if ((ret = target_states_device(rt, t, L, states, Cc, phi, scratch))) return ret;
 		if ((ret = apply_circuit_device(rt, L, ngates, gates, wires, states, cpsi, (long)Cc))) return ret;
 		k_fdot<<<nblk, HTPB, 0, rt.stream>>>(phi, cpsi, Cc * N, fpart);
 		rt.launches++;
