@@ -260,6 +260,7 @@ def gate_throughput(gpu, torch, L=28, G=256, seed=20):
             run(gates, wires, psi, out)   # warm-up
             torch.cuda.synchronize()
             e = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
+            gpu.reset_launch_count()
             e[0].record(stream)
             run(gates, wires, psi, out)
             e[1].record(stream)
@@ -267,7 +268,7 @@ def gate_throughput(gpu, torch, L=28, G=256, seed=20):
             e[2].record(stream)
             torch.cuda.synchronize()
             t_f, t_b = e[0].elapsed_time(e[1]), e[1].elapsed_time(e[2])
-            trips = G if gpp == 1 else -(-G // gpp)
+            trips = gpu.launch_count() / 2   # a launch is one read and one write of the state
             err = float(torch.max(torch.abs(back - psi)))
             r[f"gates_per_round_trip_{gpp}"] = {
                 "forward_ms": t_f, "backward_ms": t_b, "round_trips": trips,
@@ -476,7 +477,7 @@ def hmat_path(gpu, torch, stream, hbm_peak, with_reference=True, steps=3, fp64_p
     sampled()
     _, wall, dev_ms, hs_ms, hs_n, launches = timed(sampled, steps)
     r4 = {"workload": f"f + gradient vector + Hessian matrix estimated from {ns} Haar-random states, brickwall L={L} "
-                      f"depth {depth} vs brickwall target depth {tdepth} (per-gate sweep)",
+                      f"depth {depth} vs brickwall target depth {tdepth}",
           "samples_per_s_e2e": ns / wall, "ms_per_call": wall * 1e3, "sweep_ms": hs_ms, "gpu_launches": launches,
           "roofline": roofline(hess_model(L, depth, False), ns, L, hs_ms, hs_n)}
     out["sampling_L14"] = r4

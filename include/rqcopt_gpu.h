@@ -456,14 +456,18 @@ enum rqcopt_precision
 	                                complex128 once the gradient norm falls below the
 	                                refinement threshold */
 	RQCOPT_PRECISION_C64   = 2   /* complex64 passes, FP64 sums, no refinement */
+	/* complex128 sums of a brickwall against a brickwall take one basis column per orbit of the
+	 * wire relabellings that keep all layers, weighted by the orbit's size (L/2 times fewer for a
+	 * periodic brickwall); complex64 sums take every column, over which their rounding averages */
 };
 int rqcopt_gpu_set_precision(int precision);
 int rqcopt_gpu_get_precision(void);
 /* gradient-norm threshold for the switch from complex64 to complex128 (default 1e-5) */
 void rqcopt_gpu_set_refine_threshold(double gnorm);
 
-/* upper bound on the device memory (bytes) the evaluation engine may use for
- * column chunks and caches; 0 selects 75 % of the free memory at first use */
+/* upper bound on the device memory (bytes) the engines may use for column chunks, caches and
+ * the copy of a dense target; 0 selects 75 % of the free memory.  Calls that do not fit run in
+ * the form that needs less, or fail with -1 where one column does not */
 void rqcopt_gpu_set_workspace_limit(size_t bytes);
 /* number of basis columns per chunk; 0 selects it from the workspace limit */
 void rqcopt_gpu_set_column_chunk(long columns);
@@ -506,10 +510,10 @@ int rqcopt_gpu_last_config(int* gates_per_pass, long* column_chunk, int* reconst
  * B200.  Both meet the complex64 bar; fixing it keeps it for the autotuner. */
 void rqcopt_gpu_set_c64_fp32_pipe(int on);
 
-/* complex128 reverse passes over fused gates: 1 (default) rebuilds the state entering
- * each gate from the pass output with the adjoint gate when every gate is unitary to
- * 1e-14 (four tiles in shared memory, two blocks per SM); 0 recomputes those states
- * from the pass input.  Both give the same sums to rounding. */
+/* complex128 reverse passes over fused gates: 1 (default) takes the sums at the pass output
+ * (and moves states back with adjoint gates where gates of a pass share wires) when every
+ * gate is unitary to 1e-14; 0 recomputes the state entering each gate from the pass input.
+ * Both give the same sums to rounding. */
 void rqcopt_gpu_set_reconstruct(int on);
 
 /* last error recorded by a void function (0 if none); reading clears it */
