@@ -1298,10 +1298,14 @@ struct LayerSweep
 // of which the product takes longer with every tangent tile, the general sweep two a gate and one a layer, so
 // it is the faster one for long circuits on few wires; with more columns its blocks lose that again.  General
 // against layer sweep: L = 4, 8 layers, all 16 columns 334 us and 388 us, 128 samples 431 us and 422 us; 5
-// layers, all columns 266 us and 265 us.  L = 6, one sample: 8 layers 380 us and 420 us, 6 layers 322 us and
+// layers, all columns 244 us and 260 us, 24 samples 287 us and 273 us.  L = 6, one sample: 8 layers 380 us and 420 us, 6 layers 322 us and
 // 336 us, 5 layers 295 us and 296 us; 8 layers, 8 samples 428 us and 422 us.  L = 8, 10 layers, one sample
 // 530 us and 520 us.
-bool latency_bound(int L, int nl, int64_t ncols) { return nl >= L / 2 + 4 && ncols <= (int64_t)(1 << 14) >> (2 * L); }
+bool latency_bound(int L, int nl, int64_t ncols)
+{
+	const int more = nl - L / 2;   // layers more than a layer has gates
+	return ncols <= (int64_t)(more >= 4 ? 1 << 14 : more == 3 ? 1 << 12 : 0) >> (2 * L);
+}
 
 // States of the layer sweep per column: psi and phi at every layer's output, 16 tangents per
 // layer (before that a scratch state of the target), 16 cotangent states, the sample states.

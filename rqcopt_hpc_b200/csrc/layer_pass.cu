@@ -352,31 +352,4 @@ int circuit_apply_passes(Runtime& rt, int L, const std::vector<std::vector<int>>
 	return OK;
 }
 
-int circuit_apply(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, const double2* in, double2* out,
-                  double2* scratch, int64_t ncols, const ColumnSource* columns, bool neg_conj)
-{
-	// runs of gates on wires of their own
-	std::vector<std::vector<LayerGate>> runs;
-	uint64_t used = 0;
-	for (int k = 0; k < ngates; k++) {
-		const int i = wires[2 * k], j = wires[2 * k + 1];
-		const uint64_t w = ((uint64_t)1 << i) | ((uint64_t)1 << j);
-		if (runs.empty() || (used & w)) {
-			runs.emplace_back();
-			used = 0;
-		}
-		runs.back().push_back({gates + 16 * (size_t)k, i, j});
-		used |= w;
-	}
-	const int n = (int)runs.size();
-	const double2* src = in;
-	for (int r = 0; r < n; r++) {
-		double2* dst = (n - 1 - r) % 2 == 0 ? out : scratch;
-		const bool last = r == n - 1;
-		if (int e = layer_apply(rt, L, runs[r], false, src, dst, ncols, r == 0 ? columns : nullptr, last && neg_conj)) return e;
-		src = dst;
-	}
-	return OK;
-}
-
 }  // namespace rqc

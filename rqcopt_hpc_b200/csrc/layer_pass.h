@@ -24,11 +24,6 @@ bool gates_disjoint(int L, const std::vector<LayerGate>& gates);
 int layer_apply(Runtime& rt, int L, const std::vector<LayerGate>& gates, bool transposed, const double2* in, double2* out,
                 int64_t ncols, const ColumnSource* columns = nullptr, bool neg_conj = false);
 
-// out = C in for a sequential circuit (host gates and wires): runs of consecutive gates on
-// wires of their own, a layer_apply each; scratch: another array of the size of out.
-int circuit_apply(Runtime& rt, int L, int ngates, const double2* gates, const int* wires, const double2* in, double2* out,
-                  double2* scratch, int64_t ncols, const ColumnSource* columns = nullptr, bool neg_conj = false);
-
 // The gates of a circuit in passes of up to `most` (<= 5; 4 measured best: a fifth leaves tiles short
 // runs) on wires of their own, reordered where they commute.
 std::vector<std::vector<int>> reordered_passes(int L, int ngates, const int* wires, int most);
