@@ -1295,17 +1295,13 @@ struct LayerSweep
 };
 
 // Hessians of so few amplitudes that either sweep waits for its launches: the layer sweep makes five a layer,
-// of which the product takes longer with every tangent tile, the general sweep two a gate and one a layer, so
-// it is the faster one for long circuits on few wires; with more columns its blocks lose that again.  General
-// against layer sweep: L = 4, 8 layers, all 16 columns 334 us and 388 us, 128 samples 431 us and 422 us; 5
-// layers, all columns 244 us and 260 us, 24 samples 287 us and 273 us.  L = 6, one sample: 8 layers 380 us and 420 us, 6 layers 322 us and
-// 336 us, 5 layers 295 us and 296 us; 8 layers, 8 samples 428 us and 422 us.  L = 8, 10 layers, one sample
-// 530 us and 520 us.
-bool latency_bound(int L, int nl, int64_t ncols)
-{
-	const int more = nl - L / 2;   // layers more than a layer has gates
-	return ncols <= (int64_t)(more >= 4 ? 1 << 14 : more == 3 ? 1 << 12 : 0) >> (2 * L);
-}
+// of which the product takes longer with every tangent tile, the general sweep two a gate and one a layer.
+// General against layer sweep (samples unless named): L = 4, 8 layers, 8: 268 us and 394 us, 128: 353 us and
+// 425 us, 512: 436 us and 435 us, all columns 257 us and 382 us; 2 layers, 8: 135 us and 170 us.  L = 6, 8 layers,
+// 4: 337 us and 432 us, 16: 403 us and 433 us, 64: 502 us and 446 us, one column per orbit (24) 417 us and
+// 421 us.  L = 8, 8 layers, 1: 399 us and 438 us, 2: 437 us and 437 us, 4: 485 us and 437 us.  L = 10, 8 layers,
+// 1: 566 us and 458 us.
+bool latency_bound(int L, int64_t ncols) { return L <= 8 && ncols <= (1 << 16) >> (2 * L); }
 
 // States of the layer sweep per column: psi and phi at every layer's output, 16 tangents per
 // layer (before that a scratch state of the target), 16 cotangent states, the sample states.
@@ -1377,7 +1373,7 @@ int hessian_target_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t
 	const int64_t N = (int64_t)1 << L;
 	const int64_t ncols = samp ? samp->nsamples : (c.columns ? c.ncolumns : N);   // basis columns, or sample states
 	const size_t layer_bytes = layer_column_bytes(L, nl, samp != nullptr);
-	if (layer_sweep_ok(c) && !latency_bound(L, nl, ncols) && layer_bytes <= workspace_budget(rt, layer_bytes))
+	if (layer_sweep_ok(c) && !latency_bound(L, ncols) && layer_bytes <= workspace_budget(rt, layer_bytes))
 		return hessian_layers(rt, c, t, d_rec, samp);
 	// layer kernel (shared-memory tiles) up to L = 12, one kernel per gate beyond
 	const bool layered = L <= 12 && per <= HMAXPER;
@@ -1492,7 +1488,7 @@ int blockenc_device(Runtime& rt, const HessCircuit& c, const TargetSpec& t, int 
 	const int64_t layer_states = 1 + 2 * nl + 16 + (hess ? 16 * (int64_t)nl : 0);
 	const size_t layer_bytes = (size_t)layer_states * N * sizeof(double2);
 	const int64_t ncols = c.columns ? c.ncolumns : s;
-	const bool sweep = layer_sweep_ok(c) && !(hess && latency_bound(L, nl, ncols)) && layer_bytes <= workspace_budget(rt, layer_bytes);
+	const bool sweep = layer_sweep_ok(c) && !(hess && latency_bound(L, ncols)) && layer_bytes <= workspace_budget(rt, layer_bytes);
 	const int64_t nstates = sweep ? layer_states : G + (layered ? G : 3) + 1 + (hess ? 16 * (int64_t)nl : 0);
 	const size_t col_bytes = (size_t)nstates * N * sizeof(double2);
 	int64_t C = ncols;

@@ -1,7 +1,6 @@
-"""Full Hessians of few amplitudes and many layers take the general sweep, others the layer sweep:
-both sides of the rule (layers more than a layer has gates: three up to 16 columns at L = 4 and one at
-L = 6, four up to 64 and 4) against the oracle, and the
-gate launches that tell which sweep ran."""
+"""Full Hessians of few amplitudes take the general sweep, others the layer sweep: both sides of the
+rule (256 columns or samples at L = 4, 16 at L = 6, one at L = 8) against the oracle, and the gate
+launches that tell which sweep ran."""
 import numpy as np
 import pytest
 
@@ -26,9 +25,9 @@ def _launches(gpu, call):
     return out, n
 
 
-@pytest.mark.parametrize("L,depth,ns,general", [(4, 4, 0, False), (4, 5, 0, True), (4, 5, 16, True), (4, 5, 17, False),
-                                                (4, 6, 64, True), (4, 6, 65, False), (6, 6, 1, True), (6, 6, 2, False),
-                                                (6, 7, 4, True), (6, 7, 5, False), (8, 12, 1, False), (2, 1, 0, True)])
+@pytest.mark.parametrize("L,depth,ns,general", [(2, 1, 0, True), (4, 1, 0, True), (4, 6, 0, True), (4, 3, 256, True),
+                                                (4, 3, 257, False), (6, 3, 0, False), (6, 3, 16, True), (6, 3, 17, False),
+                                                (8, 3, 1, True), (8, 3, 2, False), (10, 2, 1, False)])
 def test_hessians_on_either_side_of_the_rule(gpu, oracle, L, depth, ns, general):
     v, p, tv, tp = brickwall_instance(L, depth, L, 2, L + 1)
     target, ot = gpu.Target(brickwall=(tv, tp)), oracle.target("brickwall", (tv, tp))
@@ -45,7 +44,7 @@ def test_hessians_on_either_side_of_the_rule(gpu, oracle, L, depth, ns, general)
         assert np.linalg.norm(a - b) <= 1e-12 * max(np.linalg.norm(b), np.linalg.norm(ref[1]))
 
 
-@pytest.mark.parametrize("L,depth", [(4, 4), (4, 5), (4, 9), (8, 5)])
+@pytest.mark.parametrize("L,depth", [(4, 1), (4, 5), (8, 2), (8, 5)])
 def test_block_encodings_on_either_side_of_the_rule(gpu, oracle, L, depth):
     v, p, tv, _ = brickwall_instance(L, depth, L, 2, L + 1)
     half = np.stack([np.roll(np.arange(L // 2), -(k % 2)) for k in range(2)]).astype(np.int32)

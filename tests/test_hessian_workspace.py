@@ -17,10 +17,10 @@ def _settings(gpu):
     gpu.set_workspace_limit(0)
 
 
-# states a column of the general Hessian sweep holds (phi and psi of every gate, 16 tangents a layer, the
-# sample state and a scratch state) and of the layer sweep (psi, phi and 16 tangents a layer, 16
+# states a column of the general Hessian sweep holds (phi and psi of every gate, 16 tangents a layer, samples
+# and a scratch state) and of the layer sweep (psi, phi and 16 tangents a layer, 16
 # cotangent states, the sample state): the limits lie between the two
-@pytest.mark.parametrize("L,depth,states", [(2, 1, 21), (4, 1, 24), (4, 2, 45), (14, 1, 30)])
+@pytest.mark.parametrize("L,depth,states", [(2, 1, 21), (4, 1, 24), (4, 2, 45), (8, 1, 30), (8, 2, 51), (14, 1, 30)])
 @pytest.mark.parametrize("samples", [False, True])
 def test_hessians_take_the_sweep_that_fits(gpu, L, depth, states, samples):
     if L == 14 and not samples:
@@ -41,12 +41,12 @@ def test_hessians_take_the_sweep_that_fits(gpu, L, depth, states, samples):
         assert np.linalg.norm(a - b) <= 1e-12 * max(np.linalg.norm(b), np.linalg.norm(ref[1]))
 
 
-@pytest.mark.parametrize("depth", [1, 2])
+@pytest.mark.parametrize("L,depth", [(4, 1), (4, 2), (8, 1), (8, 2)])
 @pytest.mark.parametrize("what", ["target", "gradient", "hessian"])
-def test_block_encodings_take_the_sweep_that_fits(gpu, depth, what):
-    L, G = 4, 2 * depth
+def test_block_encodings_take_the_sweep_that_fits(gpu, L, depth, what):
+    G = depth * (L // 2)
     v, p, tv, tp = brickwall_instance(L, depth, 5, 1, 6)
-    target = gpu.Target(brickwall=(tv, np.arange(2, dtype=np.int32)[None]))
+    target = gpu.Target(brickwall=(tv, np.arange(L // 2, dtype=np.int32)[None]))
     call = {"target": gpu.brickwall_blockenc_target, "gradient": gpu.brickwall_blockenc_target_and_gradient,
             "hessian": gpu.brickwall_blockenc_target_gradient_hessian}[what]
     ref = np.atleast_1d(call(target, v, p, L)) if what == "target" else call(target, v, p, L)
